@@ -404,14 +404,14 @@ def run_ours(args):
     cand = {k: breakdown[k] for k in ("pole_kernel", "transform", "tri_reduce", "tri_rows", "assemble_h", "gather")
             if k in breakdown}
     # kernels of the chosen tridiagonal configuration (TriCfg in csrc/tridiag.cu): mixed
-    # configurations 1 and 5 reduce in shared memory, all but 2 apply with resident rows
+    # configurations 0 and 4 reduce with the window on its SM, all but 2 apply with resident rows
     mixed = args.precision == "mixed"
     cfg = s.tile_config if isinstance(s.tile_config, int) else 0
     kernel_names = {"pole_kernel": "tri_pass_kernel" if route == "tridiag" else "ldl_left_kernel",
                     "transform": ("gemm_tc_kernel" if args.standard_form == "tensor" else "gemm_f32blk_kernel")
                     if (route == "tridiag" and mixed)
                     else ("gemm_f64_kernel" if args.precision == "fp64" else "gemm_df64_kernel"),
-                    "tri_reduce": "tri_reduce_res_kernel" if (mixed and cfg in (1, 5)) else "tri_reduce_kernel",
+                    "tri_reduce": "tri_reduce_reg_kernel" if (mixed and cfg in (0, 4)) else "tri_reduce_kernel",
                     "tri_rows": "tri_apply_res_kernel" if (mixed and cfg != 2) else "tri_apply_kernel",
                     "assemble_h": "assemble_h32_kernel" if mixed else "assemble_h_kernel",
                     "gather": "gather_windows_kernel"}

@@ -139,7 +139,7 @@ int lres_density_ptr(lres_ctx* ctx, const double** d_dens);
  * passes at (mu, e_lo) (LRES_MIXED configuration 4 runs the chunk products on the tensor cores,
  * tcgen05 with a 3xTF32 split; it is timed but kept only when forced, its error being ~5x that
  * of the FP32 configurations).  On the tridiagonal route it selects the reduction (working
- * copy in L2, or with LRES_MIXED the window's lower triangle in shared memory), the row
+ * copy in L2, or with LRES_MIXED the window's lower triangle on its SM), the row
  * application (rows resident in shared memory with LRES_MIXED, or one row per thread), their
  * panel widths and rows per item (six measured variants, each capped by the shared memory),
  * timed as reduction + rows (mu, e_lo unused).

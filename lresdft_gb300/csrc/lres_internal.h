@@ -124,7 +124,7 @@ int pole_sums(int nwin, const long long* offQ, const int* m_w, const long long* 
 // Tile configuration of the tridiagonal route for windows of at most nmax functions.
 struct TriPick {
     int nb = 0, nt = 0;        // reduction panel width and threads
-    int rres = 0;              // 1: the reduction holds each window in shared memory (FP32)
+    int reg = 0;               // 1: the reduction holds each window on its SM (FP32, tridiag_reg.cu)
     int nb_apply = 0;          // row application panel width
     int rpt = 1;               // rows per thread of the row-per-thread application; 0: resident rows
     int arows = 0;             // rows per application item
@@ -135,6 +135,12 @@ int tri_pick(bool fp32, int nmax, size_t smem_budget, int cfg, TriPick* out);
 int tri_reduce(bool fp32, int nwin, const int* order, int* counter, const int* n_w, const long long* offC,
                const long long* offA, const long long* offN, const void* H, void* A, void* d, void* e, void* tau,
                int* status, const TriPick& pk, int nmax, size_t smem_budget, cudaStream_t s);
+// The reduction with the window on the SM, for the last kTriRegMax columns of each window; larger
+// windows come with the columns before those reduced in panels of nb.
+constexpr int kTriRegMax = 384;
+int tri_reduce_reg(int nwin, const int* order, int* counter, const int* n_w, const long long* offC,
+                   const long long* offA, const long long* offN, const float* H, float* A, float* d, float* e,
+                   float* tau, int* status, int nb, int nmax, size_t smem_budget, cudaStream_t s);
 // tfactors: form the T factors of every (window, panel) first (once per Hamiltonian)
 int tri_apply(bool fp32, int nitems, const int4* items, const int* n_w, const int* m_w, const long long* offA,
               const long long* offN, const long long* offF, const void* A, const void* tau, const void* F, void* Y,

@@ -28,6 +28,7 @@
 //                      and applied once per panel; three barriers per column (the norm, the
 //                      dots and A x taken over the unscaled column in one phase).
 //                      Algorithmic work (4/3) n^3 flops.
+//   tri_reduce_reg_kernel  (FP32, tridiag_reg.cu) the reduction with the window held on its SM.
 //   tri_apply_res_kernel  (FP32) one CTA per (window, block of up to 128 rows) with the
 //                      rows resident in shared memory through all panels: Y = F^ Q by
 //                      panels in compact WY form, Y <- Y - ((Y V) T_p) V^T, 4 x 4 register
@@ -132,6 +133,7 @@ struct TriReduceParams {
     int* status;
     int nb;                  // panel width (<= 32)
     int ldv;                 // length of the shared vectors (multiple of 32, >= every n)
+    int keep;                // > 0: stop before the last `keep` columns (tridiag_reg.cu takes over)
 };
 
 // Shared memory of the reduction, in elements of R.
@@ -171,6 +173,10 @@ __global__ void __launch_bounds__(NT, reduce_min_ctas(NT, sizeof(R))) tri_reduce
         if (n > ldv || n < 1) {
             if (tid == 0) atomicOr(p.status, ST_BAD_SHAPE);
             __syncthreads();
+            continue;
+        }
+        if (n <= p.keep) {
+            __syncthreads();                      // item_sh is read before the next fetch
             continue;
         }
         const int ld = (n + 3) & ~3;
@@ -220,7 +226,7 @@ __global__ void __launch_bounds__(NT, reduce_min_ctas(NT, sizeof(R))) tri_reduce
         // panel-start column j+1 of the owned rows is fetched by cp.async during column j: it
         // is A e_{j+1} of column j and the start of column j+1.
         R Kprev = R(0);
-        for (int j0 = 0; j0 < n - 2; j0 += nb) {
+        for (int j0 = 0; j0 < n - 2 && n - j0 > p.keep; j0 += nb) {
             const int nbp = min(nb, n - 2 - j0);
             for (int jj = 0; jj < nbp; ++jj) {
                 const int j = j0 + jj;
@@ -399,7 +405,7 @@ __global__ void __launch_bounds__(NT, reduce_min_ctas(NT, sizeof(R))) tri_reduce
             __syncthreads();
         }
         // ---- the last (at most 2 x 2) block, fully updated
-        if (tid == 0) {
+        if (tid == 0 && !p.keep) {
             if (n >= 2) {
                 dw[n - 2] = A[(n - 2) + (long long)(n - 2) * ld];
                 ew[n - 2] = A[(n - 1) + (long long)(n - 2) * ld];
@@ -411,270 +417,6 @@ __global__ void __launch_bounds__(NT, reduce_min_ctas(NT, sizeof(R))) tri_reduce
                 dw[0] = A[0];
                 tw[0] = R(0);
                 ew[0] = R(0);
-            }
-        }
-        __syncthreads();
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Householder tridiagonalisation with the window resident in shared memory (FP32)
-// ---------------------------------------------------------------------------
-//
-// The lower triangle of the window stays in shared memory for the whole reduction, in 4 x 4
-// blocks: column c holds rows 4 (c / 4) .. ld-1, i.e. the lower part plus the upper part of
-// its diagonal block (kept equal to the lower one), from
-//     colstart(c) = c ld - 8 a (a - 1) - 4 a b,   a = c / 4, b = c % 4,
-// so that every block's four column segments start on 16-byte boundaries.  p = A v uses
-// each stored block twice: for the row quad I, block (I, K) (K <= I) directly and block (K, I)
-// (K > I) transposed; a warp takes one row quad at a time, its lanes the column quads K
-// (16-byte loads, four per block), and the lanes' partial sums are added by a butterfly in a
-// fixed order.  The trailing update touches the stored blocks only (half the FMAs of a full
-// update).  One CTA per window (work queue, largest first), windows up to ld <= 320.
-
-constexpr int kResReduceNT = 640;
-constexpr int kResReduceMaxN = 320;
-
-__host__ __device__ inline int res_cs(int c, int ld) {
-    const int a = c >> 2, b = c & 3;
-    return c * ld - 8 * a * (a - 1) - 4 * a * b;
-}
-// element (r, c) of the stored part (r >= 4 (c / 4))
-__host__ __device__ inline int res_at(int r, int c, int ld) { return res_cs(c, ld) + r - 4 * (c >> 2); }
-
-// shared memory without the partial sums of p = A v (nseg x ldv more)
-inline size_t res_reduce_smem_elems(int nb, int ldv, int nmax) {
-    const int ld = (nmax + 3) & ~3;
-    const size_t head = (size_t)res_cs(ld, ld) + 2 * (size_t)nb * ldv + 2 * (size_t)ldv + 64 + kResReduceNT / 32;
-    return ((head + 3) & ~(size_t)3) + (size_t)ldv;      // + the column-start table (16-byte aligned)
-}
-
-template <int NT>
-__global__ void __launch_bounds__(NT, 1) tri_reduce_res_kernel(TriReduceParams<float> p, int nmax, int nseg) {
-    constexpr int NW = NT / 32;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int ldv = p.ldv, nb = p.nb;
-    float* const Vs = reinterpret_cast<float*>(smem_raw);            // [nb][ldv]
-    float* const Ws = Vs + (size_t)nb * ldv;                         // [nb][ldv]
-    float* const Ls = Ws + (size_t)nb * ldv;                         // blocked lower triangle
-    float* const cv = Ls + res_cs((nmax + 3) & ~3, (nmax + 3) & ~3); // [ldv] current column
-    float* const pv = cv + ldv;                                      // [ldv] p = tau (A v)
-    float* const dots = pv + ldv;                                    // [64]
-    float* const red = dots + 64;                                    // [NW]
-    const size_t head = (size_t)(red + NW - reinterpret_cast<float*>(smem_raw));
-    int* const cst = reinterpret_cast<int*>(smem_raw) + ((head + 3) & ~(size_t)3);   // [ldv] column starts
-    float* const psum = reinterpret_cast<float*>(cst + ldv);         // [nseg][ldv] partial A v
-    __shared__ int item_sh, nseg_used;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-
-    for (;;) {
-        if (tid == 0) item_sh = atomicAdd(p.counter, 1);
-        __syncthreads();
-        const int it = item_sh;
-        if (it >= p.nwin) return;
-        const int w = p.order[it];
-        const int n = p.n_w[w];
-        const int ld = (n + 3) & ~3;
-        if (n > ldv || n > nmax || n < 1) {
-            if (tid == 0) atomicOr(p.status, ST_BAD_SHAPE);
-            __syncthreads();
-            continue;
-        }
-        const int nq = ld >> 2;
-        const float* H = p.H + p.offC[w];
-        float* A = p.A + p.offA[w];
-        float* dw = p.d + p.offN[w];
-        float* ew = p.e + p.offN[w];
-        float* tw = p.tau + p.offN[w];
-
-        for (int c = tid; c < ld; c += NT) cst[c] = res_cs(c, ld);
-        // ---- the stored part of H (lower triangle, mirrored into the diagonal blocks; zero
-        //      beyond n), warp per column, rows along the lanes
-        for (int c = warp; c < ld; c += NW) {
-            const int r0 = 4 * (c >> 2);
-            for (int r = r0 + lane; r < ld; r += 32) {
-                float x = 0.0f;
-                if (r < n && c < n) x = r >= c ? H[r + (long long)c * n] : H[c + (long long)r * n];
-                Ls[res_at(r, c, ld)] = x;
-            }
-        }
-        __syncthreads();
-
-        for (int j0 = 0; j0 < n - 2; j0 += nb) {
-            const int nbp = min(nb, n - 2 - j0);
-            for (int jj = 0; jj < nbp; ++jj) {
-                const int j = j0 + jj;
-                // (a) column j of the current matrix, rows >= j: panel-start values minus
-                //     the pending rank-2 updates; squares of rows >= j+2
-                float part = 0.0f;
-                {
-                    const int i = j + tid;
-                    if (i < n) {
-                        float c = Ls[res_at(i, j, ld)];
-                        for (int l = 0; l < jj; ++l)
-                            c -= Vs[l * ldv + i] * Ws[l * ldv + j] + Ws[l * ldv + i] * Vs[l * ldv + j];
-                        cv[i] = c;
-                        if (i >= j + 2) part = c * c;
-                    }
-                }
-                // (b) reflector H_j = I - tau v v^T, v_{j+1} = 1
-                const float s2 = block_sum<NT>(part, red);    // its barriers also publish cv
-                const float alpha = cv[j + 1];
-                float beta = alpha, tau = 0.0f, scal = 0.0f;
-                if (s2 > 0.0f) {
-                    const float nrm = sqrtf(alpha * alpha + s2);
-                    beta = alpha >= 0.0f ? -nrm : nrm;
-                    tau = (beta - alpha) / beta;
-                    scal = 1.0f / (alpha - beta);
-                }
-                if (tid == 0) {
-                    dw[j] = cv[j];
-                    ew[j] = beta;
-                    tw[j] = tau;
-                    if (!isfinite(beta) || !isfinite(cv[j])) atomicOr(p.status, ST_ZERO_PIVOT);
-                }
-                for (int i = tid; i < ldv; i += NT) {
-                    float vi = 0.0f;
-                    if (i == j + 1) vi = 1.0f;
-                    else if (i > j + 1 && i < n) vi = cv[i] * scal;
-                    Vs[jj * ldv + i] = vi;
-                    if (i > j + 1 && i < n) A[i + (long long)j * ld] = vi;   // kept for Y = F^ Q
-                }
-                __syncthreads();
-                // (c) W^T v, V^T v (warp per product) and A v on the row quads from (j+1)/4,
-                //     from the panel-start matrix (v is zero on the rows <= j)
-                for (int q = warp; q < 2 * jj; q += NW) {
-                    const float* X = q < jj ? Ws + (size_t)q * ldv : Vs + (size_t)(q - jj) * ldv;
-                    float acc = 0.0f;
-                    for (int i = j + 1 + lane; i < n; i += 32) acc += X[i] * Vs[jj * ldv + i];
-                    acc = warp_sum(acc);
-                    if (lane == 0) dots[q] = acc;
-                }
-                {
-                    // lanes over 32 row quads I, warps over (row-quad group, segment of the
-                    // column quads K); each warp's partial sums go to psum[segment] and are
-                    // added in segment order in (d)
-                    const float* vv = Vs + (size_t)jj * ldv;
-                    const int q0 = (j + 1) >> 2, mq = nq - q0;
-                    const int G = (mq + 31) >> 5;
-                    const int S = min(NW / G, nseg);
-                    const int g = warp / S, s = warp % S;
-                    if (g < G) {
-                        const int I = q0 + 32 * g + lane;
-                        const int k0 = q0 + (int)((long long)mq * s / S), k1 = q0 + (int)((long long)mq * (s + 1) / S);
-                        float pr[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                        if (I < nq) {
-                            const int4 cI = *reinterpret_cast<const int4*>(cst + 4 * I);
-                            const int csI[4] = {cI.x, cI.y, cI.z, cI.w};
-                            for (int K = k0; K < k1; ++K) {
-                                const float4 vK4 = *reinterpret_cast<const float4*>(vv + 4 * K);
-                                const float vk[4] = {vK4.x, vK4.y, vK4.z, vK4.w};
-                                if (K > I) {
-                                    // block (K, I): column 4I+c, rows 4K..4K+3: p_I[c] += b . v_K
-                                    const int base = 4 * K - 4 * I;
-#pragma unroll
-                                    for (int c = 0; c < 4; ++c) {
-                                        const float4 b = *reinterpret_cast<const float4*>(Ls + csI[c] + base);
-                                        pr[c] = fmaf(b.x, vk[0], fmaf(b.y, vk[1], fmaf(b.z, vk[2], fmaf(b.w, vk[3], pr[c]))));
-                                    }
-                                } else {
-                                    // block (I, K): column 4K+c, rows 4I..4I+3: p_I[r] += b[r] v_K[c]
-                                    const int4 cK = *reinterpret_cast<const int4*>(cst + 4 * K);
-                                    const int off = 4 * I - 4 * K;
-                                    const int cc[4] = {cK.x, cK.y, cK.z, cK.w};
-#pragma unroll
-                                    for (int c = 0; c < 4; ++c) {
-                                        const float4 b = *reinterpret_cast<const float4*>(Ls + cc[c] + off);
-                                        pr[0] = fmaf(b.x, vk[c], pr[0]);
-                                        pr[1] = fmaf(b.y, vk[c], pr[1]);
-                                        pr[2] = fmaf(b.z, vk[c], pr[2]);
-                                        pr[3] = fmaf(b.w, vk[c], pr[3]);
-                                    }
-                                }
-                            }
-                            *reinterpret_cast<float4*>(psum + (size_t)s * ldv + 4 * I) = make_float4(pr[0], pr[1], pr[2], pr[3]);
-                        }
-                    }
-                    if (tid == 0) nseg_used = S;
-                }
-                __syncthreads();
-                // (d) p *= tau (with the pending updates), K = tau/2 p.v, w = p - K v
-                float partK = 0.0f;
-                {
-                    const int i = j + 1 + tid;
-                    if (i < n) {
-                        float pi = psum[i];
-                        for (int s2 = 1; s2 < nseg_used; ++s2) pi += psum[(size_t)s2 * ldv + i];
-                        for (int l = 0; l < jj; ++l) pi -= Vs[l * ldv + i] * dots[l] + Ws[l * ldv + i] * dots[jj + l];
-                        pi *= tau;
-                        pv[i] = pi;
-                        partK = pi * Vs[jj * ldv + i];
-                    }
-                }
-                const float K = 0.5f * tau * block_sum<NT>(partK, red);
-                for (int i = tid; i < ldv; i += NT)
-                    Ws[jj * ldv + i] = (i > j && i < n) ? pv[i] - K * Vs[jj * ldv + i] : 0.0f;
-                __syncthreads();
-            }
-            // ---- trailing update of the stored blocks (I >= K >= t0 / 4): B -= V W^T + W V^T;
-            //      the blocks in column order from the last column quad, consecutive threads
-            //      on consecutive row quads of one column quad, so that the v, w of the rows
-            //      and the blocks are contiguous across a warp and those of the columns broadcast
-            const int t0 = j0 + nbp;
-            if (t0 < n) {
-                const int qa = t0 >> 2;
-                const int m = nq - qa;
-                const int ntile = m * (m + 1) / 2;
-                for (int tile = tid; tile < ntile; tile += NT) {
-                    int u = (int)((sqrtf(8.0f * tile + 1.0f) - 1.0f) * 0.5f);
-                    while ((u + 1) * (u + 2) / 2 <= tile) ++u;
-                    while (u * (u + 1) / 2 > tile) --u;
-                    const int K = qa + m - 1 - u, I = K + tile - u * (u + 1) / 2;
-                    const int i = 4 * I, c0 = 4 * K;
-                    float acc[4][4];
-#pragma unroll
-                    for (int c = 0; c < 4; ++c)
-#pragma unroll
-                        for (int r = 0; r < 4; ++r) acc[c][r] = 0.0f;
-                    for (int l = 0; l < nbp; ++l) {
-                        float vi[4], wi[4], vk[4], wk[4];
-                        ld4(Vs + (size_t)l * ldv + i, vi);
-                        ld4(Ws + (size_t)l * ldv + i, wi);
-                        ld4(Vs + (size_t)l * ldv + c0, vk);
-                        ld4(Ws + (size_t)l * ldv + c0, wk);
-#pragma unroll
-                        for (int c = 0; c < 4; ++c)
-#pragma unroll
-                            for (int r = 0; r < 4; ++r) acc[c][r] = fmaf(vi[r], wk[c], fmaf(wi[r], vk[c], acc[c][r]));
-                    }
-                    const int4 cK = *reinterpret_cast<const int4*>(cst + c0);
-                    const int cc[4] = {cK.x, cK.y, cK.z, cK.w};
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        float* dst = Ls + cc[c] + i - c0;
-                        float x[4];
-                        ld4(dst, x);
-#pragma unroll
-                        for (int r = 0; r < 4; ++r) x[r] -= acc[c][r];
-                        st4(dst, x);
-                    }
-                }
-            }
-            __syncthreads();
-        }
-        // ---- the last (at most 2 x 2) block, fully updated
-        if (tid == 0) {
-            if (n >= 2) {
-                dw[n - 2] = Ls[res_at(n - 2, n - 2, ld)];
-                ew[n - 2] = Ls[res_at(n - 1, n - 2, ld)];
-                dw[n - 1] = Ls[res_at(n - 1, n - 1, ld)];
-                tw[n - 2] = 0.0f;
-                tw[n - 1] = 0.0f;
-                ew[n - 1] = 0.0f;
-            } else {
-                dw[0] = Ls[0];
-                tw[0] = 0.0f;
-                ew[0] = 0.0f;
             }
         }
         __syncthreads();
@@ -1562,16 +1304,16 @@ __global__ void tri_mineig_kernel(int nwin, const int* n_w, const long long* off
 // the rows stay resident in shared memory (res; FP32 only).  Panel widths are capped by
 // what fits the shared memory at windows of nmax.
 struct TriCfg {
-    int nb, nt, nba, rpt, res, rres;     // rres: the reduction with the window in shared memory
+    int nb, nt, nba, rpt, res, reg;      // reg: the reduction with the window on its SM (tridiag_reg.cu)
     int rows;                            // resident application: rows per item at most
 };
-// Measured at 1024 electrons (mixed): reduction 6.7 ms with the L2-resident working copy
-// (nb 16, 512 threads, two CTAs per SM; nb 8 6.75 ms, nb 32 7.35 ms; 256 threads at four CTAs
-// per SM and 384 at three 7.8 ms), 8.1 ms with the window in shared memory (nb 8); row
-// application 2.0 ms with resident rows (NB 32), 6.3 ms one row per thread.
-static const TriCfg kTriCfg[6] = {{16, 512, 32, 1, 1, 0, 128}, {16, 512, 32, 1, 1, 1, 128},
+// Measured at 1024 electrons (mixed): reduction 3.5 ms with the window on its SM, 6.7 ms with the
+// L2-resident working copy (nb 16, 512 threads, two CTAs per SM; nb 8 6.75 ms, nb 32 7.35 ms; 256
+// threads at four CTAs per SM and 384 at three 7.8 ms); row application 2.0 ms with resident rows
+// (NB 32), 6.3 ms one row per thread.
+static const TriCfg kTriCfg[6] = {{16, 512, 32, 1, 1, 1, 128}, {16, 512, 32, 1, 1, 0, 128},
                                   {16, 512, 32, 1, 0, 0, 0},    {16, 512, 16, 1, 1, 0, 64},
-                                  {16, 512, 32, 1, 1, 0, 32},   {8, 512, 32, 1, 1, 1, 128}};
+                                  {16, 512, 32, 1, 1, 1, 32},   {8, 512, 32, 1, 1, 0, 128}};
 
 int tri_pick(bool fp32, int nmax, size_t smem_budget, int cfg, TriPick* out) {
     const int el = fp32 ? 4 : 8;
@@ -1580,13 +1322,7 @@ int tri_pick(bool fp32, int nmax, size_t smem_budget, int cfg, TriPick* out) {
     if (cfg < 0 || cfg >= 6) cfg = 0;
     const TriCfg& t = kTriCfg[cfg];
     r.nt = t.nt;
-    if (t.rres && fp32 && nmax <= kResReduceMaxN)
-        for (int b : {16, 8, 4})
-            if (b <= t.nb && !r.nb && (res_reduce_smem_elems(b, r.ldv, nmax) + r.ldv) * el <= smem_budget) {
-                r.nb = b;
-                r.nt = kResReduceNT;
-                r.rres = 1;
-            }
+    r.reg = t.reg && fp32;
     for (int b : {32, 16, 8, 4})
         if (b <= t.nb && !r.nb && reduce_smem_elems(b, r.ldv, t.nt) * el <= smem_budget) r.nb = b;
     if (t.res && fp32)
@@ -1636,29 +1372,22 @@ int tri_reduce(bool fp32, int nwin, const int* order, int* counter, const int* n
     LRES_CUDA_TRY(cudaMemsetAsync(counter, 0, sizeof(int), s));
     if (fp32) {
         TriReduceParams<float> p{nwin, order, counter, n_w, offC, offA, offN, (const float*)H, (float*)A,
-                                 (float*)d, (float*)e, (float*)tau, status, nb, ldv};
-        if (pk.rres) {
-            // as many partial-sum rows of p = A v (one per column segment) as fit, at most a warp each
-            const size_t fixed = res_reduce_smem_elems(nb, ldv, nmax) * sizeof(float);
-            const int nseg = fixed + sizeof(float) * ldv > smem_budget
-                                 ? 0
-                                 : (int)std::min<size_t>(kResReduceNT / 32, (smem_budget - fixed) / (sizeof(float) * ldv));
-            if (nseg < 1 || nmax > kResReduceMaxN) {
-                lres_set_error("resident tridiagonal reduction needs %zu B of shared memory", fixed + sizeof(float) * ldv);
-                return LRES_EINVAL;
+                                 (float*)d, (float*)e, (float*)tau, status, nb, ldv, 0};
+        if (pk.reg) {
+            // windows beyond the resident size: their first columns from the L2-resident copy
+            if (nmax > kTriRegMax) {
+                p.keep = kTriRegMax;
+                if (int rc = nt == 512 ? launch_reduce<float, 512>(p, smem_budget, s)
+                                       : launch_reduce<float, 256>(p, smem_budget, s))
+                    return rc;
             }
-            const size_t smem = fixed + sizeof(float) * (size_t)nseg * ldv;
-            int per_sm = 0;
-            if (int rc = prepare_kernel<tri_reduce_res_kernel<kResReduceNT>>(kResReduceNT, smem, &per_sm)) return rc;
-            const int grid = std::min(nwin, std::max(1, per_sm) * device_sms());
-            tri_reduce_res_kernel<kResReduceNT><<<grid, kResReduceNT, smem, s>>>(p, nmax, nseg);
-            LRES_CUDA_TRY(cudaGetLastError());
-            return LRES_OK;
+            return tri_reduce_reg(nwin, order, counter, n_w, offC, offA, offN, (const float*)H, (float*)A, (float*)d,
+                                  (float*)e, (float*)tau, status, nb, nmax, smem_budget, s);
         }
         return nt == 512 ? launch_reduce<float, 512>(p, smem_budget, s) : launch_reduce<float, 256>(p, smem_budget, s);
     }
     TriReduceParams<double> p{nwin, order, counter, n_w, offC, offA, offN, (const double*)H, (double*)A,
-                              (double*)d, (double*)e, (double*)tau, status, nb, ldv};
+                              (double*)d, (double*)e, (double*)tau, status, nb, ldv, 0};
     return nt == 512 ? launch_reduce<double, 512>(p, smem_budget, s) : launch_reduce<double, 256>(p, smem_budget, s);
 }
 
