@@ -1119,8 +1119,8 @@ extern "C" int lres_ctx_create(lres_ctx** out, const lres_system_desc* d, int pr
     LRES_CUDA_TRY(cudaMemsetAsync(c->d_dens, 0, sizeof(double) * ng, s));
     c->nw_h.resize(c->nwin);
     c->ew_h.resize(c->nwin);
-    TRY(fft3_create(&c->fft, c->shape));
-    TRY(dalloc(&c->d_fftwork, ng));
+    TRY(fft3_create(&c->fft, c->shape, c->cell));
+    TRY(dalloc(&c->d_fftwork, (size_t)c->shape[0] * c->shape[1] * (c->shape[2] / 2 + 1)));
     LRES_CUDA_TRY(cudaStreamSynchronize(s));
     *out = c.release();
     return LRES_OK;
@@ -1651,7 +1651,7 @@ extern "C" int lres_hartree(lres_ctx* c, const double* dens, double* vh, void* s
         lres_set_error("null argument");
         return LRES_EINVAL;
     }
-    return hartree_apply(c->fft, c->shape, c->cell, dens, vh, c->d_fftwork, (cudaStream_t)stream);
+    return hartree_apply(c->fft, dens, vh, c->d_fftwork, (cudaStream_t)stream);
 }
 
 extern "C" int lres_ion_potential(lres_ctx* c, int64_t natoms, const double* pos, const double* Z, const double* rc,
@@ -1668,7 +1668,7 @@ extern "C" int lres_ion_potential(lres_ctx* c, int64_t natoms, const double* pos
     LRES_CUDA_TRY(cudaMemcpyAsync(dp, pos, sizeof(double) * 3 * natoms, cudaMemcpyHostToDevice, s));
     LRES_CUDA_TRY(cudaMemcpyAsync(dz, Z, sizeof(double) * natoms, cudaMemcpyHostToDevice, s));
     LRES_CUDA_TRY(cudaMemcpyAsync(dr, rc, sizeof(double) * natoms, cudaMemcpyHostToDevice, s));
-    int r = ion_apply(c->fft, c->shape, c->cell, (int)natoms, dp, dz, dr, vion, c->d_fftwork, s);
+    int r = ion_apply(c->fft, c->cell, (int)natoms, dp, dz, dr, vion, c->d_fftwork, s);
     cudaStreamSynchronize(s);
     cudaFree(dp);
     cudaFree(dz);

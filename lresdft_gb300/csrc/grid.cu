@@ -1,23 +1,41 @@
-// Grid kernels of the SCF step: a hand-written mixed-radix complex FFT (3-D, FP64),
-// FFT Hartree, LDA exchange-correlation, the ion potential and Voronoi ownership.
-// All are HBM-bandwidth bound.
+// Grid kernels of the SCF step: a hand-written mixed-radix FFT of real grids (3-D, FP64), FFT
+// Hartree, LDA exchange-correlation, the ion potential and Voronoi ownership.
 //
-// FFT: three passes of batched 1-D transforms.  Each CTA loads a pencil of B lines
-// (coalesced along the contiguous axis) into shared memory and runs a Stockham
-// autosort transform over the factorisation of the line length (radix 4, 2, 3, 5,
-// then any remaining prime by a direct DFT), ping-ponging between two shared
-// buffers.  Bytes per 3-D transform: 3 passes x (read + write) x 16 B per point.
+// FFT: what bounds it is the FP64 pipe (1/64 of the FP32 rate: 1 TFLOP/s), not memory: a 108^3
+// Hartree step moves 0.12 GB through L2 and issues ~0.1 G FP64 instructions.  So no FP64 work
+// that a table can replace (the twiddles are read, not evaluated), and only half of the
+// spectrum is computed: two real lines make one complex line along the contiguous axis, and the
+// other two axes run over n3/2+1 wave numbers.  The x axis is transformed, divided by G^2 and
+// transformed back in one kernel: five passes per Hartree step.  Each CTA holds 8 lines in shared
+// memory ([element][line], rows of 9 so that neither direction conflicts) and runs a Stockham
+// autosort over the factors of the length (4, 2, 3, 5 in registers, any other prime by a direct
+// DFT): 8 lines per CTA give 2 or more CTAs per SM from 64^3 on.
+// Measured (LDA + Hartree): 64^3 0.48 -> 0.24 ms, 108^3 9.3 -> 0.84 ms (evaluated twiddles and
+// radix-3 and -5 factors by sincospi, six complex passes, before).
 #include "common.cuh"
 #include "lres_internal.h"
 
+#include <cmath>
 #include <vector>
 
 namespace lres {
 
+constexpr int kFftNT = 128;
+constexpr int kFftLines = 8, kFftRow = kFftLines + 1;
+constexpr int kFftFac = 14;
+
+// One axis: its length, factors and twiddle table exp(-2 pi i k / L), k < L.
+struct FftAxis {
+    int L = 0, nf = 0;
+    int fac[kFftFac] = {};
+    const double2* tw = nullptr;
+    const double* k = nullptr;        // wave numbers
+};
+
 struct FFT3 {
-    int64_t shape[3];
-    std::vector<int> fac[3];
-    int* d_fac = nullptr;     // [3][16] radices, 0-terminated
+    FftAxis ax[3];
+    double2* d_tw = nullptr;
+    double* d_k = nullptr;
 };
 
 static std::vector<int> factorise(int n) {
@@ -30,25 +48,47 @@ static std::vector<int> factorise(int n) {
     return f;
 }
 
-int fft3_create(FFT3** out, const int64_t shape[3]) {
-    FFT3* f = new FFT3();
-    std::vector<int> flat(48, 0);
+int fft3_create(FFT3** out, const int64_t shape[3], const double cell[3]) {
+    size_t total = 0;
     for (int a = 0; a < 3; ++a) {
-        f->shape[a] = shape[a];
-        f->fac[a] = factorise((int)shape[a]);
-        if (f->fac[a].size() > 15 || shape[a] > 4096) {
-            delete f;
+        if (shape[a] < 1 || shape[a] > 4096 || factorise((int)shape[a]).size() > kFftFac) {
             lres_set_error("grid axis of length %lld not supported by the FFT", (long long)shape[a]);
             return LRES_EINVAL;
         }
-        for (size_t i = 0; i < f->fac[a].size(); ++i) flat[a * 16 + i] = f->fac[a][i];
+        total += shape[a];
     }
-    if (cudaMalloc(&f->d_fac, sizeof(int) * 48) != cudaSuccess ||
-        cudaMemcpy(f->d_fac, flat.data(), sizeof(int) * 48, cudaMemcpyHostToDevice) != cudaSuccess) {
-        cudaFree(f->d_fac);
-        delete f;
+    std::vector<double2> tw(total);
+    std::vector<double> kv(total);
+    FFT3* f = new FFT3();
+    size_t off = 0;
+    for (int a = 0; a < 3; ++a) {
+        const int L = (int)shape[a];
+        const std::vector<int> fac = factorise(L);
+        f->ax[a].L = L;
+        f->ax[a].nf = (int)fac.size();
+        for (size_t i = 0; i < fac.size(); ++i) f->ax[a].fac[i] = fac[i];
+        // wave numbers as numpy: 2 pi (f (1 / (m (L / m)))) with f the fftfreq index
+        const double val = 1.0 / ((double)L * (cell[a] / (double)L));
+        for (int i = 0; i < L; ++i) {
+            const long double ph = 2.0L * acosl(-1.0L) * i / L;
+            tw[off + i] = make_double2((double)cosl(ph), (double)-sinl(ph));
+            kv[off + i] = 2.0 * M_PI * ((double)(i < (L + 1) / 2 ? i : i - L) * val);
+        }
+        off += L;
+    }
+    if (cudaMalloc(&f->d_tw, sizeof(double2) * total) != cudaSuccess ||
+        cudaMalloc(&f->d_k, sizeof(double) * total) != cudaSuccess ||
+        cudaMemcpy(f->d_tw, tw.data(), sizeof(double2) * total, cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemcpy(f->d_k, kv.data(), sizeof(double) * total, cudaMemcpyHostToDevice) != cudaSuccess) {
+        fft3_destroy(f);
         lres_set_error("FFT plan allocation failed");
         return LRES_ENOMEM;
+    }
+    off = 0;
+    for (FftAxis& x : f->ax) {
+        x.tw = f->d_tw + off;
+        x.k = f->d_k + off;
+        off += x.L;
     }
     *out = f;
     return LRES_OK;
@@ -56,212 +96,248 @@ int fft3_create(FFT3** out, const int64_t shape[3]) {
 
 void fft3_destroy(FFT3* f) {
     if (!f) return;
-    cudaFree(f->d_fac);
+    cudaFree(f->d_tw);
+    cudaFree(f->d_k);
     delete f;
 }
 
 __device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
 __device__ __forceinline__ double2 cmulc(double2 a, double2 b) {
-    return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+    return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
+}
+// a + s i b (s = -1 forward, +1 inverse)
+template <bool INV>
+__device__ __forceinline__ double2 add_i(double2 a, double2 b) {
+    return INV ? make_double2(a.x - b.y, a.y + b.x) : make_double2(a.x + b.y, a.y - b.x);
+}
+template <bool INV>
+__device__ __forceinline__ double2 twiddle(const double2* tw, int k) {
+    double2 w = tw[k];
+    if (INV) w.y = -w.y;
+    return w;
 }
 
-// One pass of 1-D transforms of length L along one axis.  Element t of line (base, b)
-// lives at data[base + t*tstride + b*bstride]; the CTA owns lines b in [b0, b0+B).
-__global__ void fft_pass_kernel(double2* data, int L, long long tstride, long long bstride, int nb_lines,
-                                int lines_per_base, long long base_stride_a, long long base_stride_b, int nbase_b,
-                                const int* fac, double sign, int B) {
-    extern __shared__ __align__(16) unsigned char smraw[];
-    double2* x = reinterpret_cast<double2*>(smraw);      // L x B
-    double2* y = x + (size_t)L * B;
-    const int tid = threadIdx.x;
-    // which lines: blockIdx.x enumerates (base, group of B lines)
-    const int groups = (lines_per_base + B - 1) / B;
-    const int gidx = blockIdx.x % groups;
-    const int base = blockIdx.x / groups;
-    const long long off = (long long)(base / nbase_b) * base_stride_a + (long long)(base % nbase_b) * base_stride_b;
-    const int b0 = gidx * B;
-    const int nbl = min(B, lines_per_base - b0);
-    (void)nb_lines;
-    // load (contiguous axis fastest)
-    if (tstride == 1) {
-        for (int idx = tid; idx < L * nbl; idx += blockDim.x) {
-            const int t = idx % L, b = idx / L;
-            x[t * B + b] = data[off + t + (long long)(b0 + b) * bstride];
-        }
+// a[t] <- sum_j a[j] exp(-+ 2 pi i j t / R)
+template <int R, bool INV>
+__device__ __forceinline__ void dft(double2 (&a)[R]) {
+    if constexpr (R == 2) {
+        const double2 t = a[0];
+        a[0] = cadd(t, a[1]);
+        a[1] = csub(t, a[1]);
+    } else if constexpr (R == 3) {
+        const double c = 0.86602540378443864676;                     // sin(2 pi / 3)
+        const double2 t = cadd(a[1], a[2]), d = make_double2(c * (a[1].x - a[2].x), c * (a[1].y - a[2].y));
+        const double2 m = make_double2(fma(-0.5, t.x, a[0].x), fma(-0.5, t.y, a[0].y));
+        a[0] = cadd(a[0], t);
+        a[1] = add_i<INV>(m, d);
+        a[2] = add_i<!INV>(m, d);
+    } else if constexpr (R == 4) {
+        const double2 t0 = cadd(a[0], a[2]), t1 = csub(a[0], a[2]), t2 = cadd(a[1], a[3]), t3 = csub(a[1], a[3]);
+        a[0] = cadd(t0, t2);
+        a[1] = add_i<INV>(t1, t3);
+        a[2] = csub(t0, t2);
+        a[3] = add_i<!INV>(t1, t3);
     } else {
-        for (int idx = tid; idx < L * nbl; idx += blockDim.x) {
-            const int b = idx % nbl, t = idx / nbl;
-            x[t * B + b] = data[off + (long long)t * tstride + (long long)(b0 + b) * bstride];
+        static_assert(R == 5, "radix");
+        const double c1 = 0.30901699437494742410, c2 = -0.80901699437494742410;   // cos(2 pi / 5), cos(4 pi / 5)
+        const double s1 = 0.95105651629515357212, s2 = 0.58778525229247312917;
+        const double2 t1 = cadd(a[1], a[4]), t2 = cadd(a[2], a[3]), t3 = csub(a[1], a[4]), t4 = csub(a[2], a[3]);
+        const double2 m1 = make_double2(fma(c1, t1.x, fma(c2, t2.x, a[0].x)), fma(c1, t1.y, fma(c2, t2.y, a[0].y)));
+        const double2 m2 = make_double2(fma(c2, t1.x, fma(c1, t2.x, a[0].x)), fma(c2, t1.y, fma(c1, t2.y, a[0].y)));
+        const double2 n1 = make_double2(fma(s1, t3.x, s2 * t4.x), fma(s1, t3.y, s2 * t4.y));
+        const double2 n2 = make_double2(fma(s2, t3.x, -s1 * t4.x), fma(s2, t3.y, -s1 * t4.y));
+        a[0] = cadd(a[0], cadd(t1, t2));
+        a[1] = add_i<INV>(m1, n1);
+        a[2] = add_i<INV>(m2, n2);
+        a[3] = add_i<!INV>(m2, n2);
+        a[4] = add_i<!INV>(m1, n1);
+    }
+}
+
+// One Stockham stage of radix R: sub-transforms of length m R, stride s (m R s = L).
+template <int R, bool INV>
+__device__ __forceinline__ void fft_stage(const double2* x, double2* y, int m, int s, const double2* tw) {
+    for (int idx = threadIdx.x; idx < m * s * kFftLines; idx += kFftNT) {
+        const int b = idx & (kFftLines - 1), pq = idx / kFftLines;
+        const int p = pq / s, q = pq - p * s;
+        double2 a[R];
+#pragma unroll
+        for (int j = 0; j < R; ++j) a[j] = x[(q + s * (p + j * m)) * kFftRow + b];
+        dft<R, INV>(a);
+#pragma unroll
+        for (int t = 0; t < R; ++t) {
+            if (t && p) a[t] = cmulc(a[t], twiddle<INV>(tw, p * t * s));
+            y[(q + s * (R * p + t)) * kFftRow + b] = a[t];
         }
     }
-    __syncthreads();
-    int n = L, s = 1;
-    for (int fi = 0; fac[fi]; ++fi) {
-        const int r = fac[fi];
-        const int m = n / r;
-        // butterflies: (p, q, b) with p < m, q < s
-        const int nbf = m * s * nbl;
-        for (int idx = tid; idx < nbf; idx += blockDim.x) {
-            const int b = idx % nbl;
-            const int pq = idx / nbl;
-            const int q = pq % s, p = pq / s;
-            double2 a[16];
-            double2 buf[16];
-            if (r <= 16) {
-                for (int j = 0; j < r; ++j) a[j] = x[(q + s * (p + j * m)) * B + b];
-                // small DFT: buf[t] = sum_j a_j exp(sign 2 pi i j t / r)
-                if (r == 2) {
-                    buf[0] = cadd(a[0], a[1]);
-                    buf[1] = make_double2(a[0].x - a[1].x, a[0].y - a[1].y);
-                } else if (r == 4) {
-                    const double2 t0 = cadd(a[0], a[2]), t1 = make_double2(a[0].x - a[2].x, a[0].y - a[2].y);
-                    const double2 t2 = cadd(a[1], a[3]), t3 = make_double2(a[1].x - a[3].x, a[1].y - a[3].y);
-                    // multiply t3 by (sign * i)
-                    const double2 t3i = make_double2(-sign * t3.y, sign * t3.x);
-                    buf[0] = cadd(t0, t2);
-                    buf[1] = cadd(t1, t3i);
-                    buf[2] = make_double2(t0.x - t2.x, t0.y - t2.y);
-                    buf[3] = make_double2(t1.x - t3i.x, t1.y - t3i.y);
-                } else {
-                    for (int t = 0; t < r; ++t) {
-                        double2 acc = make_double2(0.0, 0.0);
-                        for (int j = 0; j < r; ++j) {
-                            double sn, cs;
-                            sincospi(sign * 2.0 * (double)((j * t) % r) / (double)r, &sn, &cs);
-                            acc = cadd(acc, cmulc(a[j], make_double2(cs, sn)));
-                        }
-                        buf[t] = acc;
-                    }
-                }
-                for (int t = 0; t < r; ++t) {
-                    double2 v = buf[t];
-                    if (p && t) {
-                        double sn, cs;
-                        sincospi(sign * 2.0 * (double)(p * t) / (double)n, &sn, &cs);
-                        v = cmulc(v, make_double2(cs, sn));
-                    }
-                    y[(q + s * (r * p + t)) * B + b] = v;
-                }
-            } else {
-                // large prime radix: direct DFT from shared memory
-                for (int t = 0; t < r; ++t) {
-                    double2 acc = make_double2(0.0, 0.0);
-                    for (int j = 0; j < r; ++j) {
-                        double sn, cs;
-                        sincospi(sign * 2.0 * (double)((long long)j * t % r) / (double)r, &sn, &cs);
-                        acc = cadd(acc, cmulc(x[(q + s * (p + j * m)) * B + b], make_double2(cs, sn)));
-                    }
-                    if (p && t) {
-                        double sn, cs;
-                        sincospi(sign * 2.0 * (double)(p * t) / (double)n, &sn, &cs);
-                        acc = cmulc(acc, make_double2(cs, sn));
-                    }
-                    y[(q + s * (r * p + t)) * B + b] = acc;
-                }
-            }
+}
+
+// The same for any radix r, one output per thread.
+template <bool INV>
+__device__ __forceinline__ void fft_stage_any(const double2* x, double2* y, int r, int m, int s, const double2* tw) {
+    const int step = m * s;                                          // L / r
+    for (int idx = threadIdx.x; idx < r * m * s * kFftLines; idx += kFftNT) {
+        const int b = idx & (kFftLines - 1), k = idx / kFftLines;
+        const int q = k % s, pt = k / s, t = pt % r, p = pt / r;
+        double2 acc = make_double2(0.0, 0.0);
+        for (int j = 0, e = 0; j < r; ++j) {
+            acc = cadd(acc, cmulc(x[(q + s * (p + j * m)) * kFftRow + b], twiddle<INV>(tw, e * step)));
+            e += t;
+            if (e >= r) e -= r;
         }
+        if (p && t) acc = cmulc(acc, twiddle<INV>(tw, p * t * s));
+        y[k * kFftRow + b] = acc;
+    }
+}
+
+// The 8 lines in x transformed in place of x or y (the buffer that holds the result is returned).
+template <bool INV>
+__device__ double2* fft_lines(double2* x, double2* y, const FftAxis& ax, const double2* tw) {
+    int n = ax.L, s = 1;
+    for (int i = 0; i < ax.nf; ++i) {
+        const int r = ax.fac[i], m = n / r;
+        if (r == 4) fft_stage<4, INV>(x, y, m, s, tw);
+        else if (r == 2) fft_stage<2, INV>(x, y, m, s, tw);
+        else if (r == 3) fft_stage<3, INV>(x, y, m, s, tw);
+        else if (r == 5) fft_stage<5, INV>(x, y, m, s, tw);
+        else fft_stage_any<INV>(x, y, r, m, s, tw);
         __syncthreads();
-        double2* tmp = x;
+        double2* const t = x;
         x = y;
-        y = tmp;
+        y = t;
         n = m;
         s *= r;
     }
-    // store
-    if (tstride == 1) {
-        for (int idx = tid; idx < L * nbl; idx += blockDim.x) {
-            const int t = idx % L, b = idx / L;
-            data[off + t + (long long)(b0 + b) * bstride] = x[t * B + b];
+    return x;
+}
+
+inline size_t fft_smem(int L) { return sizeof(double2) * ((size_t)2 * L * kFftRow + L); }
+
+// Real lines of the contiguous axis: lines 2l and 2l+1 as the real and imaginary part of one.
+// Forward: the half spectra w[line * h + k], k < h; inverse: the lines scaled by `scale`.
+template <bool INV>
+__global__ void __launch_bounds__(kFftNT) fft_real_kernel(FftAxis ax, long long nlines, double* r, double2* w,
+                                                          double scale) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    const int L = ax.L, h = L / 2 + 1;
+    double2* const tw = reinterpret_cast<double2*>(smraw);
+    double2* x = tw + L;
+    double2* y = x + (size_t)L * kFftRow;
+    const long long l0 = 2 * (long long)blockIdx.x * kFftLines;      // first line
+    for (int i = threadIdx.x; i < L; i += kFftNT) tw[i] = ax.tw[i];
+    if (!INV) {
+        for (int idx = threadIdx.x; idx < L * kFftLines; idx += kFftNT) {
+            const int b = idx / L, t = idx - b * L;
+            const long long a = l0 + 2 * b;
+            x[t * kFftRow + b] = make_double2(a < nlines ? r[a * L + t] : 0.0, a + 1 < nlines ? r[(a + 1) * L + t] : 0.0);
         }
     } else {
-        for (int idx = tid; idx < L * nbl; idx += blockDim.x) {
-            const int b = idx % nbl, t = idx / nbl;
-            data[off + (long long)t * tstride + (long long)(b0 + b) * bstride] = x[t * B + b];
+        for (int idx = threadIdx.x; idx < h * kFftLines; idx += kFftNT) {
+            const int b = idx / h, k = idx - b * h;
+            const long long a = l0 + 2 * b;
+            double2 u = a < nlines ? w[a * h + k] : make_double2(0.0, 0.0);
+            double2 v = a + 1 < nlines ? w[(a + 1) * h + k] : make_double2(0.0, 0.0);
+            if (k == 0 || 2 * k == L) u.y = v.y = 0.0;              // (the real part of the line is wanted)
+            x[k * kFftRow + b] = make_double2(u.x - v.y, u.y + v.x);                    // u + i v
+            if (k && 2 * k < L) x[(L - k) * kFftRow + b] = make_double2(u.x + v.y, v.x - u.y);
+        }
+    }
+    __syncthreads();
+    const double2* z = fft_lines<INV>(x, y, ax, tw);
+    if (!INV) {
+        for (int idx = threadIdx.x; idx < h * kFftLines; idx += kFftNT) {
+            const int b = idx / h, k = idx - b * h;
+            const long long a = l0 + 2 * b;
+            const double2 p = z[k * kFftRow + b], q = z[(k ? L - k : 0) * kFftRow + b];
+            if (a < nlines) w[a * h + k] = make_double2(0.5 * (p.x + q.x), 0.5 * (p.y - q.y));
+            if (a + 1 < nlines) w[(a + 1) * h + k] = make_double2(0.5 * (p.y + q.y), 0.5 * (q.x - p.x));
+        }
+    } else {
+        for (int idx = threadIdx.x; idx < L * kFftLines; idx += kFftNT) {
+            const int b = idx / L, t = idx - b * L;
+            const long long a = l0 + 2 * b;
+            const double2 p = z[t * kFftRow + b];
+            if (a < nlines) r[a * L + t] = p.x * scale;
+            if (a + 1 < nlines) r[(a + 1) * L + t] = p.y * scale;
         }
     }
 }
 
-int fft3_exec(FFT3* f, double2* data, int inverse, cudaStream_t s) {
-    const long long n1 = f->shape[0], n2 = f->shape[1], n3 = f->shape[2];
-    const double sign = inverse ? 1.0 : -1.0;
-    const int B = 16;
-    for (int axis = 2; axis >= 0; --axis) {
-        const int L = (int)f->shape[axis];
-        long long tstride, bstride, bsa, bsb;
-        int lines_per_base, nbase, nbase_b;
-        if (axis == 2) {        // lines along k, batched along j; bases = i
-            tstride = 1; bstride = n3; lines_per_base = (int)n2; nbase = (int)n1; nbase_b = 1;
-            bsa = n2 * n3; bsb = 0;
-        } else if (axis == 1) { // lines along j, batched along k; bases = i
-            tstride = n3; bstride = 1; lines_per_base = (int)n3; nbase = (int)n1; nbase_b = 1;
-            bsa = n2 * n3; bsb = 0;
-        } else {                // lines along i, batched along k; bases = j
-            tstride = n2 * n3; bstride = 1; lines_per_base = (int)n3; nbase = (int)n2; nbase_b = 1;
-            bsa = n3; bsb = 0;
-        }
-        const int groups = (lines_per_base + B - 1) / B;
-        const size_t smem = sizeof(double2) * 2 * (size_t)L * B;
-        LRES_CUDA_TRY(cudaFuncSetAttribute(fft_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        fft_pass_kernel<<<nbase * groups, 256, smem, s>>>(data, L, tstride, bstride, lines_per_base * nbase,
-                                                        lines_per_base, bsa, bsb, nbase_b, f->d_fac + axis * 16,
-                                                        sign, B);
-        LRES_CUDA_TRY(cudaGetLastError());
+// Lines of another axis over the half spectrum, 8 neighbouring wave numbers k of the contiguous
+// axis per CTA: element t of line (o, k) at w[o * ostride + t * tstride + k].  POISSON: forward,
+// times 4 pi scale / G^2 (0 at G = 0), back (the x axis; o is then the index of the y axis).
+template <bool INV, bool POISSON>
+__global__ void __launch_bounds__(kFftNT) fft_axis_kernel(FftAxis ax, int h, long long ostride, long long tstride,
+                                                          double2* w, const double* ky, const double* kz,
+                                                          double scale) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    const int L = ax.L;
+    double2* const tw = reinterpret_cast<double2*>(smraw);
+    double2* x = tw + L;
+    double2* y = x + (size_t)L * kFftRow;
+    const int groups = (h + kFftLines - 1) / kFftLines;
+    const int o = blockIdx.x / groups, k0 = (blockIdx.x - o * groups) * kFftLines;
+    double2* const base = w + o * ostride + k0;
+    for (int i = threadIdx.x; i < L; i += kFftNT) tw[i] = ax.tw[i];
+    for (int idx = threadIdx.x; idx < L * kFftLines; idx += kFftNT) {
+        const int b = idx & (kFftLines - 1), t = idx / kFftLines;
+        x[t * kFftRow + b] = k0 + b < h ? base[t * tstride + b] : make_double2(0.0, 0.0);
     }
+    __syncthreads();
+    double2* z = fft_lines<INV>(x, y, ax, tw);
+    if (POISSON) {
+        for (int idx = threadIdx.x; idx < L * kFftLines; idx += kFftNT) {
+            const int b = idx & (kFftLines - 1), t = idx / kFftLines;
+            const double kx = ax.k[t], gy = ky[o], gz = kz[min(k0 + b, h - 1)];
+            const double g2 = kx * kx + gy * gy + gz * gz;
+            const double f = g2 > 0.0 ? 4.0 * M_PI * scale / g2 : 0.0;
+            double2& v = z[t * kFftRow + b];
+            v = make_double2(f * v.x, f * v.y);
+        }
+        __syncthreads();
+        z = fft_lines<true>(z, z == x ? y : x, ax, tw);
+    }
+    for (int idx = threadIdx.x; idx < L * kFftLines; idx += kFftNT) {
+        const int b = idx & (kFftLines - 1), t = idx / kFftLines;
+        if (k0 + b < h) base[t * tstride + b] = z[t * kFftRow + b];
+    }
+}
+
+template <bool INV>
+static int fft_real(const FFT3* f, double* r, double2* w, double scale, cudaStream_t s) {
+    const long long nlines = (long long)f->ax[0].L * f->ax[1].L;
+    const size_t smem = fft_smem(f->ax[2].L);
+    LRES_CUDA_TRY(cudaFuncSetAttribute(fft_real_kernel<INV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const long long blocks = (nlines + 2 * kFftLines - 1) / (2 * kFftLines);
+    fft_real_kernel<INV><<<(unsigned)blocks, kFftNT, smem, s>>>(f->ax[2], nlines, r, w, scale);
+    LRES_CUDA_TRY(cudaGetLastError());
+    return LRES_OK;
+}
+
+// axis 0 (x) or 1 (y) of the half spectrum
+template <bool INV, bool POISSON>
+static int fft_axis(const FFT3* f, int axis, double2* w, double scale, cudaStream_t s) {
+    const int h = f->ax[2].L / 2 + 1;
+    const long long row = h, plane = (long long)f->ax[1].L * h;
+    const size_t smem = fft_smem(f->ax[axis].L);
+    LRES_CUDA_TRY(cudaFuncSetAttribute(fft_axis_kernel<INV, POISSON>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)smem));
+    const unsigned blocks = (unsigned)(f->ax[1 - axis].L * ((h + kFftLines - 1) / kFftLines));
+    fft_axis_kernel<INV, POISSON><<<blocks, kFftNT, smem, s>>>(f->ax[axis], h, axis ? plane : row, axis ? row : plane, w,
+                                                               f->ax[1].k, f->ax[2].k, scale);
+    LRES_CUDA_TRY(cudaGetLastError());
     return LRES_OK;
 }
 
-// ---------------------------------------------------------------------------
-// wave vectors as numpy: k = 2 pi * (f * (1 / (m * (L / m)))) with f the fftfreq index
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ double kvec(int i, int m, double L) {
-    const int f = (i < (m + 1) / 2) ? i : i - m;
-    const double d = L / (double)m;
-    const double val = 1.0 / ((double)m * d);
-    return 2.0 * M_PI * ((double)f * val);
-}
-
-__global__ void real_to_complex(const double* a, double2* b, long long n) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        b[i] = make_double2(a[i], 0.0);
-}
-
-__global__ void poisson_kernel(double2* w, int n1, int n2, int n3, double L1, double L2, double L3) {
-    const long long n = (long long)n1 * n2 * n3;
-    for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < n;
-         idx += (long long)gridDim.x * blockDim.x) {
-        const int k = (int)(idx % n3), j = (int)((idx / n3) % n2), i = (int)(idx / ((long long)n2 * n3));
-        const double kx = kvec(i, n1, L1), ky = kvec(j, n2, L2), kz = kvec(k, n3, L3);
-        const double G2 = kx * kx + ky * ky + kz * kz;
-        double2 v = w[idx];
-        if (idx == 0) {
-            v = make_double2(0.0, 0.0);
-        } else {
-            const double f = 4.0 * M_PI;
-            v = make_double2(f * v.x / G2, f * v.y / G2);
-        }
-        w[idx] = v;
-    }
-}
-
-__global__ void complex_real_part(const double2* a, double* b, long long n, double scale) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        b[i] = a[i].x * scale;
-}
-
-int hartree_apply(FFT3* f, const int64_t shape[3], const double cell[3], const double* dens, double* vh,
-                  double2* work, cudaStream_t s) {
-    const long long n = shape[0] * shape[1] * shape[2];
-    real_to_complex<<<1216, 256, 0, s>>>(dens, work, n);
-    LRES_CUDA_TRY(cudaGetLastError());
-    int rc = fft3_exec(f, work, 0, s);
-    if (rc) return rc;
-    poisson_kernel<<<1216, 256, 0, s>>>(work, (int)shape[0], (int)shape[1], (int)shape[2], cell[0], cell[1], cell[2]);
-    LRES_CUDA_TRY(cudaGetLastError());
-    rc = fft3_exec(f, work, 1, s);
-    if (rc) return rc;
-    complex_real_part<<<1216, 256, 0, s>>>(work, vh, n, 1.0 / (double)n);
-    LRES_CUDA_TRY(cudaGetLastError());
-    return LRES_OK;
+int hartree_apply(FFT3* f, const double* dens, double* vh, double2* work, cudaStream_t s) {
+    const double scale = 1.0 / ((double)f->ax[0].L * f->ax[1].L * f->ax[2].L);
+    int rc = fft_real<false>(f, const_cast<double*>(dens), work, 1.0, s);
+    if (!rc) rc = fft_axis<false, false>(f, 1, work, 1.0, s);
+    if (!rc) rc = fft_axis<false, true>(f, 0, work, scale, s);
+    if (!rc) rc = fft_axis<true, false>(f, 1, work, 1.0, s);
+    if (!rc) rc = fft_real<true>(f, vh, work, 1.0, s);
+    return rc;
 }
 
 // ---------------------------------------------------------------------------
@@ -303,23 +379,35 @@ int lda_apply(long long n, const double* dens, double* exc, double* vxc, cudaStr
 // ion potential: v(G) = -4 pi / G^2 * sum_a Z_a exp(-i G.R_a - G^2 rc_a^2 / 4) / vol,
 // G = 0 removed, then v(r) = IFFT(v(G)) * ng (lrft/three_d.py:102-112,119)
 // ---------------------------------------------------------------------------
-__global__ void ion_structure_kernel(double2* w, int n1, int n2, int n3, double L1, double L2, double L3, int natoms,
-                                     const double* pos, const double* Z, const double* rc) {
-    const long long n = (long long)n1 * n2 * n3;
-    const double vol = L1 * L2 * L3;
+__global__ void ion_structure_kernel(double2* w, int n1, int n2, int n3, const double* k1, const double* k2,
+                                     const double* k3, double vol, int natoms, const double* pos, const double* Z,
+                                     const double* rc) {
+    const int h = n3 / 2 + 1;
+    const long long n = (long long)n1 * n2 * h;
     for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < n;
          idx += (long long)gridDim.x * blockDim.x) {
-        const int k = (int)(idx % n3), j = (int)((idx / n3) % n2), i = (int)(idx / ((long long)n2 * n3));
-        const double kx = kvec(i, n1, L1), ky = kvec(j, n2, L2), kz = kvec(k, n3, L3);
+        const int k = (int)(idx % h), j = (int)((idx / h) % n2), i = (int)(idx / ((long long)n2 * h));
+        const double kx = k1[i], ky = k2[j], kz = k3[k];
         const double G2 = kx * kx + ky * ky + kz * kz;
         double sx = 0.0, sy = 0.0;
-        for (int a = 0; a < natoms; ++a) {
-            const double ph = kx * pos[3 * a] + ky * pos[3 * a + 1] + kz * pos[3 * a + 2];
-            const double amp = Z[a] * exp(-G2 * rc[a] * rc[a] / 4.0);
-            double sn, cs;
-            sincos(ph, &sn, &cs);
-            sx += amp * cs;
-            sy -= amp * sn;
+        // at the highest wave number of an even axis, where +k and -k are one, the mean of both
+        // signs (the real part of the full transform is wanted; on the planes k = 0 and n3 / 2 the
+        // real lines take it)
+        const bool inner = k > 0 && 2 * k != n3, ny1 = inner && 2 * i == n1, ny2 = inner && 2 * j == n2;
+        for (int pass = 0; pass < 1 + (ny1 || ny2); ++pass) {
+            const double px = pass && ny1 ? -kx : kx, py = pass && ny2 ? -ky : ky;
+            for (int a = 0; a < natoms; ++a) {
+                const double ph = px * pos[3 * a] + py * pos[3 * a + 1] + kz * pos[3 * a + 2];
+                const double amp = Z[a] * exp(-G2 * rc[a] * rc[a] / 4.0);
+                double sn, cs;
+                sincos(ph, &sn, &cs);
+                sx += amp * cs;
+                sy -= amp * sn;
+            }
+        }
+        if (ny1 || ny2) {
+            sx *= 0.5;
+            sy *= 0.5;
         }
         double2 v;
         if (idx == 0) v = make_double2(0.0, 0.0);
@@ -331,18 +419,17 @@ __global__ void ion_structure_kernel(double2* w, int n1, int n2, int n3, double 
     }
 }
 
-int ion_apply(FFT3* f, const int64_t shape[3], const double cell[3], int natoms, const double* pos, const double* Z,
-              const double* rc, double* vion, double2* work, cudaStream_t s) {
-    const long long n = shape[0] * shape[1] * shape[2];
-    ion_structure_kernel<<<1216, 256, 0, s>>>(work, (int)shape[0], (int)shape[1], (int)shape[2], cell[0], cell[1],
-                                              cell[2], natoms, pos, Z, rc);
+int ion_apply(FFT3* f, const double cell[3], int natoms, const double* pos, const double* Z, const double* rc,
+              double* vion, double2* work, cudaStream_t s) {
+    const FftAxis* ax = f->ax;
+    ion_structure_kernel<<<1216, 256, 0, s>>>(work, ax[0].L, ax[1].L, ax[2].L, ax[0].k, ax[1].k, ax[2].k,
+                                              cell[0] * cell[1] * cell[2], natoms, pos, Z, rc);
     LRES_CUDA_TRY(cudaGetLastError());
-    int r = fft3_exec(f, work, 1, s);
-    if (r) return r;
-    // ifftn scales by 1/ng and the reference multiplies by ng again
-    complex_real_part<<<1216, 256, 0, s>>>(work, vion, n, 1.0);
-    LRES_CUDA_TRY(cudaGetLastError());
-    return LRES_OK;
+    // (the inverse transform's 1/ng and the reference's factor ng cancel)
+    int r = fft_axis<true, false>(f, 0, work, 1.0, s);
+    if (!r) r = fft_axis<true, false>(f, 1, work, 1.0, s);
+    if (!r) r = fft_real<true>(f, vion, work, 1.0, s);
+    return r;
 }
 
 // ---------------------------------------------------------------------------

@@ -175,14 +175,13 @@ int adj_point(long long ng, const long long* poff, const int2* pent, const Suppo
               const double* gH, double dV, double* dv, cudaStream_t s);
 
 struct FFT3;
-int fft3_create(FFT3** out, const int64_t shape[3]);
+int fft3_create(FFT3** out, const int64_t shape[3], const double cell[3]);
 void fft3_destroy(FFT3* f);
-int fft3_exec(FFT3* f, double2* data, int inverse, cudaStream_t s);
-int hartree_apply(FFT3* f, const int64_t shape[3], const double cell[3], const double* dens, double* vh,
-                  double2* work, cudaStream_t s);
+// work: n1 n2 (n3 / 2 + 1) complex values
+int hartree_apply(FFT3* f, const double* dens, double* vh, double2* work, cudaStream_t s);
 int lda_apply(long long n, const double* dens, double* exc, double* vxc, cudaStream_t s);
-int ion_apply(FFT3* f, const int64_t shape[3], const double cell[3], int natoms, const double* pos,
-              const double* Z, const double* rc, double* vion, double2* work, cudaStream_t s);
+int ion_apply(FFT3* f, const double cell[3], int natoms, const double* pos, const double* Z, const double* rc,
+              double* vion, double2* work, cudaStream_t s);
 int voronoi_apply(const int64_t shape[3], const double cell[3], int ncent, const double* centres, int* owner,
                   cudaStream_t s);
 
