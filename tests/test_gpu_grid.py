@@ -42,3 +42,32 @@ def test_hartree_and_ion(shape):
     # (the phases K.R of the corner of the spectrum are ~100, rounded to 1e-14)
     assert np.max(np.abs(got - want)) <= 1e-12 * np.max(np.abs(want))
     s.close()
+
+
+def test_lda_range():
+    """Densities from below the floor through both branches (rs = 1 at n = 3 / (4 pi)) to huge values,
+    inf and NaN as the formula treats them.  A handful of rounded operations per value: 4e-15."""
+    cr, s, go = _ops((8, 9, 10))
+    n = np.geomspace(1e-18, 1e40, cr.ng)
+    n[:6] = [0.0, -1.0, 1e-14, 3 / (4 * np.pi), np.nextafter(3 / (4 * np.pi), 1), np.nextafter(3 / (4 * np.pi), 0)]
+    nn = np.maximum(n, 1e-14)
+    rs = (3 / (4 * np.pi * nn)) ** (1 / 3)
+    ex = -0.75 * (3 * nn / np.pi) ** (1 / 3)
+    sr, lr = np.sqrt(rs), np.log(rs)
+    den = 1 + 1.0529 * sr + 0.3334 * rs
+    ec = np.where(rs >= 1, -0.1423 / den, 0.0311 * lr - 0.048 + 0.002 * rs * lr - 0.0116 * rs)
+    vc = np.where(rs >= 1, -0.1423 / den * (1 + 7 / 6 * 1.0529 * sr + 4 / 3 * 0.3334 * rs) / den,
+                  0.0311 * lr - 0.048 - 0.0311 / 3 + 2 / 3 * 0.002 * rs * lr + (-0.0232 - 0.002) / 3 * rs)
+    exc, vxc, _ = go.lda_hartree(n.reshape(cr.shape))
+    # (the two branches meet with a jump of 3e-5 at rs = 1: those three points are compared loosely)
+    tol = np.full(cr.ng, 4e-15)
+    tol[3:6] = 1e-4
+    assert np.all(np.abs(exc.ravel() - (ex + ec)) <= tol * np.abs(ex + ec))
+    assert np.all(np.abs(vxc.ravel() - (4 / 3 * ex + vc)) <= tol * np.abs(4 / 3 * ex + vc))
+    n[:] = 0.1
+    n[:3] = [np.inf, np.nan, 1e308]
+    exc, _, _ = go.lda_hartree(n.reshape(cr.shape))
+    e = exc.ravel()
+    assert not np.isfinite(e[0]) and np.isfinite(e[2])
+    assert e[1] == pytest.approx(-0.75 * (3 * 1e-14 / np.pi) ** (1 / 3) - 0.1423 / (1 + 1.0529 * (3 / (4e-14 * np.pi)) ** (1 / 6) + 0.3334 * (3 / (4e-14 * np.pi)) ** (1 / 3)))
+    s.close()
