@@ -36,6 +36,8 @@ struct FFT3 {
     FftAxis ax[3];
     double2* d_tw = nullptr;
     double* d_k = nullptr;
+    double2* d_ion = nullptr;         // scratch of the ion potential
+    size_t ion_size = 0;
 };
 
 static std::vector<int> factorise(int n) {
@@ -98,6 +100,7 @@ void fft3_destroy(FFT3* f) {
     if (!f) return;
     cudaFree(f->d_tw);
     cudaFree(f->d_k);
+    cudaFree(f->d_ion);
     delete f;
 }
 
@@ -413,55 +416,137 @@ int lda_apply(long long n, const double* dens, double* exc, double* vxc, cudaStr
 // ---------------------------------------------------------------------------
 // ion potential: v(G) = -4 pi / G^2 * sum_a Z_a exp(-i G.R_a - G^2 rc_a^2 / 4) / vol,
 // G = 0 removed, then v(r) = IFFT(v(G)) * ng (lrft/three_d.py:102-112,119)
+//
+// The exponential is a product over the axes, E_x E_y E_z with E = exp(-i k R - k^2 rc^2 / 4), so
+// sincos and exp run per (atom, axis, wave number) instead of per (atom, G), and what is left is
+// a contraction over the atoms on the FP64 pipe.  With Q = Z E_x E_z and E_y = c - i s, the sums
+// U = sum Q c and V = sum Q s give the structure factor at both +k_y (U - iV) and -k_y (U + iV):
+// two FP64 multiply-adds per (atom, G) plus the product Q, shared by the lanes' columns.
+// Measured (1024 atoms, 64^3): 24.7 ms one sincos and exp per (atom, G) of the full grid, 15.7 ms
+// of the half spectrum, 1.25 ms this way.
 // ---------------------------------------------------------------------------
-__global__ void ion_structure_kernel(double2* w, int n1, int n2, int n3, const double* k1, const double* k2,
-                                     const double* k3, double vol, int natoms, const double* pos, const double* Z,
-                                     const double* rc) {
-    const int h = n3 / 2 + 1;
-    const long long n = (long long)n1 * n2 * h;
-    for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < n;
-         idx += (long long)gridDim.x * blockDim.x) {
-        const int k = (int)(idx % h), j = (int)((idx / h) % n2), i = (int)(idx / ((long long)n2 * h));
-        const double kx = k1[i], ky = k2[j], kz = k3[k];
-        const double G2 = kx * kx + ky * ky + kz * kz;
-        double sx = 0.0, sy = 0.0;
-        // at the highest wave number of an even axis, where +k and -k are one, the mean of both
-        // signs (the real part of the full transform is wanted; on the planes k = 0 and n3 / 2 the
-        // real lines take it)
-        const bool inner = k > 0 && 2 * k != n3, ny1 = inner && 2 * i == n1, ny2 = inner && 2 * j == n2;
-        for (int pass = 0; pass < 1 + (ny1 || ny2); ++pass) {
-            const double px = pass && ny1 ? -kx : kx, py = pass && ny2 ? -ky : ky;
-            for (int a = 0; a < natoms; ++a) {
-                const double ph = px * pos[3 * a] + py * pos[3 * a + 1] + kz * pos[3 * a + 2];
-                const double amp = Z[a] * exp(-G2 * rc[a] * rc[a] / 4.0);
-                double sn, cs;
-                sincos(ph, &sn, &cs);
-                sx += amp * cs;
-                sy -= amp * sn;
-            }
-        }
-        if (ny1 || ny2) {
-            sx *= 0.5;
-            sy *= 0.5;
-        }
-        double2 v;
-        if (idx == 0) v = make_double2(0.0, 0.0);
-        else {
-            const double f = -4.0 * M_PI / G2 / vol;
-            v = make_double2(f * sx, f * sy);
-        }
-        w[idx] = v;
+
+// E[a * ld + i], i <= L / 2, times Z_a on the x axis: the non-negative wave numbers of x and y; of z as
+// numpy's (the highest of an even axis is negative: on that plane its sign goes with those of x and y).
+__global__ void ion_axis_kernel(int natoms, int axis, int ld, const double* k, const double* pos, const double* Z,
+                                const double* rc, double2* E) {
+    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= natoms * ld) return;
+    const int a = idx / ld, i = idx - a * ld;
+    const double q = axis == 2 ? k[i] : fabs(k[i]);
+    double sn, cs;
+    sincos(q * pos[3 * a + axis], &sn, &cs);
+    const double amp = (axis == 0 ? Z[a] : 1.0) * exp(-q * q * rc[a] * rc[a] / 4.0);
+    E[idx] = make_double2(amp * cs, -amp * sn);
+}
+
+constexpr int kIonCols = 4;                   // wave numbers k_y of a thread
+constexpr int kIonWarps = 3;                  // groups of columns of a CTA
+
+// Structure factor on the extended half grid T[(i * (2 l2) + j) * h + k]: i over 2 l1 - 1 signed wave
+// numbers of the x axis (0 .. l1-1, then -1 .. -(l1-1)), j over +0 .. +(l2-1), -0 .. -(l2-1).
+// Lane = (i, k), k fastest; a warp takes kIonCols columns.
+__global__ void __launch_bounds__(32 * kIonWarps) ion_sum_kernel(int natoms, int l1, int l2, int h, const double2* Ex,
+                                                                 const double2* Ey, const double2* Ez, double2* T) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rows = (2 * l1 - 1) * h;
+    const int row = min(blockIdx.x * 32 + lane, rows - 1);
+    const int i = row / h, k = row - i * h;
+    const int ia = i < l1 ? i : i - l1 + 1;
+    const double sx = i < l1 ? 1.0 : -1.0;
+    const int j0 = (blockIdx.y * kIonWarps + warp) * kIonCols;
+    if (j0 >= l2) return;
+    int jj[kIonCols];
+    double2 U[kIonCols], V[kIonCols];
+#pragma unroll
+    for (int c = 0; c < kIonCols; ++c) {
+        jj[c] = min(j0 + c, l2 - 1);
+        U[c] = V[c] = make_double2(0.0, 0.0);
     }
+#pragma unroll 2
+    for (int a = 0; a < natoms; ++a) {
+        double2 x = Ex[(long long)a * l1 + ia];
+        x.y *= sx;
+        const double2 z = Ez[(long long)a * h + k];
+        const double2 q = cmulc(x, z);
+#pragma unroll
+        for (int c = 0; c < kIonCols; ++c) {
+            const double2 y = Ey[(long long)a * l2 + jj[c]];       // (c, -s)
+            U[c].x = fma(q.x, y.x, U[c].x);
+            U[c].y = fma(q.y, y.x, U[c].y);
+            V[c].x = fma(q.x, y.y, V[c].x);
+            V[c].y = fma(q.y, y.y, V[c].y);
+        }
+    }
+    if (blockIdx.x * 32 + lane >= rows) return;
+    double2* const out = T + (long long)i * 2 * l2 * h + k;
+#pragma unroll
+    for (int c = 0; c < kIonCols; ++c) {
+        if (j0 + c >= l2) break;
+        out[(long long)(j0 + c) * h] = make_double2(U[c].x - V[c].y, U[c].y + V[c].x);        // U + i (-sum Q s)
+        out[(long long)(l2 + j0 + c) * h] = make_double2(U[c].x + V[c].y, U[c].y - V[c].x);
+    }
+}
+
+// v(G) on the half spectrum.  At the highest wave number of an even axis, where +k and -k are one,
+// the mean of both signs (the real part of the full transform is wanted; on the planes k = 0 and
+// n3 / 2 the real lines take it).
+__global__ void ion_potential_kernel(int n1, int n2, int n3, const double* k1, const double* k2, const double* k3,
+                                     double vol, const double2* T, double2* w) {
+    const int h = n3 / 2 + 1, l1 = n1 / 2 + 1, l2 = n2 / 2 + 1;
+    const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (idx >= (long long)n1 * n2 * h) return;
+    const int k = (int)(idx % h), j = (int)((idx / h) % n2), i = (int)(idx / ((long long)n2 * h));
+    const double kx = k1[i], ky = k2[j], kz = k3[k];
+    const double G2 = kx * kx + ky * ky + kz * kz;
+    // rows of the signed wave numbers: the highest one of an even axis is negative, as numpy's
+    const int pi = kx >= 0.0 ? i : l1 - 1 + (n1 - i), pj = ky >= 0.0 ? j : l2 + (n2 - j);
+    double2 v = T[((long long)pi * 2 * l2 + pj) * h + k];
+    const bool inner = k > 0 && 2 * k != n3, ny1 = inner && 2 * i == n1, ny2 = inner && 2 * j == n2;
+    if (ny1 || ny2) {
+        const int qi = ny1 ? i : pi, qj = ny2 ? j : pj;            // the positive sign
+        const double2 u = T[((long long)qi * 2 * l2 + qj) * h + k];
+        v = make_double2(0.5 * (v.x + u.x), 0.5 * (v.y + u.y));
+    }
+    const double f = idx == 0 ? 0.0 : -4.0 * M_PI / G2 / vol;
+    w[idx] = make_double2(f * v.x, f * v.y);
 }
 
 int ion_apply(FFT3* f, const double cell[3], int natoms, const double* pos, const double* Z, const double* rc,
               double* vion, double2* work, cudaStream_t s) {
     const FftAxis* ax = f->ax;
-    ion_structure_kernel<<<1216, 256, 0, s>>>(work, ax[0].L, ax[1].L, ax[2].L, ax[0].k, ax[1].k, ax[2].k,
-                                              cell[0] * cell[1] * cell[2], natoms, pos, Z, rc);
-    LRES_CUDA_TRY(cudaGetLastError());
+    const int l[3] = {ax[0].L / 2 + 1, ax[1].L / 2 + 1, ax[2].L / 2 + 1}, h = l[2];
+    // the axis factors and the extended structure factor
+    const size_t nE = (size_t)natoms * (l[0] + l[1] + l[2]), nT = (size_t)(2 * l[0] - 1) * 2 * l[1] * h;
+    if (f->ion_size < nE + nT) {                   // kept with the plan, grown on demand
+        if (f->d_ion) cudaFree(f->d_ion);
+        f->d_ion = nullptr;
+        f->ion_size = 0;
+        if (cudaMalloc(&f->d_ion, sizeof(double2) * (nE + nT)) != cudaSuccess) {
+            cudaGetLastError();
+            lres_set_error("ion potential: allocation of %zu bytes failed", sizeof(double2) * (nE + nT));
+            return LRES_ENOMEM;
+        }
+        f->ion_size = nE + nT;
+    }
+    double2* E[3] = {f->d_ion, nullptr, nullptr};
+    E[1] = E[0] + (size_t)natoms * l[0];
+    E[2] = E[1] + (size_t)natoms * l[1];
+    double2* const T = E[0] + nE;
+    for (int a = 0; a < 3; ++a)
+        ion_axis_kernel<<<(natoms * l[a] + 127) / 128, 128, 0, s>>>(natoms, a, l[a], ax[a].k, pos, Z, rc, E[a]);
+    const dim3 grid(((2 * l[0] - 1) * h + 31) / 32, (l[1] + kIonWarps * kIonCols - 1) / (kIonWarps * kIonCols));
+    ion_sum_kernel<<<grid, 32 * kIonWarps, 0, s>>>(natoms, l[0], l[1], h, E[0], E[1], E[2], T);
+    const long long n = (long long)ax[0].L * ax[1].L * h;
+    ion_potential_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(ax[0].L, ax[1].L, ax[2].L, ax[0].k, ax[1].k,
+                                                                     ax[2].k, cell[0] * cell[1] * cell[2], T, work);
+    int r = LRES_OK;
+    if (cudaError_t e = cudaGetLastError(); e != cudaSuccess) {
+        lres_set_error("ion potential: %s", cudaGetErrorString(e));
+        r = LRES_ECUDA;
+    }
     // (the inverse transform's 1/ng and the reference's factor ng cancel)
-    int r = fft_axis<true, false>(f, 0, work, 1.0, s);
+    if (!r) r = fft_axis<true, false>(f, 0, work, 1.0, s);
     if (!r) r = fft_axis<true, false>(f, 1, work, 1.0, s);
     if (!r) r = fft_real<true>(f, vion, work, 1.0, s);
     return r;
