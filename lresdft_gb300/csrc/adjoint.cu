@@ -19,7 +19,10 @@
 // The mixed path maps these back with L^-T ( . ) L^-1.  dE/dv(r) = dV x_r^T (sum_B dE/dH_W) x_r
 // over the atom pairs that share the point r (the adjoint of the H(v) assembly).
 #include "common.cuh"
+#include "launch.cuh"
 #include "lres_internal.h"
+
+#include <algorithm>
 
 namespace lres {
 
@@ -187,6 +190,153 @@ __global__ void __launch_bounds__(256) adj_accum_kernel(const int* wins, int P, 
         }
 }
 
+// ---------------------------------------------------------------------------
+// The same accumulations from the tridiagonal form (FP64 path on the tridiagonal route).
+//
+// With A^ = L^-1 H_W L^-T = Q T Q^T, Y = F^ Q and K = Y^T Y,
+//
+//     A_c = W X_c W^T,  W = L^-T Q,  X_c = Re sum_k c_k G_k K G_k,  G_k = (z_k - T)^-1,
+//
+// so a pole costs two tridiagonal solves with n right-hand sides instead of a dense
+// factorisation and m back-substitutions: ~23 n^2 FP64 multiply-adds against
+// 4 (n^3 / 3 + 3 m n^2).  The FP64 pipe bounds it (54 windows x 32 poles: 6.6 ms at 1.6
+// multiply-adds per clock and SM; measured 9.2 ms; forward and backward of 54 windows together
+// 626 -> 168 ms).
+// ---------------------------------------------------------------------------
+
+// Per (window, pole): the multipliers t_i = e_{i-1} / D_{i-1} and 1 / D_i of the LDL^T of z_k - T
+// (D_i = z - d_i - e_{i-1} t_i; Im D_i >= Im z), coef[item * ld + i] = (t, 1 / D).
+__global__ void adj_pivot_kernel(int nwin, int P, const int* n_w, const long long* offN, const double* d,
+                                 const double* e, const double2* z, int ld, double4* coef) {
+    const int it = blockIdx.x * blockDim.x + threadIdx.x;
+    if (it >= nwin * P) return;
+    const int w = it / P;
+    const double2 zk = z[it - w * P];
+    const int n = n_w[w];
+    const double *dw = d + offN[w], *ew = e + offN[w];
+    double4* out = coef + (size_t)it * ld;
+    double2 t = make_double2(0.0, 0.0), g = t;
+    for (int i = 0; i < n; ++i) {
+        double2 D = make_double2(zk.x - dw[i], zk.y);
+        if (i) {
+            const double el = ew[i - 1];
+            t = make_double2(el * g.x, el * g.y);
+            D.x = fma(-el, t.x, D.x);
+            D.y = fma(-el, t.y, D.y);
+        }
+        const double inv = 1.0 / (D.x * D.x + D.y * D.y);
+        g = make_double2(D.x * inv, -D.y * inv);
+        out[i] = make_double4(t.x, t.y, g.x, g.y);
+    }
+}
+
+constexpr int kSweepNT = 320;
+
+// One CTA per (window, group of poles): X_c += Re c_k G_k K G_k over its poles, the upper triangle
+// of group g at Xc[g * sizeC + offC + i + j n], i <= j.  Thread = column of K for
+// G_k K, then row of it for the second solve (whose back substitution stops at the diagonal);
+// every access but the reads of the second forward sweep runs along the threads.
+__global__ void __launch_bounds__(kSweepNT) adj_sweep_kernel(const int* wins, int P, int groups, const int* n_w,
+                                                             const long long* offC, long long sizeC, const double* K,
+                                                             const double4* coef, int ld, const double2* cw,
+                                                             double2* ws, long long ws_stride, double* Xa, double* Xb,
+                                                             double* Xc) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double4* const cf = reinterpret_cast<double4*>(smem_raw);       // [n + 1]
+    const int w = wins[blockIdx.x / groups], grp = blockIdx.x % groups;
+    const int n = n_w[w], tid = threadIdx.x;
+    const int k0 = P * grp / groups, k1 = P * (grp + 1) / groups;
+    const double* const Kw = K + offC[w];
+    double2* const B = ws + (size_t)blockIdx.x * ws_stride;         // (G K)^T: B[j + i n] = (G K)_ij
+    double2* const U = B + (size_t)n * n;                           // U[i + j n]
+    for (int k = k0; k < k1; ++k) {
+        __syncthreads();
+        const double4* const src = coef + (size_t)(w * P + k) * ld;
+        for (int i = tid; i < n; i += kSweepNT) cf[i] = src[i];
+        if (tid == 0) cf[n] = make_double4(0.0, 0.0, 0.0, 0.0);
+        __syncthreads();
+        for (int j = tid; j < n; j += kSweepNT) {
+            double2 u = make_double2(0.0, 0.0);
+#pragma unroll 4
+            for (int i = 0; i < n; ++i) {
+                const double4 c = cf[i];
+                u = make_double2(fma(c.x, u.x, fma(-c.y, u.y, Kw[j + (long long)i * n])), fma(c.x, u.y, c.y * u.x));
+                B[j + (long long)i * n] = u;
+            }
+            double2 x = make_double2(0.0, 0.0);
+#pragma unroll 4
+            for (int i = n - 1; i >= 0; --i) {
+                const double4 c = cf[i], cn = cf[i + 1];
+                const double2 v = B[j + (long long)i * n];
+                x = make_double2(fma(v.x, c.z, fma(-v.y, c.w, fma(cn.x, x.x, -cn.y * x.y))),
+                                 fma(v.x, c.w, fma(v.y, c.z, fma(cn.x, x.y, cn.y * x.x))));
+                B[j + (long long)i * n] = x;
+            }
+        }
+        __syncthreads();
+        const double2 c0 = cw[k], c1 = cw[P + k], c2 = cw[2 * P + k];
+        double* const X0 = Xa + (size_t)grp * sizeC + offC[w];
+        double* const X1 = Xb + (size_t)grp * sizeC + offC[w];
+        double* const X2 = Xc + (size_t)grp * sizeC + offC[w];
+        for (int i = tid; i < n; i += kSweepNT) {
+            double2 u = make_double2(0.0, 0.0);
+#pragma unroll 4
+            for (int j = 0; j < n; ++j) {
+                const double4 c = cf[j];
+                const double2 b = B[j + (long long)i * n];
+                u = make_double2(fma(c.x, u.x, fma(-c.y, u.y, b.x)), fma(c.x, u.y, fma(c.y, u.x, b.y)));
+                if (j >= i) U[i + (long long)j * n] = u;
+            }
+            double2 x = make_double2(0.0, 0.0);
+#pragma unroll 2
+            for (int j = n - 1; j >= i; --j) {
+                const double4 c = cf[j], cn = cf[j + 1];
+                const long long at = i + (long long)j * n;
+                const double2 v = U[at];
+                x = make_double2(fma(v.x, c.z, fma(-v.y, c.w, fma(cn.x, x.x, -cn.y * x.y))),
+                                 fma(v.x, c.w, fma(v.y, c.z, fma(cn.x, x.y, cn.y * x.x))));
+                const double y0 = k == k0 ? 0.0 : X0[at], y1 = k == k0 ? 0.0 : X1[at], y2 = k == k0 ? 0.0 : X2[at];
+                X0[at] = fma(c0.x, x.x, fma(-c0.y, x.y, y0));
+                X1[at] = fma(c1.x, x.x, fma(-c1.y, x.y, y1));
+                X2[at] = fma(c2.x, x.x, fma(-c2.y, x.y, y2));
+            }
+        }
+    }
+}
+
+// A_c = the sum of the groups' upper triangles in order, both triangles written (32 x 32 tiles; one
+// group may be in place).
+__global__ void __launch_bounds__(256) adj_groups_kernel(int groups, const int* n_w, const long long* offC,
+                                                         long long sizeC, const double* Xa, const double* Xb,
+                                                         const double* Xc, double* A0, double* A1, double* A2) {
+    __shared__ double tile[32][33];
+    const int w = blockIdx.z, n = n_w[w];
+    const int i0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
+    if (i0 > j0 || j0 >= n) return;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const double* const ins[3] = {Xa, Xb, Xc};
+    double* const outs[3] = {A0, A1, A2};
+    for (int c = 0; c < 3; ++c) {
+        const double* const src = ins[c] + offC[w];
+        double* const dst = outs[c] + offC[w];
+        __syncthreads();
+        for (int q = ty; q < 32; q += 8) {
+            const int i = i0 + tx, j = j0 + q;
+            if (i <= j && j < n) {
+                double s = 0.0;
+                for (int g = 0; g < groups; ++g) s += src[(size_t)g * sizeC + i + (long long)j * n];
+                dst[i + (long long)j * n] = s;
+                tile[q][tx] = s;
+            }
+        }
+        __syncthreads();
+        for (int q = ty; q < 32; q += 8) {
+            const int i = i0 + q, j = j0 + tx;
+            if (i < j && j < n) dst[j + (long long)i * n] = tile[tx][q];
+        }
+    }
+}
+
 // Pole weights of the three accumulations: c_0 = w_k, c_1 = w_k z_k, c_2 = w_k z_k^2,
 // nodes as the forward pass computes them (lrft/core.py:130-139).
 __global__ void adj_weights_kernel(int P, int M, double mu, double e_lo, double2* cw) {
@@ -332,6 +482,41 @@ int adj_accumulate(bool fp32, const int* wins, int nwin_batch, int P, int nmax, 
     else
         adj_accum_kernel<double2, kKeepNB128><<<grid, 256, 0, s>>>(wins, P, n_w, m_w, offC, (const double2*)ws,
                                                                    ws_stride, cw, A0, A1, A2);
+    LRES_CUDA_TRY(cudaGetLastError());
+    return LRES_OK;
+}
+
+// pole groups of a window in the sweeps: two CTAs per SM in all
+int adj_sweep_groups(int nwin, int P) {
+    return std::max(1, std::min(P, 2 * device_sms() / std::max(nwin, 1)));
+}
+
+int adj_tri(int nwin, int P, int groups, int batch, int nmax, const int* wins, const int* n_w, const long long* offN,
+            const long long* offC, long long sizeC, const double* d, const double* e, const double2* shifts,
+            const double2* cw, const double* K, double4* coef, double2* ws, double* X, double* A0, double* A1,
+            double* A2, size_t smem_budget, cudaStream_t s) {
+    if (!nwin) return LRES_OK;
+    const size_t smem = sizeof(double4) * ((size_t)nmax + 1);
+    if (smem > smem_budget || nwin > 65535) {
+        lres_set_error("adjoint sweeps: windows of %d functions (%zu B of shared memory), %d windows", nmax, smem, nwin);
+        return LRES_EINVAL;
+    }
+    adj_pivot_kernel<<<(unsigned)(((long long)nwin * P + 31) / 32), 32, 0, s>>>(nwin, P, n_w, offN, d, e, shifts, nmax,
+                                                                               coef);
+    LRES_CUDA_TRY(cudaGetLastError());
+    int per_sm = 0;
+    if (int rc = prepare_kernel<adj_sweep_kernel>(kSweepNT, smem, &per_sm)) return rc;
+    // one group accumulates in place
+    double* const Xa = groups > 1 ? X : A0;
+    double* const Xb = groups > 1 ? Xa + (size_t)groups * sizeC : A1;
+    double* const Xc = groups > 1 ? Xb + (size_t)groups * sizeC : A2;
+    for (int w0 = 0; w0 < nwin; w0 += batch) {
+        adj_sweep_kernel<<<(unsigned)std::min(batch, nwin - w0) * groups, kSweepNT, smem, s>>>(
+            wins + w0, P, groups, n_w, offC, sizeC, K, coef, nmax, cw, ws, 2LL * nmax * nmax, Xa, Xb, Xc);
+        LRES_CUDA_TRY(cudaGetLastError());
+    }
+    const int T = (nmax + 31) / 32;
+    adj_groups_kernel<<<dim3(T, T, nwin), 256, 0, s>>>(groups, n_w, offC, sizeC, Xa, Xb, Xc, A0, A1, A2);
     LRES_CUDA_TRY(cudaGetLastError());
     return LRES_OK;
 }

@@ -130,6 +130,7 @@ struct lres_ctx {
         }
     };
     RowItems ri_own, ri_tr;
+    RowItems ri_adj;                             // the rows of L^-T (adjoint)
     // pole work
     int2 *d_items = nullptr, *d_items_win = nullptr, *d_items_sub = nullptr;
     int nitems = 0;
@@ -191,6 +192,7 @@ lres_ctx::~lres_ctx() {
         if (p) cudaFree(p);
     ri_own.release();
     ri_tr.release();
+    ri_adj.release();
     if (fft) fft3_destroy(fft);
     for (cudaEvent_t e : ev)
         if (e) cudaEventDestroy(e);
@@ -1774,25 +1776,63 @@ int adj_prepare(lres_ctx* c, cudaStream_t s) {
     return LRES_OK;
 }
 
-}  // namespace
+// Workspace of the adjoint: at least `least` bytes, up to `want` as far as the free device memory
+// admits; *got receives its size.
+int adj_workspace(lres_ctx* c, size_t least, size_t want, size_t* got) {
+    if (c->adjws_bytes < want) {
+        size_t freeb = 0, totalb = 0;
+        LRES_CUDA_TRY(cudaMemGetInfo(&freeb, &totalb));
+        const size_t have = c->adjws_bytes + freeb, reserve = (size_t)4 << 30;
+        const size_t budget = have > reserve ? std::min(have - reserve, have / 4 * 3) : 0;
+        const size_t take = std::min(want, budget);
+        if (take < least) {
+            lres_set_error("adjoint: the factors of one window (%zu bytes) do not fit in free device memory", least);
+            return LRES_ENOMEM;
+        }
+        if (take > c->adjws_bytes) {
+            if (c->d_adjws) cudaFree(c->d_adjws);
+            c->d_adjws = nullptr;
+            c->adjws_bytes = 0;
+            TRY(dalloc((char**)&c->d_adjws, take));
+            c->adjws_bytes = take;
+        }
+    }
+    *got = c->adjws_bytes;
+    return LRES_OK;
+}
 
-extern "C" int lres_adjoint(lres_ctx* c, double mu, double e_lo, double* dv, int dv_on_device, double* dHW,
-                            double* dSW, int dW_on_device, double* out, void* stream) {
-    if (!c || !out) {
-        lres_set_error("null argument");
-        return LRES_EINVAL;
-    }
-    if (!c->have_h) {
-        lres_set_error("lres_adjoint before a Hamiltonian was set");
-        return LRES_ESTATE;
-    }
-    if (!(mu > e_lo) || !std::isfinite(mu) || !std::isfinite(e_lo)) {
-        lres_set_error("need finite e_lo < mu (got mu=%g, e_lo=%g)", mu, e_lo);
-        return LRES_EINVAL;
-    }
-    cudaStream_t s = (cudaStream_t)stream;
-    TRY(ensure_hhat_df(c, s));                 // the adjoint factors the double-float standard form
-    TRY(adj_prepare(c, s));
+// The accumulations of the adjoint from the tridiagonal form (FP64): N, E_band and the density by the
+// pass, A_c in the tridiagonal basis into d_adjA, W = L^-T Q in place of the standard form (which the
+// reduction has consumed).
+int adj_tri_accumulate(lres_ctx* c, cudaStream_t s) {
+    if (!c->tri_ready) TRY(tri_refresh(c, s));
+    const int P = c->npoles;
+    const int groups = adj_sweep_groups(c->nwin, P);
+    const size_t coefb = sizeof(double4) * (size_t)c->nwin * P * c->nmax;
+    const size_t xb = groups > 1 ? sizeof(double) * 3 * (size_t)groups * c->sizeC : 0;
+    const size_t perw = sizeof(double2) * 2 * (size_t)c->nmax * c->nmax * groups;
+    size_t got = 0;
+    TRY(adj_workspace(c, coefb + xb + perw, coefb + xb + perw * c->nwin, &got));
+    const int batch = (int)std::min<size_t>(c->nwin, (got - coefb - xb) / perw);
+    char* const base = static_cast<char*>(c->d_adjws);
+    double4* const coef = reinterpret_cast<double4*>(base);
+    double* const X = reinterpret_cast<double*>(base + coefb);
+    double2* const ws = reinterpret_cast<double2*>(base + coefb + xb);
+    TRY(tri_run_pass(c, c->have_trace, s));
+    // K = Y^T Y (dE/dH_W's array is free until the end)
+    TRY(batched_gram(c->nwin, c->d_n, c->have_trace ? c->d_mT : c->d_m, c->have_trace ? c->d_offFT : c->d_offF,
+                     c->d_offC, c->nmax, static_cast<const double*>(c->have_trace ? c->d_Ytr : c->d_Yown), c->d_dHW, s));
+    if (c->ri_adj.arows != c->tri.arows) TRY(build_row_items(c, c->n_w, c->ri_adj, s));
+    TRY(tri_apply(false, c->ri_adj.napply, c->ri_adj.apply, c->d_n, c->d_n, c->d_offA, c->d_offN, c->d_offC, c->d_triA,
+                  c->d_tritau, c->d_LinvT, c->d_Hhat, c->tri, c->nwin, false, c->d_triT, c->smem_budget, s));
+    return adj_tri(c->nwin, P, groups, batch, c->nmax, c->d_order, c->d_n, c->d_offN, c->d_offC, c->sizeC,
+                   static_cast<const double*>(c->d_trid), static_cast<const double*>(c->d_trie),
+                   static_cast<const double2*>(c->d_shifts), c->d_cw, c->d_dHW, coef, ws, X, c->d_adjA[0],
+                   c->d_adjA[1], c->d_adjA[2], c->smem_budget, s);
+}
+
+// The same by the LDL^T of every (window, pole), factors kept, in batches of whole windows.
+int adj_ldl_accumulate(lres_ctx* c, cudaStream_t s) {
     const bool mixed = c->precision == LRES_MIXED;
     const int P = c->npoles;
     const size_t el = mixed ? 8 : 16;
@@ -1800,33 +1840,11 @@ extern "C" int lres_adjoint(lres_ctx* c, double mu, double e_lo, double* dv, int
     const long long npmax = (c->nmax + nbk - 1) / nbk * nbk;
     const int mrows = c->have_trace ? c->mmaxT : c->mmax;
     const long long stride = ((npmax + mrows + 1) * npmax + 15) / 16 * 16;   // elements per item slot
-    const size_t item_bytes = (size_t)stride * el;
-    // items per batch: whole windows (all poles), as many as the free device memory admits
-    size_t freeb = 0, totalb = 0;
-    LRES_CUDA_TRY(cudaMemGetInfo(&freeb, &totalb));
-    size_t have = c->adjws_bytes + freeb;
-    const size_t reserve = (size_t)4 << 30;
-    size_t budget = have > reserve ? std::min(have - reserve, have / 4 * 3) : 0;
-    long long win_per_batch = (long long)(budget / (item_bytes * P));
-    if (win_per_batch < 1) {
-        lres_set_error("adjoint: one window's %d pole factors (%zu bytes) do not fit in free device memory", P,
-                       item_bytes * P);
-        return LRES_ENOMEM;
-    }
-    win_per_batch = std::min<long long>(win_per_batch, c->nwin);
-    const size_t need = item_bytes * P * (size_t)win_per_batch;
-    if (c->adjws_bytes < need) {
-        if (c->d_adjws) cudaFree(c->d_adjws);
-        c->d_adjws = nullptr;
-        c->adjws_bytes = 0;
-        TRY(dalloc((char**)&c->d_adjws, need));
-        c->adjws_bytes = need;
-    }
+    const size_t window_bytes = (size_t)stride * el * P;
+    size_t got = 0;
+    TRY(adj_workspace(c, window_bytes, window_bytes * c->nwin, &got));
+    const long long win_per_batch = std::min<long long>(got / window_bytes, c->nwin);
     const Rows rw = select_rows(c, c->have_trace);
-    poles_kernel<<<(P + 63) / 64, 64, 0, s>>>(P, c->M, mu, e_lo, mixed ? 1 : 0, c->d_shifts, c->d_wq, c->d_wzq);
-    LRES_CUDA_TRY(cudaGetLastError());
-    TRY(adj_weights(P, c->M, mu, e_lo, c->d_cw, s));
-    LRES_CUDA_TRY(cudaMemsetAsync(c->d_status, 0, sizeof(int), s));
     for (long long w0 = 0; w0 < c->nwin; w0 += win_per_batch) {
         const int nwb = (int)std::min<long long>(win_per_batch, c->nwin - w0);
         const int2* items = c->d_items + w0 * P;       // windows in work-queue order, poles inner
@@ -1866,14 +1884,48 @@ extern "C" int lres_adjoint(lres_ctx* c, double mu, double e_lo, double* dv, int
     }
     TRY(pole_sums(c->nwin, rw.offQ, rw.m, rw.Oflat, mixed, rw.q, rw.npts, P, c->d_wq, c->d_wzq, c->dV, rw.dens,
                   c->d_nw, c->d_ew, s));
-    TRY(adj_inner(c->nwin, c->d_n, c->d_offC, mixed ? nullptr : c->d_SW, c->d_adjA[0], c->d_adjA[1], c->d_adjA[2],
+    return LRES_OK;
+}
+
+}  // namespace
+
+extern "C" int lres_adjoint(lres_ctx* c, double mu, double e_lo, double* dv, int dv_on_device, double* dHW,
+                            double* dSW, int dW_on_device, double* out, void* stream) {
+    if (!c || !out) {
+        lres_set_error("null argument");
+        return LRES_EINVAL;
+    }
+    if (!c->have_h) {
+        lres_set_error("lres_adjoint before a Hamiltonian was set");
+        return LRES_ESTATE;
+    }
+    if (!(mu > e_lo) || !std::isfinite(mu) || !std::isfinite(e_lo)) {
+        lres_set_error("need finite e_lo < mu (got mu=%g, e_lo=%g)", mu, e_lo);
+        return LRES_EINVAL;
+    }
+    cudaStream_t s = (cudaStream_t)stream;
+    const bool mixed = c->precision == LRES_MIXED;
+    const bool tri = !mixed && c->route == LRES_ROUTE_TRIDIAG;
+    const int P = c->npoles;
+    if (!tri) TRY(ensure_hhat_df(c, s));       // the LDL^T path factors the double-float standard form
+    TRY(adj_prepare(c, s));
+    poles_kernel<<<(P + 63) / 64, 64, 0, s>>>(P, c->M, mu, e_lo, mixed ? 1 : 0, c->d_shifts, c->d_wq, c->d_wzq);
+    LRES_CUDA_TRY(cudaGetLastError());
+    TRY(adj_weights(P, c->M, mu, e_lo, c->d_cw, s));
+    LRES_CUDA_TRY(cudaMemsetAsync(c->d_status, 0, sizeof(int), s));
+    // the accumulations are in the basis of Wt: A_c = Wt X_c Wt^T (null: the windows' own)
+    const double* const Wt = tri ? c->d_Hhat : mixed ? c->d_LinvT : nullptr;
+    if (tri) TRY(adj_tri_accumulate(c, s));
+    else TRY(adj_ldl_accumulate(c, s));
+    TRY(adj_inner(c->nwin, c->d_n, c->d_offC, Wt ? nullptr : c->d_SW, c->d_adjA[0], c->d_adjA[1], c->d_adjA[2],
                   c->d_adju, s));
     LRES_CUDA_TRY(cudaMemcpyAsync(c->nw_h.data(), c->d_nw, sizeof(double) * c->nwin, cudaMemcpyDeviceToHost, s));
     LRES_CUDA_TRY(cudaMemcpyAsync(c->ew_h.data(), c->d_ew, sizeof(double) * c->nwin, cudaMemcpyDeviceToHost, s));
     LRES_CUDA_TRY(cudaMemcpyAsync(c->adju_h.data(), c->d_adju, sizeof(double) * 3 * c->nwin,
                                   cudaMemcpyDeviceToHost, s));
     int st = 0;
-    TRY(read_status(c, s, &st));
+    if (tri) TRY(read_pass_status(c, s, &st));
+    else TRY(read_status(c, s, &st));
     if (st) {
         lres_set_error(st & ST_ZERO_PIVOT ? "zero or non-finite pivot in a window factorisation (adjoint)"
                                           : "window kernel status %d (adjoint)", st);
@@ -1898,15 +1950,15 @@ extern "C" int lres_adjoint(lres_ctx* c, double mu, double e_lo, double* dv, int
     }
     const double kappa = dEdmu / dNdmu;
     const double sc = 4.0 * c->dV;
-    if (mixed) {
-        // B_H = 4dV (A1 - kappa A0) into A0, B_S = -4dV (A2 - kappa A1) into A2, then L^-T B L^-1
+    if (Wt) {
+        // B_H = 4dV (X1 - kappa X0) into X0, B_S = -4dV (X2 - kappa X1) into X2, then Wt B Wt^T
         TRY(adj_combine(c->sizeC, c->d_adjA[0], c->d_adjA[1], c->d_adjA[2], kappa, sc, -sc, c->d_adjA[0],
                         c->d_adjA[2], s));
         for (int which = 0; which < 2; ++which) {
             const double* B = which ? c->d_adjA[2] : c->d_adjA[0];
             double* D = which ? c->d_dSW : c->d_dHW;
-            TRY(batched_gemm(c->nwin, c->d_n, c->d_offC, c->nmax, false, c->d_LinvT, B, c->d_adjA[1], s));
-            TRY(batched_gemm(c->nwin, c->d_n, c->d_offC, c->nmax, false, c->d_adjA[1], c->d_LinvT, D, s, 0, true));
+            TRY(batched_gemm(c->nwin, c->d_n, c->d_offC, c->nmax, false, Wt, B, c->d_adjA[1], s));
+            TRY(batched_gemm(c->nwin, c->d_n, c->d_offC, c->nmax, false, c->d_adjA[1], Wt, D, s, 0, true));
         }
     } else {
         TRY(adj_combine(c->sizeC, c->d_adjA[0], c->d_adjA[1], c->d_adjA[2], kappa, sc, -sc, c->d_dHW, c->d_dSW,

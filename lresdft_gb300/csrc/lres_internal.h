@@ -164,6 +164,13 @@ int adj_backsolve(bool fp32, const int2* items, int nitems, const int* n_w, cons
 int adj_accumulate(bool fp32, const int* wins, int nwin_batch, int P, int nmax, const int* n_w, const int* m_w,
                    const long long* offC, const void* ws, long long ws_stride, const double2* cw, double* A0,
                    double* A1, double* A2, cudaStream_t s);
+// A_c in the tridiagonal basis, X_c = Re sum_k c_k G_k K G_k, in batches of windows: coef nwin * P * nmax,
+// ws batch * groups * 2 nmax^2, X 3 * groups * sizeC elements (unused with one group)
+int adj_sweep_groups(int nwin, int P);
+int adj_tri(int nwin, int P, int groups, int batch, int nmax, const int* wins, const int* n_w, const long long* offN,
+            const long long* offC, long long sizeC, const double* d, const double* e, const double2* shifts,
+            const double2* cw, const double* K, double4* coef, double2* ws, double* X, double* A0, double* A1,
+            double* A2, size_t smem_budget, cudaStream_t s);
 int adj_weights(int P, int M, double mu, double e_lo, double2* cw, cudaStream_t s);
 int adj_inner(int nwin, const int* n_w, const long long* offC, const double* S, const double* A0, const double* A1,
               const double* A2, double* u, cudaStream_t s);
