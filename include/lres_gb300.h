@@ -63,8 +63,8 @@ enum { LRES_FP64 = 0, LRES_MIXED = 1 };
  *                       tridiagonal LDL^T of z I - T and one forward sweep per row (O(n)):
  *                       the mu trials of a density call cost O(P m n) each (tridiag.cu).
  * Both evaluate the same resolvent quadratic forms; the default is the tridiagonal route
- * unless the context has fewer than 4 windows or windows too large for its shared-memory
- * panels. */
+ * unless the windows are too large for its shared-memory panels or the context has fewer
+ * than 4 of them (in FP64: fewer than 4, and under 8 poles or over 512 functions). */
 enum { LRES_ROUTE_LDL = 0, LRES_ROUTE_TRIDIAG = 1 };
 
 typedef struct lres_ctx lres_ctx;

@@ -1102,7 +1102,11 @@ extern "C" int lres_ctx_create(lres_ctx** out, const lres_system_desc* d, int pr
         TriPick pk;
         const bool fits = tri_pick(precision == LRES_MIXED, c->nmax, c->smem_budget, 0, &pk) == LRES_OK;
         lres_set_error("");
-        c->route = (fits && c->nwin >= 4) ? LRES_ROUTE_TRIDIAG : LRES_ROUTE_LDL;
+        // a few FP64 windows: the dense factorisations of 8 or more poles cost more than one CTA's
+        // reduction (one window of 96 functions, 4096 points: a warm call 32 ms against 7.5 ms; its
+        // cost grows as n^3 on one SM, 15 ms at 512)
+        const bool few = precision == LRES_FP64 && c->npoles >= 8 && c->nmax <= 512;
+        c->route = (fits && (c->nwin >= 4 || few)) ? LRES_ROUTE_TRIDIAG : LRES_ROUTE_LDL;
     }
 
     // ---- standard form (mixed path; FP64 tridiagonal route)

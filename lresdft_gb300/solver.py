@@ -157,7 +157,7 @@ class LResGPU:
     "mixed" (complex64 factor/solve of the standard-form windows
     L^-1 (z S - H) L^-T, FP64 Cholesky/orthogonalisation, FP64 pole sums, electron
     count and energies); ``route`` "auto" (the library's choice: tridiagonal unless the
-    context has fewer than 4 windows or windows too large for it), "tridiag" or "ldl"
+    windows are too large for it or too few, see lres_set_route), "tridiag" or "ldl"
     (one dense LDL^T per window and pole)."""
 
     def __init__(self, basis, cells, R_w=12.1, M=64, margin=0.3, nthreads=1, lag_mu=False, reuse_vectors=True,
