@@ -121,6 +121,11 @@ int lres_set_hamiltonian_csr(lres_ctx* ctx, const int64_t* Hp, const int64_t* Hi
  * and returns LRES_ENUMERIC (bit 1) or LRES_EINVAL (bit 2) when out[2] != 0. */
 int lres_pass(lres_ctx* ctx, double mu, double e_lo, double* dens, int dens_on_device, double* out, void* stream);
 
+/* N(mu) and E_band as lres_pass's out (and lres_window_sums), without a density: on the tridiagonal
+ * route in FP64 as traces tr((z_k - T)^-1 Y^T Y) with Y^T Y formed once per Hamiltonian, the context's
+ * density array left as it was; otherwise the same as lres_pass with dens == NULL. */
+int lres_count(lres_ctx* ctx, double mu, double e_lo, double* out, void* stream);
+
 /* The pass of lres_pass without any host synchronisation or host memory: pole nodes and
  * weights are computed on the device, d_out[0..1] (device) receives N(mu) and E_band, the
  * density stays in the context (lres_density_ptr).  Enqueues kernels and memsets only, so

@@ -131,6 +131,11 @@ struct lres_ctx {
     };
     RowItems ri_own, ri_tr;
     RowItems ri_adj;                             // the rows of L^-T (adjoint)
+    // count passes (FP64): K = Y^T Y of the current Hamiltonian, formed by the first of them
+    double* d_K = nullptr;
+    double4* d_coef = nullptr;
+    double2* d_tr = nullptr;
+    bool k_ready = false;
     // pole work
     int2 *d_items = nullptr, *d_items_win = nullptr, *d_items_sub = nullptr;
     int nitems = 0;
@@ -187,7 +192,7 @@ lres_ctx::~lres_ctx() {
                     d_wq, d_wzq, d_q, d_dens, d_nw, d_ew, d_v, d_fftwork, d_adjA[0], d_adjA[1], d_adjA[2],
                     d_dHW, d_dSW, d_gH, d_adjdv, d_adju, d_cw, d_order, d_eoff, d_poff, d_ent, d_pent, d_adjws,
                     d_mT, d_offFT, d_offQT, d_FT, d_FhatT32, d_qT, d_Fhat64, d_FhatT64, d_offN, d_offA, d_order_w, d_LinvT32, d_Linv32,
-                    d_tstatus, d_triA, d_trid, d_trie, d_tritau, d_Yown, d_Ytr, d_lam, d_triT};
+                    d_tstatus, d_K, d_coef, d_tr, d_triA, d_trid, d_trie, d_tritau, d_Yown, d_Ytr, d_lam, d_triT};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     ri_own.release();
@@ -628,6 +633,7 @@ int tri_prepare(lres_ctx* c, cudaStream_t s) {
     if (c->have_trace) TRY(tri_rows(c, true, s));
     TRY(mark(c, 7, 1, s));
     c->tri_ready = true;
+    c->k_ready = false;
     return LRES_OK;
 }
 
@@ -652,6 +658,34 @@ int tri_run_pass(lres_ctx* c, bool trace, cudaStream_t s) {
     TRY(mark(c, 1, 0, s));
     TRY(tri_window_sums(c->nwin, ri.first, ri.count, ri.part, c->dV, c->d_nw, c->d_ew, s));
     TRY(mark(c, 1, 1, s));
+    return LRES_OK;
+}
+
+// Trials of the chemical potential need no rows when K = Y^T Y is there (FP64).
+bool counts_from_k(const lres_ctx* c) { return c->route == LRES_ROUTE_TRIDIAG && c->precision == LRES_FP64; }
+
+// K of the current Hamiltonian, from the trace rows where there are any.
+int ensure_k(lres_ctx* c, cudaStream_t s) {
+    if (c->k_ready) return LRES_OK;
+    if (!c->d_K) TRY(dalloc(&c->d_K, c->sizeC));
+    const bool tr = c->have_trace;
+    TRY(batched_gram(c->nwin, c->d_n, tr ? c->d_mT : c->d_m, tr ? c->d_offFT : c->d_offF, c->d_offC, c->nmax,
+                     static_cast<const double*>(tr ? c->d_Ytr : c->d_Yown), c->d_K, s));
+    c->k_ready = true;
+    return LRES_OK;
+}
+
+// Per-window N and E_band at the nodes already set, into d_nw / d_ew; the density is left as it is.
+int tri_run_count(lres_ctx* c, cudaStream_t s) {
+    const int P = c->npoles;
+    if (!c->d_coef) TRY(dalloc(&c->d_coef, (size_t)c->nwin * P * c->nmax));
+    if (!c->d_tr) TRY(dalloc(&c->d_tr, (size_t)c->nwin * P));
+    TRY(ensure_k(c, s));
+    TRY(mark(c, 0, 0, s));
+    TRY(tri_count(c->nwin, P, c->nmax, c->d_n, c->d_offN, c->d_offC, static_cast<const double*>(c->d_trid),
+                  static_cast<const double*>(c->d_trie), c->d_K, static_cast<const double2*>(c->d_shifts), c->d_wq,
+                  c->d_wzq, c->dV, c->d_coef, c->d_tr, c->d_nw, c->d_ew, c->d_status, c->smem_budget, s));
+    TRY(mark(c, 0, 1, s));
     return LRES_OK;
 }
 
@@ -1181,8 +1215,8 @@ extern "C" int lres_set_hamiltonian_csr(lres_ctx* c, const int64_t* Hp, const in
     return LRES_OK;
 }
 
-extern "C" int lres_pass(lres_ctx* c, double mu, double e_lo, double* dens, int dens_on_device, double* out,
-                         void* stream) {
+static int run_pass(lres_ctx* c, double mu, double e_lo, double* dens, int dens_on_device, bool count, double* out,
+                    void* stream) {
     if (!c || !out) {
         lres_set_error("null argument");
         return LRES_EINVAL;
@@ -1207,7 +1241,8 @@ extern "C" int lres_pass(lres_ctx* c, double mu, double e_lo, double* dens, int 
     const bool trace = !dens && c->have_trace;
     if (c->route == LRES_ROUTE_TRIDIAG) {
         if (!c->tri_ready) TRY(tri_refresh(c, s));
-        TRY(tri_run_pass(c, trace, s));
+        if ((count || trace) && counts_from_k(c)) TRY(tri_run_count(c, s));
+        else TRY(tri_run_pass(c, trace, s));
     } else {
         const Rows rw = select_rows(c, trace);
         TRY(ensure_hhat_df(c, s));
@@ -1248,6 +1283,15 @@ extern "C" int lres_pass(lres_ctx* c, double mu, double e_lo, double* dens, int 
         return LRES_EINVAL;
     }
     return LRES_OK;
+}
+
+extern "C" int lres_pass(lres_ctx* c, double mu, double e_lo, double* dens, int dens_on_device, double* out,
+                         void* stream) {
+    return run_pass(c, mu, e_lo, dens, dens_on_device, false, out, stream);
+}
+
+extern "C" int lres_count(lres_ctx* c, double mu, double e_lo, double* out, void* stream) {
+    return run_pass(c, mu, e_lo, nullptr, 0, true, out, stream);
 }
 
 extern "C" int lres_autotune(lres_ctx* c, double mu, double e_lo, int32_t force_config, int32_t* chosen,
@@ -1823,15 +1867,13 @@ int adj_tri_accumulate(lres_ctx* c, cudaStream_t s) {
     double* const X = reinterpret_cast<double*>(base + coefb);
     double2* const ws = reinterpret_cast<double2*>(base + coefb + xb);
     TRY(tri_run_pass(c, c->have_trace, s));
-    // K = Y^T Y (dE/dH_W's array is free until the end)
-    TRY(batched_gram(c->nwin, c->d_n, c->have_trace ? c->d_mT : c->d_m, c->have_trace ? c->d_offFT : c->d_offF,
-                     c->d_offC, c->nmax, static_cast<const double*>(c->have_trace ? c->d_Ytr : c->d_Yown), c->d_dHW, s));
+    TRY(ensure_k(c, s));
     if (c->ri_adj.arows != c->tri.arows) TRY(build_row_items(c, c->n_w, c->ri_adj, s));
     TRY(tri_apply(false, c->ri_adj.napply, c->ri_adj.apply, c->d_n, c->d_n, c->d_offA, c->d_offN, c->d_offC, c->d_triA,
                   c->d_tritau, c->d_LinvT, c->d_Hhat, c->tri, c->nwin, false, c->d_triT, c->smem_budget, s));
     return adj_tri(c->nwin, P, groups, batch, c->nmax, c->d_order, c->d_n, c->d_offN, c->d_offC, c->sizeC,
                    static_cast<const double*>(c->d_trid), static_cast<const double*>(c->d_trie),
-                   static_cast<const double2*>(c->d_shifts), c->d_cw, c->d_dHW, coef, ws, X, c->d_adjA[0],
+                   static_cast<const double2*>(c->d_shifts), c->d_cw, c->d_K, coef, ws, X, c->d_adjA[0],
                    c->d_adjA[1], c->d_adjA[2], c->smem_budget, s);
 }
 

@@ -151,6 +151,11 @@ int tri_pass(bool fp32, int nitems, const int4* items, int* counter, const int* 
              const void* Y, const void* d, const void* e, int P, const void* shifts, const double2* wq,
              const double2* wzq, double* dens, double* part, int* status, int ldv, size_t smem_budget,
              cudaStream_t s);
+// N and E_band of every window from K = Y^T Y (FP64): coef nwin * P * nmax, trace nwin * P elements
+int tri_count(int nwin, int P, int nmax, const int* n_w, const long long* offN, const long long* offC, const double* d,
+              const double* e, const double* K, const double2* shifts, const double2* wq, const double2* wzq,
+              double dV, double4* coef, double2* trace, double* nw, double* ew, int* status, size_t smem_budget,
+              cudaStream_t s);
 int tri_window_sums(int nwin, const int* first, const int* count, const double* part, double dV, double* nw,
                     double* ew, cudaStream_t s);
 int tri_sturm(bool fp32, int nwin, const int* n_w, const long long* offN, const void* d, const void* e,

@@ -1244,6 +1244,141 @@ __global__ void __launch_bounds__(NT) tri_pass_kernel(TriPassParams<R> p) {
     }
 }
 
+// ---------------------------------------------------------------------------
+// electron count and band energy without rows (FP64): tr((z_k - T)^-1 K), K = Y^T Y
+// ---------------------------------------------------------------------------
+//
+// A trial of the chemical potential needs N and E_band only, and those depend on the rows through
+// K (n x n, formed once per Hamiltonian).  The upper triangle of G = (z - T)^-1 is
+// G_ij = G_jj t_{i+1} ... t_j (t_i = e_{i-1} / D_{i-1}), so
+//
+//     tr(G K) = sum_j G_jj (K_jj + 2 h_j),  h_j = sum_{i<j} K_ij t_{i+1} ... t_j   (Horner in i):
+//
+// 5 FP64 instructions per (pole, i < j), 2.5 n^2 against the 11 m n of the rows.  The FP64 pipe
+// bounds it: 54 windows of 276-300 functions (256 rows) 4.7 -> 1.0 ms per trial.
+
+// 1 / x: from the FP32 reciprocal by one third-order step (y (1 + e + e^2), e = 1 - x y), by the
+// division outside its range.
+__device__ __forceinline__ double recip_f64(double x) {
+    if (x > 1e-30 && x < 1e30) {
+        const double y = (double)(1.0f / (float)x);
+        const double e = fma(-x, y, 1.0);
+        return fma(y * e, 1.0 + e, y);
+    }
+    return 1.0 / x;
+}
+
+// Per (window, pole): coef[item * ld + i] = (t_i, G_ii), G_ii = 1 / D_i + t_{i+1}^2 G_{i+1,i+1}.  Two
+// serial chains of n steps, bound by their latency; the second reads what the first stored four
+// steps ahead.
+__global__ void tri_diag_kernel(int nwin, int P, const int* n_w, const long long* offN, const double* __restrict__ d,
+                                const double* __restrict__ e, const double2* z, int ld, double4* coef) {
+    const int it = blockIdx.x * blockDim.x + threadIdx.x;
+    if (it >= nwin * P) return;
+    const int w = it / P;
+    const double2 zk = z[it - w * P];
+    const int n = n_w[w];
+    const double *dw = d + offN[w], *ew = e + offN[w];
+    double4* out = coef + (size_t)it * ld;
+    double2 t = make_double2(0.0, 0.0), g = t;
+    double el = 0.0;                                                 // e_{i-1}
+#pragma unroll 4
+    for (int i = 0; i < n; ++i) {
+        t = make_double2(el * g.x, el * g.y);
+        const double2 D = make_double2(fma(-el, t.x, zk.x - dw[i]), fma(-el, t.y, zk.y));
+        const double inv = recip_f64(D.x * D.x + D.y * D.y);
+        g = make_double2(D.x * inv, -D.y * inv);
+        out[i] = make_double4(t.x, t.y, g.x, g.y);
+        el = ew[i];
+    }
+    double2 G = make_double2(0.0, 0.0);
+    double2 tn = make_double2(0.0, 0.0);                             // t_{i+1}
+    for (int i1 = n - 1; i1 >= 0; i1 -= 4) {
+        double4 c[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) c[u] = out[max(i1 - u, 0)];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (i1 - u < 0) break;
+            const double2 t2 = make_double2(tn.x * tn.x - tn.y * tn.y, 2.0 * tn.x * tn.y);
+            G = make_double2(fma(t2.x, G.x, fma(-t2.y, G.y, c[u].z)), fma(t2.x, G.y, fma(t2.y, G.x, c[u].w)));
+            tn = make_double2(c[u].x, c[u].y);
+            reinterpret_cast<double2*>(out + i1 - u)[1] = G;
+        }
+    }
+}
+
+constexpr int kCountNT = 320, kCountPoles = 4;
+
+// One CTA per (window, 4 poles), thread = column j; the lanes of a warp run over the same i, so that
+// K is read along its rows and t is one broadcast.
+__global__ void __launch_bounds__(kCountNT) tri_count_kernel(int P, int groups, const int* n_w, const long long* offC,
+                                                             const double* K, const double4* coef, int ld,
+                                                             double2* trace) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double2* const ts = reinterpret_cast<double2*>(smem_raw);       // [n][kCountPoles]
+    __shared__ double red[kCountNT / 32];
+    const int w = blockIdx.x / groups, k0 = (blockIdx.x % groups) * kCountPoles;
+    const int n = n_w[w], tid = threadIdx.x;
+    const double* const Kw = K + offC[w];
+    const double4* const cf = coef + ((size_t)w * P + k0) * ld;
+    const int np = min(kCountPoles, P - k0);
+    for (int idx = tid; idx < n * kCountPoles; idx += kCountNT) {
+        const int q = idx / n, i = idx - q * n;
+        const double4 c = q < np ? cf[(size_t)q * ld + i] : make_double4(0.0, 0.0, 0.0, 0.0);
+        ts[i * kCountPoles + q] = make_double2(c.x, c.y);
+    }
+    __syncthreads();
+    double2 acc[kCountPoles];
+#pragma unroll
+    for (int q = 0; q < kCountPoles; ++q) acc[q] = make_double2(0.0, 0.0);
+    for (int j = tid; j < n; j += kCountNT) {
+        double2 h[kCountPoles];
+#pragma unroll
+        for (int q = 0; q < kCountPoles; ++q) h[q] = make_double2(0.0, 0.0);
+#pragma unroll 4
+        for (int i = 0; i < j; ++i) {
+            const double x = Kw[j + (long long)i * n];
+#pragma unroll
+            for (int q = 0; q < kCountPoles; ++q) {
+                const double2 t = ts[(i + 1) * kCountPoles + q];
+                const double u = h[q].x + x;
+                h[q] = make_double2(fma(t.x, u, -t.y * h[q].y), fma(t.y, u, t.x * h[q].y));
+            }
+        }
+        const double kjj = Kw[j + (long long)j * n];
+#pragma unroll
+        for (int q = 0; q < kCountPoles; ++q) {
+            if (q >= np) break;
+            const double4 c = cf[(size_t)q * ld + j];
+            const double u = fma(2.0, h[q].x, kjj), v = 2.0 * h[q].y;
+            acc[q].x += c.z * u - c.w * v;
+            acc[q].y += c.z * v + c.w * u;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < kCountPoles; ++q) {
+        const double x = block_sum<kCountNT>(acc[q].x, red), y = block_sum<kCountNT>(acc[q].y, red);
+        if (tid == 0 && q < np) trace[(size_t)w * P + k0 + q] = make_double2(x, y);
+    }
+}
+
+// per-window N and E_band from the traces, poles in order
+__global__ void tri_count_sums_kernel(int nwin, int P, const double2* trace, const double2* wq, const double2* wzq,
+                                      double dV, double* nw, double* ew, int* status) {
+    const int w = blockIdx.x * blockDim.x + threadIdx.x;
+    if (w >= nwin) return;
+    double sn = 0.0, se = 0.0;
+    for (int k = 0; k < P; ++k) {
+        const double2 x = trace[(size_t)w * P + k], a = wq[k], b = wzq[k];
+        sn += a.x * x.x - a.y * x.y;
+        se += b.x * x.x - b.y * x.y;
+    }
+    if (!isfinite(sn) || !isfinite(se)) atomicOr(status, ST_ZERO_PIVOT);
+    nw[w] = 4.0 * sn * dV;
+    ew[w] = 4.0 * se * dV;
+}
+
 // per-window totals from the items of each window (contiguous, fixed order)
 __global__ void tri_window_sums_kernel(int nwin, const int* first, const int* count, const double* part, double dV,
                                        double* nw, double* ew) {
@@ -1529,6 +1664,29 @@ int tri_pass(bool fp32, int nitems, const int4* items, int* counter, const int* 
                             (const double*)d, (const double*)e, P, (const double2*)shifts, wq, wzq, dens, part,
                             status, ldv};
     return launch_pass<double, 4>(p, smem_budget, s);
+}
+
+int tri_count(int nwin, int P, int nmax, const int* n_w, const long long* offN, const long long* offC, const double* d,
+              const double* e, const double* K, const double2* shifts, const double2* wq, const double2* wzq,
+              double dV, double4* coef, double2* trace, double* nw, double* ew, int* status, size_t smem_budget,
+              cudaStream_t s) {
+    if (!nwin) return LRES_OK;
+    const size_t smem = sizeof(double2) * kCountPoles * (size_t)nmax;
+    if (smem > smem_budget) {
+        lres_set_error("count pass needs %zu B of shared memory", smem);
+        return LRES_EINVAL;
+    }
+    tri_diag_kernel<<<(unsigned)(((long long)nwin * P + 31) / 32), 32, 0, s>>>(nwin, P, n_w, offN, d, e, shifts, nmax,
+                                                                              coef);
+    LRES_CUDA_TRY(cudaGetLastError());
+    int per_sm = 0;
+    if (int rc = prepare_kernel<tri_count_kernel>(kCountNT, smem, &per_sm)) return rc;
+    const int groups = (P + kCountPoles - 1) / kCountPoles;
+    tri_count_kernel<<<(unsigned)nwin * groups, kCountNT, smem, s>>>(P, groups, n_w, offC, K, coef, nmax, trace);
+    LRES_CUDA_TRY(cudaGetLastError());
+    tri_count_sums_kernel<<<(nwin + 63) / 64, 64, 0, s>>>(nwin, P, trace, wq, wzq, dV, nw, ew, status);
+    LRES_CUDA_TRY(cudaGetLastError());
+    return LRES_OK;
 }
 
 int tri_window_sums(int nwin, const int* first, const int* count, const double* part, double dV, double* nw,

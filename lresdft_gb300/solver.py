@@ -160,6 +160,8 @@ class LResGPU:
     windows are too large for it or too few, see lres_set_route), "tridiag" or "ldl"
     (one dense LDL^T per window and pole)."""
 
+    _counts = False             # trial passes as counts without rows (FP64, tridiagonal route)
+
     def __init__(self, basis, cells, R_w=12.1, M=64, margin=0.3, nthreads=1, lag_mu=False, reuse_vectors=True,
                  precision="fp64", tile_config=None, trace_rows="auto", merge_windows="auto", route="auto"):
         if M % 2 or M < 2:
@@ -223,6 +225,7 @@ class LResGPU:
         self._keep = (X, S, T, cWflat, cWoff, cOflat, cOoff)   # referenced by the descriptor
         if route != "auto":
             self.set_route(route)
+        self._counts = precision == "fp64" and self.route == "tridiag"
         # tile configuration of the pole kernel: an index, or "auto" to time all of them on
         # the first Hamiltonian (see autotune); None keeps the library default
         self.tile_config = tile_config
@@ -280,6 +283,7 @@ class LResGPU:
         """Switch the route of the pole solves ("tridiag" or "ldl")."""
         code = {"tridiag": _lib.LRES_ROUTE_TRIDIAG, "ldl": _lib.LRES_ROUTE_LDL}[route]
         _lib.check(_lib.lib.lres_set_route(self._ctx, code, None))
+        self._counts = self.precision == "fp64" and route == "tridiag"
 
     def set_potential(self, v):
         """H(v) for all windows: assembled on the GPU from v (a host array or a CUDA tensor of
@@ -464,7 +468,10 @@ class LResGPU:
         """One pole pass: returns (density or None, N(mu), E_band); the density is a host
         array, or a CUDA tensor while a density_device call runs."""
         self.passes += 1
-        if want_density and self._device_out:
+        if not want_density and self._counts:
+            dens = None
+            _lib.check(_lib.lib.lres_count(self._ctx, float(mu), float(e_lo), _lib.ptrd(self._out), None))
+        elif want_density and self._device_out:
             import torch
             dens = torch.empty(self.b.cr.ng, dtype=torch.float64, device="cuda")
             torch.cuda.synchronize()               # the device copy below runs on the legacy stream
@@ -541,7 +548,7 @@ class LResGPU:
         hist = []
 
         def f(x):
-            dens, n, eb = self.pole_pass(x, e_lo, want_density=not self._trace)
+            dens, n, eb = self.pole_pass(x, e_lo, want_density=not (self._trace or self._counts))
             cache[x] = (dens, eb)
             hist.append((x, n - N))
             return n - N
@@ -720,7 +727,7 @@ class LResGPU:
         if self._mu_last is not None and self._mu_last > lo:
             # the root of the (monotone) count is unique: start from the previous mu
             try:
-                dens, n, eb = self.pole_pass(self._mu_last, e_lo, want_density=not self._trace)
+                dens, n, eb = self.pole_pass(self._mu_last, e_lo, want_density=not (self._trace or self._counts))
                 mu, dens, eb = self._solve_mu(e_lo, N, ftol, start=(self._mu_last, n - N, dens, eb))
                 found = True
             except StaleMu:
