@@ -410,7 +410,7 @@ def run_ours(args):
     kernel_names = {"pole_kernel": "tri_pass_kernel" if route == "tridiag" else "ldl_left_kernel",
                     "transform": ("gemm_tc_kernel" if args.standard_form == "tensor" else "gemm_f32blk_kernel")
                     if (route == "tridiag" and mixed)
-                    else ("gemm_f64_kernel" if args.precision == "fp64" else "gemm_df64_kernel"),
+                    else ("oz_gemm_kernel" if args.precision == "fp64" else "gemm_df64_kernel"),
                     "tri_reduce": "tri_reduce_reg_kernel" if (mixed and cfg in (0, 4)) else "tri_reduce_kernel",
                     "tri_rows": "tri_apply_res_kernel" if (mixed and cfg != 2) else "tri_apply_kernel",
                     "assemble_h": "assemble_h32_kernel" if mixed else "assemble_h_kernel",

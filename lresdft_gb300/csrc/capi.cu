@@ -136,6 +136,7 @@ struct lres_ctx {
     double4* d_coef = nullptr;
     double2* d_tr = nullptr;
     bool k_ready = false;
+    OzWork oz;                                   // digits of the FP64 products on the tensor cores
     // pole work
     int2 *d_items = nullptr, *d_items_win = nullptr, *d_items_sub = nullptr;
     int nitems = 0;
@@ -198,6 +199,7 @@ lres_ctx::~lres_ctx() {
     ri_own.release();
     ri_tr.release();
     ri_adj.release();
+    oz.release();
     if (fft) fft3_destroy(fft);
     for (cudaEvent_t e : ev)
         if (e) cudaEventDestroy(e);
@@ -371,6 +373,12 @@ int transform_f32(lres_ctx* c, cudaStream_t s) {
     return LRES_OK;
 }
 
+// FP64 product of window matrices (n x n, column-major): C = op(A) op(B), (at) A^T B, (not bk) A B^T.
+int square_gemm(lres_ctx* c, const double* A, bool at, const double* B, bool bk, double* C, int klim, cudaStream_t s) {
+    return oz_gemm(c->oz, c->nwin, c->nmax, c->nmax, c->nmax, c->d_n, c->d_n, c->d_n, A, c->d_offC, at, B, c->d_offC, bk,
+                   C, c->d_offC, klim, c->smem_budget, s);
+}
+
 // FP64 (the FP64 tridiagonal route); the product H LinvT lives in the working blocks of the
 // reduction (at least sizeC elements), which the reduction overwrites afterwards.
 int transform_fp64(lres_ctx* c, cudaStream_t s) {
@@ -379,8 +387,8 @@ int transform_fp64(lres_ctx* c, cudaStream_t s) {
         lres_set_error("FP64 standard form without the tridiagonal buffers");
         return LRES_ESTATE;
     }
-    TRY(batched_gemm(c->nwin, c->d_n, c->d_offC, c->nmax, false, c->d_HW, c->d_LinvT, Y, s, 1));
-    TRY(batched_gemm(c->nwin, c->d_n, c->d_offC, c->nmax, true, c->d_LinvT, Y, c->d_Hhat, s, 2));
+    TRY(square_gemm(c, c->d_HW, false, c->d_LinvT, true, Y, 1, s));
+    TRY(square_gemm(c, c->d_LinvT, true, Y, true, c->d_Hhat, 2, s));
     return LRES_OK;
 }
 
@@ -2003,8 +2011,8 @@ extern "C" int lres_adjoint(lres_ctx* c, double mu, double e_lo, double* dv, int
         for (int which = 0; which < 2; ++which) {
             const double* B = which ? c->d_adjA[2] : c->d_adjA[0];
             double* D = which ? c->d_dSW : c->d_dHW;
-            TRY(batched_gemm(c->nwin, c->d_n, c->d_offC, c->nmax, false, Wt, B, c->d_adjA[1], s));
-            TRY(batched_gemm(c->nwin, c->d_n, c->d_offC, c->nmax, false, c->d_adjA[1], Wt, D, s, 0, true));
+            TRY(square_gemm(c, Wt, false, B, true, c->d_adjA[1], 0, s));
+            TRY(square_gemm(c, c->d_adjA[1], false, Wt, false, D, 0, s));
         }
     } else {
         TRY(adj_combine(c->sizeC, c->d_adjA[0], c->d_adjA[1], c->d_adjA[2], kappa, sc, -sc, c->d_dHW, c->d_dSW,

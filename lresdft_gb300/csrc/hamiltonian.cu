@@ -1,6 +1,6 @@
 // Atom-pair assembly of H(v) = T + X^T diag(v) X dV, gathers of the dense window
-// blocks, the owned-point basis blocks F_W, a batched FP64 GEMM for the standard-form
-// transform, and the pole-weighted reductions to density / electron count / band
+// blocks, the owned-point basis blocks F_W, batched FP64 products of the set-up and the FP32 and
+// double-float GEMMs of the standard form, and the pole-weighted reductions to density / electron count / band
 // energy.  All bandwidth-bound except the GEMM.
 //
 // H(v) (lrft/lcao3d.py:98-100): functions of one atom share one support, so
@@ -430,65 +430,8 @@ int build_F(int nwin, const long long* Xp, const int* Xi, const double* Xv, cons
 }
 
 // ---------------------------------------------------------------------------
-// batched FP64 GEMM  C_w = op(A_w) B_w  (n_w x n_w, column-major, same offsets)
+// batched FP64 products of the set-up (those of every Hamiltonian: oz_gemm.cu)
 // ---------------------------------------------------------------------------
-
-// KLIM = 0: full product.  KLIM = 1: B upper triangular (k <= column).  KLIM = 2: op(A)
-// lower triangular (k <= row) and only the lower triangle of C is needed.  TB: C = op(A) B^T.
-template <bool TA, int KLIM, bool TB = false>
-__global__ void __launch_bounds__(256) gemm_f64_kernel(const int* n_w, const long long* off, const double* A,
-                                                       const double* B, double* C) {
-    constexpr int BM = 64, BN = 64, BK = 16;
-    const int w = blockIdx.z;
-    const int n = n_w[w];
-    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
-    if (m0 >= n || n0 >= n) return;
-    if (KLIM == 2 && m0 + BM - 1 < n0) return;
-    const int kend = KLIM == 1 ? min(n, n0 + BN) : KLIM == 2 ? min(n, m0 + BM) : n;
-    const double* Aw = A + off[w];
-    const double* Bw = B + off[w];
-    double* Cw = C + off[w];
-    __shared__ double As[BK][BM + 1];
-    __shared__ double Bs[BK][BN + 1];
-    const int tid = threadIdx.x;
-    const int tx = tid % 16, ty = tid / 16;   // 16 x 16 threads, 4 x 4 outputs each
-    double acc[4][4] = {};
-    for (int k0 = 0; k0 < kend; k0 += BK) {
-        for (int idx = tid; idx < BK * BM; idx += 256) {
-            const int kk = idx / BM, i = idx % BM;
-            const int gi = m0 + i, gk = k0 + kk;
-            double a = 0.0;
-            if (gi < n && gk < n) a = TA ? Aw[gk + (long long)gi * n] : Aw[gi + (long long)gk * n];
-            As[kk][i] = a;
-        }
-        for (int idx = tid; idx < BK * BN; idx += 256) {
-            const int j = TB ? idx % BN : idx / BK, kk = TB ? idx / BN : idx % BK;
-            const int gj = n0 + j, gk = k0 + kk;
-            Bs[kk][j] = (gj < n && gk < n) ? (TB ? Bw[gj + (long long)gk * n] : Bw[gk + (long long)gj * n]) : 0.0;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
-            double a[4], b[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) a[u] = As[kk][tx + 16 * u];
-#pragma unroll
-            for (int v = 0; v < 4; ++v) b[v] = Bs[kk][ty + 16 * v];
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int v = 0; v < 4; ++v) acc[u][v] = fma(a[u], b[v], acc[u][v]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            const int gi = m0 + tx + 16 * u, gj = n0 + ty + 16 * v;
-            if (gi < n && gj < n) Cw[gi + (long long)gj * n] = acc[u][v];
-        }
-}
 
 // C_w = A_w U_w with A_w m_w x n_w (column-major, leading dimension m_w, offsets offA) and
 // U_w n_w x n_w upper triangular (column-major, offsets offU): the owned-point rows in the
@@ -613,27 +556,6 @@ int batched_gemm_rect_upper(int nwin, const int* n_w, const int* m_w, const long
     return LRES_OK;
 }
 
-int batched_gemm(int nwin, const int* n_w, const long long* offA, int nmax, bool transA, const double* A,
-                 const double* B, double* C, cudaStream_t s, int klim, bool transB) {
-    if (!nwin) return LRES_OK;
-    dim3 grid((nmax + 63) / 64, (nmax + 63) / 64, nwin);
-    if (transB) {
-        if (transA || klim) {
-            lres_set_error("unsupported FP64 GEMM variant");
-            return LRES_EINVAL;
-        }
-        gemm_f64_kernel<false, 0, true><<<grid, 256, 0, s>>>(n_w, offA, A, B, C);
-    } else if (transA) {
-        if (klim == 2) gemm_f64_kernel<true, 2><<<grid, 256, 0, s>>>(n_w, offA, A, B, C);
-        else gemm_f64_kernel<true, 0><<<grid, 256, 0, s>>>(n_w, offA, A, B, C);
-    } else {
-        if (klim == 1) gemm_f64_kernel<false, 1><<<grid, 256, 0, s>>>(n_w, offA, A, B, C);
-        else gemm_f64_kernel<false, 0><<<grid, 256, 0, s>>>(n_w, offA, A, B, C);
-    }
-    LRES_CUDA_TRY(cudaGetLastError());
-    return LRES_OK;
-}
-
 __global__ void convert_kernel(const double* a, float* b, long long n) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         b[i] = (float)a[i];
@@ -746,7 +668,8 @@ __device__ __forceinline__ void df_mac(float2 a, float2 b, float& sh, float& sl)
     sh = t;
 }
 
-// KLIM as gemm_f64_kernel.  OUT32: write fl32(hi + lo) to a float array, else (hi, lo).
+// KLIM = 1: B upper triangular (k <= column).  KLIM = 2: op(A) lower triangular (k <= row) and only the
+// lower triangle of C is needed.  OUT32: write fl32(hi + lo) to a float array, else (hi, lo).
 template <bool TA, int KLIM, bool OUT32>
 __global__ void __launch_bounds__(256) gemm_df64_kernel(const int* n_w, const long long* off, const float2* A,
                                                         const float2* B, float2* C, float* C32) {
@@ -814,7 +737,7 @@ __global__ void __launch_bounds__(256) gemm_df64_kernel(const int* n_w, const lo
 // ---------------------------------------------------------------------------
 // batched FP32 GEMM with blocked sums  C_w = A_w B_w  (n_w x n_w, offsets off)
 // ---------------------------------------------------------------------------
-// KLIM as gemm_f64_kernel (1: B upper triangular, k <= column; 2: A lower triangular, k <= row,
+// KLIM as gemm_df64_kernel (1: B upper triangular, k <= column; 2: A lower triangular, k <= row,
 // lower triangle of C only).  A is column-major, FP64 (converted on load) or FP32; B is given
 // k-major (Bt[j + k n] = B[k][j], i.e. B stored row-major), so that both operand tiles are
 // staged with coalesced loads and conflict-free stores and read as 16-byte vectors; C is

@@ -96,8 +96,18 @@ int gather_windows(int nwin, int nmax, const int* fn, const long long* fnoff, co
 int build_F(int nwin, const long long* Xp, const int* Xi, const double* Xv, const int* group_of_fn,
             const int* gptr, const int* gloc, int ngroups, const long long* Ooff, const long long* Oflat,
             const long long* offF, const int* m_w, int mmax, double* F, cudaStream_t s);
-int batched_gemm(int nwin, const int* n_w, const long long* offA, int nmax, bool transA, const double* A,
-                 const double* B, double* C, cudaStream_t s, int klim = 0, bool transB = false);
+// FP64 products on the tensor cores (oz_gemm.cu): C_w = op(A_w) op(B_w), C_w m_w x n_w column-major at
+// offC, K = k_w terms.  op(A)(i, k) at A[i + k m] or (a_kcontig) A[k + i K]; op(B)(k, j) at B[j + k n] or
+// (b_kcontig) B[k + j K]; klim 1: op(B) upper triangular, 2: op(A) lower triangular and the lower triangle
+// of C only.  The workspace grows on demand.
+struct OzWork {
+    void* buf = nullptr;
+    size_t bytes = 0;
+    void release();
+};
+int oz_gemm(OzWork& wk, int nwin, int mmax, int nmax, int kmax, const int* m_w, const int* n_w, const int* k_w,
+            const double* A, const long long* offA, bool a_kcontig, const double* B, const long long* offB,
+            bool b_kcontig, double* C, const long long* offC, int klim, size_t smem_budget, cudaStream_t s);
 int batched_gram(int nwin, const int* n_w, const int* m_w, const long long* offF, const long long* offK, int nmax,
                  const double* F, double* K, cudaStream_t s);
 int batched_gemm_rect_upper(int nwin, const int* n_w, const int* m_w, const long long* offA, const long long* offU,
@@ -107,7 +117,7 @@ int split_f64(const double* a, float2* b, long long n, cudaStream_t s);
 int batched_gemm_df64(int nwin, const int* n_w, const long long* off, int nmax, bool transA, int klim,
                       const float2* A, const float2* B, float2* C, float* C32, cudaStream_t s);
 // C = A B for every window block: A column-major (FP64 or FP32), B k-major (Bt[j + k n] =
-// B[k][j]), C column-major or row-major (c_rowmajor); klim as batched_gemm.
+// B[k][j]), C column-major or row-major (c_rowmajor); klim as oz_gemm.
 int batched_gemm_f32(int nwin, const int* n_w, const long long* off, int nmax, int klim, const void* A, bool a_f64,
                      const float* Bt, float* C, bool c_rowmajor, cudaStream_t s);
 // batched_gemm_f32's products on the tensor cores (tcgen05, 3xTF32, 32-term chunks); a timed-out

@@ -1,0 +1,362 @@
+// Batched FP64 matrix products on the tensor cores (sm_103a): C_w = op(A_w) op(B_w).
+//
+// GB300 issues 1.6 FP64 multiply-adds per clock and SM, its bf16 tensor cores ~1000 (mma.sync).  Every
+// operand row (column of B) is scaled by a power of two to 56-bit fixed point and cut into 8 signed
+// digits of 7 bits, exact in bf16 (the error-free splitting of Ozaki, Ogita, Oishi and Rump, Numer.
+// Algorithms 59 (2012) 95-118).  Products of digits sum exactly in the FP32 accumulators: 64 x 64 x
+// 8 pairs x 512 terms = 2^24 (longer sums are taken in runs of 512).  The 36 digit pairs s + t <= 7
+// are kept, summed by s + t in 8 accumulators, joined in 64-bit integers and rounded twice; what is
+// dropped is below 2^-55 of the row's and the column's largest value per term, so the error is that
+// of a fixed-point product with 55 bits: at least FP64's relative to the largest elements.
+//
+// Two kernels: oz_slice_kernel writes the digits of an operand ([digit][row][k], k contiguous), each
+// element once; oz_gemm_kernel, one CTA per 64 x 64 tile, stages 32 terms of all digits of both
+// operands by cp.async (three stages of 64 KB) and issues 36 m16n8k16 products per warp tile and 16
+// terms, 8 warps of 32 x 16.  The digit pairs bound it: 36 x 4096 flops per 2048 multiply-adds at
+// ~600 TFLOP/s is 26 FP64 multiply-adds per clock and SM.  The windows go in batches, so that the
+// digits take at most ~1 GB whatever the context's size.
+//
+// Measured (432 windows of 270-306 functions): the standard form's two products 23.5 -> 4.5 ms (54
+// windows 3.7 -> 0.67), density error against 64 bits unchanged (2e-14).
+#include "common.cuh"
+#include "launch.cuh"
+#include "lres_internal.h"
+
+#include <algorithm>
+
+namespace lres {
+namespace {
+
+constexpr int kDig = 8;                       // digits of an operand
+constexpr int kBits = 7;                      // bits of a digit
+constexpr int kOzT = 64;                      // tile edge
+constexpr int kOzK = 32;                      // terms of a stage
+constexpr int kOzStages = 3;
+constexpr int kOzNT = 256;
+constexpr int kOzRun = 512;                   // terms that sum exactly
+constexpr int kOzBad = 1 << 20;               // exponent of a row with a non-finite value
+constexpr int kStageBytes = 2 * kDig * kOzT * kOzK * 2;
+constexpr int kOzSmem = kOzStages * kStageBytes;
+
+// One operand of a batch: window w's matrix at X[off[w]], element (r, k) at r + k rows (k_contig = 0)
+// or k + r cols (k_contig = 1); rows, cols per window, or one array for both.
+struct Operand {
+    const double* X;
+    const long long* off;
+    const int* rows;
+    const int* cols;
+    int k_contig;
+};
+
+__device__ __forceinline__ int ilogb_bits(double x) {
+    const int e = (int)((__double_as_longlong(x) >> 52) & 0x7ff);
+    return e == 0 ? -1022 : e - 1023;
+}
+
+// Digits of 32 rows of one window: dig[((slot * kDig + s) * Rp + r) * Kp + k], ex[slot * Rp + r].
+__global__ void __launch_bounds__(256) oz_slice_kernel(int w0, Operand o, int Rp, int Kp, unsigned short* dig, int* ex) {
+    __shared__ double tile[32][33];
+    __shared__ int emax[32];
+    const int slot = blockIdx.y, w = w0 + slot, r0 = blockIdx.x * 32;
+    const int R = o.rows[w], K = o.cols[w];
+    if (r0 >= (R + kOzT - 1) / kOzT * kOzT) return;                 // (tiles beyond are never read)
+    const double* const X = o.X + o.off[w];
+    const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
+    if (tid < 32) emax[tid] = -1100;
+    __syncthreads();
+    // the largest exponent of every row
+    if (o.k_contig) {
+        for (int r = ty; r < 32; r += 8) {
+            int e = -1100;
+            if (r0 + r < R)
+                for (int k = tx; k < K; k += 32) {
+                    const double x = X[k + (long long)(r0 + r) * K];
+                    if (x != 0.0) e = max(e, ilogb_bits(x));
+                }
+            e = __reduce_max_sync(0xffffffffu, e);
+            if (tx == 0) emax[r] = e;
+        }
+    } else {
+        int e = -1100;
+        if (r0 + tx < R)
+            for (int k = ty; k < K; k += 8) {
+                const double x = X[r0 + tx + (long long)k * R];
+                if (x != 0.0) e = max(e, ilogb_bits(x));
+            }
+        atomicMax(&emax[tx], e);
+    }
+    __syncthreads();
+    if (tid < 32) ex[(size_t)slot * Rp + r0 + tid] = emax[tid] == 1024 ? kOzBad : emax[tid];
+    const int r = tid >> 3, kq = (tid & 7) * 4;                     // this thread: row r, 4 terms
+    const int E = emax[r];
+    for (int k0 = 0; k0 < Kp; k0 += 32) {
+        if (k0 >= (K + kOzK - 1) / kOzK * kOzK) break;
+        __syncthreads();
+        for (int q = ty; q < 32; q += 8) {
+            double x = 0.0;
+            if (o.k_contig) {
+                if (r0 + q < R && k0 + tx < K) x = X[k0 + tx + (long long)(r0 + q) * K];
+                tile[q][tx] = x;
+            } else {
+                if (r0 + tx < R && k0 + q < K) x = X[r0 + tx + (long long)(k0 + q) * R];
+                tile[tx][q] = x;
+            }
+        }
+        __syncthreads();
+        unsigned short d[kDig][4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const long long b = __double_as_longlong(tile[r][kq + u]);
+            const int ef = (int)((b >> 52) & 0x7ff);
+            long long m = b & 0xfffffffffffffLL;
+            if (ef) m |= 1LL << 52;
+            const int sh = (ef ? ef - 1023 : -1022) - E + 2;        // q = x 2^(54 - E)
+            long long q = 0;
+            if (m == 0) q = 0;
+            else if (sh >= 0) q = m << sh;                           // (sh <= 2)
+            else if (sh > -60) q = (m + (1LL << (-sh - 1))) >> -sh;
+            if (b < 0) q = -q;
+#pragma unroll
+            for (int s = kDig - 1; s >= 0; --s) {
+                const int t = s ? (int)((q + 64) & 127) - 64 : (int)q;
+                q = (q - t) >> kBits;
+                d[s][u] = (unsigned short)(__float_as_uint((float)t) >> 16);    // exact: |t| <= 64
+            }
+        }
+#pragma unroll
+        for (int s = 0; s < kDig; ++s) {
+            const uint2 v = make_uint2((unsigned)d[s][0] | (unsigned)d[s][1] << 16,
+                                       (unsigned)d[s][2] | (unsigned)d[s][3] << 16);
+            *reinterpret_cast<uint2*>(dig + (((size_t)slot * kDig + s) * Rp + r0 + r) * Kp + k0 + kq) = v;
+        }
+    }
+}
+
+__device__ __forceinline__ void cp16(unsigned dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src));
+}
+__device__ __forceinline__ void ldm4(unsigned (&r)[4], unsigned addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr));
+}
+__device__ __forceinline__ void mma(float (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+                 "{%0,%1,%2,%3};\n"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// sum_d acc_d 2^(-7 d), in units of 2^21 (exact up to the last rounding)
+__device__ __forceinline__ double oz_join(const float (&a)[kDig]) {
+    long long hi = 0, lo = 0;
+#pragma unroll
+    for (int d = 0; d < 4; ++d) hi = (hi << kBits) + __float2int_rn(a[d]);
+#pragma unroll
+    for (int d = 4; d < 8; ++d) lo = (lo << kBits) + __float2int_rn(a[d]);
+    // |hi|, |lo| < 2^47: to double by the exponent of 1.5 2^52
+    const double magic = 6755399441055744.0;
+    const double h = __longlong_as_double(0x4338000000000000LL + hi) - magic;
+    const double l = __longlong_as_double(0x4338000000000000LL + lo) - magic;
+    return fma(l, 3.7252902984619140625e-09, h);                    // 2^-28
+}
+
+// KLIM: 1, B upper triangular (k <= column); 2, A lower triangular (k <= row) and the
+// lower triangle of C only.  LONG: sums of more than 512 terms.
+template <int KLIM, bool LONG>
+__global__ void __launch_bounds__(kOzNT, 1) oz_gemm_kernel(int w0, const int* m_w, const int* n_w, const int* k_w,
+                                                           int Rp, int Cp, int Kp, const unsigned short* da,
+                                                           const unsigned short* db, const int* ea, const int* eb,
+                                                           const long long* offC, double* C) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int slot = blockIdx.z, w = w0 + slot;
+    const int M = m_w[w], N = n_w[w], K = k_w[w];
+    const int m0 = blockIdx.x * kOzT, n0 = blockIdx.y * kOzT;
+    if (m0 >= M || n0 >= N) return;
+    if (KLIM == 2 && m0 + kOzT - 1 < n0) return;
+    const int kend = KLIM == 1 ? min(K, n0 + kOzT) : KLIM == 2 ? min(K, m0 + kOzT) : K;
+    const int nk = (kend + kOzK - 1) / kOzK;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned short* const A = da + ((size_t)slot * kDig * Rp + m0) * Kp;
+    const unsigned short* const B = db + ((size_t)slot * kDig * Cp + n0) * Kp;
+    const unsigned sbase = (unsigned)__cvta_generic_to_shared(smem);
+    // stage: [operand][digit][row][4 chunks of 16 bytes], chunk c of row r at c ^ (r >> 1 & 3)
+    auto load = [&](int kt, int buf) {
+        const unsigned dst = sbase + buf * kStageBytes;
+#pragma unroll
+        for (int q = 0; q < 2 * kDig * kOzT * 4 / kOzNT; ++q) {
+            const int idx = tid + q * kOzNT;
+            const int c = idx & 3, r = (idx >> 2) & (kOzT - 1), s = (idx >> 8) & (kDig - 1), op = idx >> 11;
+            const unsigned short* src = op ? B + ((size_t)s * Cp + r) * Kp : A + ((size_t)s * Rp + r) * Kp;
+            cp16(dst + (((op * kDig + s) * kOzT + r) * 4 + (c ^ (r >> 1 & 3))) * 16, src + kt * kOzK + c * 8);
+        }
+        asm volatile("cp.async.commit_group;\n" ::);
+    };
+    const int wm = (warp & 1) * 32, wn = (warp >> 1) * 16;
+    const int ar = (lane & 7) + ((lane >> 3) & 1) * 8, ac = lane >> 4;       // ldmatrix rows and chunks
+    const int br = (lane & 7) + (lane >> 4) * 8, bc = (lane >> 3) & 1;
+    float acc[kDig][2][2][4];
+    double sum[2][2][4];
+    auto clear = [&]() {
+#pragma unroll
+        for (int d = 0; d < kDig; ++d)
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) acc[d][i][j][e] = 0.0f;
+    };
+    auto flush = [&]() {
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    float a[kDig];
+#pragma unroll
+                    for (int d = 0; d < kDig; ++d) a[d] = acc[d][i][j][e];
+                    const double x = oz_join(a);
+                    if constexpr (LONG) sum[i][j][e] += x;
+                    else sum[i][j][e] = x;
+                }
+    };
+    if constexpr (LONG) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) sum[i][j][e] = 0.0;
+    }
+    clear();
+#pragma unroll
+    for (int q = 0; q < kOzStages - 1; ++q) {
+        if (q < nk) load(q, q);
+        else asm volatile("cp.async.commit_group;\n" ::);
+    }
+    for (int kt = 0; kt < nk; ++kt) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(kOzStages - 2) : "memory");
+        __syncthreads();                                            // stage kt here; stage kt - 1 consumed
+        if (kt + kOzStages - 1 < nk) load(kt + kOzStages - 1, (kt + kOzStages - 1) % kOzStages);
+        else asm volatile("cp.async.commit_group;\n" ::);
+        const unsigned st = sbase + (kt % kOzStages) * kStageBytes;
+#pragma unroll
+        for (int h = 0; h < kOzK / 16; ++h) {
+            unsigned bf[kDig][4];
+#pragma unroll
+            for (int t = 0; t < kDig; ++t) {
+                const int r = wn + br;
+                ldm4(bf[t], st + (((kDig + t) * kOzT + r) * 4 + ((2 * h + bc) ^ (r >> 1 & 3))) * 16);
+            }
+#pragma unroll
+            for (int s = 0; s < kDig; ++s) {
+                unsigned af[2][4];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const int r = wm + 16 * i + ar;
+                    ldm4(af[i], st + ((s * kOzT + r) * 4 + ((2 * h + ac) ^ (r >> 1 & 3))) * 16);
+                }
+#pragma unroll
+                for (int t = 0; t < kDig - s; ++t)
+#pragma unroll
+                    for (int i = 0; i < 2; ++i)
+#pragma unroll
+                        for (int j = 0; j < 2; ++j) mma(acc[s + t][i][j], af[i], bf[t][2 * j], bf[t][2 * j + 1]);
+            }
+        }
+        if constexpr (LONG) {
+            if ((kt + 1) % (kOzRun / kOzK) == 0 && kt + 1 < nk) {
+                flush();
+                clear();
+            }
+        }
+    }
+    flush();
+    double* const Cw = C + offC[w];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int gi = m0 + wm + 16 * i + (lane >> 2) + 8 * (e >> 1), gj = n0 + wn + 8 * j + 2 * (lane & 3) + (e & 1);
+                if (gi >= M || gj >= N) continue;
+                const int xa = ea[(size_t)slot * Rp + gi], xb = eb[(size_t)slot * Cp + gj];
+                const int p = xa + xb - 31;                          // hi is in units of 2^(Ea + Eb - 10 - 21)
+                double x = sum[i][j][e];
+                if (xa >= kOzBad || xb >= kOzBad) x = __longlong_as_double(0x7ff8000000000000LL);
+                else if (p > -960 && p < 960) x *= __longlong_as_double((long long)(p + 1023) << 52);
+                else x = ldexp(x, p);
+                Cw[gi + (long long)gj * M] = x;
+            }
+}
+
+}  // namespace
+
+void OzWork::release() {
+    if (buf) cudaFree(buf);
+    *this = OzWork{};
+}
+
+int oz_gemm(OzWork& wk, int nwin, int mmax, int nmax, int kmax, const int* m_w, const int* n_w, const int* k_w,
+            const double* A, const long long* offA, bool a_kcontig, const double* B, const long long* offB,
+            bool b_kcontig, double* C, const long long* offC, int klim, size_t smem_budget, cudaStream_t s) {
+    if (!nwin || !mmax || !nmax) return LRES_OK;
+    if ((size_t)kOzSmem > smem_budget) {
+        lres_set_error("tensor-core FP64 product needs %d B of shared memory", kOzSmem);
+        return LRES_EINVAL;
+    }
+    const int Rp = (mmax + kOzT - 1) / kOzT * kOzT, Cp = (nmax + kOzT - 1) / kOzT * kOzT;
+    const int Kp = (std::max(kmax, 1) + kOzK - 1) / kOzK * kOzK;
+    const size_t perw = sizeof(unsigned short) * kDig * (size_t)(Rp + Cp) * Kp + sizeof(int) * (size_t)(Rp + Cp);
+    // about 1 GB of digits at most (one window at least), kept with the context
+    const int batch = (int)std::min<size_t>({(size_t)nwin, std::max<size_t>(((size_t)1 << 30) / perw, 1), (size_t)65535});
+    if (wk.bytes < perw * batch) {
+        wk.release();
+        if (cudaMalloc(&wk.buf, perw * batch) != cudaSuccess) {
+            cudaGetLastError();
+            wk.buf = nullptr;
+            lres_set_error("tensor-core FP64 product: allocation of %zu bytes failed", perw * batch);
+            return LRES_ENOMEM;
+        }
+        wk.bytes = perw * batch;
+    }
+    unsigned short* const da = static_cast<unsigned short*>(wk.buf);
+    unsigned short* const db = da + (size_t)batch * kDig * Rp * Kp;
+    int* const ea = reinterpret_cast<int*>(db + (size_t)batch * kDig * Cp * Kp);
+    int* const eb = ea + (size_t)batch * Rp;
+    const bool lng = kmax > kOzRun;
+    int per_sm = 0;
+    auto launch = [&](auto kern, int w0, int nb) {
+        const dim3 grid((mmax + kOzT - 1) / kOzT, (nmax + kOzT - 1) / kOzT, nb);
+        kern<<<grid, kOzNT, kOzSmem, s>>>(w0, m_w, n_w, k_w, Rp, Cp, Kp, da, db, ea, eb, offC, C);
+    };
+    for (int w0 = 0; w0 < nwin; w0 += batch) {
+        const int nb = std::min(batch, nwin - w0);
+        oz_slice_kernel<<<dim3(Rp / 32, nb), 256, 0, s>>>(w0, Operand{A, offA, m_w, k_w, a_kcontig}, Rp, Kp, da, ea);
+        oz_slice_kernel<<<dim3(Cp / 32, nb), 256, 0, s>>>(w0, Operand{B, offB, n_w, k_w, b_kcontig}, Cp, Kp, db, eb);
+        LRES_CUDA_TRY(cudaGetLastError());
+#define OZ_RUN(KL, LG)                                                                  \
+    do {                                                                                \
+        if (int rc = prepare_kernel<oz_gemm_kernel<KL, LG>>(kOzNT, kOzSmem, &per_sm)) return rc; \
+        launch(oz_gemm_kernel<KL, LG>, w0, nb);                                         \
+    } while (0)
+        if (klim == 1) {
+            if (lng) OZ_RUN(1, true);
+            else OZ_RUN(1, false);
+        } else if (klim == 2) {
+            if (lng) OZ_RUN(2, true);
+            else OZ_RUN(2, false);
+        } else {
+            if (lng) OZ_RUN(0, true);
+            else OZ_RUN(0, false);
+        }
+#undef OZ_RUN
+        LRES_CUDA_TRY(cudaGetLastError());
+    }
+    return LRES_OK;
+}
+
+}  // namespace lres

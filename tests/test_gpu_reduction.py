@@ -59,3 +59,56 @@ def test_reduction_sizes(n, config):
     assert abs(N - cr.dV * want.sum()) <= (M * dA / (2 * R) + 1e-6) * 2 * cr.dV * Y2.sum()
     assert abs(E - 2 * cr.dV * np.sum(Y2 @ (r * lam))) <= (M * dA / R + 1e-6) * 2 * cr.dV * Y2.sum() * (np.abs(lam).max() + 1)
     s.close()
+
+
+@pytest.mark.parametrize("n", [1, 2, 5, 31, 33, 63, 64, 65, 130, 257, 300, 511, 513, 600])
+def test_fp64_sizes(n):
+    """The FP64 tridiagonal route (products on the tensor cores, reduction, rows, pass, count, adjoint)
+    on one window against numpy, around the edges of its 32- and 64-wide tiles and the 512-term runs.
+    S_W has condition ~4 and the spectrum is of order one, so every step is a backward-stable sum of
+    n terms: errors of a small multiple of n u ~ 1e-13 of the result; 1e-11 leaves a factor of 100."""
+    from lresdft_gb300 import LResGPU
+    cr, b = _system(n)
+    M = 32
+    s = LResGPU(b, cr.pos[:1], R_w=1e3, M=M, precision="fp64", route="tridiag", trace_rows=False)
+    rng = np.random.default_rng(n)
+    Q = np.linalg.qr(rng.normal(size=(n, n)))[0]
+    H = (Q * np.linspace(-1, 1, n)) @ Q.T + 0.1 * np.diag(rng.normal(size=n))
+    H = 0.5 * (H + H.T)
+    Q = np.linalg.qr(rng.normal(size=(n, n)))[0]
+    S = (Q * np.geomspace(0.5, 2.0, n)) @ Q.T
+    S = 0.5 * (S + S.T)
+    s.set_windows(HW=s.flatten_windows([H]), SW=s.flatten_windows([S]))
+    L = np.linalg.cholesky(S)
+    A = np.linalg.solve(L, np.linalg.solve(L, H).T)
+    lam, C = np.linalg.eigh(0.5 * (A + A.T))
+    e_lo, mu = lam[0] - 0.3, float(np.median(lam)) + 0.05
+    R = 0.5 * (mu - e_lo)
+    r = 1 / (1 + ((lam - 0.5 * (mu + e_lo)) / R) ** M)
+    F = np.zeros((cr.ng, n))
+    F[s.ctx_own[0]] = b.Xr[s.ctx_own[0]][:, s.ctx_windows[0]].toarray()
+    Y2 = (F @ np.linalg.solve(L.T, C)) ** 2
+    want, N0, E0 = 2 * Y2 @ r, 2 * cr.dV * float((Y2 @ r).sum()), 2 * cr.dV * float((Y2 @ (r * lam)).sum())
+    dens, N, E = s.pole_pass(mu, e_lo)
+    assert np.linalg.norm(dens - want) <= 1e-11 * np.linalg.norm(2 * Y2.sum(axis=1))
+    assert abs(N - N0) <= 1e-11 * abs(N0) + 1e-13 and abs(E - E0) <= 1e-11 * (abs(E0) + abs(N0))
+    _, N1, E1 = s.pole_pass(mu, e_lo, want_density=False)
+    assert abs(N1 - N0) <= 1e-11 * abs(N0) + 1e-13 and abs(E1 - E0) <= 1e-11 * (abs(E0) + abs(N0))
+    for sigma in (e_lo, 0.5 * (lam[0] + lam[-1]), lam[-1] + 0.1):
+        got = s.inertia(float(sigma))
+        assert np.sum(lam < sigma - 1e-11) <= got <= np.sum(lam < sigma + 1e-11)
+    if n > 1:
+        z = 0.5 * (mu + e_lo) + R * np.exp(1j * np.pi * (2 * np.arange(M // 2) + 1) / M)
+        wk = (z - 0.5 * (mu + e_lo)) / M
+        K = F.T @ F
+        a = [np.zeros((n, n)) for _ in range(3)]
+        for zk, w in zip(z, wk):
+            G = np.linalg.inv(zk * S - H)
+            for q in range(3):
+                a[q] += np.real(w * zk ** q * (G @ K @ G))
+        out = s.adjoint(mu, e_lo, windows=True)
+        k = out["kappa"]
+        for got, ref in ((out["dHW"], a[1] - k * a[0]), (out["dSW"], -(a[2] - k * a[1]))):
+            ref = 4 * cr.dV * ref
+            assert np.linalg.norm(got - ref.ravel(order="F")) <= 1e-10 * np.linalg.norm(4 * cr.dV * a[0])
+    s.close()
