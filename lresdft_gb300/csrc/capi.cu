@@ -136,6 +136,12 @@ struct lres_ctx {
     double4* d_coef = nullptr;
     double2* d_tr = nullptr;
     bool k_ready = false;
+    // density passes through P (FP64): V = Y P in batches of windows
+    bool by_matrix = false;
+    double* d_V = nullptr;
+    long long* d_offV = nullptr;
+    std::vector<int> vbatch;                     // first window of every batch, then nwin
+    int max_pass_items = 0;                      // pass items of a window at most
     OzWork oz;                                   // digits of the FP64 products on the tensor cores
     // pole work
     int2 *d_items = nullptr, *d_items_win = nullptr, *d_items_sub = nullptr;
@@ -193,7 +199,7 @@ lres_ctx::~lres_ctx() {
                     d_wq, d_wzq, d_q, d_dens, d_nw, d_ew, d_v, d_fftwork, d_adjA[0], d_adjA[1], d_adjA[2],
                     d_dHW, d_dSW, d_gH, d_adjdv, d_adju, d_cw, d_order, d_eoff, d_poff, d_ent, d_pent, d_adjws,
                     d_mT, d_offFT, d_offQT, d_FT, d_FhatT32, d_qT, d_Fhat64, d_FhatT64, d_offN, d_offA, d_order_w, d_LinvT32, d_Linv32,
-                    d_tstatus, d_K, d_coef, d_tr, d_triA, d_trid, d_trie, d_tritau, d_Yown, d_Ytr, d_lam, d_triT};
+                    d_tstatus, d_K, d_coef, d_tr, d_V, d_offV, d_triA, d_trid, d_trie, d_tritau, d_Yown, d_Ytr, d_lam, d_triT};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     ri_own.release();
@@ -588,6 +594,47 @@ int ensure_tfactors(lres_ctx* c) {
     return LRES_OK;
 }
 
+// Buffers of the FP64 density pass through P, where that is the cheaper one: 2.5 n^2 FP64 instructions
+// a pole and a product of m n^2 multiply-adds on the tensor cores (16 times the FP64 rate) against
+// 11 m n a pole.  Every size of the benchmark and the tests is on this side except windows of one
+// or two atoms' points.
+int tri_setup_matrix(lres_ctx* c, cudaStream_t s) {
+    double rows = 0.0, mat = 0.0;
+    for (int w = 0; w < c->nwin; ++w) {
+        const double n = c->n_w[w], m = c->m_w[w];
+        rows += 11.0 * c->npoles * m * n;
+        mat += 2.5 * c->npoles * n * n + m * n * n / 16 + 12.0 * m * n;
+    }
+    if (mat > rows || c->nwin > 65535) return LRES_OK;
+    const long long most = std::max<long long>((long long)1 << 27, 1);       // 1 GB of V
+    std::vector<long long> offV(c->nwin, 0);
+    long long size = 0, cur = 0;
+    c->vbatch.assign(1, 0);
+    for (int w = 0; w < c->nwin; ++w) {
+        const long long mine = (long long)c->n_w[w] * c->m_w[w];
+        if (cur && cur + mine > most) {
+            c->vbatch.push_back(w);
+            cur = 0;
+        }
+        offV[w] = cur;
+        cur += mine;
+        size = std::max(size, cur);
+    }
+    c->vbatch.push_back(c->nwin);
+    const int rb = tri_rows_per_item(false, c->npoles);
+    c->max_pass_items = (c->mmax + rb - 1) / rb;
+    int nb = 0;
+    for (size_t i = 0; i + 1 < c->vbatch.size(); ++i) nb = std::max(nb, c->vbatch[i + 1] - c->vbatch[i]);
+    TRY(upload(&c->d_offV, offV, s));
+    TRY(dalloc(&c->d_V, size));
+    TRY(oz_reserve(c->oz, nb, c->mmax, c->nmax, c->nmax));
+    TRY(oz_reserve(c->oz, c->nwin, c->nmax, c->nmax, c->nmax));
+    if (!c->d_coef) TRY(dalloc(&c->d_coef, (size_t)c->nwin * c->npoles * c->nmax));
+    LRES_CUDA_TRY(cudaStreamSynchronize(s));     // offV goes out of scope
+    c->by_matrix = true;
+    return LRES_OK;
+}
+
 // Buffers of the tridiagonal route (once per context).
 int tri_setup(lres_ctx* c, cudaStream_t s) {
     if (c->tri_alloc) return LRES_OK;
@@ -610,6 +657,7 @@ int tri_setup(lres_ctx* c, cudaStream_t s) {
         TRY(build_row_items(c, mT, c->ri_tr, s));
         TRY(dalloc((char**)&c->d_Ytr, el * (size_t)std::max<long long>(c->sizeFT, 1)));
     }
+    if (!fp32) TRY(tri_setup_matrix(c, s));
     c->tri_alloc = true;
     return LRES_OK;
 }
@@ -695,6 +743,36 @@ int tri_run_count(lres_ctx* c, cudaStream_t s) {
                   c->d_wzq, c->dV, c->d_coef, c->d_tr, c->d_nw, c->d_ew, c->d_status, c->smem_budget, s));
     TRY(mark(c, 0, 1, s));
     return LRES_OK;
+}
+
+// The FP64 density pass through P (in place of the standard form, which the reduction has consumed).
+int tri_run_matrix(lres_ctx* c, cudaStream_t s) {
+    const int P = c->npoles;
+    const lres_ctx::RowItems& ri = c->ri_own;
+    const double *d = static_cast<const double*>(c->d_trid), *e = static_cast<const double*>(c->d_trie);
+    const double* Y = static_cast<const double*>(c->d_Yown);
+    TRY(mark(c, 0, 0, s));
+    TRY(tri_pmat(c->nwin, P, c->nmax, c->d_n, c->d_offN, c->d_offC, d, e, static_cast<const double2*>(c->d_shifts),
+                 c->d_wq, c->d_coef, c->d_Hhat, s));
+    for (size_t i = 0; i + 1 < c->vbatch.size(); ++i) {
+        const int w0 = c->vbatch[i], nb = c->vbatch[i + 1] - w0;
+        TRY(oz_gemm(c->oz, nb, c->mmax, c->nmax, c->nmax, c->d_m + w0, c->d_n + w0, c->d_n + w0, Y, c->d_offF + w0, false,
+                    c->d_Hhat, c->d_offC + w0, true, c->d_V, c->d_offV + w0, 0, c->smem_budget, s));
+        TRY(tri_rowdot(w0, nb, c->max_pass_items, ri.pass, ri.first, ri.count, c->d_n, c->d_m, c->d_offN, c->d_offF,
+                       c->d_offV, c->d_offQ, c->d_Oflat, Y, c->d_V, d, e, c->d_dens, ri.part, c->d_status, s));
+    }
+    TRY(mark(c, 0, 1, s));
+    TRY(mark(c, 1, 0, s));
+    TRY(tri_window_sums(c->nwin, ri.first, ri.count, ri.part, c->dV, c->d_nw, c->d_ew, s));
+    TRY(mark(c, 1, 1, s));
+    return LRES_OK;
+}
+
+// A pass at the nodes already set: the density and the windows' sums, or (count) the sums only.
+int tri_any_pass(lres_ctx* c, bool count, bool trace, cudaStream_t s) {
+    if ((count || trace) && counts_from_k(c)) return tri_run_count(c, s);
+    if (!trace && c->by_matrix) return tri_run_matrix(c, s);
+    return tri_run_pass(c, trace, s);
 }
 
 int find_block(const std::vector<int>& bptr, const std::vector<int>& bcol, int g, int h) {
@@ -1249,8 +1327,7 @@ static int run_pass(lres_ctx* c, double mu, double e_lo, double* dens, int dens_
     const bool trace = !dens && c->have_trace;
     if (c->route == LRES_ROUTE_TRIDIAG) {
         if (!c->tri_ready) TRY(tri_refresh(c, s));
-        if ((count || trace) && counts_from_k(c)) TRY(tri_run_count(c, s));
-        else TRY(tri_run_pass(c, trace, s));
+        TRY(tri_any_pass(c, count, trace, s));
     } else {
         const Rows rw = select_rows(c, trace);
         TRY(ensure_hhat_df(c, s));
@@ -1490,7 +1567,7 @@ extern "C" int lres_pass_async(lres_ctx* c, double mu, double e_lo, double* d_ou
     LRES_CUDA_TRY(cudaMemsetAsync(c->d_status, 0, sizeof(int), s));
     if (c->route == LRES_ROUTE_TRIDIAG) {
         if (!c->tri_ready) TRY(tri_refresh(c, s));
-        TRY(tri_run_pass(c, false, s));
+        TRY(tri_any_pass(c, false, false, s));
     } else {
         TRY(ensure_hhat_df(c, s));
         if (mixed)
@@ -1874,7 +1951,7 @@ int adj_tri_accumulate(lres_ctx* c, cudaStream_t s) {
     double4* const coef = reinterpret_cast<double4*>(base);
     double* const X = reinterpret_cast<double*>(base + coefb);
     double2* const ws = reinterpret_cast<double2*>(base + coefb + xb);
-    TRY(tri_run_pass(c, c->have_trace, s));
+    TRY(tri_any_pass(c, false, c->have_trace, s));
     TRY(ensure_k(c, s));
     if (c->ri_adj.arows != c->tri.arows) TRY(build_row_items(c, c->n_w, c->ri_adj, s));
     TRY(tri_apply(false, c->ri_adj.napply, c->ri_adj.apply, c->d_n, c->d_n, c->d_offA, c->d_offN, c->d_offC, c->d_triA,

@@ -105,6 +105,8 @@ struct OzWork {
     size_t bytes = 0;
     void release();
 };
+// Workspace for products of up to these sizes (a call within them allocates nothing).
+int oz_reserve(OzWork& wk, int nwin, int mmax, int nmax, int kmax);
 int oz_gemm(OzWork& wk, int nwin, int mmax, int nmax, int kmax, const int* m_w, const int* n_w, const int* k_w,
             const double* A, const long long* offA, bool a_kcontig, const double* B, const long long* offB,
             bool b_kcontig, double* C, const long long* offC, int klim, size_t smem_budget, cudaStream_t s);
@@ -166,6 +168,14 @@ int tri_count(int nwin, int P, int nmax, const int* n_w, const long long* offN, 
               const double* e, const double* K, const double2* shifts, const double2* wq, const double2* wzq,
               double dV, double4* coef, double2* trace, double* nw, double* ew, int* status, size_t smem_budget,
               cudaStream_t s);
+// P = Re sum_k w_k (z_k - T)^-1 of every window (FP64), and the rows' n, e from V = Y P for windows
+// w0 .. w0 + nwin - 1 (V of window w at offV[w], maxitems pass items of a window at most)
+int tri_pmat(int nwin, int P, int nmax, const int* n_w, const long long* offN, const long long* offC, const double* d,
+             const double* e, const double2* shifts, const double2* wq, double4* coef, double* Pm, cudaStream_t s);
+int tri_rowdot(int w0, int nwin, int maxitems, const int4* items, const int* first, const int* count, const int* n_w,
+               const int* m_w, const long long* offN, const long long* offF, const long long* offV,
+               const long long* offQ, const long long* Oflat, const double* Y, const double* V, const double* d,
+               const double* e, double* dens, double* part, int* status, cudaStream_t s);
 int tri_window_sums(int nwin, const int* first, const int* count, const double* part, double dV, double* nw,
                     double* ew, cudaStream_t s);
 int tri_sturm(bool fp32, int nwin, const int* n_w, const long long* offN, const void* d, const void* e,

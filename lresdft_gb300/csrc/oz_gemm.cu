@@ -300,6 +300,36 @@ void OzWork::release() {
     *this = OzWork{};
 }
 
+// Padded sizes and windows per batch: about 1 GB of digits at most (one window at least).
+struct OzPlan {
+    int Rp, Cp, Kp, batch;
+    size_t perw;
+};
+static OzPlan oz_plan(int nwin, int mmax, int nmax, int kmax) {
+    OzPlan p;
+    p.Rp = (mmax + kOzT - 1) / kOzT * kOzT;
+    p.Cp = (nmax + kOzT - 1) / kOzT * kOzT;
+    p.Kp = (std::max(kmax, 1) + kOzK - 1) / kOzK * kOzK;
+    p.perw = sizeof(unsigned short) * kDig * (size_t)(p.Rp + p.Cp) * p.Kp + sizeof(int) * (size_t)(p.Rp + p.Cp);
+    p.batch = (int)std::min<size_t>({(size_t)nwin, std::max<size_t>(((size_t)1 << 30) / p.perw, 1), (size_t)65535});
+    return p;
+}
+
+int oz_reserve(OzWork& wk, int nwin, int mmax, int nmax, int kmax) {
+    const OzPlan p = oz_plan(nwin, mmax, nmax, kmax);
+    const size_t need = p.perw * p.batch;
+    if (wk.bytes >= need) return LRES_OK;
+    wk.release();
+    if (cudaMalloc(&wk.buf, need) != cudaSuccess) {
+        cudaGetLastError();
+        wk.buf = nullptr;
+        lres_set_error("tensor-core FP64 product: allocation of %zu bytes failed", need);
+        return LRES_ENOMEM;
+    }
+    wk.bytes = need;
+    return LRES_OK;
+}
+
 int oz_gemm(OzWork& wk, int nwin, int mmax, int nmax, int kmax, const int* m_w, const int* n_w, const int* k_w,
             const double* A, const long long* offA, bool a_kcontig, const double* B, const long long* offB,
             bool b_kcontig, double* C, const long long* offC, int klim, size_t smem_budget, cudaStream_t s) {
@@ -308,21 +338,9 @@ int oz_gemm(OzWork& wk, int nwin, int mmax, int nmax, int kmax, const int* m_w, 
         lres_set_error("tensor-core FP64 product needs %d B of shared memory", kOzSmem);
         return LRES_EINVAL;
     }
-    const int Rp = (mmax + kOzT - 1) / kOzT * kOzT, Cp = (nmax + kOzT - 1) / kOzT * kOzT;
-    const int Kp = (std::max(kmax, 1) + kOzK - 1) / kOzK * kOzK;
-    const size_t perw = sizeof(unsigned short) * kDig * (size_t)(Rp + Cp) * Kp + sizeof(int) * (size_t)(Rp + Cp);
-    // about 1 GB of digits at most (one window at least), kept with the context
-    const int batch = (int)std::min<size_t>({(size_t)nwin, std::max<size_t>(((size_t)1 << 30) / perw, 1), (size_t)65535});
-    if (wk.bytes < perw * batch) {
-        wk.release();
-        if (cudaMalloc(&wk.buf, perw * batch) != cudaSuccess) {
-            cudaGetLastError();
-            wk.buf = nullptr;
-            lres_set_error("tensor-core FP64 product: allocation of %zu bytes failed", perw * batch);
-            return LRES_ENOMEM;
-        }
-        wk.bytes = perw * batch;
-    }
+    if (int rc = oz_reserve(wk, nwin, mmax, nmax, kmax)) return rc;
+    const OzPlan p = oz_plan(nwin, mmax, nmax, kmax);
+    const int Rp = p.Rp, Cp = p.Cp, Kp = p.Kp, batch = p.batch;
     unsigned short* const da = static_cast<unsigned short*>(wk.buf);
     unsigned short* const db = da + (size_t)batch * kDig * Rp * Kp;
     int* const ea = reinterpret_cast<int*>(db + (size_t)batch * kDig * Cp * Kp);

@@ -1379,6 +1379,138 @@ __global__ void tri_count_sums_kernel(int nwin, int P, const double2* trace, con
     ew[w] = 4.0 * se * dV;
 }
 
+// ---------------------------------------------------------------------------
+// density pass through the pole-weighted matrix (FP64)
+// ---------------------------------------------------------------------------
+//
+// n(r) = 4 y_r P y_r^T and, since Re sum_k w_k = 0, e(r) = 4 y_r T P y_r^T with P = Re sum_k w_k G_k (n x n,
+// real).  P costs 2.5 n^2 FP64 instructions a pole instead of the rows' 11 m n, and V = Y P is a
+// dense product for the tensor cores (oz_gemm.cu); what is left per row is two inner products.
+// Measured: 54 windows of 276-300 functions and 256 rows 4.7 -> 2.3 ms, 432 windows 29.4 ->
+// 10.5 ms.
+
+constexpr int kPmatWarps = 4, kPmatPoles = 8;
+
+// One CTA per (window, 32 columns), lane = column j, the poles dealt to the warps; row i from the
+// diagonal up: G_ij = G_{i+1,j} t_{i+1}.  The warps' sums of 32 rows are joined in shared memory and
+// written with their mirror image.
+__global__ void __launch_bounds__(32 * kPmatWarps) tri_pmat_kernel(int P, const int* n_w, const long long* offC,
+                                                                   const double4* coef, int ld, const double2* wq,
+                                                                   double* Pm) {
+    __shared__ double part[kPmatWarps][32][33];
+    const int w = blockIdx.y, n = n_w[w];
+    const int b = blockIdx.x;
+    if (32 * b >= n) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int j = 32 * b + lane;
+    double* const Pw = Pm + offC[w];
+    const double4* const cw = coef + (size_t)w * P * ld;
+    for (int k0 = 0; k0 < P; k0 += kPmatWarps * kPmatPoles) {
+        const double4* cf[kPmatPoles];                              // this warp's poles
+        double2 s[kPmatPoles], init[kPmatPoles];
+#pragma unroll
+        for (int q = 0; q < kPmatPoles; ++q) {
+            const int k = k0 + warp + q * kPmatWarps;
+            cf[q] = cw + (size_t)min(k, P - 1) * ld;
+            init[q] = s[q] = make_double2(0.0, 0.0);
+            if (k < P && j < n) {
+                const double4 g = cf[q][j];
+                const double2 wk = wq[k];
+                init[q] = make_double2(wk.x * g.z - wk.y * g.w, wk.x * g.w + wk.y * g.z);
+            }
+        }
+        for (int ib = b; ib >= 0; --ib) {
+#pragma unroll 2
+            for (int r = 31; r >= 0; --r) {
+                const int i = 32 * ib + r;
+                if (i >= n) continue;                               // (the same for every lane)
+                double sum = 0.0;
+#pragma unroll
+                for (int q = 0; q < kPmatPoles; ++q) {
+                    if (i == j) s[q] = init[q];
+                    sum += s[q].x;
+                    const double2 t = *reinterpret_cast<const double2*>(cf[q] + i);
+                    s[q] = make_double2(fma(t.x, s[q].x, -t.y * s[q].y), fma(t.x, s[q].y, t.y * s[q].x));
+                }
+                part[warp][r][lane] = sum;                          // (zero above the diagonal: s is zero there)
+            }
+            __syncthreads();
+            for (int r = warp; r < 32; r += kPmatWarps) {
+                const int i = 32 * ib + r;
+                if (i < n && j < n && i <= j) {
+                    double x = part[0][r][lane];
+#pragma unroll
+                    for (int q = 1; q < kPmatWarps; ++q) x += part[q][r][lane];
+                    if (k0) x += Pw[j + (long long)i * n];
+                    Pw[j + (long long)i * n] = x;
+                    part[0][r][lane] = x;
+                }
+            }
+            __syncthreads();
+            for (int c = warp; c < 32; c += kPmatWarps) {           // column 32 b + c, rows along the lanes
+                const int i = 32 * ib + lane, jc = 32 * b + c;
+                if (jc < n && i < jc) Pw[i + (long long)jc * n] = part[0][lane][c];
+            }
+            __syncthreads();
+        }
+    }
+}
+
+// n(r) and e(r) of an item's rows from V = Y P, sums of the item; rows along the lanes, the columns
+// split over the warps.
+__global__ void __launch_bounds__(128) tri_rowdot_kernel(int w0, const int4* items, const int* first, const int* count,
+                                                         const int* n_w, const int* m_w, const long long* offN,
+                                                         const long long* offF, const long long* offV,
+                                                         const long long* offQ, const long long* Oflat, const double* Y,
+                                                         const double* V, const double* d, const double* e, double* dens,
+                                                         double* part, int* status) {
+    __shared__ double sn[4][32], se[4][32];
+    if ((int)blockIdx.x >= count[w0 + blockIdx.y]) return;
+    const int it = first[w0 + blockIdx.y] + blockIdx.x;
+    const int4 item = items[it];
+    const int w = item.x, r0 = item.y, nr = item.z;
+    const int n = n_w[w], m = m_w[w];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const double *dw = d + offN[w], *ew = e + offN[w];
+    double tn = 0.0, te = 0.0;                                      // (warp 0: sums of the item)
+    for (int rb = 0; rb < nr; rb += 32) {
+        double an = 0.0, ae = 0.0;
+        if (rb + lane < nr) {
+            const double* const y = Y + offF[w] + r0 + rb + lane;
+            const double* const v = V + offV[w] + r0 + rb + lane;
+            const int j0 = n * warp / 4, j1 = n * (warp + 1) / 4;
+            double yp = j0 > 0 ? y[(long long)(j0 - 1) * m] : 0.0, yc = j0 < n ? y[(long long)j0 * m] : 0.0;
+            for (int j = j0; j < j1; ++j) {
+                const double yn = j + 1 < n ? y[(long long)(j + 1) * m] : 0.0;
+                const double x = v[(long long)j * m];
+                const double ty = fma(dw[j], yc, fma(j > 0 ? ew[j - 1] : 0.0, yp, (j + 1 < n ? ew[j] : 0.0) * yn));
+                an = fma(x, yc, an);
+                ae = fma(x, ty, ae);
+                yp = yc;
+                yc = yn;
+            }
+        }
+        __syncthreads();
+        sn[warp][lane] = an;
+        se[warp][lane] = ae;
+        __syncthreads();
+        if (warp == 0) {
+            const double nrow = 4.0 * ((sn[0][lane] + sn[1][lane]) + (sn[2][lane] + sn[3][lane]));
+            const double erow = 4.0 * ((se[0][lane] + se[1][lane]) + (se[2][lane] + se[3][lane]));
+            if (rb + lane < nr) {
+                if (!isfinite(nrow) || !isfinite(erow)) atomicOr(status, ST_ZERO_PIVOT);
+                if (dens) dens[Oflat[offQ[w] + r0 + rb + lane]] = nrow;
+            }
+            tn += warp_sum(nrow);
+            te += warp_sum(erow);
+        }
+    }
+    if (threadIdx.x == 0) {
+        part[2 * (size_t)it] = tn;
+        part[2 * (size_t)it + 1] = te;
+    }
+}
+
 // per-window totals from the items of each window (contiguous, fixed order)
 __global__ void tri_window_sums_kernel(int nwin, const int* first, const int* count, const double* part, double dV,
                                        double* nw, double* ew) {
@@ -1685,6 +1817,28 @@ int tri_count(int nwin, int P, int nmax, const int* n_w, const long long* offN, 
     tri_count_kernel<<<(unsigned)nwin * groups, kCountNT, smem, s>>>(P, groups, n_w, offC, K, coef, nmax, trace);
     LRES_CUDA_TRY(cudaGetLastError());
     tri_count_sums_kernel<<<(nwin + 63) / 64, 64, 0, s>>>(nwin, P, trace, wq, wzq, dV, nw, ew, status);
+    LRES_CUDA_TRY(cudaGetLastError());
+    return LRES_OK;
+}
+
+int tri_pmat(int nwin, int P, int nmax, const int* n_w, const long long* offN, const long long* offC, const double* d,
+             const double* e, const double2* shifts, const double2* wq, double4* coef, double* Pm, cudaStream_t s) {
+    if (!nwin) return LRES_OK;
+    tri_diag_kernel<<<(unsigned)(((long long)nwin * P + 31) / 32), 32, 0, s>>>(nwin, P, n_w, offN, d, e, shifts, nmax,
+                                                                              coef);
+    LRES_CUDA_TRY(cudaGetLastError());
+    tri_pmat_kernel<<<dim3((nmax + 31) / 32, nwin), 32 * kPmatWarps, 0, s>>>(P, n_w, offC, coef, nmax, wq, Pm);
+    LRES_CUDA_TRY(cudaGetLastError());
+    return LRES_OK;
+}
+
+int tri_rowdot(int w0, int nwin, int maxitems, const int4* items, const int* first, const int* count, const int* n_w,
+               const int* m_w, const long long* offN, const long long* offF, const long long* offV,
+               const long long* offQ, const long long* Oflat, const double* Y, const double* V, const double* d,
+               const double* e, double* dens, double* part, int* status, cudaStream_t s) {
+    if (!nwin || !maxitems) return LRES_OK;
+    tri_rowdot_kernel<<<dim3(maxitems, nwin), 128, 0, s>>>(w0, items, first, count, n_w, m_w, offN, offF, offV, offQ,
+                                                           Oflat, Y, V, d, e, dens, part, status);
     LRES_CUDA_TRY(cudaGetLastError());
     return LRES_OK;
 }
