@@ -130,12 +130,13 @@ struct lres_ctx {
         }
     };
     RowItems ri_own, ri_tr;
-    RowItems ri_adj;                             // the rows of L^-T (adjoint)
     // count passes (FP64): K = Y^T Y of the current Hamiltonian, formed by the first of them
     double* d_K = nullptr;
     double4* d_coef = nullptr;
     double2* d_tr = nullptr;
     bool k_ready = false;
+    OzRows ozr;                                  // rows through the reflectors on the tensor cores (FP64)
+    OzRowSet oz_own, oz_trc, oz_adj;
     // density passes through P (FP64): V = Y P in batches of windows
     bool by_matrix = false;
     double* d_V = nullptr;
@@ -204,8 +205,11 @@ lres_ctx::~lres_ctx() {
         if (p) cudaFree(p);
     ri_own.release();
     ri_tr.release();
-    ri_adj.release();
     oz.release();
+    ozr.release();
+    oz_own.release();
+    oz_trc.release();
+    oz_adj.release();
     if (fft) fft3_destroy(fft);
     for (cudaEvent_t e : ev)
         if (e) cudaEventDestroy(e);
@@ -381,8 +385,8 @@ int transform_f32(lres_ctx* c, cudaStream_t s) {
 
 // FP64 product of window matrices (n x n, column-major): C = op(A) op(B), (at) A^T B, (not bk) A B^T.
 int square_gemm(lres_ctx* c, const double* A, bool at, const double* B, bool bk, double* C, int klim, cudaStream_t s) {
-    return oz_gemm(c->oz, c->nwin, c->nmax, c->nmax, c->nmax, c->d_n, c->d_n, c->d_n, A, c->d_offC, at, B, c->d_offC, bk,
-                   C, c->d_offC, klim, c->smem_budget, s);
+    return oz_gemm(c->oz, c->nwin, c->nmax, c->nmax, c->nmax, c->d_n, c->d_n, c->d_n, A, c->d_offC, OzForm(at),
+                   B, c->d_offC, OzForm(bk), C, c->d_offC, klim, false, c->smem_budget, s);
 }
 
 // FP64 (the FP64 tridiagonal route); the product H LinvT lives in the working blocks of the
@@ -594,6 +598,63 @@ int ensure_tfactors(lres_ctx* c) {
     return LRES_OK;
 }
 
+// Panels of the FP64 rows on the tensor cores (once per context).
+int oz_setup(lres_ctx* c, cudaStream_t s) {
+    OzRows& o = c->ozr;
+    o.panels = (std::max(c->nmax - 2, 0) + kOzPanel - 1) / kOzPanel;
+    const size_t cnt = (size_t)o.panels * c->nwin;
+    std::vector<int> q(cnt, 0), r(cnt, 0);
+    std::vector<long long> offV(cnt, 0), offT(cnt, 0);
+    long long offA = 0, size = 0;
+    for (int w = 0; w < c->nwin; ++w) {
+        const int n = c->n_w[w];
+        const long long ld = (n + 3) & ~3;
+        for (int p = 0; p < o.panels; ++p) {
+            const size_t i = (size_t)p * c->nwin + w;
+            const int j0 = p * kOzPanel;
+            q[i] = std::clamp(n - 2 - j0, 0, kOzPanel);
+            r[i] = q[i] ? n - 1 - j0 : 0;
+            offV[i] = q[i] ? offA + j0 + 1 + j0 * ld : 0;
+            offT[i] = size;
+            size += (long long)q[i] * q[i];
+        }
+        offA += ld * n;
+    }
+    TRY(upload(&o.q, q, s));
+    TRY(upload(&o.r, r, s));
+    TRY(upload(&o.offV, offV, s));
+    TRY(upload(&o.offT, offT, s));
+    TRY(dalloc(&o.T, size));
+    LRES_CUDA_TRY(cudaStreamSynchronize(s));     // the host vectors go out of scope
+    return LRES_OK;
+}
+
+// One row set of m[w] rows for them.
+int oz_setup_rows(lres_ctx* c, const std::vector<int>& m, OzRowSet& rs, cudaStream_t s) {
+    rs.release();
+    const int np = c->ozr.panels;
+    std::vector<long long> offS(c->nwin, 0), offY((size_t)np * c->nwin, 0);
+    long long size = 0, off = 0;
+    for (int w = 0; w < c->nwin; ++w) {
+        rs.mmax = std::max(rs.mmax, m[w]);
+        offS[w] = size;
+        size += (long long)m[w] * kOzPanel;
+        for (int p = 0; p < np; ++p)
+            offY[(size_t)p * c->nwin + w] = off + (long long)std::min(p * kOzPanel + 1, c->n_w[w]) * m[w];
+        off += (long long)m[w] * c->n_w[w];
+    }
+    TRY(upload(&rs.offS, offS, s));
+    TRY(upload(&rs.offY, offY, s));
+    TRY(dalloc(&rs.S, size));
+    TRY(dalloc(&rs.S2, size));
+    // the products' workspace for these sizes
+    const int q = std::min(kOzPanel, std::max(c->nmax - 2, 1));
+    TRY(oz_reserve(c->oz, c->nwin, rs.mmax, q, c->nmax));
+    TRY(oz_reserve(c->oz, c->nwin, rs.mmax, c->nmax, q));
+    LRES_CUDA_TRY(cudaStreamSynchronize(s));     // the host vectors go out of scope
+    return LRES_OK;
+}
+
 // Buffers of the FP64 density pass through P, where that is the cheaper one: 2.5 n^2 FP64 instructions
 // a pole and a product of m n^2 multiply-adds on the tensor cores (16 times the FP64 rate) against
 // 11 m n a pole.  Every size of the benchmark and the tests is on this side except windows of one
@@ -657,21 +718,44 @@ int tri_setup(lres_ctx* c, cudaStream_t s) {
         TRY(build_row_items(c, mT, c->ri_tr, s));
         TRY(dalloc((char**)&c->d_Ytr, el * (size_t)std::max<long long>(c->sizeFT, 1)));
     }
-    if (!fp32) TRY(tri_setup_matrix(c, s));
+    if (!fp32) {
+        TRY(oz_setup(c, s));
+        TRY(oz_setup_rows(c, c->m_w, c->oz_own, s));
+        if (c->have_trace) {
+            std::vector<int> mT(c->nwin);
+            LRES_CUDA_TRY(cudaMemcpy(mT.data(), c->d_mT, sizeof(int) * c->nwin, cudaMemcpyDeviceToHost));
+            TRY(oz_setup_rows(c, mT, c->oz_trc, s));
+        }
+        TRY(tri_setup_matrix(c, s));
+    }
     c->tri_alloc = true;
     return LRES_OK;
 }
 
+// FP64 rows F (m_w x n_w at offF, `size` values) through the reflectors into Y.
+int rows_fp64(lres_ctx* c, const OzRowSet& rs, const int* m_w, const double* F, long long size, double* Y,
+              cudaStream_t s) {
+    LRES_CUDA_TRY(cudaMemcpyAsync(Y, F, sizeof(double) * size, cudaMemcpyDeviceToDevice, s));
+    return oz_rows(c->oz, c->ozr, rs, c->nwin, c->nmax, c->d_n, m_w, static_cast<const double*>(c->d_triA), Y,
+                   c->smem_budget, s);
+}
+
 // Rows of one row set (owned points or trace rows) through the reflectors.
 int tri_rows(lres_ctx* c, bool trace, cudaStream_t s) {
-    const bool fp32 = c->precision == LRES_MIXED;
-    const lres_ctx::RowItems& ri = trace ? c->ri_tr : c->ri_own;
-    const void* F = trace ? (fp32 ? (const void*)c->d_FhatT32 : (const void*)c->d_FhatT64)
-                          : (fp32 ? (const void*)c->d_Fhat32 : (const void*)c->d_Fhat64);
     // the T factors depend on the reflectors only: formed with the owned rows
-    return tri_apply(fp32, ri.napply, ri.apply, c->d_n, trace ? c->d_mT : c->d_m, c->d_offA, c->d_offN,
-                     trace ? c->d_offFT : c->d_offF, c->d_triA, c->d_tritau, F, trace ? c->d_Ytr : c->d_Yown,
-                     c->tri, c->nwin, !trace, c->d_triT, c->smem_budget, s);
+    if (c->precision != LRES_MIXED) {
+        if (!trace)
+            TRY(oz_tfactors(c->oz, c->ozr, c->nwin, c->nmax, c->d_n, static_cast<const double*>(c->d_triA),
+                            static_cast<const double*>(c->d_tritau), c->d_offN, c->smem_budget, s));
+        return trace ? rows_fp64(c, c->oz_trc, c->d_mT, c->d_FhatT64, c->sizeFT, static_cast<double*>(c->d_Ytr), s)
+                     : rows_fp64(c, c->oz_own, c->d_m, c->d_Fhat64, c->sizeF, static_cast<double*>(c->d_Yown), s);
+    }
+    const lres_ctx::RowItems& ri = trace ? c->ri_tr : c->ri_own;
+    return tri_apply(ri.napply, ri.apply, c->d_n, trace ? c->d_mT : c->d_m, c->d_offA, c->d_offN,
+                     trace ? c->d_offFT : c->d_offF, static_cast<const float*>(c->d_triA),
+                     static_cast<const float*>(c->d_tritau), trace ? c->d_FhatT32 : c->d_Fhat32,
+                     static_cast<float*>(trace ? c->d_Ytr : c->d_Yown), c->tri, c->nwin, !trace, c->d_triT,
+                     c->smem_budget, s);
 }
 
 // Tridiagonal form of the current standard-form windows and the rows through its reflectors
@@ -756,8 +840,9 @@ int tri_run_matrix(lres_ctx* c, cudaStream_t s) {
                  c->d_wq, c->d_coef, c->d_Hhat, s));
     for (size_t i = 0; i + 1 < c->vbatch.size(); ++i) {
         const int w0 = c->vbatch[i], nb = c->vbatch[i + 1] - w0;
-        TRY(oz_gemm(c->oz, nb, c->mmax, c->nmax, c->nmax, c->d_m + w0, c->d_n + w0, c->d_n + w0, Y, c->d_offF + w0, false,
-                    c->d_Hhat, c->d_offC + w0, true, c->d_V, c->d_offV + w0, 0, c->smem_budget, s));
+        TRY(oz_gemm(c->oz, nb, c->mmax, c->nmax, c->nmax, c->d_m + w0, c->d_n + w0, c->d_n + w0, Y, c->d_offF + w0,
+                    OzForm(false), c->d_Hhat, c->d_offC + w0, OzForm(true), c->d_V, c->d_offV + w0, 0, false,
+                    c->smem_budget, s));
         TRY(tri_rowdot(w0, nb, c->max_pass_items, ri.pass, ri.first, ri.count, c->d_n, c->d_m, c->d_offN, c->d_offF,
                        c->d_offV, c->d_offQ, c->d_Oflat, Y, c->d_V, d, e, c->d_dens, ri.part, c->d_status, s));
     }
@@ -1953,9 +2038,8 @@ int adj_tri_accumulate(lres_ctx* c, cudaStream_t s) {
     double2* const ws = reinterpret_cast<double2*>(base + coefb + xb);
     TRY(tri_any_pass(c, false, c->have_trace, s));
     TRY(ensure_k(c, s));
-    if (c->ri_adj.arows != c->tri.arows) TRY(build_row_items(c, c->n_w, c->ri_adj, s));
-    TRY(tri_apply(false, c->ri_adj.napply, c->ri_adj.apply, c->d_n, c->d_n, c->d_offA, c->d_offN, c->d_offC, c->d_triA,
-                  c->d_tritau, c->d_LinvT, c->d_Hhat, c->tri, c->nwin, false, c->d_triT, c->smem_budget, s));
+    if (!c->oz_adj.offS) TRY(oz_setup_rows(c, c->n_w, c->oz_adj, s));
+    TRY(rows_fp64(c, c->oz_adj, c->d_n, c->d_LinvT, c->sizeC, c->d_Hhat, s));
     return adj_tri(c->nwin, P, groups, batch, c->nmax, c->d_order, c->d_n, c->d_offN, c->d_offC, c->sizeC,
                    static_cast<const double*>(c->d_trid), static_cast<const double*>(c->d_trie),
                    static_cast<const double2*>(c->d_shifts), c->d_cw, c->d_K, coef, ws, X, c->d_adjA[0],
@@ -2197,6 +2281,7 @@ extern "C" int lres_set_trace_rows(lres_ctx* c, const int32_t* r_w, const double
     }
     if (c->tri_alloc) {
         TRY(build_row_items(c, m, c->ri_tr, s));
+        if (!mixed) TRY(oz_setup_rows(c, m, c->oz_trc, s));
         TRY(dalloc((char**)&c->d_Ytr, (mixed ? sizeof(float) : sizeof(double)) * (size_t)std::max<long long>(c->sizeFT, 1)));
         if (c->tri_ready) TRY(tri_rows(c, true, s));
     }

@@ -96,10 +96,15 @@ int gather_windows(int nwin, int nmax, const int* fn, const long long* fnoff, co
 int build_F(int nwin, const long long* Xp, const int* Xi, const double* Xv, const int* group_of_fn,
             const int* gptr, const int* gloc, int ngroups, const long long* Ooff, const long long* Oflat,
             const long long* offF, const int* m_w, int mmax, double* F, cudaStream_t s);
-// FP64 products on the tensor cores (oz_gemm.cu): C_w = op(A_w) op(B_w), C_w m_w x n_w column-major at
-// offC, K = k_w terms.  op(A)(i, k) at A[i + k m] or (a_kcontig) A[k + i K]; op(B)(k, j) at B[j + k n] or
-// (b_kcontig) B[k + j K]; klim 1: op(B) upper triangular, 2: op(A) lower triangular and the lower triangle
-// of C only.  The workspace grows on demand.
+// FP64 products on the tensor cores (oz_gemm.cu): C_w = op(A_w) op(B_w) (or C_w -= it), C_w m_w x n_w
+// column-major at offC, K = k_w terms.  klim 1: op(B) upper triangular, 2: op(A) lower triangular and
+// the lower triangle of C only.  The workspace grows on demand.
+struct OzForm {                       // how an operand is stored
+    bool k_contig;                    // op(A)(i, k) at A[k + i ld] (op(B)(k, j) at B[k + j ld]), else at A[i + k ld] (B[j + k ld])
+    const int* ld = nullptr;          // leading dimension ld[w] rounded up to 4; none: that of a dense block
+    bool refl = false;                // Householder vectors (row i, reflector l): 1 on the diagonal, 0 above
+    OzForm(bool kc, const int* l = nullptr, bool r = false) : k_contig(kc), ld(l), refl(r) {}
+};
 struct OzWork {
     void* buf = nullptr;
     size_t bytes = 0;
@@ -108,8 +113,8 @@ struct OzWork {
 // Workspace for products of up to these sizes (a call within them allocates nothing).
 int oz_reserve(OzWork& wk, int nwin, int mmax, int nmax, int kmax);
 int oz_gemm(OzWork& wk, int nwin, int mmax, int nmax, int kmax, const int* m_w, const int* n_w, const int* k_w,
-            const double* A, const long long* offA, bool a_kcontig, const double* B, const long long* offB,
-            bool b_kcontig, double* C, const long long* offC, int klim, size_t smem_budget, cudaStream_t s);
+            const double* A, const long long* offA, OzForm fa, const double* B, const long long* offB, OzForm fb,
+            double* C, const long long* offC, int klim, bool subtract, size_t smem_budget, cudaStream_t s);
 int batched_gram(int nwin, const int* n_w, const int* m_w, const long long* offF, const long long* offK, int nmax,
                  const double* F, double* K, cudaStream_t s);
 int batched_gemm_rect_upper(int nwin, const int* n_w, const int* m_w, const long long* offA, const long long* offU,
@@ -154,9 +159,28 @@ int tri_reduce_reg(int nwin, const int* order, int* counter, const int* n_w, con
                    const long long* offA, const long long* offN, const float* H, float* A, float* d, float* e,
                    float* tau, int* status, int nb, int nmax, size_t smem_budget, cudaStream_t s);
 // tfactors: form the T factors of every (window, panel) first (once per Hamiltonian)
-int tri_apply(bool fp32, int nitems, const int4* items, const int* n_w, const int* m_w, const long long* offA,
-              const long long* offN, const long long* offF, const void* A, const void* tau, const void* F, void* Y,
-              const TriPick& pk, int nwin, bool tfactors, void* T, size_t smem_budget, cudaStream_t s);
+int tri_apply(int nitems, const int4* items, const int* n_w, const int* m_w, const long long* offA,
+              const long long* offN, const long long* offF, const float* A, const float* tau, const float* F, float* Y,
+              const TriPick& pk, int nwin, bool tfactors, float* T, size_t smem_budget, cudaStream_t s);
+// Rows of a set through the reflectors on the tensor cores (FP64): panels of kOzPanel reflectors.
+constexpr int kOzPanel = 128;
+struct OzRows {                       // per panel and window, panel-major: reflectors, rows below, offsets of
+    int panels = 0;                   // the panel's reflectors, its T (kOzPanel^2 apart)
+    int *q = nullptr, *r = nullptr;
+    long long *offV = nullptr, *offT = nullptr;
+    double* T = nullptr;
+    void release();
+};
+struct OzRowSet {                     // one row set: S scratch and, per panel and window, offsets of Y's block
+    long long *offS = nullptr, *offY = nullptr;
+    double *S = nullptr, *S2 = nullptr;
+    int mmax = 0;
+    void release();
+};
+int oz_tfactors(OzWork& wk, const OzRows& o, int nwin, int nmax, const int* n_w, const double* A, const double* tau,
+                const long long* offN, size_t smem_budget, cudaStream_t s);
+int oz_rows(OzWork& wk, const OzRows& o, const OzRowSet& rs, int nwin, int nmax, const int* n_w, const int* m_w,
+            const double* A, double* Y, size_t smem_budget, cudaStream_t s);
 int tri_rows_per_item(bool fp32, int P);
 int tri_pass(bool fp32, int nitems, const int4* items, int* counter, const int* n_w, const int* m_w,
              const long long* offN, const long long* offF, const long long* offQ, const long long* Oflat,

@@ -38,14 +38,15 @@ constexpr int kOzBad = 1 << 20;               // exponent of a row with a non-fi
 constexpr int kStageBytes = 2 * kDig * kOzT * kOzK * 2;
 constexpr int kOzSmem = kOzStages * kStageBytes;
 
-// One operand of a batch: window w's matrix at X[off[w]], element (r, k) at r + k rows (k_contig = 0)
-// or k + r cols (k_contig = 1); rows, cols per window, or one array for both.
+// One operand of a batch: window w's matrix at X[off[w]], element (r, k) at r + k ld (k_contig = 0) or
+// k + r ld (k_contig = 1), ld = rows or cols unless given.  Reflectors (OzForm::refl): the stored entry
+// (row i, reflector l) counts below the diagonal, is 1 on it and 0 above.
 struct Operand {
     const double* X;
     const long long* off;
     const int* rows;
     const int* cols;
-    int k_contig;
+    OzForm f;
 };
 
 __device__ __forceinline__ int ilogb_bits(double x) {
@@ -61,16 +62,22 @@ __global__ void __launch_bounds__(256) oz_slice_kernel(int w0, Operand o, int Rp
     const int R = o.rows[w], K = o.cols[w];
     if (r0 >= (R + kOzT - 1) / kOzT * kOzT) return;                 // (tiles beyond are never read)
     const double* const X = o.X + o.off[w];
+    const long long ld = o.f.ld ? (o.f.ld[w] + 3) & ~3 : o.f.k_contig ? K : R;
+    auto at = [&](int r, int k) -> double {
+        const int i = o.f.k_contig ? k : r, l = o.f.k_contig ? r : k;
+        if (o.f.refl && i <= l) return i == l ? 1.0 : 0.0;
+        return X[i + l * ld];
+    };
     const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
     if (tid < 32) emax[tid] = -1100;
     __syncthreads();
     // the largest exponent of every row
-    if (o.k_contig) {
+    if (o.f.k_contig) {
         for (int r = ty; r < 32; r += 8) {
             int e = -1100;
             if (r0 + r < R)
                 for (int k = tx; k < K; k += 32) {
-                    const double x = X[k + (long long)(r0 + r) * K];
+                    const double x = at(r0 + r, k);
                     if (x != 0.0) e = max(e, ilogb_bits(x));
                 }
             e = __reduce_max_sync(0xffffffffu, e);
@@ -80,7 +87,7 @@ __global__ void __launch_bounds__(256) oz_slice_kernel(int w0, Operand o, int Rp
         int e = -1100;
         if (r0 + tx < R)
             for (int k = ty; k < K; k += 8) {
-                const double x = X[r0 + tx + (long long)k * R];
+                const double x = at(r0 + tx, k);
                 if (x != 0.0) e = max(e, ilogb_bits(x));
             }
         atomicMax(&emax[tx], e);
@@ -94,11 +101,11 @@ __global__ void __launch_bounds__(256) oz_slice_kernel(int w0, Operand o, int Rp
         __syncthreads();
         for (int q = ty; q < 32; q += 8) {
             double x = 0.0;
-            if (o.k_contig) {
-                if (r0 + q < R && k0 + tx < K) x = X[k0 + tx + (long long)(r0 + q) * K];
+            if (o.f.k_contig) {
+                if (r0 + q < R && k0 + tx < K) x = at(r0 + q, k0 + tx);
                 tile[q][tx] = x;
             } else {
-                if (r0 + tx < R && k0 + q < K) x = X[r0 + tx + (long long)(k0 + q) * R];
+                if (r0 + tx < R && k0 + q < K) x = at(r0 + tx, k0 + q);
                 tile[tx][q] = x;
             }
         }
@@ -167,7 +174,7 @@ template <int KLIM, bool LONG>
 __global__ void __launch_bounds__(kOzNT, 1) oz_gemm_kernel(int w0, const int* m_w, const int* n_w, const int* k_w,
                                                            int Rp, int Cp, int Kp, const unsigned short* da,
                                                            const unsigned short* db, const int* ea, const int* eb,
-                                                           const long long* offC, double* C) {
+                                                           const long long* offC, double* C, int subtract) {
     extern __shared__ __align__(128) unsigned char smem[];
     const int slot = blockIdx.z, w = w0 + slot;
     const int M = m_w[w], N = n_w[w], K = k_w[w];
@@ -289,7 +296,8 @@ __global__ void __launch_bounds__(kOzNT, 1) oz_gemm_kernel(int w0, const int* m_
                 if (xa >= kOzBad || xb >= kOzBad) x = __longlong_as_double(0x7ff8000000000000LL);
                 else if (p > -960 && p < 960) x *= __longlong_as_double((long long)(p + 1023) << 52);
                 else x = ldexp(x, p);
-                Cw[gi + (long long)gj * M] = x;
+                double* const dst = Cw + gi + (long long)gj * M;
+                *dst = subtract ? *dst - x : x;
             }
 }
 
@@ -331,9 +339,9 @@ int oz_reserve(OzWork& wk, int nwin, int mmax, int nmax, int kmax) {
 }
 
 int oz_gemm(OzWork& wk, int nwin, int mmax, int nmax, int kmax, const int* m_w, const int* n_w, const int* k_w,
-            const double* A, const long long* offA, bool a_kcontig, const double* B, const long long* offB,
-            bool b_kcontig, double* C, const long long* offC, int klim, size_t smem_budget, cudaStream_t s) {
-    if (!nwin || !mmax || !nmax) return LRES_OK;
+            const double* A, const long long* offA, OzForm fa, const double* B, const long long* offB, OzForm fb,
+            double* C, const long long* offC, int klim, bool subtract, size_t smem_budget, cudaStream_t s) {
+    if (nwin < 1 || mmax < 1 || nmax < 1) return LRES_OK;
     if ((size_t)kOzSmem > smem_budget) {
         lres_set_error("tensor-core FP64 product needs %d B of shared memory", kOzSmem);
         return LRES_EINVAL;
@@ -349,12 +357,12 @@ int oz_gemm(OzWork& wk, int nwin, int mmax, int nmax, int kmax, const int* m_w, 
     int per_sm = 0;
     auto launch = [&](auto kern, int w0, int nb) {
         const dim3 grid((mmax + kOzT - 1) / kOzT, (nmax + kOzT - 1) / kOzT, nb);
-        kern<<<grid, kOzNT, kOzSmem, s>>>(w0, m_w, n_w, k_w, Rp, Cp, Kp, da, db, ea, eb, offC, C);
+        kern<<<grid, kOzNT, kOzSmem, s>>>(w0, m_w, n_w, k_w, Rp, Cp, Kp, da, db, ea, eb, offC, C, subtract ? 1 : 0);
     };
     for (int w0 = 0; w0 < nwin; w0 += batch) {
         const int nb = std::min(batch, nwin - w0);
-        oz_slice_kernel<<<dim3(Rp / 32, nb), 256, 0, s>>>(w0, Operand{A, offA, m_w, k_w, a_kcontig}, Rp, Kp, da, ea);
-        oz_slice_kernel<<<dim3(Cp / 32, nb), 256, 0, s>>>(w0, Operand{B, offB, n_w, k_w, b_kcontig}, Cp, Kp, db, eb);
+        oz_slice_kernel<<<dim3(Rp / 32, nb), 256, 0, s>>>(w0, Operand{A, offA, m_w, k_w, fa}, Rp, Kp, da, ea);
+        oz_slice_kernel<<<dim3(Cp / 32, nb), 256, 0, s>>>(w0, Operand{B, offB, n_w, k_w, fb}, Cp, Kp, db, eb);
         LRES_CUDA_TRY(cudaGetLastError());
 #define OZ_RUN(KL, LG)                                                                  \
     do {                                                                                \
@@ -373,6 +381,107 @@ int oz_gemm(OzWork& wk, int nwin, int mmax, int nmax, int kmax, const int* m_w, 
         }
 #undef OZ_RUN
         LRES_CUDA_TRY(cudaGetLastError());
+    }
+    return LRES_OK;
+}
+
+// ---------------------------------------------------------------------------
+// rows through the Householder reflectors, compact WY panels of 128 (FP64)
+// ---------------------------------------------------------------------------
+//
+// Y <- Y - ((Y V) T) V^T per panel, three products on the tensor cores; V^T V (for T) a fourth, once per
+// Hamiltonian for all row sets.  Panels of 128 rather than the 32 of tri_apply_kernel: a product over
+// 32 terms would spend more on the digits and the joining than on its terms.  The FP64 pipe does the
+// T recurrence only.  Measured (with T): 54 windows of 256 rows 7.5 -> 2.6 ms, 432 windows 32.5 ->
+// 12.5 ms.
+
+namespace {
+
+constexpr int kTNT = 128;
+
+// T of one (window, panel) from G = V^T V in its slot: T_ll = tau_l, T[0:l, l] = -tau_l T[0:l, 0:l] G[0:l, l],
+// T in place of G (column-major, zero below the diagonal).  Thread = row of T; the upper triangles packed
+// by columns in shared memory.
+__global__ void __launch_bounds__(kTNT) oz_tfactor_kernel(const int* q_w, const long long* offT, const long long* offN,
+                                                          const double* tau, int j0, double* T) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    double* const Gs = reinterpret_cast<double*>(smem);             // (a, b), a <= b at b (b + 1) / 2 + a
+    const int w = blockIdx.x, q = q_w[w], a = threadIdx.x;
+    if (q < 1) return;
+    double* const Ts = Gs + q * (q + 1) / 2;
+    double* const Tw = T + offT[w];
+    for (int b = 0; b < q; ++b)
+        for (int i = a; i <= b; i += kTNT) Gs[b * (b + 1) / 2 + i] = Tw[i + (long long)b * q];
+    __syncthreads();
+    const double* const tw = tau + offN[w] + j0;
+    for (int l = 0; l < q; ++l) {
+        const double tl = tw[l];
+        const double* const g = Gs + l * (l + 1) / 2;
+        if (a < l) {
+            double s[4] = {0.0, 0.0, 0.0, 0.0};
+            int b = a;
+            for (; b + 3 < l; b += 4)
+#pragma unroll
+                for (int u = 0; u < 4; ++u) s[u] = fma(Ts[(b + u) * (b + u + 1) / 2 + a], g[b + u], s[u]);
+            for (; b < l; ++b) s[0] = fma(Ts[b * (b + 1) / 2 + a], g[b], s[0]);
+            Ts[l * (l + 1) / 2 + a] = -tl * ((s[0] + s[1]) + (s[2] + s[3]));
+        } else if (a == l) {
+            Ts[l * (l + 1) / 2 + a] = tl;
+        }
+        // (row a is read by thread a only)
+    }
+    __syncthreads();
+    for (int b = 0; b < q; ++b)
+        if (a < q) Tw[a + (long long)b * q] = a <= b ? Ts[b * (b + 1) / 2 + a] : 0.0;
+}
+
+}  // namespace
+
+void OzRows::release() {
+    for (void* p : {(void*)q, (void*)r, (void*)offV, (void*)offT, (void*)T})
+        if (p) cudaFree(p);
+    *this = OzRows{};
+}
+void OzRowSet::release() {
+    for (void* p : {(void*)offS, (void*)offY, (void*)S, (void*)S2})
+        if (p) cudaFree(p);
+    *this = OzRowSet{};
+}
+
+int oz_tfactors(OzWork& wk, const OzRows& o, int nwin, int nmax, const int* n_w, const double* A, const double* tau,
+                const long long* offN, size_t smem_budget, cudaStream_t s) {
+    for (int p = 0; p < o.panels; ++p) {
+        const int j0 = p * kOzPanel, qm = std::min(kOzPanel, nmax - 2 - j0), rm = nmax - 1 - j0;
+        const int *q = o.q + (size_t)p * nwin, *r = o.r + (size_t)p * nwin;
+        const long long *offV = o.offV + (size_t)p * nwin, *offT = o.offT + (size_t)p * nwin;
+        const OzForm v(true, n_w, true);
+        if (int rc = oz_gemm(wk, nwin, qm, qm, rm, q, q, r, A, offV, v, A, offV, v, o.T, offT, 0, false, smem_budget, s))
+            return rc;
+        const size_t smem = sizeof(double) * (size_t)qm * (qm + 1);
+        int per_sm = 0;
+        if (int rc = prepare_kernel<oz_tfactor_kernel>(kTNT, smem, &per_sm)) return rc;
+        oz_tfactor_kernel<<<nwin, kTNT, smem, s>>>(q, offT, offN, tau, j0, o.T);
+        LRES_CUDA_TRY(cudaGetLastError());
+    }
+    return LRES_OK;
+}
+
+int oz_rows(OzWork& wk, const OzRows& o, const OzRowSet& rs, int nwin, int nmax, const int* n_w, const int* m_w,
+            const double* A, double* Y, size_t smem_budget, cudaStream_t s) {
+    for (int p = 0; p < o.panels; ++p) {
+        const int j0 = p * kOzPanel, qm = std::min(kOzPanel, nmax - 2 - j0), rm = nmax - 1 - j0;
+        const int *q = o.q + (size_t)p * nwin, *r = o.r + (size_t)p * nwin;
+        const long long *offV = o.offV + (size_t)p * nwin, *offT = o.offT + (size_t)p * nwin;
+        const long long* offY = rs.offY + (size_t)p * nwin;
+        if (int rc = oz_gemm(wk, nwin, rs.mmax, qm, rm, m_w, q, r, Y, offY, OzForm(false), A, offV,
+                             OzForm(true, n_w, true), rs.S, rs.offS, 0, false, smem_budget, s))
+            return rc;
+        if (int rc = oz_gemm(wk, nwin, rs.mmax, qm, qm, m_w, q, q, rs.S, rs.offS, OzForm(false), o.T, offT,
+                             OzForm(true), rs.S2, rs.offS, 1, false, smem_budget, s))
+            return rc;
+        if (int rc = oz_gemm(wk, nwin, rs.mmax, rm, qm, m_w, r, q, rs.S2, rs.offS, OzForm(false), A, offV,
+                             OzForm(false, n_w, true), Y, offY, 0, true, smem_budget, s))
+            return rc;
     }
     return LRES_OK;
 }

@@ -1728,31 +1728,22 @@ static int launch_apply_res(const TriApplyParams<float>& p, const TriTParams& tp
     return LRES_OK;
 }
 
-int tri_apply(bool fp32, int nitems, const int4* items, const int* n_w, const int* m_w, const long long* offA,
-              const long long* offN, const long long* offF, const void* A, const void* tau, const void* F, void* Y,
-              const TriPick& pk, int nwin, bool tfactors, void* T, size_t smem_budget, cudaStream_t s) {
+int tri_apply(int nitems, const int4* items, const int* n_w, const int* m_w, const long long* offA,
+              const long long* offN, const long long* offF, const float* A, const float* tau, const float* F, float* Y,
+              const TriPick& pk, int nwin, bool tfactors, float* T, size_t smem_budget, cudaStream_t s) {
     if (!nitems) return LRES_OK;
-    if (fp32) {
-        TriApplyParams<float> p{nitems, items, n_w, m_w, offA, offN, offF, (const float*)A, (const float*)tau,
-                                (const float*)F, (float*)Y, pk.ldv};
-        if (pk.rpt == 0) {
-            if (!T) {
-                lres_set_error("resident row application without a T-factor buffer");
-                return LRES_ESTATE;
-            }
-            const int maxp = tfactors ? (pk.ldv + pk.nb_apply - 1) / pk.nb_apply : 0;
-            TriTParams tp{nwin, maxp, n_w, offA, offN, (const float*)A, (const float*)tau, (float*)T, pk.tstride,
-                          pk.ldv};
-            if (pk.nb_apply == 32) return launch_apply_res<32>(p, tp, pk.arows, smem_budget, s);
-            if (pk.nb_apply == 16) return launch_apply_res<16>(p, tp, pk.arows, smem_budget, s);
-            lres_set_error("resident row application: panel width %d not compiled", pk.nb_apply);
-            return LRES_EINVAL;
-        }
-        return dispatch_apply(p, pk.nb_apply, pk.rpt, s);
+    TriApplyParams<float> p{nitems, items, n_w, m_w, offA, offN, offF, A, tau, F, Y, pk.ldv};
+    if (pk.rpt) return dispatch_apply(p, pk.nb_apply, pk.rpt, s);
+    if (!T) {
+        lres_set_error("resident row application without a T-factor buffer");
+        return LRES_ESTATE;
     }
-    TriApplyParams<double> p{nitems, items, n_w, m_w, offA, offN, offF, (const double*)A, (const double*)tau,
-                             (const double*)F, (double*)Y, pk.ldv};
-    return dispatch_apply(p, pk.nb_apply, pk.rpt, s);
+    const int maxp = tfactors ? (pk.ldv + pk.nb_apply - 1) / pk.nb_apply : 0;
+    TriTParams tp{nwin, maxp, n_w, offA, offN, A, tau, T, pk.tstride, pk.ldv};
+    if (pk.nb_apply == 32) return launch_apply_res<32>(p, tp, pk.arows, smem_budget, s);
+    if (pk.nb_apply == 16) return launch_apply_res<16>(p, tp, pk.arows, smem_budget, s);
+    lres_set_error("resident row application: panel width %d not compiled", pk.nb_apply);
+    return LRES_EINVAL;
 }
 
 int tri_rows_per_item(bool fp32, int P) {
