@@ -1,23 +1,24 @@
 // Batched FP64 matrix products on the tensor cores (sm_103a): C_w = op(A_w) op(B_w).
 //
 // GB300 issues 1.6 FP64 multiply-adds per clock and SM, its bf16 tensor cores ~1000 (mma.sync).  Every
-// operand row (column of B) is scaled by a power of two to 56-bit fixed point and cut into 8 signed
+// operand row (column of B) is scaled by a power of two to 63-bit fixed point and cut into 9 signed
 // digits of 7 bits, exact in bf16 (the error-free splitting of Ozaki, Ogita, Oishi and Rump, Numer.
 // Algorithms 59 (2012) 95-118).  Products of digits sum exactly in the FP32 accumulators: 64 x 64 x
-// 8 pairs x 512 terms = 2^24 (longer sums are taken in runs of 512).  The 36 digit pairs s + t <= 7
-// are kept, summed by s + t in 8 accumulators, joined in 64-bit integers and rounded twice; what is
-// dropped is below 2^-55 of the row's and the column's largest value per term, so the error is that
-// of a fixed-point product with 55 bits: at least FP64's relative to the largest elements.
+// 9 pairs x 448 terms < 2^24 (longer sums are taken in runs of 448).  The 45 digit pairs s + t <= 8
+// are kept, summed by s + t in 9 accumulators and joined with two roundings.  What is dropped is below
+// 2^-62 of the row's and the column's largest value per term: 9 bits less than FP64's rounding of
+// the largest elements, so that the smaller ones keep FP64's accuracy too (8 digits: 2^-55, a fifth
+// less time, and the density of 54 windows 2.1e-14 off 64 bits against 1.6e-14, the FP64 pipe's error).
 //
 // Two kernels: oz_slice_kernel writes the digits of an operand ([digit][row][k], k contiguous), each
 // element once; oz_gemm_kernel, one CTA per 64 x 64 tile, stages 32 terms of all digits of both
-// operands by cp.async (three stages of 64 KB) and issues 36 m16n8k16 products per warp tile and 16
-// terms, 8 warps of 32 x 16.  The digit pairs bound it: 36 x 4096 flops per 2048 multiply-adds at
-// ~600 TFLOP/s is 26 FP64 multiply-adds per clock and SM.  The windows go in batches, so that the
+// operands by cp.async (three stages of 72 KB) and issues 45 m16n8k16 products per warp tile and 16
+// terms, 8 warps of 32 x 16.  The digit pairs bound it: 45 x 4096 flops per 2048 multiply-adds at
+// ~600 TFLOP/s is 21 FP64 multiply-adds per clock and SM.  The windows go in batches, so that the
 // digits take at most ~1 GB whatever the context's size.
 //
-// Measured (432 windows of 270-306 functions): the standard form's two products 23.5 -> 4.5 ms (54
-// windows 3.7 -> 0.67), density error against 64 bits unchanged (2e-14).
+// Measured (432 windows of 270-306 functions): the standard form's two products 23.5 -> 6.1 ms (54
+// windows 3.7 -> 0.90).
 #include "common.cuh"
 #include "launch.cuh"
 #include "lres_internal.h"
@@ -27,13 +28,14 @@
 namespace lres {
 namespace {
 
-constexpr int kDig = 8;                       // digits of an operand
+constexpr int kDig = 9;                       // digits of an operand
 constexpr int kBits = 7;                      // bits of a digit
+constexpr int kTop = kBits * (kDig - 1) + 5 - 52;    // bits below FP64's last of a row's largest value
 constexpr int kOzT = 64;                      // tile edge
 constexpr int kOzK = 32;                      // terms of a stage
 constexpr int kOzStages = 3;
 constexpr int kOzNT = 256;
-constexpr int kOzRun = 512;                   // terms that sum exactly
+constexpr int kOzRun = 448;                   // terms that sum exactly: kDig 64 64 kOzRun <= 2^24
 constexpr int kOzBad = 1 << 20;               // exponent of a row with a non-finite value
 constexpr int kStageBytes = 2 * kDig * kOzT * kOzK * 2;
 constexpr int kOzSmem = kOzStages * kStageBytes;
@@ -117,10 +119,10 @@ __global__ void __launch_bounds__(256) oz_slice_kernel(int w0, Operand o, int Rp
             const int ef = (int)((b >> 52) & 0x7ff);
             long long m = b & 0xfffffffffffffLL;
             if (ef) m |= 1LL << 52;
-            const int sh = (ef ? ef - 1023 : -1022) - E + 2;        // q = x 2^(54 - E)
+            const int sh = (ef ? ef - 1023 : -1022) - E + kTop;     // q = x 2^(52 + kTop - E) < 2^62
             long long q = 0;
             if (m == 0) q = 0;
-            else if (sh >= 0) q = m << sh;                           // (sh <= 2)
+            else if (sh >= 0) q = m << sh;                           // (sh <= kTop)
             else if (sh > -60) q = (m + (1LL << (-sh - 1))) >> -sh;
             if (b < 0) q = -q;
 #pragma unroll
@@ -154,18 +156,20 @@ __device__ __forceinline__ void mma(float (&c)[4], const unsigned (&a)[4], unsig
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// sum_d acc_d 2^(-7 d), in units of 2^21 (exact up to the last rounding)
+// sum_d acc_d 2^(-7 d) in units of 2^-14: groups of three exact in integers, joined with two roundings
 __device__ __forceinline__ double oz_join(const float (&a)[kDig]) {
-    long long hi = 0, lo = 0;
+    static_assert(kDig == 9, "three groups of three");
+    double g[3];
 #pragma unroll
-    for (int d = 0; d < 4; ++d) hi = (hi << kBits) + __float2int_rn(a[d]);
+    for (int q = 0; q < 3; ++q) {
+        long long v = 0;
 #pragma unroll
-    for (int d = 4; d < 8; ++d) lo = (lo << kBits) + __float2int_rn(a[d]);
-    // |hi|, |lo| < 2^47: to double by the exponent of 1.5 2^52
-    const double magic = 6755399441055744.0;
-    const double h = __longlong_as_double(0x4338000000000000LL + hi) - magic;
-    const double l = __longlong_as_double(0x4338000000000000LL + lo) - magic;
-    return fma(l, 3.7252902984619140625e-09, h);                    // 2^-28
+        for (int d = 0; d < 3; ++d) v = (v << kBits) + __float2int_rn(a[3 * q + d]);
+        // |v| < 2^39: to double by the exponent of 1.5 2^52
+        g[q] = __longlong_as_double(0x4338000000000000LL + v) - 6755399441055744.0;
+    }
+    const double u = 4.76837158203125e-07;                          // 2^-21
+    return fma(fma(g[2], u, g[1]), u, g[0]);
 }
 
 // KLIM: 1, B upper triangular (k <= column); 2, A lower triangular (k <= row) and the
@@ -191,9 +195,8 @@ __global__ void __launch_bounds__(kOzNT, 1) oz_gemm_kernel(int w0, const int* m_
     auto load = [&](int kt, int buf) {
         const unsigned dst = sbase + buf * kStageBytes;
 #pragma unroll
-        for (int q = 0; q < 2 * kDig * kOzT * 4 / kOzNT; ++q) {
-            const int idx = tid + q * kOzNT;
-            const int c = idx & 3, r = (idx >> 2) & (kOzT - 1), s = (idx >> 8) & (kDig - 1), op = idx >> 11;
+        for (int q = 0; q < 2 * kDig; ++q) {                        // (a digit of an operand: 256 chunks)
+            const int c = tid & 3, r = tid >> 2, s = q % kDig, op = q / kDig;
             const unsigned short* src = op ? B + ((size_t)s * Cp + r) * Kp : A + ((size_t)s * Rp + r) * Kp;
             cp16(dst + (((op * kDig + s) * kOzT + r) * 4 + (c ^ (r >> 1 & 3))) * 16, src + kt * kOzK + c * 8);
         }
@@ -291,7 +294,7 @@ __global__ void __launch_bounds__(kOzNT, 1) oz_gemm_kernel(int w0, const int* m_
                 const int gi = m0 + wm + 16 * i + (lane >> 2) + 8 * (e >> 1), gj = n0 + wn + 8 * j + 2 * (lane & 3) + (e & 1);
                 if (gi >= M || gj >= N) continue;
                 const int xa = ea[(size_t)slot * Rp + gi], xb = eb[(size_t)slot * Cp + gj];
-                const int p = xa + xb - 31;                          // hi is in units of 2^(Ea + Eb - 10 - 21)
+                const int p = xa + xb - 24;                          // the join is in units of 2^(Ea + Eb - 10 - 14)
                 double x = sum[i][j][e];
                 if (xa >= kOzBad || xb >= kOzBad) x = __longlong_as_double(0x7ff8000000000000LL);
                 else if (p > -960 && p < 960) x *= __longlong_as_double((long long)(p + 1023) << 52);
@@ -392,8 +395,8 @@ int oz_gemm(OzWork& wk, int nwin, int mmax, int nmax, int kmax, const int* m_w, 
 // Y <- Y - ((Y V) T) V^T per panel, three products on the tensor cores; V^T V (for T) a fourth, once per
 // Hamiltonian for all row sets.  Panels of 128 rather than the 32 of tri_apply_kernel: a product over
 // 32 terms would spend more on the digits and the joining than on its terms.  The FP64 pipe does the
-// T recurrence only.  Measured (with T): 54 windows of 256 rows 7.5 -> 2.6 ms, 432 windows 32.5 ->
-// 12.5 ms.
+// T recurrence only.  Measured (with T): 54 windows of 256 rows 7.5 -> 2.9 ms, 432 windows 32.5 ->
+// 14.4 ms.
 
 namespace {
 
