@@ -37,7 +37,7 @@
 //                      T_p of the compact WY form (one warp), once per Hamiltonian for all
 //                      row sets.
 //   tri_apply_kernel   one CTA per (window, block of up to 256 rows), one thread per row,
-//                      the rows re-read from global memory per panel (FP64 path, and the
+//                      the rows re-read from global memory per panel (FP32, the
 //                      configurations without resident rows).
 //   tri_pass_kernel    one CTA per (window, batch of rows) from a work queue: thread =
 //                      (pole, rows); the pivot recurrence of its pole is shared by its rows,
@@ -137,17 +137,43 @@ struct TriReduceParams {
 };
 
 // Shared memory of the reduction, in elements of R.
-inline size_t reduce_smem_elems(int nb, int ldv, int nt) {
+inline size_t reduce_smem_elems(int nb, int ldv, int nt, int cl = 1) {
     const size_t big = std::max((size_t)2 * nb * ldv, (size_t)(nt / 32) * 32 * 33);
-    return big + 5 * (size_t)ldv + 4 * (size_t)nt + 64 + nt / 32;
+    return big + (4 + cl) * (size_t)ldv + 4 * (size_t)nt + 64 + nt / 32;
 }
 
-// CTAs per SM that the FP32 reduction is compiled for (registers: 65536 / (NT * that)).
-constexpr int reduce_min_ctas(int nt, int elem) { return elem != 4 ? 1 : 1024 / nt; }
+// CTAs per SM that the reduction is compiled for (registers: 65536 / (NT * that)).
+constexpr int reduce_min_ctas(int nt, int elem) { return elem != 4 ? 512 / nt : 1024 / nt; }
 
-template <class R, int NT>
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// Barrier of the cluster; what its CTAs wrote before (global and shared memory) is visible after.
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// x to the same shared variable of CTA `rank` of the cluster
+__device__ __forceinline__ void st_cluster(double* dst, unsigned rank, double x) {
+    unsigned a = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(a), "r"(rank));
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(x) : "memory");
+}
+__device__ __forceinline__ void st_cluster(float* dst, unsigned rank, float x) {
+    unsigned a = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(a), "r"(rank));
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(x) : "memory");
+}
+
+// CL = 2: a cluster of two CTAs per window, for fewer windows than half the SMs (FP64, 54 windows of 276-300
+// functions 9.2 -> 7.6 ms; one window of 96, where the barriers outweigh the work, 1.64 -> 1.84 ms).  Both form the columns, reflectors and vectors (the same bits); the row quads of q = A x and the
+// blocks of the trailing update, which hold the FP64 pipe, are dealt to them, q exchanged through
+// distributed shared memory (two buffers by column parity: the other CTA may be a phase ahead).
+template <class R, int NT, int CL = 1>
 __global__ void __launch_bounds__(NT, reduce_min_ctas(NT, sizeof(R))) tri_reduce_kernel(TriReduceParams<R> p) {
     constexpr int NW = NT / 32;
+    const int rank = CL > 1 ? (int)cluster_rank() : 0;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int ldv = p.ldv, nb = p.nb;
     R* const big = reinterpret_cast<R*>(smem_raw);
@@ -155,8 +181,8 @@ __global__ void __launch_bounds__(NT, reduce_min_ctas(NT, sizeof(R))) tri_reduce
     R* const Ws = big + (size_t)nb * ldv;                // [nb][ldv]
     R* const cv = big + std::max((size_t)2 * nb * ldv, (size_t)NW * 32 * 33);   // [ldv] current column
     R* const pv = cv + ldv;                              // [ldv] p = tau (A v)
-    R* const qx = pv + ldv;                              // [ldv] q = A x (unsplit)
-    R* const acol = qx + ldv;                            // [2][ldv] panel-start columns j, j+1
+    R* const qx0 = pv + ldv;                             // [CL][ldv] q = A x (unsplit)
+    R* const acol = qx0 + CL * ldv;                      // [2][ldv] panel-start columns j, j+1
     R* const psum = acol + 2 * ldv;                      // [4 NT] split sums of A x
     R* const dots = psum + 4 * NT;                       // [64] W^T x, V^T x, x^T x
     R* const red = dots + 64;                            // [NW]
@@ -164,18 +190,25 @@ __global__ void __launch_bounds__(NT, reduce_min_ctas(NT, sizeof(R))) tri_reduce
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
     for (;;) {
-        if (tid == 0) item_sh = atomicAdd(p.counter, 1);
-        __syncthreads();
-        const int it = item_sh;
+        int it;
+        if constexpr (CL > 1) {                           // one window per cluster
+            it = blockIdx.x / CL;
+        } else {
+            if (tid == 0) item_sh = atomicAdd(p.counter, 1);
+            __syncthreads();
+            it = item_sh;
+        }
         if (it >= p.nwin) return;
         const int w = p.order[it];
         const int n = p.n_w[w];
         if (n > ldv || n < 1) {
             if (tid == 0) atomicOr(p.status, ST_BAD_SHAPE);
+            if constexpr (CL > 1) return;
             __syncthreads();
             continue;
         }
         if (n <= p.keep) {
+            if constexpr (CL > 1) return;
             __syncthreads();                      // item_sh is read before the next fetch
             continue;
         }
@@ -192,7 +225,7 @@ __global__ void __launch_bounds__(NT, reduce_min_ctas(NT, sizeof(R))) tri_reduce
         {
             R* tile = big + (size_t)warp * 32 * 33;
             const int nt = (n + 31) / 32;
-            for (int t = warp; t < nt * (nt + 1) / 2; t += NW) {
+            for (int t = warp + rank * NW; t < nt * (nt + 1) / 2; t += NW * CL) {
                 int bi = 0, bk = t;                      // t-th block of the lower block triangle
                 while (bk > bi) {
                     bk -= bi + 1;
@@ -217,7 +250,8 @@ __global__ void __launch_bounds__(NT, reduce_min_ctas(NT, sizeof(R))) tri_reduce
                 __syncwarp();
             }
         }
-        __syncthreads();
+        if constexpr (CL > 1) cluster_sync();
+        else __syncthreads();
 
         // Each column takes three barriers.  Rows are owned by threads (row i by thread i mod NT)
         // for the column, the reflector and w; the norm, the dots W^T x, V^T x and q = A x are
@@ -257,12 +291,20 @@ __global__ void __launch_bounds__(NT, reduce_min_ctas(NT, sizeof(R))) tri_reduce
                 //     32 terms from zero.
                 const int i0 = (j + 1) & ~3;
                 const int nq = (ld - i0) >> 2;
-                const int nsplit = nq >= NT ? 1 : NT / nq;
+                const int nqo = (nq + CL - 1) / CL;             // this CTA's quads: rank, rank + CL, ...
+                const int nsplit = nqo >= NT ? 1 : NT / nqo;
+                R* const qx = qx0 + (j & (CL - 1)) * ldv;
+                auto publish = [&](int i, R x) {
+                    qx[i] = x;
+                    if constexpr (CL > 1) st_cluster(qx + i, rank ^ 1, x);
+                };
                 {
-                    const int qstep = nq >= NT ? NT : nq;
+                    const int qstep = nqo >= NT ? NT : nqo;
                     if (tid < qstep * nsplit) {
                         const int sp = tid / qstep;
-                        for (int q = tid % qstep; q < nq; q += qstep) {
+                        for (int u = tid % qstep; u < nqo; u += qstep) {
+                            const int q = u * CL + rank;
+                            if (q >= nq) break;
                             const R* Aq = A + i0 + 4 * q;
                             R a[4] = {R(0), R(0), R(0), R(0)};
                             for (int kb = j + 2 + sp; kb < n; kb += 32 * nsplit) {
@@ -280,12 +322,12 @@ __global__ void __launch_bounds__(NT, reduce_min_ctas(NT, sizeof(R))) tri_reduce
                                 for (int r = 0; r < 4; ++r) a[r] += c[r];
                             }
                             if (nsplit > 1) {
-                                st4(psum + (sp * nq + q) * 4, a);    // 16-byte stores: no bank conflicts
+                                st4(psum + (sp * nqo + u) * 4, a);   // 16-byte stores: no bank conflicts
                             } else {
 #pragma unroll
                                 for (int r = 0; r < 4; ++r) {
                                     const int i = i0 + 4 * q + r;
-                                    if (i > j && i < n) qx[i] = a[r];
+                                    if (i > j && i < n) publish(i, a[r]);
                                 }
                             }
                         }
@@ -300,7 +342,21 @@ __global__ void __launch_bounds__(NT, reduce_min_ctas(NT, sizeof(R))) tri_reduce
                     acc = warp_sum(acc);
                     if (lane == 0) dots[q] = acc;
                 }
-                __syncthreads();
+                if constexpr (CL > 1) {
+                    if (nsplit > 1) {
+                        __syncthreads();
+                        for (int idx = tid; idx < 4 * nqo; idx += NT) {
+                            const int u = idx >> 2, r = idx & 3, i = i0 + 4 * (u * CL + rank) + r;
+                            if (i <= j || i >= n) continue;
+                            R qi = R(0);
+                            for (int sp = 0; sp < nsplit; ++sp) qi += psum[(sp * nqo + u) * 4 + r];
+                            publish(i, qi);
+                        }
+                    }
+                    cluster_sync();
+                } else {
+                    __syncthreads();
+                }
                 // (c) reflector H_j = I - tau v v^T with v_{j+1} = 1 mapping rows j+1.. of the
                 //     column onto beta e_{j+1} (every thread, the same bits); p = tau (A v - V (W^T v)
                 //     - W (V^T v)) on the owned rows, partial sums of p^T v
@@ -313,7 +369,7 @@ __global__ void __launch_bounds__(NT, reduce_min_ctas(NT, sizeof(R))) tri_reduce
                     tau = (beta - alpha) / beta;
                     scal = R(1) / (alpha - beta);
                 }
-                if (tid == 0) {
+                if (tid == 0 && rank == 0) {
                     dw[j] = cv[j];
                     ew[j] = beta;
                     tw[j] = tau;
@@ -327,9 +383,9 @@ __global__ void __launch_bounds__(NT, reduce_min_ctas(NT, sizeof(R))) tri_reduce
                     else if (i > j + 1 && i < n) vi = cv[i] * scal;
                     Vs[jj * ldv + i] = vi;
                     if (i > j && i < n) {
-                        if (i > j + 1) A[i + (long long)j * ld] = vi;      // kept for Y = F^ Q
+                        if (i > j + 1 && rank == 0) A[i + (long long)j * ld] = vi;      // kept for Y = F^ Q
                         R qi;
-                        if (nsplit > 1) {
+                        if (CL == 1 && nsplit > 1) {
                             const int q = (i - i0) >> 2, r = (i - i0) & 3;
                             qi = R(0);
                             for (int sp = 0; sp < nsplit; ++sp) qi += psum[(sp * nq + q) * 4 + r];
@@ -369,7 +425,7 @@ __global__ void __launch_bounds__(NT, reduce_min_ctas(NT, sizeof(R))) tri_reduce
             if (t0 < n) {
                 const int q0 = t0 & ~3;
                 const int nq = (ld - q0) >> 2;
-                for (int tile = tid; tile < nq * (nq + 1) / 2; tile += NT) {
+                for (int tile = tid + rank * NT; tile < nq * (nq + 1) / 2; tile += NT * CL) {
                     // column quads from the last: quad nq-1-u has u + 1 blocks
                     int u = (int)((sqrtf(8.0f * tile + 1.0f) - 1.0f) * 0.5f);
                     while ((u + 1) * (u + 2) / 2 <= tile) ++u;
@@ -422,10 +478,11 @@ __global__ void __launch_bounds__(NT, reduce_min_ctas(NT, sizeof(R))) tri_reduce
                     }
                 }
             }
-            __syncthreads();
+            if constexpr (CL > 1) cluster_sync();
+            else __syncthreads();
         }
         // ---- the last (at most 2 x 2) block, fully updated
-        if (tid == 0 && !p.keep) {
+        if (tid == 0 && rank == 0 && !p.keep) {
             if (n >= 2) {
                 dw[n - 2] = A[(n - 2) + (long long)(n - 2) * ld];
                 ew[n - 2] = A[(n - 1) + (long long)(n - 2) * ld];
@@ -439,6 +496,7 @@ __global__ void __launch_bounds__(NT, reduce_min_ctas(NT, sizeof(R))) tri_reduce
                 ew[0] = R(0);
             }
         }
+        if constexpr (CL > 1) return;                     // (the last cluster barrier is behind every exchange)
         __syncthreads();
     }
 }
@@ -1651,6 +1709,27 @@ static int launch_reduce(const TriReduceParams<R>& p, size_t smem_budget, cudaSt
     return LRES_OK;
 }
 
+// Two CTAs per window.
+static int launch_reduce_cluster(const TriReduceParams<double>& p, cudaStream_t s) {
+    constexpr int NT = 512;
+    const size_t smem = reduce_smem_elems(p.nb, p.ldv, NT, 2) * sizeof(double);
+    int per_sm = 0;
+    if (int rc = prepare_kernel<tri_reduce_kernel<double, NT, 2>>(NT, smem, &per_sm)) return rc;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * (unsigned)p.nwin);
+    cfg.blockDim = dim3(NT);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    LRES_CUDA_TRY(cudaLaunchKernelEx(&cfg, tri_reduce_kernel<double, NT, 2>, p));
+    return LRES_OK;
+}
+
 int tri_reduce(bool fp32, int nwin, const int* order, int* counter, const int* n_w, const long long* offC,
                const long long* offA, const long long* offN, const void* H, void* A, void* d, void* e, void* tau,
                int* status, const TriPick& pk, int nmax, size_t smem_budget, cudaStream_t s) {
@@ -1675,7 +1754,17 @@ int tri_reduce(bool fp32, int nwin, const int* order, int* counter, const int* n
     }
     TriReduceParams<double> p{nwin, order, counter, n_w, offC, offA, offN, (const double*)H, (double*)A,
                               (double*)d, (double*)e, (double*)tau, status, nb, ldv, 0};
-    return nt == 512 ? launch_reduce<double, 512>(p, smem_budget, s) : launch_reduce<double, 256>(p, smem_budget, s);
+    if (nt == 512) {
+        // two CTAs per window while they find an SM each and the windows are large enough to share; one
+        // CTA of 512 threads while the windows find one;
+        // beyond, two of 256 threads per SM, which fill each other's barriers (432 windows 26.5 -> 23.3 ms)
+        if (2 * nwin <= device_sms() && nmax >= 192 && reduce_smem_elems(nb, ldv, 512, 2) * sizeof(double) <= smem_budget)
+            return launch_reduce_cluster(p, s);
+        if (nwin > device_sms() && 2 * (reduce_smem_elems(nb, ldv, 256) * sizeof(double) + 1024) <= smem_budget + 1024)
+            return launch_reduce<double, 256>(p, smem_budget, s);
+        return launch_reduce<double, 512>(p, smem_budget, s);
+    }
+    return launch_reduce<double, 256>(p, smem_budget, s);
 }
 
 template <class R, int NB, int RPT>
