@@ -232,73 +232,88 @@ __global__ void adj_pivot_kernel(int nwin, int P, const int* n_w, const long lon
 
 constexpr int kSweepNT = 320;
 
-// One CTA per (window, group of poles): X_c += Re c_k G_k K G_k over its poles, the upper triangle
-// of group g at Xc[g * sizeC + offC + i + j n], i <= j.  Thread = column of K for
-// G_k K, then row of it for the second solve (whose back substitution stops at the diagonal);
-// every access but the reads of the second forward sweep runs along the threads.
+template <class R> struct Sweep;
+template <> struct Sweep<double> { using C2 = double2; using C4 = double4; };
+template <> struct Sweep<float> { using C2 = float2; using C4 = float4; };
+
+// One CTA per (window, group of poles): X_c += Re c_k G_k K G_k over its poles, the upper triangle of
+// group g at Xc[g * sizeC + offC + i + j n], i <= j.  Thread = column of K for G_k K, then row of it for
+// the second solve (whose back substitution stops at the diagonal); every access but the reads of the
+// second forward sweep runs along the threads.  R = float (mixed precision): the sweeps in FP32 from the
+// FP64 pivots, the poles still summed in FP64.
+template <class R>
 __global__ void __launch_bounds__(kSweepNT) adj_sweep_kernel(const int* wins, int P, int groups, const int* n_w,
-                                                             const long long* offC, long long sizeC, const double* K,
+                                                             const long long* offC, long long sizeC, const R* K,
                                                              const double4* coef, int ld, const double2* cw,
-                                                             double2* ws, long long ws_stride, double* Xa, double* Xb,
-                                                             double* Xc) {
+                                                             typename Sweep<R>::C2* ws, long long ws_stride, double* Xa,
+                                                             double* Xb, double* Xc) {
+    using C2 = typename Sweep<R>::C2;
+    using C4 = typename Sweep<R>::C4;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    double4* const cf = reinterpret_cast<double4*>(smem_raw);       // [n + 1]
+    C4* const cf = reinterpret_cast<C4*>(smem_raw);                 // [n + 1]
     const int w = wins[blockIdx.x / groups], grp = blockIdx.x % groups;
     const int n = n_w[w], tid = threadIdx.x;
     const int k0 = P * grp / groups, k1 = P * (grp + 1) / groups;
-    const double* const Kw = K + offC[w];
-    double2* const B = ws + (size_t)blockIdx.x * ws_stride;         // (G K)^T: B[j + i n] = (G K)_ij
-    double2* const U = B + (size_t)n * n;                           // U[i + j n]
+    const R* const Kw = K + offC[w];
+    C2* const B = ws + (size_t)blockIdx.x * ws_stride;              // (G K)^T: B[j + i n] = (G K)_ij
+    C2* const U = B + (size_t)n * n;                                // U[i + j n]
     for (int k = k0; k < k1; ++k) {
         __syncthreads();
         const double4* const src = coef + (size_t)(w * P + k) * ld;
-        for (int i = tid; i < n; i += kSweepNT) cf[i] = src[i];
-        if (tid == 0) cf[n] = make_double4(0.0, 0.0, 0.0, 0.0);
+        for (int i = tid; i < n; i += kSweepNT) cf[i] = C4{(R)src[i].x, (R)src[i].y, (R)src[i].z, (R)src[i].w};
+        if (tid == 0) cf[n] = C4{R(0), R(0), R(0), R(0)};
         __syncthreads();
         for (int j = tid; j < n; j += kSweepNT) {
-            double2 u = make_double2(0.0, 0.0);
+            C2 u = C2{R(0), R(0)};
 #pragma unroll 4
             for (int i = 0; i < n; ++i) {
-                const double4 c = cf[i];
-                u = make_double2(fma(c.x, u.x, fma(-c.y, u.y, Kw[j + (long long)i * n])), fma(c.x, u.y, c.y * u.x));
+                const C4 c = cf[i];
+                u = C2{fma(c.x, u.x, fma(-c.y, u.y, Kw[j + (long long)i * n])), fma(c.x, u.y, c.y * u.x)};
                 B[j + (long long)i * n] = u;
             }
-            double2 x = make_double2(0.0, 0.0);
+            C2 x = C2{R(0), R(0)};
 #pragma unroll 4
             for (int i = n - 1; i >= 0; --i) {
-                const double4 c = cf[i], cn = cf[i + 1];
-                const double2 v = B[j + (long long)i * n];
-                x = make_double2(fma(v.x, c.z, fma(-v.y, c.w, fma(cn.x, x.x, -cn.y * x.y))),
-                                 fma(v.x, c.w, fma(v.y, c.z, fma(cn.x, x.y, cn.y * x.x))));
+                const C4 c = cf[i], cn = cf[i + 1];
+                const C2 v = B[j + (long long)i * n];
+                x = C2{fma(v.x, c.z, fma(-v.y, c.w, fma(cn.x, x.x, -cn.y * x.y))),
+                       fma(v.x, c.w, fma(v.y, c.z, fma(cn.x, x.y, cn.y * x.x)))};
                 B[j + (long long)i * n] = x;
             }
         }
         __syncthreads();
-        const double2 c0 = cw[k], c1 = cw[P + k], c2 = cw[2 * P + k];
+        const C2 c0 = C2{(R)cw[k].x, (R)cw[k].y}, c1 = C2{(R)cw[P + k].x, (R)cw[P + k].y},
+                 c2 = C2{(R)cw[2 * P + k].x, (R)cw[2 * P + k].y};
         double* const X0 = Xa + (size_t)grp * sizeC + offC[w];
         double* const X1 = Xb + (size_t)grp * sizeC + offC[w];
         double* const X2 = Xc + (size_t)grp * sizeC + offC[w];
         for (int i = tid; i < n; i += kSweepNT) {
-            double2 u = make_double2(0.0, 0.0);
+            C2 u = C2{R(0), R(0)};
 #pragma unroll 4
             for (int j = 0; j < n; ++j) {
-                const double4 c = cf[j];
-                const double2 b = B[j + (long long)i * n];
-                u = make_double2(fma(c.x, u.x, fma(-c.y, u.y, b.x)), fma(c.x, u.y, fma(c.y, u.x, b.y)));
+                const C4 c = cf[j];
+                const C2 b = B[j + (long long)i * n];
+                u = C2{fma(c.x, u.x, fma(-c.y, u.y, b.x)), fma(c.x, u.y, fma(c.y, u.x, b.y))};
                 if (j >= i) U[i + (long long)j * n] = u;
             }
-            double2 x = make_double2(0.0, 0.0);
+            C2 x = C2{R(0), R(0)};
 #pragma unroll 2
             for (int j = n - 1; j >= i; --j) {
-                const double4 c = cf[j], cn = cf[j + 1];
+                const C4 c = cf[j], cn = cf[j + 1];
                 const long long at = i + (long long)j * n;
-                const double2 v = U[at];
-                x = make_double2(fma(v.x, c.z, fma(-v.y, c.w, fma(cn.x, x.x, -cn.y * x.y))),
-                                 fma(v.x, c.w, fma(v.y, c.z, fma(cn.x, x.y, cn.y * x.x))));
+                const C2 v = U[at];
+                x = C2{fma(v.x, c.z, fma(-v.y, c.w, fma(cn.x, x.x, -cn.y * x.y))),
+                       fma(v.x, c.w, fma(v.y, c.z, fma(cn.x, x.y, cn.y * x.x)))};
                 const double y0 = k == k0 ? 0.0 : X0[at], y1 = k == k0 ? 0.0 : X1[at], y2 = k == k0 ? 0.0 : X2[at];
-                X0[at] = fma(c0.x, x.x, fma(-c0.y, x.y, y0));
-                X1[at] = fma(c1.x, x.x, fma(-c1.y, x.y, y1));
-                X2[at] = fma(c2.x, x.x, fma(-c2.y, x.y, y2));
+                if constexpr (sizeof(R) == 8) {
+                    X0[at] = fma(c0.x, x.x, fma(-c0.y, x.y, y0));
+                    X1[at] = fma(c1.x, x.x, fma(-c1.y, x.y, y1));
+                    X2[at] = fma(c2.x, x.x, fma(-c2.y, x.y, y2));
+                } else {
+                    X0[at] = y0 + (double)fma(c0.x, x.x, -c0.y * x.y);
+                    X1[at] = y1 + (double)fma(c1.x, x.x, -c1.y * x.y);
+                    X2[at] = y2 + (double)fma(c2.x, x.x, -c2.y * x.y);
+                }
             }
         }
     }
@@ -431,7 +446,8 @@ __global__ void __launch_bounds__(256) adj_point_kernel(long long ng, const long
         const int nfg = gptr[g + 1] - gptr[g];
         const double* xg = sval + (size_t)gs.y * 8;
         const int b0 = bptr[g], b1 = bptr[g + 1];
-        for (long long f = e0; f < e1; ++f) {
+        for (long long f = e; f < e1; ++f) {                         // (gH is symmetric: pairs once)
+            const double twice = f == e ? 1.0 : 2.0;
             const int2 hs = pent[f];
             const int h = hs.x;
             int lo = b0, hi = b1;              // block (g, h) in the sorted block row g
@@ -447,7 +463,7 @@ __global__ void __launch_bounds__(256) adj_point_kernel(long long ng, const long
             for (int a = 0; a < nfg; ++a) {
                 double t = 0.0;
                 for (int c = 0; c < nfh; ++c) t = fma(blk[a * nfh + c], xh[c], t);
-                s = fma(xg[a], t, s);
+                s = fma(twice * xg[a], t, s);
             }
         }
     }
@@ -491,30 +507,47 @@ int adj_sweep_groups(int nwin, int P) {
     return std::max(1, std::min(P, 2 * device_sms() / std::max(nwin, 1)));
 }
 
+template <class R>
+static int launch_sweeps(int nwin, int P, int groups, int batch, int nmax, const int* wins, const int* n_w,
+                         const long long* offC, long long sizeC, const R* K, const double4* coef, const double2* cw,
+                         void* ws, double* Xa, double* Xb, double* Xc, size_t smem_budget, cudaStream_t s) {
+    const size_t smem = sizeof(typename Sweep<R>::C4) * ((size_t)nmax + 1);
+    if (smem > smem_budget) {
+        lres_set_error("adjoint sweeps need %zu B of shared memory", smem);
+        return LRES_EINVAL;
+    }
+    int per_sm = 0;
+    if (int rc = prepare_kernel<adj_sweep_kernel<R>>(kSweepNT, smem, &per_sm)) return rc;
+    for (int w0 = 0; w0 < nwin; w0 += batch) {
+        adj_sweep_kernel<R><<<(unsigned)std::min(batch, nwin - w0) * groups, kSweepNT, smem, s>>>(
+            wins + w0, P, groups, n_w, offC, sizeC, K, coef, nmax, cw, static_cast<typename Sweep<R>::C2*>(ws),
+            2LL * nmax * nmax, Xa, Xb, Xc);
+        LRES_CUDA_TRY(cudaGetLastError());
+    }
+    return LRES_OK;
+}
+
 int adj_tri(int nwin, int P, int groups, int batch, int nmax, const int* wins, const int* n_w, const long long* offN,
             const long long* offC, long long sizeC, const double* d, const double* e, const double2* shifts,
-            const double2* cw, const double* K, double4* coef, double2* ws, double* X, double* A0, double* A1,
-            double* A2, size_t smem_budget, cudaStream_t s) {
+            const double2* cw, const double* K, const float* K32, double4* coef, void* ws, double* X, double* A0,
+            double* A1, double* A2, size_t smem_budget, cudaStream_t s) {
     if (!nwin) return LRES_OK;
-    const size_t smem = sizeof(double4) * ((size_t)nmax + 1);
-    if (smem > smem_budget || nwin > 65535) {
-        lres_set_error("adjoint sweeps: windows of %d functions (%zu B of shared memory), %d windows", nmax, smem, nwin);
+    if (nwin > 65535) {
+        lres_set_error("adjoint supports at most 65535 windows (got %d)", nwin);
         return LRES_EINVAL;
     }
     adj_pivot_kernel<<<(unsigned)(((long long)nwin * P + 31) / 32), 32, 0, s>>>(nwin, P, n_w, offN, d, e, shifts, nmax,
                                                                                coef);
     LRES_CUDA_TRY(cudaGetLastError());
-    int per_sm = 0;
-    if (int rc = prepare_kernel<adj_sweep_kernel>(kSweepNT, smem, &per_sm)) return rc;
     // one group accumulates in place
     double* const Xa = groups > 1 ? X : A0;
     double* const Xb = groups > 1 ? Xa + (size_t)groups * sizeC : A1;
     double* const Xc = groups > 1 ? Xb + (size_t)groups * sizeC : A2;
-    for (int w0 = 0; w0 < nwin; w0 += batch) {
-        adj_sweep_kernel<<<(unsigned)std::min(batch, nwin - w0) * groups, kSweepNT, smem, s>>>(
-            wins + w0, P, groups, n_w, offC, sizeC, K, coef, nmax, cw, ws, 2LL * nmax * nmax, Xa, Xb, Xc);
-        LRES_CUDA_TRY(cudaGetLastError());
-    }
+    if (int rc = K32 ? launch_sweeps<float>(nwin, P, groups, batch, nmax, wins, n_w, offC, sizeC, K32, coef, cw, ws, Xa,
+                                            Xb, Xc, smem_budget, s)
+                     : launch_sweeps<double>(nwin, P, groups, batch, nmax, wins, n_w, offC, sizeC, K, coef, cw, ws, Xa,
+                                             Xb, Xc, smem_budget, s))
+        return rc;
     const int T = (nmax + 31) / 32;
     adj_groups_kernel<<<dim3(T, T, nwin), 256, 0, s>>>(groups, n_w, offC, sizeC, Xa, Xb, Xc, A0, A1, A2);
     LRES_CUDA_TRY(cudaGetLastError());

@@ -137,6 +137,19 @@ struct lres_ctx {
     bool k_ready = false;
     OzRows ozr;                                  // rows through the reflectors on the tensor cores (FP64)
     OzRowSet oz_own, oz_trc, oz_adj;
+    // FP64 tridiagonal form of the mixed adjoint (on its first use): reflectors, T, its standard form and
+    // then W = L^-T Q, K = W^T (F^T F) W, FP64 nodes
+    struct AdjTri {
+        double *A = nullptr, *d = nullptr, *e = nullptr, *tau = nullptr, *H = nullptr, *K = nullptr;
+        double2* shifts = nullptr;
+        bool tried = false;
+        bool ok() const { return shifts != nullptr; }
+        void release() {
+            for (void* q : {(void*)A, (void*)d, (void*)e, (void*)tau, (void*)H, (void*)K, (void*)shifts})
+                if (q) cudaFree(q);
+            *this = AdjTri{};
+        }
+    } at;
     // density passes through P (FP64): V = Y P in batches of windows
     bool by_matrix = false;
     double* d_V = nullptr;
@@ -210,6 +223,7 @@ lres_ctx::~lres_ctx() {
     oz_own.release();
     oz_trc.release();
     oz_adj.release();
+    at.release();
     if (fft) fft3_destroy(fft);
     for (cudaEvent_t e : ev)
         if (e) cudaEventDestroy(e);
@@ -801,6 +815,13 @@ int tri_run_pass(lres_ctx* c, bool trace, cudaStream_t s) {
     return LRES_OK;
 }
 
+// C_w = R_w^T R_w of owned or trace rows R (m x n).
+int gram_product(lres_ctx* c, const double* R, bool trace, double* C, cudaStream_t s) {
+    const long long* off = trace ? c->d_offFT : c->d_offF;
+    return oz_gemm(c->oz, c->nwin, c->nmax, c->nmax, trace ? c->mmaxT : c->mmax, c->d_n, c->d_n, trace ? c->d_mT : c->d_m,
+                   R, off, OzForm(true), R, off, OzForm(true), C, c->d_offC, 0, false, c->smem_budget, s);
+}
+
 // Trials of the chemical potential need no rows when K = Y^T Y is there (FP64).
 bool counts_from_k(const lres_ctx* c) { return c->route == LRES_ROUTE_TRIDIAG && c->precision == LRES_FP64; }
 
@@ -809,8 +830,7 @@ int ensure_k(lres_ctx* c, cudaStream_t s) {
     if (c->k_ready) return LRES_OK;
     if (!c->d_K) TRY(dalloc(&c->d_K, c->sizeC));
     const bool tr = c->have_trace;
-    TRY(batched_gram(c->nwin, c->d_n, tr ? c->d_mT : c->d_m, tr ? c->d_offFT : c->d_offF, c->d_offC, c->nmax,
-                     static_cast<const double*>(tr ? c->d_Ytr : c->d_Yown), c->d_K, s));
+    TRY(gram_product(c, static_cast<const double*>(tr ? c->d_Ytr : c->d_Yown), tr, c->d_K, s));
     c->k_ready = true;
     return LRES_OK;
 }
@@ -2019,31 +2039,96 @@ int adj_workspace(lres_ctx* c, size_t least, size_t want, size_t* got) {
     return LRES_OK;
 }
 
-// The accumulations of the adjoint from the tridiagonal form (FP64): N, E_band and the density by the
-// pass, A_c in the tridiagonal basis into d_adjA, W = L^-T Q in place of the standard form (which the
-// reduction has consumed).
-int adj_tri_accumulate(lres_ctx* c, cudaStream_t s) {
+// Buffers of the mixed adjoint's FP64 tridiagonal form; false (once and for all) if they do not fit, the
+// adjoint then factors every (window, pole).
+bool adj_tri_buffers(lres_ctx* c, cudaStream_t s) {
+    lres_ctx::AdjTri& a = c->at;
+    if (a.tried) return a.ok();
+    a.tried = true;
+    TriPick pk;
+    int rc = tri_pick(false, c->nmax, c->smem_budget, 0, &pk);
+    if (!rc) rc = dalloc(&a.A, c->sizeA);
+    if (!rc) rc = dalloc(&a.d, c->sizeN);
+    if (!rc) rc = dalloc(&a.e, c->sizeN);
+    if (!rc) rc = dalloc(&a.tau, c->sizeN);
+    if (!rc) rc = dalloc(&a.H, c->sizeC);
+    if (!rc) rc = dalloc(&a.K, c->sizeC);
+    if (!rc) rc = oz_setup(c, s);
+    if (!rc) rc = oz_setup_rows(c, c->n_w, c->oz_adj, s);
+    if (!rc) rc = dalloc(&a.shifts, c->npoles);
+    if (rc) {
+        cudaGetLastError();
+        a.release();
+        c->ozr.release();
+        c->oz_adj.release();
+        a.tried = true;
+    }
+    return a.ok();
+}
+
+// The accumulations of the adjoint from the FP64 tridiagonal form: per-window N and E_band, the density by
+// the pass, A_c in the tridiagonal basis into d_adjA, W = L^-T Q in *Wt (over the standard form, which the
+// reduction has consumed).  In mixed precision the tridiagonal form is made here (d_HW and L^-T are FP64)
+// and the sweeps run in FP32: 128 windows 89 -> 45 ms, the gradients 1.8e-6 off 64 bits against the
+// 2.2e-6 of FP32 factors.
+int adj_tri_accumulate(lres_ctx* c, double mu, double e_lo, const double** Wt, cudaStream_t s) {
+    const bool mixed = c->precision == LRES_MIXED;
     if (!c->tri_ready) TRY(tri_refresh(c, s));
     const int P = c->npoles;
     const int groups = adj_sweep_groups(c->nwin, P);
     const size_t coefb = sizeof(double4) * (size_t)c->nwin * P * c->nmax;
+    const size_t trb = sizeof(double2) * (size_t)c->nwin * P;
+    const size_t k32b = mixed ? (sizeof(float) * (size_t)c->sizeC + 15) / 16 * 16 : 0;
     const size_t xb = groups > 1 ? sizeof(double) * 3 * (size_t)groups * c->sizeC : 0;
-    const size_t perw = sizeof(double2) * 2 * (size_t)c->nmax * c->nmax * groups;
+    const size_t perw = (mixed ? sizeof(float2) : sizeof(double2)) * 2 * (size_t)c->nmax * c->nmax * groups;
+    const size_t head = coefb + trb + k32b + xb;
     size_t got = 0;
-    TRY(adj_workspace(c, coefb + xb + perw, coefb + xb + perw * c->nwin, &got));
-    const int batch = (int)std::min<size_t>(c->nwin, (got - coefb - xb) / perw);
+    TRY(adj_workspace(c, head + perw, head + perw * c->nwin, &got));
+    const int batch = (int)std::min<size_t>(c->nwin, (got - head) / perw);
     char* const base = static_cast<char*>(c->d_adjws);
     double4* const coef = reinterpret_cast<double4*>(base);
-    double* const X = reinterpret_cast<double*>(base + coefb);
-    double2* const ws = reinterpret_cast<double2*>(base + coefb + xb);
-    TRY(tri_any_pass(c, false, c->have_trace, s));
-    TRY(ensure_k(c, s));
-    if (!c->oz_adj.offS) TRY(oz_setup_rows(c, c->n_w, c->oz_adj, s));
-    TRY(rows_fp64(c, c->oz_adj, c->d_n, c->d_LinvT, c->sizeC, c->d_Hhat, s));
-    return adj_tri(c->nwin, P, groups, batch, c->nmax, c->d_order, c->d_n, c->d_offN, c->d_offC, c->sizeC,
-                   static_cast<const double*>(c->d_trid), static_cast<const double*>(c->d_trie),
-                   static_cast<const double2*>(c->d_shifts), c->d_cw, c->d_K, coef, ws, X, c->d_adjA[0],
-                   c->d_adjA[1], c->d_adjA[2], c->smem_budget, s);
+    double2* const trace = reinterpret_cast<double2*>(base + coefb);
+    float* const K32 = mixed ? reinterpret_cast<float*>(base + coefb + trb) : nullptr;
+    double* const X = reinterpret_cast<double*>(base + coefb + trb + k32b);
+    void* const ws = base + head;
+    const double2* shifts = static_cast<const double2*>(c->d_shifts);
+    const double *d = static_cast<const double*>(c->d_trid), *e = static_cast<const double*>(c->d_trie);
+    double *W = c->d_Hhat, *K = c->d_K;
+    if (!mixed || !c->have_trace) TRY(tri_any_pass(c, false, c->have_trace, s));   // (trace rows: no density)
+    if (!mixed) {
+        TRY(ensure_k(c, s));
+        K = c->d_K;
+        if (!c->oz_adj.offS) TRY(oz_setup_rows(c, c->n_w, c->oz_adj, s));
+        TRY(rows_fp64(c, c->oz_adj, c->d_n, c->d_LinvT, c->sizeC, W, s));
+    } else {
+        lres_ctx::AdjTri& a = c->at;
+        TriPick pk;
+        TRY(tri_pick(false, c->nmax, c->smem_budget, 0, &pk));
+        poles_kernel<<<(P + 63) / 64, 64, 0, s>>>(P, c->M, mu, e_lo, 0, a.shifts, c->d_wq, c->d_wzq);
+        LRES_CUDA_TRY(cudaGetLastError());
+        TRY(square_gemm(c, c->d_HW, false, c->d_LinvT, true, a.A, 1, s));
+        TRY(square_gemm(c, c->d_LinvT, true, a.A, true, a.H, 2, s));
+        TRY(tri_reduce(false, c->nwin, c->d_order_w, c->d_counter, c->d_n, c->d_offC, c->d_offA, c->d_offN, a.H, a.A, a.d,
+                       a.e, a.tau, c->d_status, pk, c->nmax, c->smem_budget, s));
+        TRY(oz_tfactors(c->oz, c->ozr, c->nwin, c->nmax, c->d_n, a.A, a.tau, c->d_offN, c->smem_budget, s));
+        LRES_CUDA_TRY(cudaMemcpyAsync(a.H, c->d_LinvT, sizeof(double) * c->sizeC, cudaMemcpyDeviceToDevice, s));
+        TRY(oz_rows(c->oz, c->ozr, c->oz_adj, c->nwin, c->nmax, c->d_n, c->d_n, a.A, a.H, c->smem_budget, s));
+        // K = W^T (F^T F) W
+        TRY(gram_product(c, c->have_trace ? c->d_FT : c->d_F, c->have_trace, a.K, s));
+        TRY(square_gemm(c, a.K, false, a.H, true, c->d_adjA[0], 0, s));
+        TRY(square_gemm(c, a.H, true, c->d_adjA[0], true, a.K, 0, s));
+        TRY(tri_count(c->nwin, P, c->nmax, c->d_n, c->d_offN, c->d_offC, a.d, a.e, a.K, a.shifts, c->d_wq, c->d_wzq, c->dV,
+                      coef, trace, c->d_nw, c->d_ew, c->d_status, c->smem_budget, s));
+        TRY(convert_f64_f32(a.K, K32, c->sizeC, s));
+        shifts = a.shifts;
+        d = a.d;
+        e = a.e;
+        W = a.H;
+        K = a.K;
+    }
+    *Wt = W;
+    return adj_tri(c->nwin, P, groups, batch, c->nmax, c->d_order, c->d_n, c->d_offN, c->d_offC, c->sizeC, d, e, shifts,
+                   c->d_cw, K, K32, coef, ws, X, c->d_adjA[0], c->d_adjA[1], c->d_adjA[2], c->smem_budget, s);
 }
 
 // The same by the LDL^T of every (window, pole), factors kept, in batches of whole windows.
@@ -2120,7 +2205,7 @@ extern "C" int lres_adjoint(lres_ctx* c, double mu, double e_lo, double* dv, int
     }
     cudaStream_t s = (cudaStream_t)stream;
     const bool mixed = c->precision == LRES_MIXED;
-    const bool tri = !mixed && c->route == LRES_ROUTE_TRIDIAG;
+    const bool tri = c->route == LRES_ROUTE_TRIDIAG && (!mixed || adj_tri_buffers(c, s));
     const int P = c->npoles;
     if (!tri) TRY(ensure_hhat_df(c, s));       // the LDL^T path factors the double-float standard form
     TRY(adj_prepare(c, s));
@@ -2129,8 +2214,8 @@ extern "C" int lres_adjoint(lres_ctx* c, double mu, double e_lo, double* dv, int
     TRY(adj_weights(P, c->M, mu, e_lo, c->d_cw, s));
     LRES_CUDA_TRY(cudaMemsetAsync(c->d_status, 0, sizeof(int), s));
     // the accumulations are in the basis of Wt: A_c = Wt X_c Wt^T (null: the windows' own)
-    const double* const Wt = tri ? c->d_Hhat : mixed ? c->d_LinvT : nullptr;
-    if (tri) TRY(adj_tri_accumulate(c, s));
+    const double* Wt = mixed ? c->d_LinvT : nullptr;
+    if (tri) TRY(adj_tri_accumulate(c, mu, e_lo, &Wt, s));
     else TRY(adj_ldl_accumulate(c, s));
     TRY(adj_inner(c->nwin, c->d_n, c->d_offC, Wt ? nullptr : c->d_SW, c->d_adjA[0], c->d_adjA[1], c->d_adjA[2],
                   c->d_adju, s));

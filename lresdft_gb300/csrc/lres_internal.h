@@ -214,12 +214,13 @@ int adj_accumulate(bool fp32, const int* wins, int nwin_batch, int P, int nmax, 
                    const long long* offC, const void* ws, long long ws_stride, const double2* cw, double* A0,
                    double* A1, double* A2, cudaStream_t s);
 // A_c in the tridiagonal basis, X_c = Re sum_k c_k G_k K G_k, in batches of windows: coef nwin * P * nmax,
-// ws batch * groups * 2 nmax^2, X 3 * groups * sizeC elements (unused with one group)
+// ws batch * groups * 2 nmax^2 complex values, X 3 * groups * sizeC elements (unused with one group); with
+// K32 the sweeps run in FP32
 int adj_sweep_groups(int nwin, int P);
 int adj_tri(int nwin, int P, int groups, int batch, int nmax, const int* wins, const int* n_w, const long long* offN,
             const long long* offC, long long sizeC, const double* d, const double* e, const double2* shifts,
-            const double2* cw, const double* K, double4* coef, double2* ws, double* X, double* A0, double* A1,
-            double* A2, size_t smem_budget, cudaStream_t s);
+            const double2* cw, const double* K, const float* K32, double4* coef, void* ws, double* X, double* A0,
+            double* A1, double* A2, size_t smem_budget, cudaStream_t s);
 int adj_weights(int P, int M, double mu, double e_lo, double2* cw, cudaStream_t s);
 int adj_inner(int nwin, const int* n_w, const long long* offC, const double* S, const double* A0, const double* A1,
               const double* A2, double* u, cudaStream_t s);
