@@ -31,6 +31,8 @@ namespace {
 constexpr int kDig = 9;                       // digits of an operand
 constexpr int kBits = 7;                      // bits of a digit
 constexpr int kTop = kBits * (kDig - 1) + 5 - 52;    // bits below FP64's last of a row's largest value
+constexpr unsigned long long bias_of(int digits) { return digits ? 64ull << (7 * (digits - 1)) | bias_of(digits - 1) : 0; }
+constexpr unsigned long long kBias = bias_of(kDig);
 constexpr int kOzT = 64;                      // tile edge
 constexpr int kOzK = 32;                      // terms of a stage
 constexpr int kOzStages = 3;
@@ -112,7 +114,7 @@ __global__ void __launch_bounds__(256) oz_slice_kernel(int w0, Operand o, int Rp
             }
         }
         __syncthreads();
-        unsigned short d[kDig][4];
+        unsigned d[kDig][4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const long long b = __double_as_longlong(tile[r][kq + u]);
@@ -125,17 +127,18 @@ __global__ void __launch_bounds__(256) oz_slice_kernel(int w0, Operand o, int Rp
             else if (sh >= 0) q = m << sh;                           // (sh <= kTop)
             else if (sh > -60) q = (m + (1LL << (-sh - 1))) >> -sh;
             if (b < 0) q = -q;
+            // all digits at once: with 64 added at every place they are the 7-bit fields (the first may
+            // be 128); to float by the exponent of 2^23, exact in bf16
+            const unsigned long long z = (unsigned long long)q + kBias;
 #pragma unroll
-            for (int s = kDig - 1; s >= 0; --s) {
-                const int t = s ? (int)((q + 64) & 127) - 64 : (int)q;
-                q = (q - t) >> kBits;
-                d[s][u] = (unsigned short)(__float_as_uint((float)t) >> 16);    // exact: |t| <= 64
+            for (int s = 0; s < kDig; ++s) {
+                const unsigned t = (unsigned)(z >> (kBits * (kDig - 1 - s))) & (s ? 127u : 255u);
+                d[s][u] = __float_as_uint(__uint_as_float(0x4B000000u | t) - 8388672.0f);   // 2^23 + 64
             }
         }
 #pragma unroll
         for (int s = 0; s < kDig; ++s) {
-            const uint2 v = make_uint2((unsigned)d[s][0] | (unsigned)d[s][1] << 16,
-                                       (unsigned)d[s][2] | (unsigned)d[s][3] << 16);
+            const uint2 v = make_uint2(__byte_perm(d[s][0], d[s][1], 0x7632), __byte_perm(d[s][2], d[s][3], 0x7632));
             *reinterpret_cast<uint2*>(dig + (((size_t)slot * kDig + s) * Rp + r0 + r) * Kp + k0 + kq) = v;
         }
     }
@@ -353,9 +356,12 @@ int oz_gemm(OzWork& wk, int nwin, int mmax, int nmax, int kmax, const int* m_w, 
     const OzPlan p = oz_plan(nwin, mmax, nmax, kmax);
     const int Rp = p.Rp, Cp = p.Cp, Kp = p.Kp, batch = p.batch;
     unsigned short* const da = static_cast<unsigned short*>(wk.buf);
-    unsigned short* const db = da + (size_t)batch * kDig * Rp * Kp;
-    int* const ea = reinterpret_cast<int*>(db + (size_t)batch * kDig * Cp * Kp);
-    int* const eb = ea + (size_t)batch * Rp;
+    // (a Gram product has one operand)
+    const bool same = A == B && offA == offB && m_w == n_w && fa.k_contig == fb.k_contig && fa.ld == fb.ld &&
+                      fa.refl == fb.refl && Rp == Cp;
+    unsigned short* const db = same ? da : da + (size_t)batch * kDig * Rp * Kp;
+    int* const ea = reinterpret_cast<int*>(da + (size_t)batch * kDig * (Rp + Cp) * Kp);
+    int* const eb = same ? ea : ea + (size_t)batch * Rp;
     const bool lng = kmax > kOzRun;
     int per_sm = 0;
     auto launch = [&](auto kern, int w0, int nb) {
@@ -365,7 +371,8 @@ int oz_gemm(OzWork& wk, int nwin, int mmax, int nmax, int kmax, const int* m_w, 
     for (int w0 = 0; w0 < nwin; w0 += batch) {
         const int nb = std::min(batch, nwin - w0);
         oz_slice_kernel<<<dim3(Rp / 32, nb), 256, 0, s>>>(w0, Operand{A, offA, m_w, k_w, fa}, Rp, Kp, da, ea);
-        oz_slice_kernel<<<dim3(Cp / 32, nb), 256, 0, s>>>(w0, Operand{B, offB, n_w, k_w, fb}, Cp, Kp, db, eb);
+        if (!same)
+            oz_slice_kernel<<<dim3(Cp / 32, nb), 256, 0, s>>>(w0, Operand{B, offB, n_w, k_w, fb}, Cp, Kp, db, eb);
         LRES_CUDA_TRY(cudaGetLastError());
 #define OZ_RUN(KL, LG)                                                                  \
     do {                                                                                \
