@@ -77,7 +77,7 @@ __host__ __device__ constexpr int row_ld(int NB) { return 4 * NB + 4; }
 // Shared memory of windows of NB column blocks, in floats.
 inline size_t reg_smem_floats(int NB) {
     const int N = 32 * NB;
-    return (size_t)(8 + 1 + 1 + kRegNW) * N + kRegNW * row_ld(NB) + 64 + (size_t)kRegNT * sh_slots(NB);
+    return (size_t)(8 + 1 + 1 + kRegNW) * N + kRegNW * row_ld(NB) + 64 + kRegNT + (size_t)kRegNT * sh_slots(NB);
 }
 
 __device__ __forceinline__ float warp_sum(float x) {
@@ -89,7 +89,7 @@ __device__ __forceinline__ float warp_sum(float x) {
 // Sums of NR values (rows) over the lanes: halves the rows held at each step, then sums the
 // groups of lanes that hold the same row.  Lane group g (of NR) ends with row rowof(lane).
 template <int NR>
-__device__ __forceinline__ float rows_sum(float (&r)[NR], int lane) {
+__device__ __forceinline__ float rows_sum(float* r, int lane) {
     int o = 16;
 #pragma unroll
     for (int half = NR / 2; half; half >>= 1, o >>= 1) {
@@ -151,10 +151,10 @@ __global__ void __launch_bounds__(kRegNT, 1) tri_reduce_reg_kernel(TriRegParams 
         float* const xr = xs + N;                                   // [8][row_ld] x by rows of a warp
         float* const rowp = xr + kRegNW * row_ld(NB);               // [N] row products of q
         float* const colp = rowp + N;                               // [8][N] column products of q
-        float* const xq = colp + kRegNW * N;                        // [8] x^T A x by warp
-        float* const dots = xq + 8;                                 // [8] (v_l^T x, w_l^T x)
-        float* const pub = dots + 8;                                // alpha = x_{c+1}
-        float* const S = xq + 64 + tid;                             // [slot][256]: this thread's
+        float* const xq = colp + kRegNW * N;                        // [256] x^T A x by thread
+        float* const dots = xq + kRegNT;                            // [8] (v_l^T x, w_l^T x)
+        float* const pub = dots + 8;                                // alpha = x_{c+1}, tau, scal
+        float* const S = dots + 64 + tid;                           // [slot][256]: this thread's
         const int ld = (n + 3) & ~3;
         float* const Aw = p.A + p.offA[w];
         const float* const src = first ? Aw : p.H + p.offC[w];
@@ -373,12 +373,15 @@ __global__ void __launch_bounds__(kRegNT, 1) tri_reduce_reg_kernel(TriRegParams 
             float cpr[kRegBlk];
 #pragma unroll
             for (int b = 0; b < kRegBlk; ++b) cpr[b] = 0.0f;
+            constexpr int NR = SB >= 0 ? 8 * (kRegBlk / 2 - SB / 2) : 8;
+            float rows[NR];
             static_for<(SB > 0 ? SB / 2 : 0), kRegBlk / 2>([&](auto gc) {
                 constexpr int g = decltype(gc)::value;
                 const float* const xw = xr + warp * row_ld(NB) + 4 * B0 + 8 * g;
                 const float4 x4 = *reinterpret_cast<const float4*>(xw), x5 = *reinterpret_cast<const float4*>(xw + 4);
                 const float rx[8] = {x4.x, x4.y, x4.z, x4.w, x5.x, x5.y, x5.z, x5.w};
-                float rp[8];
+                constexpr int R0 = SB >= 0 ? 8 * (g - SB / 2) : 0;
+                float* const rp = rows + R0;
 #pragma unroll
                 for (int r = 0; r < 8; ++r) rp[r] = 0.0f;
                 if constexpr (SB >= 0) {
@@ -419,19 +422,38 @@ __global__ void __launch_bounds__(kRegNT, 1) tri_reduce_reg_kernel(TriRegParams 
                 });
 #pragma unroll
                 for (int r = 0; r < 8; ++r) qx = fmaf(rp[r], rx[r], qx);
-                const float sum = rows_sum<8>(rp, lane);
-                if ((lane & 3) == 0) rowp[32 * B0 + 64 * g + warp + 8 * (lane >> 2)] = sum;
+                if constexpr (SB < 0) {
+                    const float sum = rows_sum<8>(rows, lane);
+                    if ((lane & 3) == 0) rowp[32 * B0 + 64 * g + warp + 8 * (lane >> 2)] = sum;
+                }
             });
+            if constexpr (SB >= 0) {
+                // all rows in one butterfly (its five exchanges are waited for once)
+                float* const dst = rowp + 32 * B0 + 64 * (SB / 2) + warp;
+                if constexpr (NR >= 32) {
+                    dst[8 * lane] = rows_sum<32>(rows, lane);
+                } else if constexpr (NR >= 16) {
+                    const float sum = rows_sum<16>(rows, lane);
+                    if ((lane & 1) == 0) dst[8 * (lane >> 1)] = sum;
+                }
+                if constexpr (NR == 8 || NR == 24) {
+                    const float sum = rows_sum<8>(rows + NR - 8, lane);
+                    if ((lane & 3) == 0) dst[8 * (NR - 8) + 8 * (lane >> 2)] = sum;
+                }
+            }
             static_for<(SB > 0 ? SB : 0), kRegBlk>([&](auto bc) {
                 constexpr int b = decltype(bc)::value;
                 colp[warp * N + 32 * (B0 + b) + lane] = cpr[b];
                 qx = fmaf(cpr[b], xc[b], qx);
             });
-            qx = warp_sum(qx);
-            if (lane == 0) xq[warp] = qx;
+            xq[tid] = qx;
             __syncthreads();
 
             // ---- C
+            // x^T A x: every warp sums the threads' parts (beside the loads below)
+            const float4 xa = *reinterpret_cast<const float4*>(xq + 4 * lane);
+            const float4 xb4 = *reinterpret_cast<const float4*>(xq + 128 + 4 * lane);
+            const float xax = warp_sum(((xa.x + xa.y) + (xa.z + xa.w)) + ((xb4.x + xb4.y) + (xb4.z + xb4.w)));
             const int c1 = c + 1;
             // column c1 at row i: lane c1 % 32 of warp i % 8
             const float* const col = S - tid + (c1 & 31);
@@ -460,8 +482,6 @@ __global__ void __launch_bounds__(kRegNT, 1) tri_reduce_reg_kernel(TriRegParams 
             const float4 f1 = *reinterpret_cast<const float4*>(VW + 4 * c1);
             const float2 h1 = *reinterpret_cast<const float2*>(VW + 4 * (N + c1));
             float p1[6] = {f1.x, f1.y, f1.z, f1.w, h1.x, h1.y};     // (v_l, w_l) of row c1
-            const float4 xa = *reinterpret_cast<const float4*>(xq), xb4 = *reinterpret_cast<const float4*>(xq + 4);
-            const float xax = ((xa.x + xa.y) + (xa.z + xa.w)) + ((xb4.x + xb4.y) + (xb4.z + xb4.w));
             float y1 = fmaf(scal, q1, a1);
             float s = a1 + scal * (2.0f * q1 + scal * xax);
             float DV[3], DW[3];                                     // V^T v, W^T v
