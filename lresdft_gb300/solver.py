@@ -421,44 +421,53 @@ class LResGPU:
         self.trace_rows = None
 
     def solve_mu_fixed_n(self, N=None, mu0=None, tol=1e-10, maxiter=60):
-        """mu with |N(mu) - N| <= tol (absolute) on the current Hamiltonian, e_lo fixed: a
-        bracket grown from mu0 (default: the current mu) by steps of the stored slope, then
-        Brent's method, on passes without density.  Returns (mu, N(mu), E_band(mu))."""
+        """mu with |N(mu) - N| <= tol (absolute) on the current Hamiltonian, e_lo fixed: from mu0
+        (default: the current mu) a step with the slope dN/dmu of the last solve, secant steps until
+        the count changes sign, then Brent's method, on passes without density (54 windows from
+        0.02 Ha away: 19 passes with steps that doubled, 8 to 13 this way).  Returns (mu, N(mu),
+        E_band(mu))."""
         N = self.b.cr.n_elec if N is None else N
         mu = self.mu if mu0 is None else mu0
         if mu is None or self.e_lo is None:
             raise RuntimeError("solve_mu_fixed_n needs (mu, e_lo): call density() first or set them")
         lo_bound = self.e_lo + 1e-6
         mu = max(mu, lo_bound + 1e-6)
-        cache = {}
+        cache, hist = {}, []
 
         def f(x):
             _, n, e = self.pole_pass(x, self.e_lo, want_density=False)
             cache[x] = (n, e)
+            hist.append((x, n - N))
             return n - N
+
+        def found(x):
+            self._note_slope(hist, x)
+            return x, cache[x][0], cache[x][1]
 
         f0 = f(mu)
         if abs(f0) <= tol:
             return mu, cache[mu][0], cache[mu][1]
         slope = self._slope if self._slope and self._slope > 0 else max(N, 1.0)
-        step = min(max(abs(f0) / slope, 1e-6), 0.1)
+        step = math.copysign(min(max(abs(f0) / slope, 1e-6), 0.1), -f0)
         a, fa = mu, f0
         for _ in range(maxiter):
-            x = a - step if fa > 0 else a + step
+            x = a + step
             if x <= lo_bound:
                 x = 0.5 * (a + lo_bound)
             fx = f(x)
             if abs(fx) <= tol:
-                return x, cache[x][0], cache[x][1]
+                return found(x)
             if (fx > 0) != (fa > 0):
                 b, fb = x, fx
                 break
+            # secant step, 10% past its root so that the next point brackets; at least twice the last
+            # step where the count hardly moved
+            sec = -fx * (x - a) / (fx - fa) if fx != fa else 2 * step
+            step = math.copysign(min(1.1 * abs(sec) if abs(sec) > 0 else 2 * abs(step), 0.5), step)
             a, fa = x, fx
-            step *= 2.0
         else:
             raise RuntimeError("solve_mu_fixed_n: no sign change of N(mu) - N")
-        x = self._brent(f, a, fa, b, fb, tol, xtol=1e-15, maxit=maxiter)
-        return x, cache[x][0], cache[x][1]
+        return found(self._brent(f, a, fa, b, fb, tol, xtol=1e-15, maxit=maxiter))
 
     def set_hamiltonian(self, H):
         Hp, Hi, Hv = csr64(H)
