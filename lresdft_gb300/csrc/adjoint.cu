@@ -200,8 +200,8 @@ __global__ void __launch_bounds__(256) adj_accum_kernel(const int* wins, int P, 
 // so a pole costs two tridiagonal solves with n right-hand sides instead of a dense
 // factorisation and m back-substitutions: ~23 n^2 FP64 multiply-adds against
 // 4 (n^3 / 3 + 3 m n^2).  The FP64 pipe bounds it (54 windows x 32 poles: 6.6 ms at 1.6
-// multiply-adds per clock and SM; measured 9.2 ms; forward and backward of 54 windows together
-// 626 -> 168 ms).
+// multiply-adds per clock and SM; measured 7.9 ms, 9.2 without the loads ahead of the chain; in FP32, 128
+// windows, 6.9 ms, 14.8 without).
 // ---------------------------------------------------------------------------
 
 // Per (window, pole): the multipliers t_i = e_{i-1} / D_{i-1} and 1 / D_i of the LDL^T of z_k - T
@@ -239,7 +239,7 @@ template <> struct Sweep<float> { using C2 = float2; using C4 = float4; };
 // One CTA per (window, group of poles): X_c += Re c_k G_k K G_k over its poles, the upper triangle of
 // group g at Xc[g * sizeC + offC + i + j n], i <= j.  Thread = column of K for G_k K, then row of it for
 // the second solve (whose back substitution stops at the diagonal); every access but the reads of the
-// second forward sweep runs along the threads.  R = float (mixed precision): the sweeps in FP32 from the
+// second forward sweep runs along the threads, and CH steps are loaded ahead of the chain.  R = float (mixed precision): the sweeps in FP32 from the
 // FP64 pivots, the poles still summed in FP64.
 template <class R>
 __global__ void __launch_bounds__(kSweepNT) adj_sweep_kernel(const int* wins, int P, int groups, const int* n_w,
@@ -249,6 +249,7 @@ __global__ void __launch_bounds__(kSweepNT) adj_sweep_kernel(const int* wins, in
                                                              double* Xb, double* Xc) {
     using C2 = typename Sweep<R>::C2;
     using C4 = typename Sweep<R>::C4;
+    constexpr int CH = 8;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C4* const cf = reinterpret_cast<C4*>(smem_raw);                 // [n + 1]
     const int w = wins[blockIdx.x / groups], grp = blockIdx.x % groups;
@@ -265,20 +266,31 @@ __global__ void __launch_bounds__(kSweepNT) adj_sweep_kernel(const int* wins, in
         __syncthreads();
         for (int j = tid; j < n; j += kSweepNT) {
             C2 u = C2{R(0), R(0)};
-#pragma unroll 4
-            for (int i = 0; i < n; ++i) {
-                const C4 c = cf[i];
-                u = C2{fma(c.x, u.x, fma(-c.y, u.y, Kw[j + (long long)i * n])), fma(c.x, u.y, c.y * u.x)};
-                B[j + (long long)i * n] = u;
+            for (int i0 = 0; i0 < n; i0 += CH) {
+                R kv[CH];
+#pragma unroll
+                for (int q = 0; q < CH; ++q) kv[q] = Kw[j + (long long)min(i0 + q, n - 1) * n];
+#pragma unroll
+                for (int q = 0; q < CH; ++q) {
+                    if (i0 + q >= n) break;
+                    const C4 c = cf[i0 + q];
+                    u = C2{fma(c.x, u.x, fma(-c.y, u.y, kv[q])), fma(c.x, u.y, c.y * u.x)};
+                    B[j + (long long)(i0 + q) * n] = u;
+                }
             }
             C2 x = C2{R(0), R(0)};
-#pragma unroll 4
-            for (int i = n - 1; i >= 0; --i) {
-                const C4 c = cf[i], cn = cf[i + 1];
-                const C2 v = B[j + (long long)i * n];
-                x = C2{fma(v.x, c.z, fma(-v.y, c.w, fma(cn.x, x.x, -cn.y * x.y))),
-                       fma(v.x, c.w, fma(v.y, c.z, fma(cn.x, x.y, cn.y * x.x)))};
-                B[j + (long long)i * n] = x;
+            for (int i1 = n - 1; i1 >= 0; i1 -= CH) {
+                C2 v[CH];
+#pragma unroll
+                for (int q = 0; q < CH; ++q) v[q] = B[j + (long long)max(i1 - q, 0) * n];
+#pragma unroll
+                for (int q = 0; q < CH; ++q) {
+                    if (i1 - q < 0) break;
+                    const C4 c = cf[i1 - q], cn = cf[i1 - q + 1];
+                    x = C2{fma(v[q].x, c.z, fma(-v[q].y, c.w, fma(cn.x, x.x, -cn.y * x.y))),
+                           fma(v[q].x, c.w, fma(v[q].y, c.z, fma(cn.x, x.y, cn.y * x.x)))};
+                    B[j + (long long)(i1 - q) * n] = x;
+                }
             }
         }
         __syncthreads();
@@ -289,30 +301,52 @@ __global__ void __launch_bounds__(kSweepNT) adj_sweep_kernel(const int* wins, in
         double* const X2 = Xc + (size_t)grp * sizeC + offC[w];
         for (int i = tid; i < n; i += kSweepNT) {
             C2 u = C2{R(0), R(0)};
-#pragma unroll 4
-            for (int j = 0; j < n; ++j) {
-                const C4 c = cf[j];
-                const C2 b = B[j + (long long)i * n];
-                u = C2{fma(c.x, u.x, fma(-c.y, u.y, b.x)), fma(c.x, u.y, fma(c.y, u.x, b.y))};
-                if (j >= i) U[i + (long long)j * n] = u;
+            for (int j0 = 0; j0 < n; j0 += CH) {
+                C2 bv[CH];
+#pragma unroll
+                for (int q = 0; q < CH; ++q) bv[q] = B[min(j0 + q, n - 1) + (long long)i * n];
+#pragma unroll
+                for (int q = 0; q < CH; ++q) {
+                    const int j = j0 + q;
+                    if (j >= n) break;
+                    const C4 c = cf[j];
+                    u = C2{fma(c.x, u.x, fma(-c.y, u.y, bv[q].x)), fma(c.x, u.y, fma(c.y, u.x, bv[q].y))};
+                    if (j >= i) U[i + (long long)j * n] = u;
+                }
             }
             C2 x = C2{R(0), R(0)};
-#pragma unroll 2
-            for (int j = n - 1; j >= i; --j) {
-                const C4 c = cf[j], cn = cf[j + 1];
-                const long long at = i + (long long)j * n;
-                const C2 v = U[at];
-                x = C2{fma(v.x, c.z, fma(-v.y, c.w, fma(cn.x, x.x, -cn.y * x.y))),
-                       fma(v.x, c.w, fma(v.y, c.z, fma(cn.x, x.y, cn.y * x.x)))};
-                const double y0 = k == k0 ? 0.0 : X0[at], y1 = k == k0 ? 0.0 : X1[at], y2 = k == k0 ? 0.0 : X2[at];
-                if constexpr (sizeof(R) == 8) {
-                    X0[at] = fma(c0.x, x.x, fma(-c0.y, x.y, y0));
-                    X1[at] = fma(c1.x, x.x, fma(-c1.y, x.y, y1));
-                    X2[at] = fma(c2.x, x.x, fma(-c2.y, x.y, y2));
-                } else {
-                    X0[at] = y0 + (double)fma(c0.x, x.x, -c0.y * x.y);
-                    X1[at] = y1 + (double)fma(c1.x, x.x, -c1.y * x.y);
-                    X2[at] = y2 + (double)fma(c2.x, x.x, -c2.y * x.y);
+            constexpr int CX = 4;
+            for (int j1 = n - 1; j1 >= i; j1 -= CX) {
+                C2 v[CX];
+                double y[CX][3];
+#pragma unroll
+                for (int q = 0; q < CX; ++q) {
+                    const long long at = i + (long long)max(j1 - q, i) * n;
+                    v[q] = U[at];
+                    y[q][0] = y[q][1] = y[q][2] = 0.0;
+                    if (k != k0) {
+                        y[q][0] = X0[at];
+                        y[q][1] = X1[at];
+                        y[q][2] = X2[at];
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < CX; ++q) {
+                    const int j = j1 - q;
+                    if (j < i) break;
+                    const C4 c = cf[j], cn = cf[j + 1];
+                    const long long at = i + (long long)j * n;
+                    x = C2{fma(v[q].x, c.z, fma(-v[q].y, c.w, fma(cn.x, x.x, -cn.y * x.y))),
+                           fma(v[q].x, c.w, fma(v[q].y, c.z, fma(cn.x, x.y, cn.y * x.x)))};
+                    if constexpr (sizeof(R) == 8) {
+                        X0[at] = fma(c0.x, x.x, fma(-c0.y, x.y, y[q][0]));
+                        X1[at] = fma(c1.x, x.x, fma(-c1.y, x.y, y[q][1]));
+                        X2[at] = fma(c2.x, x.x, fma(-c2.y, x.y, y[q][2]));
+                    } else {
+                        X0[at] = y[q][0] + (double)fma(c0.x, x.x, -c0.y * x.y);
+                        X1[at] = y[q][1] + (double)fma(c1.x, x.x, -c1.y * x.y);
+                        X2[at] = y[q][2] + (double)fma(c2.x, x.x, -c2.y * x.y);
+                    }
                 }
             }
         }
