@@ -407,42 +407,42 @@ int oz_gemm(OzWork& wk, int nwin, int mmax, int nmax, int kmax, const int* m_w, 
 
 namespace {
 
-constexpr int kTNT = 128;
+constexpr int kTNT = kOzPanel;
 
-// T of one (window, panel) from G = V^T V in its slot: T_ll = tau_l, T[0:l, l] = -tau_l T[0:l, 0:l] G[0:l, l],
-// T in place of G (column-major, zero below the diagonal).  Thread = row of T; the upper triangles packed
-// by columns in shared memory.
-__global__ void __launch_bounds__(kTNT) oz_tfactor_kernel(const int* q_w, const long long* offT, const long long* offN,
-                                                          const double* tau, int j0, double* T) {
+// T of every (window, panel) from G = V^T V in its slot: T_ll = tau_l, T[0:l, l] = -tau_l T[0:l, 0:l] G[0:l, l],
+// T in place of G (column-major, zero below the diagonal).  Thread = row of T, which only it reads; T by
+// columns and G's upper triangle packed by columns in shared memory.  Bound by the FP64 pipe (q^3 / 6
+// multiply-adds, 20 clocks a warp's).
+__global__ void __launch_bounds__(kTNT) oz_tfactor_kernel(int nwin, const int* q_w, const long long* offT,
+                                                          const long long* offN, const double* tau, int qmax, double* T) {
     extern __shared__ __align__(16) unsigned char smem[];
-    double* const Gs = reinterpret_cast<double*>(smem);             // (a, b), a <= b at b (b + 1) / 2 + a
-    const int w = blockIdx.x, q = q_w[w], a = threadIdx.x;
+    double* const Ts = reinterpret_cast<double*>(smem);             // [qmax][kTNT]
+    double* const Gs = Ts + (size_t)qmax * kTNT;                    // (a, b), a <= b at b (b + 1) / 2 + a
+    const int w = blockIdx.x % nwin, p = blockIdx.x / nwin, a = threadIdx.x;
+    const int q = q_w[blockIdx.x];
     if (q < 1) return;
-    double* const Ts = Gs + q * (q + 1) / 2;
-    double* const Tw = T + offT[w];
+    double* const Tw = T + offT[blockIdx.x];
     for (int b = 0; b < q; ++b)
-        for (int i = a; i <= b; i += kTNT) Gs[b * (b + 1) / 2 + i] = Tw[i + (long long)b * q];
+        if (a <= b) Gs[b * (b + 1) / 2 + a] = Tw[a + (long long)b * q];
     __syncthreads();
-    const double* const tw = tau + offN[w] + j0;
+    const double* const tw = tau + offN[w] + p * kOzPanel;
     for (int l = 0; l < q; ++l) {
         const double tl = tw[l];
         const double* const g = Gs + l * (l + 1) / 2;
+        double val = a == l ? tl : 0.0;
         if (a < l) {
             double s[4] = {0.0, 0.0, 0.0, 0.0};
             int b = a;
             for (; b + 3 < l; b += 4)
 #pragma unroll
-                for (int u = 0; u < 4; ++u) s[u] = fma(Ts[(b + u) * (b + u + 1) / 2 + a], g[b + u], s[u]);
-            for (; b < l; ++b) s[0] = fma(Ts[b * (b + 1) / 2 + a], g[b], s[0]);
-            Ts[l * (l + 1) / 2 + a] = -tl * ((s[0] + s[1]) + (s[2] + s[3]));
-        } else if (a == l) {
-            Ts[l * (l + 1) / 2 + a] = tl;
+                for (int u = 0; u < 4; ++u) s[u] = fma(Ts[(b + u) * kTNT + a], g[b + u], s[u]);
+            for (; b < l; ++b) s[0] = fma(Ts[b * kTNT + a], g[b], s[0]);
+            val = -tl * ((s[0] + s[1]) + (s[2] + s[3]));
         }
-        // (row a is read by thread a only)
+        Ts[l * kTNT + a] = val;
     }
-    __syncthreads();
     for (int b = 0; b < q; ++b)
-        if (a < q) Tw[a + (long long)b * q] = a <= b ? Ts[b * (b + 1) / 2 + a] : 0.0;
+        if (a < q) Tw[a + (long long)b * q] = Ts[b * kTNT + a];
 }
 
 }  // namespace
@@ -467,10 +467,13 @@ int oz_tfactors(OzWork& wk, const OzRows& o, int nwin, int nmax, const int* n_w,
         const OzForm v(true, n_w, true);
         if (int rc = oz_gemm(wk, nwin, qm, qm, rm, q, q, r, A, offV, v, A, offV, v, o.T, offT, 0, false, smem_budget, s))
             return rc;
-        const size_t smem = sizeof(double) * (size_t)qm * (qm + 1);
+    }
+    if (o.panels) {
+        const int qm = std::min(kOzPanel, nmax - 2);
+        const size_t smem = sizeof(double) * ((size_t)qm * kTNT + (size_t)qm * (qm + 1) / 2);
         int per_sm = 0;
         if (int rc = prepare_kernel<oz_tfactor_kernel>(kTNT, smem, &per_sm)) return rc;
-        oz_tfactor_kernel<<<nwin, kTNT, smem, s>>>(q, offT, offN, tau, j0, o.T);
+        oz_tfactor_kernel<<<(unsigned)nwin * o.panels, kTNT, smem, s>>>(nwin, o.q, o.offT, offN, tau, qm, o.T);
         LRES_CUDA_TRY(cudaGetLastError());
     }
     return LRES_OK;
