@@ -152,6 +152,7 @@ struct lres_ctx {
     } at;
     // density passes through P (FP64): V = Y P in batches of windows
     bool by_matrix = false;
+    bool no_room_for_k = false;                  // K did not fit: counts over the rows
     double* d_V = nullptr;
     long long* d_offV = nullptr;
     std::vector<int> vbatch;                     // first window of every batch, then nwin
@@ -639,6 +640,10 @@ int oz_setup(lres_ctx* c, cudaStream_t s) {
     TRY(upload(&o.offV, offV, s));
     TRY(upload(&o.offT, offT, s));
     TRY(dalloc(&o.T, size));
+    // the workspace of every product of the context (standard form, rows, P, K, adjoint), so that none
+    // of them replaces it later under a captured pass
+    TRY(oz_reserve(c->oz, c->nwin, std::max(c->mmax, c->nmax), c->nmax, c->nmax));
+    TRY(oz_reserve(c->oz, c->nwin, c->nmax, c->nmax, std::max(c->mmax, c->nmax)));
     LRES_CUDA_TRY(cudaStreamSynchronize(s));     // the host vectors go out of scope
     return LRES_OK;
 }
@@ -661,10 +666,6 @@ int oz_setup_rows(lres_ctx* c, const std::vector<int>& m, OzRowSet& rs, cudaStre
     TRY(upload(&rs.offY, offY, s));
     TRY(dalloc(&rs.S, size));
     TRY(dalloc(&rs.S2, size));
-    // the products' workspace for these sizes
-    const int q = std::min(kOzPanel, std::max(c->nmax - 2, 1));
-    TRY(oz_reserve(c->oz, c->nwin, rs.mmax, q, c->nmax));
-    TRY(oz_reserve(c->oz, c->nwin, rs.mmax, c->nmax, q));
     LRES_CUDA_TRY(cudaStreamSynchronize(s));     // the host vectors go out of scope
     return LRES_OK;
 }
@@ -698,13 +699,13 @@ int tri_setup_matrix(lres_ctx* c, cudaStream_t s) {
     c->vbatch.push_back(c->nwin);
     const int rb = tri_rows_per_item(false, c->npoles);
     c->max_pass_items = (c->mmax + rb - 1) / rb;
-    int nb = 0;
-    for (size_t i = 0; i + 1 < c->vbatch.size(); ++i) nb = std::max(nb, c->vbatch[i + 1] - c->vbatch[i]);
+    if (dalloc(&c->d_V, size) || (!c->d_coef && dalloc(&c->d_coef, (size_t)c->nwin * c->npoles * c->nmax))) {
+        cudaGetLastError();                      // no room: the passes run over the rows
+        cudaFree(c->d_V);
+        c->d_V = nullptr;
+        return LRES_OK;
+    }
     TRY(upload(&c->d_offV, offV, s));
-    TRY(dalloc(&c->d_V, size));
-    TRY(oz_reserve(c->oz, nb, c->mmax, c->nmax, c->nmax));
-    TRY(oz_reserve(c->oz, c->nwin, c->nmax, c->nmax, c->nmax));
-    if (!c->d_coef) TRY(dalloc(&c->d_coef, (size_t)c->nwin * c->npoles * c->nmax));
     LRES_CUDA_TRY(cudaStreamSynchronize(s));     // offV goes out of scope
     c->by_matrix = true;
     return LRES_OK;
@@ -799,15 +800,15 @@ int tri_refresh(lres_ctx* c, cudaStream_t s) {
 }
 
 // The pole pass of the tridiagonal route over one row set (nodes and weights already set):
-// per-window N and E_band into d_nw / d_ew, the density into d_dens for the owned points.
-int tri_run_pass(lres_ctx* c, bool trace, cudaStream_t s) {
+// per-window N and E_band into d_nw / d_ew, the density (unless count) into d_dens for the owned points.
+int tri_run_pass(lres_ctx* c, bool count, bool trace, cudaStream_t s) {
     const bool fp32 = c->precision == LRES_MIXED;
     const lres_ctx::RowItems& ri = trace ? c->ri_tr : c->ri_own;
     TRY(mark(c, 0, 0, s));
     TRY(tri_pass(fp32, ri.npass, ri.pass, c->d_counter, c->d_n, trace ? c->d_mT : c->d_m, c->d_offN,
-                 trace ? c->d_offFT : c->d_offF, trace ? c->d_offQT : c->d_offQ, trace ? nullptr : c->d_Oflat,
+                 trace ? c->d_offFT : c->d_offF, trace ? c->d_offQT : c->d_offQ, trace || count ? nullptr : c->d_Oflat,
                  trace ? c->d_Ytr : c->d_Yown, c->d_trid, c->d_trie, c->npoles, c->d_shifts, c->d_wq, c->d_wzq,
-                 trace ? nullptr : c->d_dens, ri.part, c->d_status, c->tri.ldv, c->smem_budget, s));
+                 trace || count ? nullptr : c->d_dens, ri.part, c->d_status, c->tri.ldv, c->smem_budget, s));
     TRY(mark(c, 0, 1, s));
     TRY(mark(c, 1, 0, s));
     TRY(tri_window_sums(c->nwin, ri.first, ri.count, ri.part, c->dV, c->d_nw, c->d_ew, s));
@@ -822,8 +823,18 @@ int gram_product(lres_ctx* c, const double* R, bool trace, double* C, cudaStream
                    R, off, OzForm(true), R, off, OzForm(true), C, c->d_offC, 0, false, c->smem_budget, s);
 }
 
-// Trials of the chemical potential need no rows when K = Y^T Y is there (FP64).
-bool counts_from_k(const lres_ctx* c) { return c->route == LRES_ROUTE_TRIDIAG && c->precision == LRES_FP64; }
+// Trials of the chemical potential need no rows when K = Y^T Y is there (FP64); where its buffers do
+// not fit, the trials run over the rows.
+bool counts_from_k(lres_ctx* c) {
+    if (c->route != LRES_ROUTE_TRIDIAG || c->precision != LRES_FP64 || c->no_room_for_k) return false;
+    const size_t items = (size_t)c->nwin * c->npoles;
+    if ((c->d_K || !dalloc(&c->d_K, c->sizeC)) && (c->d_coef || !dalloc(&c->d_coef, items * c->nmax)) &&
+        (c->d_tr || !dalloc(&c->d_tr, items)))
+        return true;
+    cudaGetLastError();
+    c->no_room_for_k = true;
+    return false;
+}
 
 // K of the current Hamiltonian, from the trace rows where there are any.
 int ensure_k(lres_ctx* c, cudaStream_t s) {
@@ -838,8 +849,6 @@ int ensure_k(lres_ctx* c, cudaStream_t s) {
 // Per-window N and E_band at the nodes already set, into d_nw / d_ew; the density is left as it is.
 int tri_run_count(lres_ctx* c, cudaStream_t s) {
     const int P = c->npoles;
-    if (!c->d_coef) TRY(dalloc(&c->d_coef, (size_t)c->nwin * P * c->nmax));
-    if (!c->d_tr) TRY(dalloc(&c->d_tr, (size_t)c->nwin * P));
     TRY(ensure_k(c, s));
     TRY(mark(c, 0, 0, s));
     TRY(tri_count(c->nwin, P, c->nmax, c->d_n, c->d_offN, c->d_offC, static_cast<const double*>(c->d_trid),
@@ -877,7 +886,7 @@ int tri_run_matrix(lres_ctx* c, cudaStream_t s) {
 int tri_any_pass(lres_ctx* c, bool count, bool trace, cudaStream_t s) {
     if ((count || trace) && counts_from_k(c)) return tri_run_count(c, s);
     if (!trace && c->by_matrix) return tri_run_matrix(c, s);
-    return tri_run_pass(c, trace, s);
+    return tri_run_pass(c, count && c->precision == LRES_FP64, trace, s);
 }
 
 int find_block(const std::vector<int>& bptr, const std::vector<int>& bcol, int g, int h) {

@@ -110,7 +110,7 @@ struct OzWork {
     size_t bytes = 0;
     void release();
 };
-// Workspace for products of up to these sizes (a call within them allocates nothing).
+// Workspace for products of these sizes; a product whose windows fit one by one allocates nothing.
 int oz_reserve(OzWork& wk, int nwin, int mmax, int nmax, int kmax);
 int oz_gemm(OzWork& wk, int nwin, int mmax, int nmax, int kmax, const int* m_w, const int* n_w, const int* k_w,
             const double* A, const long long* offA, OzForm fa, const double* B, const long long* offB, OzForm fb,

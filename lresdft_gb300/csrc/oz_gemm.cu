@@ -352,9 +352,12 @@ int oz_gemm(OzWork& wk, int nwin, int mmax, int nmax, int kmax, const int* m_w, 
         lres_set_error("tensor-core FP64 product needs %d B of shared memory", kOzSmem);
         return LRES_EINVAL;
     }
-    if (int rc = oz_reserve(wk, nwin, mmax, nmax, kmax)) return rc;
+    // within the workspace that is there (a captured graph keeps its address): it grows only where one
+    // window does not fit
     const OzPlan p = oz_plan(nwin, mmax, nmax, kmax);
-    const int Rp = p.Rp, Cp = p.Cp, Kp = p.Kp, batch = p.batch;
+    if (wk.bytes < p.perw)
+        if (int rc = oz_reserve(wk, nwin, mmax, nmax, kmax)) return rc;
+    const int Rp = p.Rp, Cp = p.Cp, Kp = p.Kp, batch = (int)std::min<size_t>(p.batch, wk.bytes / p.perw);
     unsigned short* const da = static_cast<unsigned short*>(wk.buf);
     // (a Gram product has one operand)
     const bool same = A == B && offA == offB && m_w == n_w && fa.k_contig == fb.k_contig && fa.ld == fb.ld &&
