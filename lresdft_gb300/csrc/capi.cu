@@ -699,7 +699,7 @@ int tri_setup_matrix(lres_ctx* c, cudaStream_t s) {
     c->vbatch.push_back(c->nwin);
     const int rb = tri_rows_per_item(false, c->npoles);
     c->max_pass_items = (c->mmax + rb - 1) / rb;
-    if (dalloc(&c->d_V, size) || (!c->d_coef && dalloc(&c->d_coef, (size_t)c->nwin * c->npoles * c->nmax))) {
+    if (dalloc(&c->d_V, size) || (!c->d_coef && dalloc(&c->d_coef, tri_coef_elems(c->nwin, c->npoles, c->nmax)))) {
         cudaGetLastError();                      // no room: the passes run over the rows
         cudaFree(c->d_V);
         c->d_V = nullptr;
@@ -828,7 +828,7 @@ int gram_product(lres_ctx* c, const double* R, bool trace, double* C, cudaStream
 bool counts_from_k(lres_ctx* c) {
     if (c->route != LRES_ROUTE_TRIDIAG || c->precision != LRES_FP64 || c->no_room_for_k) return false;
     const size_t items = (size_t)c->nwin * c->npoles;
-    if ((c->d_K || !dalloc(&c->d_K, c->sizeC)) && (c->d_coef || !dalloc(&c->d_coef, items * c->nmax)) &&
+    if ((c->d_K || !dalloc(&c->d_K, c->sizeC)) && (c->d_coef || !dalloc(&c->d_coef, tri_coef_elems(c->nwin, c->npoles, c->nmax))) &&
         (c->d_tr || !dalloc(&c->d_tr, items)))
         return true;
     cudaGetLastError();
@@ -2085,7 +2085,7 @@ int adj_tri_accumulate(lres_ctx* c, double mu, double e_lo, const double** Wt, c
     if (!c->tri_ready) TRY(tri_refresh(c, s));
     const int P = c->npoles;
     const int groups = adj_sweep_groups(c->nwin, P);
-    const size_t coefb = sizeof(double4) * (size_t)c->nwin * P * c->nmax;
+    const size_t coefb = sizeof(double4) * tri_coef_elems(c->nwin, P, c->nmax);
     const size_t trb = sizeof(double2) * (size_t)c->nwin * P;
     const size_t k32b = mixed ? (sizeof(float) * (size_t)c->sizeC + 15) / 16 * 16 : 0;
     const size_t xb = groups > 1 ? sizeof(double) * 3 * (size_t)groups * c->sizeC : 0;

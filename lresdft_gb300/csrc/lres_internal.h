@@ -187,7 +187,9 @@ int tri_pass(bool fp32, int nitems, const int4* items, int* counter, const int* 
              const void* Y, const void* d, const void* e, int P, const void* shifts, const double2* wq,
              const double2* wzq, double* dens, double* part, int* status, int ldv, size_t smem_budget,
              cudaStream_t s);
-// N and E_band of every window from K = Y^T Y (FP64): coef nwin * P * nmax, trace nwin * P elements
+// Elements of the coefficients of G_k: (t_i, G_ii) of nwin * P * nmax, then the products of t within blocks.
+inline size_t tri_coef_elems(int nwin, int P, int nmax) { return ((size_t)nwin * P * nmax * 3 + 1) / 2; }
+// N and E_band of every window from K = Y^T Y (FP64): coef tri_coef_elems, trace nwin * P elements
 int tri_count(int nwin, int P, int nmax, const int* n_w, const long long* offN, const long long* offC, const double* d,
               const double* e, const double* K, const double2* shifts, const double2* wq, const double2* wzq,
               double dV, double4* coef, double2* trace, double* nw, double* ew, int* status, size_t smem_budget,

@@ -1355,10 +1355,13 @@ __global__ void __launch_bounds__(NT) tri_pass_kernel(TriPassParams<R> p) {
 // K (n x n, formed once per Hamiltonian).  The upper triangle of G = (z - T)^-1 is
 // G_ij = G_jj t_{i+1} ... t_j (t_i = e_{i-1} / D_{i-1}), so
 //
-//     tr(G K) = sum_j G_jj (K_jj + 2 h_j),  h_j = sum_{i<j} K_ij t_{i+1} ... t_j   (Horner in i):
+//     tr(G K) = sum_j G_jj (K_jj + 2 h_j),  h_j = sum_{i<j} K_ij t_{i+1} ... t_j.
 //
-// 5 FP64 instructions per (pole, i < j), 2.5 n^2 against the 11 m n of the rows.  The FP64 pipe
-// bounds it: 54 windows of 276-300 functions (256 rows) 4.7 -> 1.0 ms per trial.
+// By blocks of 32 rows: with L_i = t_{i+1} ... t_e, e the end of i's block, h_j grows by sum_i K_ij L_i
+// per block (2 FP64 multiply-adds per pole, i and j) and takes the factor of the whole block (L of its first
+// row) from one to the next; Horner in i (5) is left for the diagonal blocks.  1.2 n^2 FP64 instructions a
+// pole against the 11 m n of the rows.  The FP64 pipe bounds it: 54 windows of 276-300 functions (256
+// rows) 4.7 -> 0.61 ms per trial (0.95 ms by Horner alone).
 
 // 1 / x: from the FP32 reciprocal by one third-order step (y (1 + e + e^2), e = 1 - x y), by the
 // division outside its range.
@@ -1371,9 +1374,16 @@ __device__ __forceinline__ double recip_f64(double x) {
     return 1.0 / x;
 }
 
-// Per (window, pole): coef[item * ld + i] = (t_i, G_ii), G_ii = 1 / D_i + t_{i+1}^2 G_{i+1,i+1}.  Two
-// serial chains of n steps, bound by their latency; the second reads what the first stored four
-// steps ahead.
+constexpr int kSemi = 32;                      // rows of a block of G
+
+// The products L_i behind the (t, G) pairs.
+__device__ __forceinline__ const double2* semi_products(const double4* coef, int nitems, int ld) {
+    return reinterpret_cast<const double2*>(coef + (size_t)nitems * ld);
+}
+
+// Per (window, pole): coef[item * ld + i] = (t_i, G_ii), G_ii = 1 / D_i + t_{i+1}^2 G_{i+1,i+1}, and the
+// products L_i = t_{i+1} ... t_e to the end e of i's block.  Two serial chains of n steps, bound by their
+// latency; the second reads what the first stored four steps ahead.
 __global__ void tri_diag_kernel(int nwin, int P, const int* n_w, const long long* offN, const double* __restrict__ d,
                                 const double* __restrict__ e, const double2* z, int ld, double4* coef) {
     const int it = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1394,7 +1404,8 @@ __global__ void tri_diag_kernel(int nwin, int P, const int* n_w, const long long
         out[i] = make_double4(t.x, t.y, g.x, g.y);
         el = ew[i];
     }
-    double2 G = make_double2(0.0, 0.0);
+    double2* const Lo = reinterpret_cast<double2*>(coef + (size_t)nwin * P * ld) + (size_t)it * ld;
+    double2 G = make_double2(0.0, 0.0), L = G;
     double2 tn = make_double2(0.0, 0.0);                             // t_{i+1}
     for (int i1 = n - 1; i1 >= 0; i1 -= 4) {
         double4 c[4];
@@ -1405,6 +1416,9 @@ __global__ void tri_diag_kernel(int nwin, int P, const int* n_w, const long long
             if (i1 - u < 0) break;
             const double2 t2 = make_double2(tn.x * tn.x - tn.y * tn.y, 2.0 * tn.x * tn.y);
             G = make_double2(fma(t2.x, G.x, fma(-t2.y, G.y, c[u].z)), fma(t2.x, G.y, fma(t2.y, G.x, c[u].w)));
+            const bool last = (i1 - u) % kSemi == kSemi - 1;
+            L = last ? tn : make_double2(fma(tn.x, L.x, -tn.y * L.y), fma(tn.x, L.y, tn.y * L.x));
+            Lo[i1 - u] = L;
             tn = make_double2(c[u].x, c[u].y);
             reinterpret_cast<double2*>(out + i1 - u)[1] = G;
         }
@@ -1414,10 +1428,11 @@ __global__ void tri_diag_kernel(int nwin, int P, const int* n_w, const long long
 constexpr int kCountNT = 320, kCountPoles = 4;
 
 // One CTA per (window, 4 poles), thread = column j; the lanes of a warp run over the same i, so that
-// K is read along its rows and t is one broadcast.
+// K is read along its rows and t or L is one broadcast.  A warp's columns lie in one block.
 __global__ void __launch_bounds__(kCountNT) tri_count_kernel(int P, int groups, const int* n_w, const long long* offC,
                                                              const double* K, const double4* coef, int ld,
                                                              double2* trace) {
+    static_assert(kSemi == 32 && kCountNT % 32 == 0, "a warp's columns lie in one block");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double2* const ts = reinterpret_cast<double2*>(smem_raw);       // [n][kCountPoles]
     __shared__ double red[kCountNT / 32];
@@ -1432,15 +1447,39 @@ __global__ void __launch_bounds__(kCountNT) tri_count_kernel(int P, int groups, 
         ts[i * kCountPoles + q] = make_double2(c.x, c.y);
     }
     __syncthreads();
+    const double2* Lq[kCountPoles];
+    const int nitems = (int)(gridDim.x / groups) * P;
     double2 acc[kCountPoles];
 #pragma unroll
-    for (int q = 0; q < kCountPoles; ++q) acc[q] = make_double2(0.0, 0.0);
+    for (int q = 0; q < kCountPoles; ++q) {
+        Lq[q] = semi_products(coef, nitems, ld) + ((size_t)w * P + min(k0 + q, P - 1)) * ld;
+        acc[q] = make_double2(0.0, 0.0);
+    }
     for (int j = tid; j < n; j += kCountNT) {
         double2 h[kCountPoles];
 #pragma unroll
         for (int q = 0; q < kCountPoles; ++q) h[q] = make_double2(0.0, 0.0);
+        const int jb = j / kSemi * kSemi;
+        for (int i0 = 0; i0 < jb; i0 += kSemi) {
+            if (i0) {
+#pragma unroll
+                for (int q = 0; q < kCountPoles; ++q) {
+                    const double2 f = Lq[q][i0];
+                    h[q] = make_double2(fma(f.x, h[q].x, -f.y * h[q].y), fma(f.x, h[q].y, f.y * h[q].x));
+                }
+            }
 #pragma unroll 4
-        for (int i = 0; i < j; ++i) {
+            for (int i = i0; i < i0 + kSemi; ++i) {
+                const double x = Kw[j + (long long)i * n];
+#pragma unroll
+                for (int q = 0; q < kCountPoles; ++q) {
+                    const double2 f = Lq[q][i];
+                    h[q] = make_double2(fma(x, f.x, h[q].x), fma(x, f.y, h[q].y));
+                }
+            }
+        }
+#pragma unroll 4
+        for (int i = jb; i < j; ++i) {
             const double x = Kw[j + (long long)i * n];
 #pragma unroll
             for (int q = 0; q < kCountPoles; ++q) {
@@ -1487,15 +1526,17 @@ __global__ void tri_count_sums_kernel(int nwin, int P, const double2* trace, con
 // ---------------------------------------------------------------------------
 //
 // n(r) = 4 y_r P y_r^T and, since Re sum_k w_k = 0, e(r) = 4 y_r T P y_r^T with P = Re sum_k w_k G_k (n x n,
-// real).  P costs 2.5 n^2 FP64 instructions a pole instead of the rows' 11 m n, and V = Y P is a
+// real).  P costs 1.2 n^2 FP64 instructions a pole instead of the rows' 11 m n, and V = Y P is a
 // dense product for the tensor cores (oz_gemm.cu); what is left per row is two inner products.
-// Measured: 54 windows of 276-300 functions and 256 rows 4.7 -> 2.3 ms, 432 windows 29.4 ->
-// 10.5 ms.
+// Measured: 54 windows of 276-300 functions and 256 rows 4.7 -> 1.6 ms, 432 windows 29.4 ->
+// 8.0 ms.
 
 constexpr int kPmatWarps = 4, kPmatPoles = 8;
 
-// One CTA per (window, 32 columns), lane = column j, the poles dealt to the warps; row i from the
-// diagonal up: G_ij = G_{i+1,j} t_{i+1}.  The warps' sums of 32 rows are joined in shared memory and
+// One CTA per (window, 32 columns), lane = column j, the poles dealt to the warps.  In the diagonal block row
+// by row up, G_ij = G_{i+1,j} t_{i+1} (5 FP64 instructions per pole, row and column); above it
+// G_ij = L_i s_j with s_j = t_{e+1} ... t_j G_jj carried from block to block (2; with 5 throughout: 54 windows
+// 2.39 ms, 432 windows 11.1 ms a pass).  The warps' sums of 32 rows are joined in shared memory and
 // written with their mirror image.
 __global__ void __launch_bounds__(32 * kPmatWarps) tri_pmat_kernel(int P, const int* n_w, const long long* offC,
                                                                    const double4* coef, int ld, const double2* wq,
@@ -1507,14 +1548,18 @@ __global__ void __launch_bounds__(32 * kPmatWarps) tri_pmat_kernel(int P, const 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int j = 32 * b + lane;
     double* const Pw = Pm + offC[w];
+    static_assert(kSemi == 32, "a CTA's columns are a block");
     const double4* const cw = coef + (size_t)w * P * ld;
+    const double2* const lw = semi_products(coef, (int)gridDim.y * P, ld) + (size_t)w * P * ld;
     for (int k0 = 0; k0 < P; k0 += kPmatWarps * kPmatPoles) {
         const double4* cf[kPmatPoles];                              // this warp's poles
+        const double2* lf[kPmatPoles];
         double2 s[kPmatPoles], init[kPmatPoles];
 #pragma unroll
         for (int q = 0; q < kPmatPoles; ++q) {
             const int k = k0 + warp + q * kPmatWarps;
             cf[q] = cw + (size_t)min(k, P - 1) * ld;
+            lf[q] = lw + (size_t)min(k, P - 1) * ld;
             init[q] = s[q] = make_double2(0.0, 0.0);
             if (k < P && j < n) {
                 const double4 g = cf[q][j];
@@ -1523,19 +1568,39 @@ __global__ void __launch_bounds__(32 * kPmatWarps) tri_pmat_kernel(int P, const 
             }
         }
         for (int ib = b; ib >= 0; --ib) {
-#pragma unroll 2
-            for (int r = 31; r >= 0; --r) {
-                const int i = 32 * ib + r;
-                if (i >= n) continue;                               // (the same for every lane)
-                double sum = 0.0;
+            if (ib < b) {
+#pragma unroll 4
+                for (int r = 0; r < 32; ++r) {
+                    double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+                    for (int q = 0; q < kPmatPoles; ++q) {
+                        const double2 f = lf[q][32 * ib + r];
+                        s0 = fma(f.x, s[q].x, s0);
+                        s1 = fma(f.y, s[q].y, s1);
+                    }
+                    part[warp][r][lane] = s0 - s1;
+                }
 #pragma unroll
                 for (int q = 0; q < kPmatPoles; ++q) {
-                    if (i == j) s[q] = init[q];
-                    sum += s[q].x;
-                    const double2 t = *reinterpret_cast<const double2*>(cf[q] + i);
-                    s[q] = make_double2(fma(t.x, s[q].x, -t.y * s[q].y), fma(t.x, s[q].y, t.y * s[q].x));
+                    const double2 f = lf[q][32 * ib];
+                    s[q] = make_double2(fma(f.x, s[q].x, -f.y * s[q].y), fma(f.x, s[q].y, f.y * s[q].x));
                 }
-                part[warp][r][lane] = sum;                          // (zero above the diagonal: s is zero there)
+            } else {
+#pragma unroll 2
+                for (int r = 31; r >= 0; --r) {
+                    const int i = 32 * ib + r;
+                    if (i >= n) continue;                           // (the same for every lane)
+                    double sum = 0.0;
+#pragma unroll
+                    for (int q = 0; q < kPmatPoles; ++q) {
+                        if (i == j) s[q] = init[q];
+                        sum += s[q].x;
+                        if (r == 0) continue;                       // (s stays G_ij of the block's first row)
+                        const double2 t = *reinterpret_cast<const double2*>(cf[q] + i);
+                        s[q] = make_double2(fma(t.x, s[q].x, -t.y * s[q].y), fma(t.x, s[q].y, t.y * s[q].x));
+                    }
+                    part[warp][r][lane] = sum;                      // (zero below the diagonal: s is zero there)
+                }
             }
             __syncthreads();
             for (int r = warp; r < 32; r += kPmatWarps) {
