@@ -1383,7 +1383,9 @@ __device__ __forceinline__ const double2* semi_products(const double4* coef, int
 
 // Per (window, pole): coef[item * ld + i] = (t_i, G_ii), G_ii = 1 / D_i + t_{i+1}^2 G_{i+1,i+1}, and the
 // products L_i = t_{i+1} ... t_e to the end e of i's block.  Two serial chains of n steps, bound by their
-// latency; the second reads what the first stored four steps ahead.
+// latency and the issue of FP64 instructions (27 a step, 80 clocks each on a quarter of an SM: a form with one reciprocal
+// per two steps, 32 instructions for 28, measured 8 % slower); the second reads what the first stored four
+// steps ahead.
 __global__ void tri_diag_kernel(int nwin, int P, const int* n_w, const long long* offN, const double* __restrict__ d,
                                 const double* __restrict__ e, const double2* z, int ld, double4* coef) {
     const int it = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1425,10 +1427,11 @@ __global__ void tri_diag_kernel(int nwin, int P, const int* n_w, const long long
     }
 }
 
-constexpr int kCountNT = 320, kCountPoles = 4;
+constexpr int kCountNT = 320;
 
-// One CTA per (window, 4 poles), thread = column j; the lanes of a warp run over the same i, so that
+// One CTA per (window, kCountPoles poles), thread = column j; the lanes of a warp run over the same i, so that
 // K is read along its rows and t or L is one broadcast.  A warp's columns lie in one block.
+template <int kCountPoles>
 __global__ void __launch_bounds__(kCountNT) tri_count_kernel(int P, int groups, const int* n_w, const long long* offC,
                                                              const double* K, const double4* coef, int ld,
                                                              double2* trace) {
@@ -1993,7 +1996,10 @@ int tri_count(int nwin, int P, int nmax, const int* n_w, const long long* offN, 
               double dV, double4* coef, double2* trace, double* nw, double* ew, int* status, size_t smem_budget,
               cudaStream_t s) {
     if (!nwin) return LRES_OK;
-    const size_t smem = sizeof(double2) * kCountPoles * (size_t)nmax;
+    // four poles a CTA share the reads of K and the broadcasts; one where that leaves SMs without a CTA (one
+    // window of 96 functions, 32 poles: 85 -> COUNT1 us)
+    const int np = (long long)nwin * ((P + 3) / 4) < device_sms() ? 1 : 4;
+    const size_t smem = sizeof(double2) * np * (size_t)nmax;
     if (smem > smem_budget) {
         lres_set_error("count pass needs %zu B of shared memory", smem);
         return LRES_EINVAL;
@@ -2002,9 +2008,14 @@ int tri_count(int nwin, int P, int nmax, const int* n_w, const long long* offN, 
                                                                               coef);
     LRES_CUDA_TRY(cudaGetLastError());
     int per_sm = 0;
-    if (int rc = prepare_kernel<tri_count_kernel>(kCountNT, smem, &per_sm)) return rc;
-    const int groups = (P + kCountPoles - 1) / kCountPoles;
-    tri_count_kernel<<<(unsigned)nwin * groups, kCountNT, smem, s>>>(P, groups, n_w, offC, K, coef, nmax, trace);
+    const int groups = (P + np - 1) / np;
+    if (np == 1) {
+        if (int rc = prepare_kernel<tri_count_kernel<1>>(kCountNT, smem, &per_sm)) return rc;
+        tri_count_kernel<1><<<(unsigned)nwin * groups, kCountNT, smem, s>>>(P, groups, n_w, offC, K, coef, nmax, trace);
+    } else {
+        if (int rc = prepare_kernel<tri_count_kernel<4>>(kCountNT, smem, &per_sm)) return rc;
+        tri_count_kernel<4><<<(unsigned)nwin * groups, kCountNT, smem, s>>>(P, groups, n_w, offC, K, coef, nmax, trace);
+    }
     LRES_CUDA_TRY(cudaGetLastError());
     tri_count_sums_kernel<<<(nwin + 63) / 64, 64, 0, s>>>(nwin, P, trace, wq, wzq, dV, nw, ew, status);
     LRES_CUDA_TRY(cudaGetLastError());
