@@ -166,13 +166,20 @@ __device__ __forceinline__ void st_cluster(float* dst, unsigned rank, float x) {
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(x) : "memory");
 }
 
+// In FP64 every warp instruction holds its quarter of the SM for 80 clocks, so nothing is computed twice that
+// one warp can publish: the root and divisions of the reflector run in the last warp beside the others' A x,
+// the sum of p^T v in the warps that own rows only (in every warp, the same bits: a third of the FP64
+// instructions; 54 windows 7.6 -> 5.55 ms, one of 96 functions 1.64 -> 1.03 ms).
+//
 // CL = 2: a cluster of two CTAs per window, for fewer windows than half the SMs (FP64, 54 windows of 276-300
-// functions 9.2 -> 7.6 ms; one window of 96, where the barriers outweigh the work, 1.64 -> 1.84 ms).  Both form the columns, reflectors and vectors (the same bits); the row quads of q = A x and the
+// functions 9.2 -> 7.6 ms, before the above; one window of 96, where the barriers outweigh the work, 1.64 -> 1.84 ms).  Both form the columns, reflectors and vectors (the same bits); the row quads of q = A x and the
 // blocks of the trailing update, which hold the FP64 pipe, are dealt to them, q exchanged through
 // distributed shared memory (two buffers by column parity: the other CTA may be a phase ahead).
 template <class R, int NT, int CL = 1>
 __global__ void __launch_bounds__(NT, reduce_min_ctas(NT, sizeof(R))) tri_reduce_kernel(TriReduceParams<R> p) {
     constexpr int NW = NT / 32;
+    constexpr bool FP64 = sizeof(R) == 8;
+    constexpr int NA = FP64 ? NT - 32 : NT;              // threads of q = A x (FP64: the last warp forms the reflector)
     const int rank = CL > 1 ? (int)cluster_rank() : 0;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int ldv = p.ldv, nb = p.nb;
@@ -187,6 +194,7 @@ __global__ void __launch_bounds__(NT, reduce_min_ctas(NT, sizeof(R))) tri_reduce
     R* const dots = psum + 4 * NT;                       // [64] W^T x, V^T x, x^T x
     R* const red = dots + 64;                            // [NW]
     __shared__ int item_sh;
+    __shared__ R refl[3];                                // beta, tau, 1 / (alpha - beta) of the column
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
     for (;;) {
@@ -273,13 +281,14 @@ __global__ void __launch_bounds__(NT, reduce_min_ctas(NT, sizeof(R))) tri_reduce
                 //     updates of this panel) on the owned rows >= j.  w_{jj-1} at row j is
                 //     p_j - K (v_{jj-1} is 1 there); every thread forms it from the published p.
                 {
-                    const R wlast = jj > 0 ? pv[j] - Kprev : R(0);
                     for (int i = tid; i < n; i += NT) {
                         if (i < j) continue;
+                        const R wlast = jj > 0 ? pv[j] - Kprev : R(0);
                         R c = jj > 0 ? acur[i] : A[i + (long long)j * ld];
                         for (int l = 0; l < jj; ++l) {
                             const R wlj = l == jj - 1 ? wlast : Ws[l * ldv + j];
-                            c -= Vs[l * ldv + i] * wlj + Ws[l * ldv + i] * Vs[l * ldv + j];
+                            if constexpr (FP64) c = fma(-Ws[l * ldv + i], Vs[l * ldv + j], fma(-Vs[l * ldv + i], wlj, c));
+                            else c -= Vs[l * ldv + i] * wlj + Ws[l * ldv + i] * Vs[l * ldv + j];
                         }
                         cv[i] = c;
                     }
@@ -292,14 +301,14 @@ __global__ void __launch_bounds__(NT, reduce_min_ctas(NT, sizeof(R))) tri_reduce
                 const int i0 = (j + 1) & ~3;
                 const int nq = (ld - i0) >> 2;
                 const int nqo = (nq + CL - 1) / CL;             // this CTA's quads: rank, rank + CL, ...
-                const int nsplit = nqo >= NT ? 1 : NT / nqo;
+                const int nsplit = nqo >= NA ? 1 : NA / nqo;
                 R* const qx = qx0 + (j & (CL - 1)) * ldv;
                 auto publish = [&](int i, R x) {
                     qx[i] = x;
                     if constexpr (CL > 1) st_cluster(qx + i, rank ^ 1, x);
                 };
                 {
-                    const int qstep = nqo >= NT ? NT : nqo;
+                    const int qstep = nqo >= NA ? NA : nqo;
                     if (tid < qstep * nsplit) {
                         const int sp = tid / qstep;
                         for (int u = tid % qstep; u < nqo; u += qstep) {
@@ -319,7 +328,7 @@ __global__ void __launch_bounds__(NT, reduce_min_ctas(NT, sizeof(R))) tri_reduce
                                     for (int r = 0; r < 4; ++r) c[r] = fma(x[r], xk, c[r]);
                                 }
 #pragma unroll
-                                for (int r = 0; r < 4; ++r) a[r] += c[r];
+                                for (int r = 0; r < 4; ++r) a[r] = kb == j + 2 + sp ? c[r] : a[r] + c[r];
                             }
                             if (nsplit > 1) {
                                 st4(psum + (sp * nqo + u) * 4, a);   // 16-byte stores: no bank conflicts
@@ -333,14 +342,34 @@ __global__ void __launch_bounds__(NT, reduce_min_ctas(NT, sizeof(R))) tri_reduce
                         }
                     }
                 }
-                //     dots[l] = W_l^T x, dots[jj + l] = V_l^T x, dots[2 jj] = x^T x over rows >= j+2,
-                //     a warp each (the last warps first: they have the fewest row quads)
-                for (int q = NW - 1 - warp; q <= 2 * jj; q += NW) {
-                    const R* X = q < jj ? Ws + (size_t)q * ldv : q < 2 * jj ? Vs + (size_t)(q - jj) * ldv : cv;
+                //     dots[l] = W_l^T x, dots[jj + l] = V_l^T x over rows >= j+2, a warp each; the last warp:
+                //     x^T x and from it the reflector H_j = I - tau v v^T with v_{j+1} = 1 mapping rows j+1..
+                //     of the column onto beta e_{j+1}
+                auto dot = [&](const R* X) {
                     R acc = R(0);
                     for (int i = j + 2 + lane; i < n; i += 32) acc += X[i] * cv[i];
-                    acc = warp_sum(acc);
-                    if (lane == 0) dots[q] = acc;
+                    return warp_sum(acc);
+                };
+                if (warp == NW - 1) {
+                    const R s2 = dot(cv);
+                    const R alpha = cv[j + 1];
+                    R beta = alpha, tau = R(0), scal = R(0);
+                    if (s2 > R(0)) {
+                        const R nrm = sqrt(alpha * alpha + s2);
+                        beta = alpha >= R(0) ? -nrm : nrm;
+                        tau = (beta - alpha) / beta;
+                        scal = R(1) / (alpha - beta);
+                    }
+                    if (lane == 0) {
+                        refl[0] = beta;
+                        refl[1] = tau;
+                        refl[2] = scal;
+                    }
+                } else {
+                    for (int q = NW - 2 - warp; q < 2 * jj; q += NW - 1) {
+                        const R acc = dot(q < jj ? Ws + (size_t)q * ldv : Vs + (size_t)(q - jj) * ldv);
+                        if (lane == 0) dots[q] = acc;
+                    }
                 }
                 if constexpr (CL > 1) {
                     if (nsplit > 1) {
@@ -357,18 +386,9 @@ __global__ void __launch_bounds__(NT, reduce_min_ctas(NT, sizeof(R))) tri_reduce
                 } else {
                     __syncthreads();
                 }
-                // (c) reflector H_j = I - tau v v^T with v_{j+1} = 1 mapping rows j+1.. of the
-                //     column onto beta e_{j+1} (every thread, the same bits); p = tau (A v - V (W^T v)
-                //     - W (V^T v)) on the owned rows, partial sums of p^T v
-                const R s2 = dots[2 * jj];
-                const R alpha = cv[j + 1];
-                R beta = alpha, tau = R(0), scal = R(0);
-                if (s2 > R(0)) {
-                    const R nrm = sqrt(alpha * alpha + s2);
-                    beta = alpha >= R(0) ? -nrm : nrm;
-                    tau = (beta - alpha) / beta;
-                    scal = R(1) / (alpha - beta);
-                }
+                // (c) p = tau (A v - V (W^T v) - W (V^T v)) on the owned rows, partial sums of p^T v
+                const R beta = refl[0], tau = refl[1], scal = refl[2];
+                const bool owner = n > NT || (32 * warp + 31 > j && 32 * warp < n);     // rows > j in this warp
                 if (tid == 0 && rank == 0) {
                     dw[j] = cv[j];
                     ew[j] = beta;
@@ -396,21 +416,20 @@ __global__ void __launch_bounds__(NT, reduce_min_ctas(NT, sizeof(R))) tri_reduce
                         for (int l = 0; l < jj; ++l) {
                             const R dW = Ws[l * ldv + j + 1] + scal * dots[l];
                             const R dV = Vs[l * ldv + j + 1] + scal * dots[jj + l];
-                            pi -= Vs[l * ldv + i] * dW + Ws[l * ldv + i] * dV;
+                            if constexpr (FP64) pi = fma(-Ws[l * ldv + i], dV, fma(-Vs[l * ldv + i], dW, pi));
+                            else pi -= Vs[l * ldv + i] * dW + Ws[l * ldv + i] * dV;
                         }
                         pi *= tau;
                         pv[i] = pi;
                         partK += pi * vi;
                     }
                 }
-                partK = warp_sum(partK);
+                if (owner) partK = warp_sum(partK);
                 if (lane == 0) red[warp] = partK;
                 __syncthreads();
                 // (d) K = tau/2 p^T v, w = p - K v on the owned rows
-                R sK = red[0];
-#pragma unroll
-                for (int w2 = 1; w2 < NW; ++w2) sK += red[w2];
-                const R K = R(0.5) * tau * sK;
+                R K = R(0);
+                if (owner) K = R(0.5) * tau * warp_sum(lane < NW ? red[lane] : R(0));
                 Kprev = K;
                 for (int i = tid; i < ldv; i += NT)
                     Ws[jj * ldv + i] = (i > j && i < n) ? pv[i] - K * Vs[jj * ldv + i] : R(0);
