@@ -169,7 +169,7 @@ __device__ __forceinline__ void st_cluster(float* dst, unsigned rank, float x) {
 // In FP64 every warp instruction holds its quarter of the SM for 80 clocks, so nothing is computed twice that
 // one warp can publish: the root and divisions of the reflector run in the last warp beside the others' A x,
 // the sum of p^T v in the warps that own rows only (in every warp, the same bits: a third of the FP64
-// instructions; 54 windows 7.6 -> 5.55 ms, one of 96 functions 1.64 -> 1.03 ms).
+// instructions; 54 windows 7.6 -> 5.55 ms, one of 96 functions 1.64 -> 1.03 ms; with panels of 8 5.17 and 0.92).
 //
 // CL = 2: a cluster of two CTAs per window, for fewer windows than half the SMs (FP64, 54 windows of 276-300
 // functions 9.2 -> 7.6 ms, before the above; one window of 96, where the barriers outweigh the work, 1.64 -> 1.84 ms).  Both form the columns, reflectors and vectors (the same bits); the row quads of q = A x and the
@@ -1800,8 +1800,12 @@ int tri_pick(bool fp32, int nmax, size_t smem_budget, int cfg, TriPick* out) {
     const TriCfg& t = kTriCfg[cfg];
     r.nt = t.nt;
     r.reg = t.reg && fp32;
+    // FP64: panels of 8, the pending updates cost instructions of its pipe and the L2 traffic of more frequent
+    // updates does not bound it (54 windows: panels of 4, 8, 16 take 5.21, 5.17, 5.56 ms; 432 windows 19.6,
+    // 18.3, 19.4 to 20.7 ms; one window of 96 functions 0.88, 0.92, 1.03 ms)
+    const int nbmax = fp32 ? t.nb : std::min(t.nb, 8);
     for (int b : {32, 16, 8, 4})
-        if (b <= t.nb && !r.nb && reduce_smem_elems(b, r.ldv, t.nt) * el <= smem_budget) r.nb = b;
+        if (b <= nbmax && !r.nb && reduce_smem_elems(b, r.ldv, t.nt) * el <= smem_budget) r.nb = b;
     if (t.res && fp32)
         for (int b : {32, 16})
             for (int rows = std::min(kResRows, t.rows); rows >= 32 && !r.nb_apply; rows -= 32)
@@ -1889,7 +1893,7 @@ int tri_reduce(bool fp32, int nwin, const int* order, int* counter, const int* n
     if (nt == 512) {
         // two CTAs per window while they find an SM each and the windows are large enough to share; one
         // CTA of 512 threads while the windows find one;
-        // beyond, two of 256 threads per SM, which fill each other's barriers (432 windows 26.5 -> 23.3 ms)
+        // beyond, two of 256 threads per SM, which fill each other's barriers (432 windows 19.7 -> 18.3 ms)
         if (2 * nwin <= device_sms() && nmax >= 192 && reduce_smem_elems(nb, ldv, 512, 2) * sizeof(double) <= smem_budget)
             return launch_reduce_cluster(p, s);
         if (nwin > device_sms() && 2 * (reduce_smem_elems(nb, ldv, 256) * sizeof(double) + 1024) <= smem_budget + 1024)
