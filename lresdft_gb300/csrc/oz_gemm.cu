@@ -17,8 +17,8 @@
 // ~600 TFLOP/s is 21 FP64 multiply-adds per clock and SM.  The windows go in batches, so that the
 // digits take at most ~1 GB whatever the context's size.
 //
-// Measured (432 windows of 270-306 functions): the standard form's two products 23.5 -> 6.1 ms (54
-// windows 3.7 -> 0.90).
+// Measured (432 windows of 270-306 functions): the standard form's two products 23.5 -> 5.6 ms (54
+// windows 3.7 -> 0.79).
 #include "common.cuh"
 #include "launch.cuh"
 #include "lres_internal.h"
@@ -405,47 +405,55 @@ int oz_gemm(OzWork& wk, int nwin, int mmax, int nmax, int kmax, const int* m_w, 
 // Y <- Y - ((Y V) T) V^T per panel, three products on the tensor cores; V^T V (for T) a fourth, once per
 // Hamiltonian for all row sets.  Panels of 128 rather than the 32 of tri_apply_kernel: a product over
 // 32 terms would spend more on the digits and the joining than on its terms.  The FP64 pipe does the
-// T recurrence only.  Measured (with T): 54 windows of 256 rows 7.5 -> 2.9 ms, 432 windows 32.5 ->
-// 14.4 ms.
+// T recurrence only.  Measured (with T): 54 windows of 256 rows 7.5 -> 1.86 ms, 432 windows 32.5 ->
+// 11.4 ms.
 
 namespace {
 
-constexpr int kTNT = kOzPanel;
+constexpr int kTNT = 4 * kOzPanel;             // four threads a row
+constexpr int kTLd = kOzPanel + 8;            // (four columns of eight rows in 16 banks each)
 
 // T of every (window, panel) from G = V^T V in its slot: T_ll = tau_l, T[0:l, l] = -tau_l T[0:l, 0:l] G[0:l, l],
-// T in place of G (column-major, zero below the diagonal).  Thread = row of T, which only it reads; T by
-// columns and G's upper triangle packed by columns in shared memory.  Bound by the FP64 pipe (q^3 / 6
-// multiply-adds, 20 clocks a warp's).
+// T in place of G (column-major, zero below the diagonal).  T by columns and G's upper triangle packed by
+// columns in shared memory.  Bound by the FP64 pipe (q^3 / 6 multiply-adds, 80 clocks a warp's on a quarter of
+// the SM): a row's sum is dealt to four threads of a warp, so that the rows of a warp have nearly the same
+// length and sixteen warps share the pipe (a thread per row, the first warp's the longest: 432 windows of 290
+// functions 2.54 -> 1.17 ms, 54 windows 0.43 -> 0.20 ms).
 __global__ void __launch_bounds__(kTNT) oz_tfactor_kernel(int nwin, const int* q_w, const long long* offT,
                                                           const long long* offN, const double* tau, int qmax, double* T) {
     extern __shared__ __align__(16) unsigned char smem[];
-    double* const Ts = reinterpret_cast<double*>(smem);             // [qmax][kTNT]
-    double* const Gs = Ts + (size_t)qmax * kTNT;                    // (a, b), a <= b at b (b + 1) / 2 + a
-    const int w = blockIdx.x % nwin, p = blockIdx.x / nwin, a = threadIdx.x;
+    double* const Ts = reinterpret_cast<double*>(smem);             // [qmax][kTLd]
+    double* const Gs = Ts + (size_t)qmax * kTLd;                    // (a, b), a <= b at b (b + 1) / 2 + a
+    const int w = blockIdx.x % nwin, p = blockIdx.x / nwin, a = threadIdx.x >> 2, part = threadIdx.x & 3;
     const int q = q_w[blockIdx.x];
     if (q < 1) return;
     double* const Tw = T + offT[blockIdx.x];
-    for (int b = 0; b < q; ++b)
-        if (a <= b) Gs[b * (b + 1) / 2 + a] = Tw[a + (long long)b * q];
+    for (int b = threadIdx.x >> 7; b < q; b += kTNT / kOzPanel) {
+        const int r = threadIdx.x & (kOzPanel - 1);
+        if (r <= b) Gs[b * (b + 1) / 2 + r] = Tw[r + (long long)b * q];
+    }
     __syncthreads();
     const double* const tw = tau + offN[w] + p * kOzPanel;
+    const int first = a & ~7;                                       // the warp's first row
     for (int l = 0; l < q; ++l) {
         const double tl = tw[l];
-        const double* const g = Gs + l * (l + 1) / 2;
         double val = a == l ? tl : 0.0;
-        if (a < l) {
-            double s[4] = {0.0, 0.0, 0.0, 0.0};
-            int b = a;
-            for (; b + 3 < l; b += 4)
-#pragma unroll
-                for (int u = 0; u < 4; ++u) s[u] = fma(Ts[(b + u) * kTNT + a], g[b + u], s[u]);
-            for (; b < l; ++b) s[0] = fma(Ts[b * kTNT + a], g[b], s[0]);
-            val = -tl * ((s[0] + s[1]) + (s[2] + s[3]));
+        if (first < l) {                                            // (the same for the warp)
+            const double* const g = Gs + l * (l + 1) / 2;
+            double s = 0.0;
+            for (int b = a + part; b < l; b += 4) s = fma(Ts[b * kTLd + a], g[b], s);
+            s += __shfl_xor_sync(0xffffffffu, s, 1);
+            s += __shfl_xor_sync(0xffffffffu, s, 2);
+            if (a < l) val = -tl * s;
         }
-        Ts[l * kTNT + a] = val;
+        if (part == 0) Ts[l * kTLd + a] = val;
+        __syncwarp();
     }
-    for (int b = 0; b < q; ++b)
-        if (a < q) Tw[a + (long long)b * q] = Ts[b * kTNT + a];
+    __syncthreads();
+    for (int b = threadIdx.x >> 7; b < q; b += kTNT / kOzPanel) {
+        const int r = threadIdx.x & (kOzPanel - 1);
+        if (r < q) Tw[r + (long long)b * q] = Ts[b * kTLd + r];
+    }
 }
 
 }  // namespace
@@ -473,7 +481,7 @@ int oz_tfactors(OzWork& wk, const OzRows& o, int nwin, int nmax, const int* n_w,
     }
     if (o.panels) {
         const int qm = std::min(kOzPanel, nmax - 2);
-        const size_t smem = sizeof(double) * ((size_t)qm * kTNT + (size_t)qm * (qm + 1) / 2);
+        const size_t smem = sizeof(double) * ((size_t)qm * kTLd + (size_t)qm * (qm + 1) / 2);
         int per_sm = 0;
         if (int rc = prepare_kernel<oz_tfactor_kernel>(kTNT, smem, &per_sm)) return rc;
         oz_tfactor_kernel<<<(unsigned)nwin * o.panels, kTNT, smem, s>>>(nwin, o.q, o.offT, offN, tau, qm, o.T);
