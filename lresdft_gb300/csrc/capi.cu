@@ -2078,14 +2078,14 @@ bool adj_tri_buffers(lres_ctx* c, cudaStream_t s) {
 // The accumulations of the adjoint from the FP64 tridiagonal form: per-window N and E_band, the density by
 // the pass, A_c in the tridiagonal basis into d_adjA, W = L^-T Q in *Wt (over the standard form, which the
 // reduction has consumed).  In mixed precision the tridiagonal form is made here (d_HW and L^-T are FP64)
-// and the sweeps run in FP32: 128 windows 89 -> 45 ms, the gradients 1.8e-6 off 64 bits against the
+// and the sweeps run in FP32: 128 windows 89 -> 35 ms, the gradients 1.8e-6 off 64 bits against the
 // 2.2e-6 of FP32 factors.
 int adj_tri_accumulate(lres_ctx* c, double mu, double e_lo, const double** Wt, cudaStream_t s) {
     const bool mixed = c->precision == LRES_MIXED;
     if (!c->tri_ready) TRY(tri_refresh(c, s));
     const int P = c->npoles;
     const int groups = adj_sweep_groups(c->nwin, P);
-    const size_t coefb = sizeof(double4) * tri_coef_elems(c->nwin, P, c->nmax);
+    const size_t coefb = sizeof(double4) * tri_coef_elems(c->nwin, P, c->nmax) * (mixed ? 2 : 1);   // (and derivatives)
     const size_t trb = sizeof(double2) * (size_t)c->nwin * P;
     const size_t k32b = mixed ? (sizeof(float) * (size_t)c->sizeC + 15) / 16 * 16 : 0;
     const size_t xb = groups > 1 ? sizeof(double) * 3 * (size_t)groups * c->sizeC : 0;
@@ -2128,6 +2128,9 @@ int adj_tri_accumulate(lres_ctx* c, double mu, double e_lo, const double** Wt, c
         TRY(square_gemm(c, a.H, true, c->d_adjA[0], true, a.K, 0, s));
         TRY(tri_count(c->nwin, P, c->nmax, c->d_n, c->d_offN, c->d_offC, a.d, a.e, a.K, a.shifts, c->d_wq, c->d_wzq, c->dV,
                       coef, trace, c->d_nw, c->d_ew, c->d_status, c->smem_budget, s));
+        // the inner products <S, A_c> = tr(X_c) in FP64 (the FP32 X_c leave 1e-6 of N in dN/dmu)
+        TRY(tri_slopes(c->nwin, P, c->nmax, c->d_n, c->d_offN, c->d_offC, a.d, a.e, a.K, a.shifts, c->d_cw, coef,
+                       coef + tri_coef_elems(c->nwin, P, c->nmax), trace, c->d_adju, s));
         TRY(convert_f64_f32(a.K, K32, c->sizeC, s));
         shifts = a.shifts;
         d = a.d;
@@ -2226,8 +2229,9 @@ extern "C" int lres_adjoint(lres_ctx* c, double mu, double e_lo, double* dv, int
     const double* Wt = mixed ? c->d_LinvT : nullptr;
     if (tri) TRY(adj_tri_accumulate(c, mu, e_lo, &Wt, s));
     else TRY(adj_ldl_accumulate(c, s));
-    TRY(adj_inner(c->nwin, c->d_n, c->d_offC, Wt ? nullptr : c->d_SW, c->d_adjA[0], c->d_adjA[1], c->d_adjA[2],
-                  c->d_adju, s));
+    if (!tri || !mixed)                        // (with their accumulations otherwise)
+        TRY(adj_inner(c->nwin, c->d_n, c->d_offC, Wt ? nullptr : c->d_SW, c->d_adjA[0], c->d_adjA[1], c->d_adjA[2],
+                      c->d_adju, s));
     LRES_CUDA_TRY(cudaMemcpyAsync(c->nw_h.data(), c->d_nw, sizeof(double) * c->nwin, cudaMemcpyDeviceToHost, s));
     LRES_CUDA_TRY(cudaMemcpyAsync(c->ew_h.data(), c->d_ew, sizeof(double) * c->nwin, cudaMemcpyDeviceToHost, s));
     LRES_CUDA_TRY(cudaMemcpyAsync(c->adju_h.data(), c->d_adju, sizeof(double) * 3 * c->nwin,

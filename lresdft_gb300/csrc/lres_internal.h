@@ -195,6 +195,11 @@ int tri_count(int nwin, int P, int nmax, const int* n_w, const long long* offN, 
               double dV, double4* coef, double2* trace, double* nw, double* ew, int* status, size_t smem_budget,
               cudaStream_t s);
 // P = Re sum_k w_k (z_k - T)^-1 of every window (FP64), and the rows' n, e from V = Y P for windows
+// u[c * nwin + w] = Re sum_k cw[c P + k] tr(G_k K G_k), c = 0, 1, 2, after tri_count: its coef, dcoef as coef,
+// slope nwin * P elements.
+int tri_slopes(int nwin, int P, int nmax, const int* n_w, const long long* offN, const long long* offC, const double* d,
+               const double* e, const double* K, const double2* shifts, const double2* cw, const double4* coef,
+               double4* dcoef, double2* slope, double* u, cudaStream_t s);
 // w0 .. w0 + nwin - 1 (V of window w at offV[w], maxitems pass items of a window at most)
 int tri_pmat(int nwin, int P, int nmax, const int* n_w, const long long* offN, const long long* offC, const double* d,
              const double* e, const double2* shifts, const double2* wq, double4* coef, double* Pm, cudaStream_t s);

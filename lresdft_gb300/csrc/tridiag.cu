@@ -1527,6 +1527,121 @@ __global__ void __launch_bounds__(kCountNT) tri_count_kernel(int P, int groups, 
     }
 }
 
+// tr(G_k K G_k) = -d/dz tr(G_k K) of every (window, pole): the sums above with their derivatives in z, from
+// t', G' (dcoef) and L' behind them.  FP64, for the derivatives of N and E_band in the chemical potential, which
+// are small differences of large sums: from the FP32 sweeps of the mixed adjoint they carry an error of 1e-6 of
+// N, whatever their size.
+constexpr int kSlopePoles = 2;
+
+// (t'_i, G'_ii) and L'_i from (t_i, G_ii) and L_i: D' = 1 - e t', (1 / D)' = -D' / D^2.
+__global__ void tri_slope_diag_kernel(int nwin, int P, const int* n_w, const long long* offN, const double* __restrict__ d,
+                                      const double* __restrict__ e, const double2* z, int ld, const double4* coef,
+                                      double4* dcoef) {
+    const int it = blockIdx.x * blockDim.x + threadIdx.x;
+    if (it >= nwin * P) return;
+    const int w = it / P, n = n_w[w];
+    const double2 zk = z[it - w * P];
+    const double *dw = d + offN[w], *ew = e + offN[w];
+    const double4* const in = coef + (size_t)it * ld;
+    const double2* const L = semi_products(coef, nwin * P, ld) + (size_t)it * ld;
+    double4* const out = dcoef + (size_t)it * ld;
+    double2* const Ld = reinterpret_cast<double2*>(dcoef + (size_t)nwin * P * ld) + (size_t)it * ld;
+    auto mul = [](double2 a, double2 b) { return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x)); };
+    double2 td = make_double2(0.0, 0.0), gd = td;
+    double el = 0.0;                                                 // e_{i-1}
+    for (int i = 0; i < n; ++i) {
+        const double2 t = make_double2(in[i].x, in[i].y);
+        td = make_double2(el * gd.x, el * gd.y);
+        const double2 D = make_double2(fma(-el, t.x, zk.x - dw[i]), fma(-el, t.y, zk.y));
+        const double inv = recip_f64(D.x * D.x + D.y * D.y);
+        const double2 g = make_double2(D.x * inv, -D.y * inv);
+        const double2 g2 = mul(g, g), Dd = make_double2(fma(-el, td.x, 1.0), -el * td.y);
+        gd = mul(make_double2(-g2.x, -g2.y), Dd);
+        out[i] = make_double4(td.x, td.y, gd.x, gd.y);
+        el = ew[i];
+    }
+    double2 G = make_double2(0.0, 0.0), Gd = G, tn = G, tnd = G, Lp = G, Lc = G;     // of i + 1; L', L
+    for (int i = n - 1; i >= 0; --i) {
+        const double4 c = in[i], o = out[i];
+        const double2 t2 = mul(tn, tn), x = mul(mul(make_double2(2.0 * tn.x, 2.0 * tn.y), tnd), G), y = mul(t2, Gd);
+        Gd = make_double2(o.z + x.x + y.x, o.w + x.y + y.y);
+        G = make_double2(c.z, c.w);
+        if (i % kSemi == kSemi - 1) {
+            Lp = tnd;
+        } else {
+            const double2 a = mul(tn, Lp), b = mul(tnd, Lc);
+            Lp = make_double2(a.x + b.x, a.y + b.y);
+        }
+        Lc = L[i];
+        Ld[i] = Lp;
+        tn = make_double2(c.x, c.y);
+        tnd = make_double2(o.x, o.y);
+        out[i] = make_double4(o.x, o.y, Gd.x, Gd.y);
+    }
+}
+
+__global__ void __launch_bounds__(kCountNT) tri_slope_kernel(int P, int groups, const int* n_w, const long long* offC,
+                                                             const double* K, const double4* coef, const double4* dcoef,
+                                                             int ld, double2* slope) {
+    __shared__ double red[kCountNT / 32];
+    const int w = blockIdx.x / groups, k0 = (blockIdx.x % groups) * kSlopePoles;
+    const int n = n_w[w], tid = threadIdx.x, nitems = (int)(gridDim.x / groups) * P;
+    const double* const Kw = K + offC[w];
+    auto mul = [](double2 a, double2 b) { return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x)); };
+    for (int q = 0; q < kSlopePoles && k0 + q < P; ++q) {
+        const size_t it = ((size_t)w * P + k0 + q) * ld;
+        const double4 *cf = coef + it, *cd = dcoef + it;
+        const double2 *L = semi_products(coef, nitems, ld) + it, *Ld = semi_products(dcoef, nitems, ld) + it;
+        double2 acc = make_double2(0.0, 0.0);
+        for (int j = tid; j < n; j += kCountNT) {
+            double2 h = make_double2(0.0, 0.0), hd = h;
+            const int jb = j / kSemi * kSemi;
+            for (int i0 = 0; i0 < jb; i0 += kSemi) {
+                if (i0) {
+                    const double2 f = L[i0], fd = Ld[i0], a = mul(hd, f), b = mul(h, fd);
+                    hd = make_double2(a.x + b.x, a.y + b.y);
+                    h = mul(h, f);
+                }
+#pragma unroll 8
+                for (int i = i0; i < i0 + kSemi; ++i) {
+                    const double x = Kw[j + (long long)i * n];
+                    const double2 f = L[i], fd = Ld[i];
+                    h = make_double2(fma(x, f.x, h.x), fma(x, f.y, h.y));
+                    hd = make_double2(fma(x, fd.x, hd.x), fma(x, fd.y, hd.y));
+                }
+            }
+#pragma unroll 4
+            for (int i = jb; i < j; ++i) {
+                const double4 t4 = cf[i + 1], d4 = cd[i + 1];
+                const double2 t = make_double2(t4.x, t4.y), td = make_double2(d4.x, d4.y);
+                const double2 u = make_double2(h.x + Kw[j + (long long)i * n], h.y), a = mul(hd, t), b = mul(u, td);
+                hd = make_double2(a.x + b.x, a.y + b.y);
+                h = mul(u, t);
+            }
+            const double2 u = make_double2(fma(2.0, h.x, Kw[j + (long long)j * n]), 2.0 * h.y);
+            const double2 a = mul(make_double2(cd[j].z, cd[j].w), u);
+            const double2 b = mul(make_double2(cf[j].z, cf[j].w), make_double2(2.0 * hd.x, 2.0 * hd.y));
+            acc = make_double2(acc.x + a.x + b.x, acc.y + a.y + b.y);
+        }
+        const double x = block_sum<kCountNT>(acc.x, red), y = block_sum<kCountNT>(acc.y, red);
+        if (tid == 0) slope[(size_t)w * P + k0 + q] = make_double2(-x, -y);
+    }
+}
+
+// u[c * nwin + w] = Re sum_k c_k tr(G_k K G_k), poles in order
+__global__ void tri_slope_sums_kernel(int nwin, int P, const double2* slope, const double2* cw, double* u) {
+    const int w = blockIdx.x * blockDim.x + threadIdx.x;
+    if (w >= nwin) return;
+    for (int c = 0; c < 3; ++c) {
+        double s = 0.0;
+        for (int k = 0; k < P; ++k) {
+            const double2 x = slope[(size_t)w * P + k], a = cw[c * P + k];
+            s += a.x * x.x - a.y * x.y;
+        }
+        u[(size_t)c * nwin + w] = s;
+    }
+}
+
 // per-window N and E_band from the traces, poles in order
 __global__ void tri_count_sums_kernel(int nwin, int P, const double2* trace, const double2* wq, const double2* wzq,
                                       double dV, double* nw, double* ew, int* status) {
@@ -2041,6 +2156,21 @@ int tri_count(int nwin, int P, int nmax, const int* n_w, const long long* offN, 
     }
     LRES_CUDA_TRY(cudaGetLastError());
     tri_count_sums_kernel<<<(nwin + 63) / 64, 64, 0, s>>>(nwin, P, trace, wq, wzq, dV, nw, ew, status);
+    LRES_CUDA_TRY(cudaGetLastError());
+    return LRES_OK;
+}
+
+int tri_slopes(int nwin, int P, int nmax, const int* n_w, const long long* offN, const long long* offC, const double* d,
+               const double* e, const double* K, const double2* shifts, const double2* cw, const double4* coef,
+               double4* dcoef, double2* slope, double* u, cudaStream_t s) {
+    if (!nwin) return LRES_OK;
+    tri_slope_diag_kernel<<<(unsigned)(((long long)nwin * P + 31) / 32), 32, 0, s>>>(nwin, P, n_w, offN, d, e, shifts,
+                                                                                    nmax, coef, dcoef);
+    LRES_CUDA_TRY(cudaGetLastError());
+    const int groups = (P + kSlopePoles - 1) / kSlopePoles;
+    tri_slope_kernel<<<(unsigned)nwin * groups, kCountNT, 0, s>>>(P, groups, n_w, offC, K, coef, dcoef, nmax, slope);
+    LRES_CUDA_TRY(cudaGetLastError());
+    tri_slope_sums_kernel<<<(nwin + 63) / 64, 64, 0, s>>>(nwin, P, slope, cw, u);
     LRES_CUDA_TRY(cudaGetLastError());
     return LRES_OK;
 }
