@@ -183,16 +183,37 @@ def roofline_of(name, ms, nW, mW, P, nnz_h, peaks):
             "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)" if peaks else "fallback"}
 
 
-def launches_per_step(route, precision, tile_config=0, standard_form="simt"):
+def oz_launches(nwin, m, n, k, gram=False):
+    """Launches of one FP64 product of all windows on the tensor cores (csrc/oz_gemm.cu): the digits
+    of both operands (one of a Gram product) and the product, per batch of 1 GB of digits."""
+    up = lambda x, t: -(-max(x, 1) // t) * t
+    per_window = 18 * (up(m, 64) + up(n, 64)) * up(k, 32) + 4 * (up(m, 64) + up(n, 64))
+    batch = min(nwin, max((1 << 30) // per_window, 1))
+    return (2 if gram else 3) * -(-nwin // batch)
+
+
+def launches_per_step(route, precision, tile_config=0, standard_form="simt", nW=(), mW=()):
     """Our kernels in one step (H(v) + window blocks + standard form + pass)."""
+    nwin, n, m = len(nW), int(max(nW, default=0)), int(max(mW, default=0))
     if route == "tridiag":
         # assemble_h, gather, 2 standard-form GEMMs, reduction, rows, pole nodes, pass, window
-        # sums; mixed: + the FP32 potential per slot, + V^T V and the T factors of the
+        # sums; + the FP32 potential per slot, + V^T V and the T factors of the
         # resident-row application (every configuration but 2), + the FP32 copy of the H
-        # blocks that the SIMT standard form's FP32 windows are gathered from
+        # blocks that the SIMT standard form's FP32 windows are gathered from, + the first columns
+        # of windows beyond 384 functions
         if precision == "mixed":
-            return 10 + 2 * (tile_config != 2) + (standard_form == "simt")
-        return 9
+            return 10 + 2 * (tile_config != 2) + (standard_form == "simt") + (tile_config in (0, 4) and n > 384)
+        # FP64: assemble_h, gather, reduction, T factors, pole nodes, diagonals of G, P, rows' sums
+        # (V a batch of windows at a time, 1 GB), window sums; the products: 2 of the standard form,
+        # V^T V and 3 of the rows per panel of 128 reflectors, V = Y P
+        total = 9 + 2 * oz_launches(nwin, n, n, n)
+        for j0 in range(0, n - 2, 128):
+            q, r = min(128, n - 2 - j0), n - 1 - j0
+            total += oz_launches(nwin, q, q, r, gram=True) + oz_launches(nwin, m, q, r)
+            total += oz_launches(nwin, m, q, q) + oz_launches(nwin, m, r, q)
+        vb = max(1, min(nwin, (1 << 27) // max(m * n, 1)))
+        batches = -(-nwin // vb)
+        return total + (batches - 1) + sum(oz_launches(min(vb, nwin - i * vb), m, n, n) for i in range(batches))
     # assemble_h, gather, [split + 2 double-float GEMMs], pole nodes, LDL^T kernel, pole sums
     return 8 if precision == "mixed" else 5
 
@@ -304,7 +325,7 @@ def run_ours(args):
     P = s.M // 2
     units = len(s.nW) * P
     lps = launches_per_step(route, args.precision, s.tile_config if isinstance(s.tile_config, int) else 0,
-                            args.standard_form)
+                            args.standard_form, nW, mW)
 
     def step():
         s.set_potential_device(v_dev.data_ptr())
@@ -407,12 +428,13 @@ def run_ours(args):
     # configurations 0 and 4 reduce with the window on its SM, all but 2 apply with resident rows
     mixed = args.precision == "mixed"
     cfg = s.tile_config if isinstance(s.tile_config, int) else 0
-    kernel_names = {"pole_kernel": "tri_pass_kernel" if route == "tridiag" else "ldl_left_kernel",
+    kernel_names = {"pole_kernel": ("tri_pass_kernel" if mixed else "tri_pmat_kernel")
+                    if route == "tridiag" else "ldl_left_kernel",
                     "transform": ("gemm_tc_kernel" if args.standard_form == "tensor" else "gemm_f32blk_kernel")
                     if (route == "tridiag" and mixed)
-                    else ("oz_gemm_kernel" if args.precision == "fp64" else "gemm_df64_kernel"),
+                    else ("oz_gemm_kernel (standard form)" if args.precision == "fp64" else "gemm_df64_kernel"),
                     "tri_reduce": "tri_reduce_reg_kernel" if (mixed and cfg in (0, 4)) else "tri_reduce_kernel",
-                    "tri_rows": "tri_apply_res_kernel" if (mixed and cfg != 2) else "tri_apply_kernel",
+                    "tri_rows": ("tri_apply_res_kernel" if cfg != 2 else "tri_apply_kernel") if mixed else "oz_gemm_kernel (rows)",
                     "assemble_h": "assemble_h32_kernel" if mixed else "assemble_h_kernel",
                     "gather": "gather_windows_kernel"}
 
