@@ -138,18 +138,19 @@ struct lres_ctx {
     OzRows ozr;                                  // rows through the reflectors on the tensor cores (FP64)
     OzRowSet oz_own, oz_trc, oz_adj;
     // FP64 tridiagonal form of the mixed adjoint (on its first use): reflectors, T, its standard form and
-    // then W = L^-T Q, K = W^T (F^T F) W, FP64 nodes
+    // then W = L^-T Q, K = W^T (F^T F) W, H(v) in FP64, FP64 nodes
     struct AdjTri {
-        double *A = nullptr, *d = nullptr, *e = nullptr, *tau = nullptr, *H = nullptr, *K = nullptr;
+        double *A = nullptr, *d = nullptr, *e = nullptr, *tau = nullptr, *H = nullptr, *K = nullptr, *Hblk = nullptr;
         double2* shifts = nullptr;
         bool tried = false;
         bool ok() const { return shifts != nullptr; }
         void release() {
-            for (void* q : {(void*)A, (void*)d, (void*)e, (void*)tau, (void*)H, (void*)K, (void*)shifts})
+            for (void* q : {(void*)A, (void*)d, (void*)e, (void*)tau, (void*)H, (void*)K, (void*)Hblk, (void*)shifts})
                 if (q) cudaFree(q);
             *this = AdjTri{};
         }
     } at;
+    bool h_from_v = false;                       // mixed: H_W is the FP32 H(v) of d_v
     // density passes through P (FP64): V = Y P in batches of windows
     bool by_matrix = false;
     bool no_room_for_k = false;                  // K did not fit: counts over the rows
@@ -1388,9 +1389,11 @@ extern "C" int lres_set_potential(lres_ctx* c, const double* v, int v_on_device,
         LRES_CUDA_TRY(cudaMemcpyAsync(c->d_v, v, sizeof(double) * c->ng, cudaMemcpyHostToDevice, s));
         dv = c->d_v;
     }
+    c->h_from_v = c->sp.sval32 != nullptr;
     TRY(mark(c, 2, 0, s));
     if (c->sp.sval32)
-        TRY(assemble_h32(c->bp, c->sp, c->d_Tblk, dv, c->dV, c->d_Hblk, s));
+        // (v is kept: the mixed adjoint assembles H(v) again in FP64)
+        TRY(assemble_h32(c->bp, c->sp, c->d_Tblk, dv, c->dV, c->d_Hblk, c->ng, dv == c->d_v ? nullptr : c->d_v, s));
     else
         TRY(assemble_h(c->bp, c->sp, c->d_Tblk, dv, c->dV, c->d_Hblk, s));
     TRY(mark(c, 2, 1, s));
@@ -1409,6 +1412,7 @@ extern "C" int lres_set_hamiltonian_csr(lres_ctx* c, const int64_t* Hp, const in
         for (int f = c->gptr_h[g]; f < c->gptr_h[g + 1]; ++f) group_of_fn[f] = g;
     std::vector<double> blk;
     TRY(scatter_csr(c, group_of_fn, Hp, Hi, Hv, blk));
+    c->h_from_v = false;
     LRES_CUDA_TRY(cudaMemcpyAsync(c->d_Hblk, blk.data(), sizeof(double) * blk.size(), cudaMemcpyHostToDevice, s));
     TRY(after_h_blocks(c, s));
     LRES_CUDA_TRY(cudaStreamSynchronize(s));   // blk is a host temporary
@@ -1942,6 +1946,7 @@ extern "C" int lres_set_windows(lres_ctx* c, const double* HW, const double* SW,
     const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     c->h32_dense = false;                // the FP32 windows, if any, are of the previous H
     if (HW) LRES_CUDA_TRY(cudaMemcpyAsync(c->d_HW, HW, sizeof(double) * c->sizeC, kind, s));
+    if (HW) c->h_from_v = false;
     if (SW) {
         LRES_CUDA_TRY(cudaMemcpyAsync(c->d_SW, SW, sizeof(double) * c->sizeC, kind, s));
         if (needs_standard_form(c)) TRY(setup_standard_form(c, s));
@@ -2062,6 +2067,7 @@ bool adj_tri_buffers(lres_ctx* c, cudaStream_t s) {
     if (!rc) rc = dalloc(&a.tau, c->sizeN);
     if (!rc) rc = dalloc(&a.H, c->sizeC);
     if (!rc) rc = dalloc(&a.K, c->sizeC);
+    if (!rc) rc = dalloc(&a.Hblk, c->bp.nval);
     if (!rc) rc = oz_setup(c, s);
     if (!rc) rc = oz_setup_rows(c, c->n_w, c->oz_adj, s);
     if (!rc) rc = dalloc(&a.shifts, c->npoles);
@@ -2078,8 +2084,8 @@ bool adj_tri_buffers(lres_ctx* c, cudaStream_t s) {
 // The accumulations of the adjoint from the FP64 tridiagonal form: per-window N and E_band, the density by
 // the pass, A_c in the tridiagonal basis into d_adjA, W = L^-T Q in *Wt (over the standard form, which the
 // reduction has consumed).  In mixed precision the tridiagonal form is made here (d_HW and L^-T are FP64)
-// and the sweeps run in FP32: 128 windows 89 -> 35 ms, the gradients 1.8e-6 off 64 bits against the
-// 2.2e-6 of FP32 factors.
+// and the sweeps run in FP32: 128 windows 89 -> 36 ms, the gradients 5e-7 off 64 bits against the
+// 2e-6 of FP32 factors.
 int adj_tri_accumulate(lres_ctx* c, double mu, double e_lo, const double** Wt, cudaStream_t s) {
     const bool mixed = c->precision == LRES_MIXED;
     if (!c->tri_ready) TRY(tri_refresh(c, s));
@@ -2115,7 +2121,15 @@ int adj_tri_accumulate(lres_ctx* c, double mu, double e_lo, const double** Wt, c
         TRY(tri_pick(false, c->nmax, c->smem_budget, 0, &pk));
         poles_kernel<<<(P + 63) / 64, 64, 0, s>>>(P, c->M, mu, e_lo, 0, a.shifts, c->d_wq, c->d_wzq);
         LRES_CUDA_TRY(cudaGetLastError());
-        TRY(square_gemm(c, c->d_HW, false, c->d_LinvT, true, a.A, 1, s));
+        // H_W: where it is an FP32 H(v) again in FP64 (its 1e-8 Ha of the levels are 2e-6 of dN/dmu)
+        const double* HW = c->d_HW;
+        if (c->h_from_v) {
+            TRY(assemble_h(c->bp, c->sp, c->d_Tblk, c->d_v, c->dV, a.Hblk, s));
+            TRY(gather_windows(c->nwin, c->nmax, c->d_gfn, c->d_gfnoff, c->d_gbtab, c->d_gbtoff, c->d_gnlg, c->d_offC,
+                               c->d_n, a.Hblk, a.K, nullptr, nullptr, s));
+            HW = a.K;
+        }
+        TRY(square_gemm(c, HW, false, c->d_LinvT, true, a.A, 1, s));
         TRY(square_gemm(c, c->d_LinvT, true, a.A, true, a.H, 2, s));
         TRY(tri_reduce(false, c->nwin, c->d_order_w, c->d_counter, c->d_n, c->d_offC, c->d_offA, c->d_offN, a.H, a.A, a.d,
                        a.e, a.tau, c->d_status, pk, c->nmax, c->smem_budget, s));

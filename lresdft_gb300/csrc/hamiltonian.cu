@@ -191,9 +191,11 @@ int assemble_h(const BlockPattern& bp, const Supports& sp, const double* Tblk, c
 // ---------------------------------------------------------------------------
 
 // v at every support slot, FP32 (the FP32 kernel reads it next to the basis values)
-__global__ void slot_potential_kernel(long long nslot, const int* sgrid, const double* v, float* vslot) {
-    const long long a = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (a < nslot) vslot[a] = (float)v[sgrid[a]];
+__global__ void slot_potential_kernel(long long nslot, const int* sgrid, const double* v, float* vslot, long long ng,
+                                      double* vcopy) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < nslot) vslot[i] = (float)v[sgrid[i]];
+    if (vcopy && i < ng) vcopy[i] = v[i];
 }
 
 template <int NF>
@@ -315,14 +317,15 @@ __global__ void __launch_bounds__(kAsmThreads, 5) assemble_h32_kernel(int npair,
 bool assemble_h32_supported(const BlockPattern& bp) { return bp.nfmax <= 6; }
 
 int assemble_h32(const BlockPattern& bp, const Supports& sp, const double* Tblk, const double* v, double dV,
-                 double* Hblk, cudaStream_t s) {
+                 double* Hblk, long long ng, double* vcopy, cudaStream_t s) {
     if (!sp.sval32 || !sp.vslot || bp.nfmax > 6) {
         lres_set_error("FP32 H(v) assembly needs the FP32 basis values and at most 6 functions per atom");
         return LRES_ESTATE;
     }
     if (!bp.npair) return LRES_OK;
-    if (sp.nslot)
-        slot_potential_kernel<<<(unsigned)((sp.nslot + 255) / 256), 256, 0, s>>>(sp.nslot, sp.sgrid, v, sp.vslot);
+    const long long top = std::max<long long>(sp.nslot, vcopy ? ng : 0);
+    if (top)
+        slot_potential_kernel<<<(unsigned)((top + 255) / 256), 256, 0, s>>>(sp.nslot, sp.sgrid, v, sp.vslot, ng, vcopy);
     LRES_CUDA_TRY(cudaGetLastError());
     const int threads = kAsmThreads;
     const int blocks = (int)(((long long)bp.npair * 32 + threads - 1) / threads);

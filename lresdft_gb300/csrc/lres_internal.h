@@ -87,7 +87,7 @@ int assemble_h(const BlockPattern& bp, const Supports& sp, const double* Tblk, c
                double* Hblk, cudaStream_t s);
 bool assemble_h32_supported(const BlockPattern& bp);
 int assemble_h32(const BlockPattern& bp, const Supports& sp, const double* Tblk, const double* v, double dV,
-                 double* Hblk, cudaStream_t s);
+                 double* Hblk, long long ng, double* vcopy, cudaStream_t s);   // vcopy (nullable): ng values of v
 // Dense window blocks (column-major, every element written) from the atom-pair blocks; with
 // blk32 and dense32, also the FP32 windows from the FP32 copy of the blocks.
 int gather_windows(int nwin, int nmax, const int* fn, const long long* fnoff, const int* btab, const long long* btoff,
