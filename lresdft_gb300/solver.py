@@ -460,10 +460,11 @@ class LResGPU:
             if (fx > 0) != (fa > 0):
                 b, fb = x, fx
                 break
-            # secant step, 10% past its root so that the next point brackets; at least twice the last
-            # step where the count hardly moved
+            # secant step, 10% past its root so that the next point brackets (twice the last step where
+            # the count did not move); 0.5 Ha or twice the last step at most, so that a gap of any width
+            # is crossed
             sec = -fx * (x - a) / (fx - fa) if fx != fa else 2 * step
-            step = math.copysign(min(1.1 * abs(sec) if abs(sec) > 0 else 2 * abs(step), 0.5), step)
+            step = math.copysign(min(1.1 * abs(sec) if abs(sec) > 0 else 2 * abs(step), max(0.5, 2 * abs(step))), step)
             a, fa = x, fx
         else:
             raise RuntimeError("solve_mu_fixed_n: no sign change of N(mu) - N")
