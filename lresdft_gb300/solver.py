@@ -422,27 +422,22 @@ class LResGPU:
 
     def solve_mu_fixed_n(self, N=None, mu0=None, tol=1e-10, maxiter=60):
         """mu with |N(mu) - N| <= tol (absolute) on the current Hamiltonian, e_lo fixed: from mu0
-        (default: the current mu) a step with the slope dN/dmu of the last solve, secant steps until
-        the count changes sign, then Brent's method, on passes without density (54 windows from
-        0.02 Ha away: 19 passes with steps that doubled, 8 to 13 this way).  Returns (mu, N(mu),
-        E_band(mu))."""
+        (default: the current mu) a step with the slope dN/dmu of the last density call, secant steps
+        until the count changes sign, then Brent's method, on passes without density.  Leaves the
+        stored slope as it is, so that a repeated search runs over the same points.  Returns (mu,
+        N(mu), E_band(mu))."""
         N = self.b.cr.n_elec if N is None else N
         mu = self.mu if mu0 is None else mu0
         if mu is None or self.e_lo is None:
             raise RuntimeError("solve_mu_fixed_n needs (mu, e_lo): call density() first or set them")
         lo_bound = self.e_lo + 1e-6
         mu = max(mu, lo_bound + 1e-6)
-        cache, hist = {}, []
+        cache = {}
 
         def f(x):
             _, n, e = self.pole_pass(x, self.e_lo, want_density=False)
             cache[x] = (n, e)
-            hist.append((x, n - N))
             return n - N
-
-        def found(x):
-            self._note_slope(hist, x)
-            return x, cache[x][0], cache[x][1]
 
         f0 = f(mu)
         if abs(f0) <= tol:
@@ -456,7 +451,7 @@ class LResGPU:
                 x = 0.5 * (a + lo_bound)
             fx = f(x)
             if abs(fx) <= tol:
-                return found(x)
+                return x, cache[x][0], cache[x][1]
             if (fx > 0) != (fa > 0):
                 b, fb = x, fx
                 break
@@ -468,7 +463,8 @@ class LResGPU:
             a, fa = x, fx
         else:
             raise RuntimeError("solve_mu_fixed_n: no sign change of N(mu) - N")
-        return found(self._brent(f, a, fa, b, fb, tol, xtol=1e-15, maxit=maxiter))
+        x = self._brent(f, a, fa, b, fb, tol, xtol=1e-15, maxit=maxiter)
+        return x, cache[x][0], cache[x][1]
 
     def set_hamiltonian(self, H):
         Hp, Hi, Hv = csr64(H)

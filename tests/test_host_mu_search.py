@@ -21,6 +21,13 @@ def _levels(lam, width):
     return lambda mu: sum(2 / (1 + math.exp(min(max((x - mu) / width, -700), 700))) for x in lam)
 
 
+def test_a_search_leaves_nothing_for_the_next():
+    count = _levels([-1.0, -0.4, -0.3, 0.5], 0.05)
+    first, a = _search(count, -0.2, 6.0 - 1e-3)
+    again, b = _search(count, -0.2, 6.0 - 1e-3, slope=first._slope)
+    assert first._slope is None and a == b and first.calls == again.calls
+
+
 @pytest.mark.parametrize("slope", [None, 1e-9, 1e-3, 1.0, 1e9])
 def test_any_stored_slope_finds_the_root(slope):
     """A slope left by another crystal or state only costs passes."""
