@@ -135,6 +135,9 @@ struct lres_ctx {
     double4* d_coef = nullptr;
     double2* d_tr = nullptr;
     bool k_ready = false;
+    // an update of the Hamiltonian was captured in a graph: a replay exchanges T, the rows and H_W without
+    // running host code, so what is formed from them on demand is formed at every use
+    bool replayable = false;
     OzRows ozr;                                  // rows through the reflectors on the tensor cores (FP64)
     OzRowSet oz_own, oz_trc, oz_adj;
     // FP64 tridiagonal form of the mixed adjoint (on its first use): reflectors, T, its standard form and
@@ -151,6 +154,7 @@ struct lres_ctx {
         }
     } at;
     bool h_from_v = false;                       // mixed: H_W is the FP32 H(v) of d_v
+    bool hw_replayable = false;                  // a replay may set H_W from window matrices at any time
     // density passes through P (FP64): V = Y P in batches of windows
     bool by_matrix = false;
     bool no_room_for_k = false;                  // K did not fit: counts over the rows
@@ -424,9 +428,11 @@ int window_transform(lres_ctx* c, cudaStream_t s) {
     return transform_fp64(c, s);
 }
 
-// The double-float standard form for the LDL^T consumers (passes on that route, the adjoint).
+// The double-float standard form for the LDL^T consumers (passes on that route, whose updates of the
+// Hamiltonian form it themselves; the adjoint).
 int ensure_hhat_df(lres_ctx* c, cudaStream_t s) {
-    if (c->precision == LRES_MIXED && !c->hhat_df) return transform_df64(c, s);
+    const bool stale = !c->hhat_df || (c->replayable && c->route == LRES_ROUTE_TRIDIAG);
+    if (c->precision == LRES_MIXED && stale) return transform_df64(c, s);
     return LRES_OK;
 }
 
@@ -435,11 +441,18 @@ bool needs_standard_form(const lres_ctx* c) {
     return c->precision == LRES_MIXED || c->route == LRES_ROUTE_TRIDIAG;
 }
 
-int mark(lres_ctx* c, int which, int end, cudaStream_t s) {
-    // a stream being captured into a graph records no timing events
+int capturing(cudaStream_t s, bool* yes) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     LRES_CUDA_TRY(cudaStreamIsCapturing(s, &cs));
-    if (cs != cudaStreamCaptureStatusNone) return LRES_OK;
+    *yes = cs != cudaStreamCaptureStatusNone;
+    return LRES_OK;
+}
+
+int mark(lres_ctx* c, int which, int end, cudaStream_t s) {
+    // a stream being captured into a graph records no timing events
+    bool cap = false;
+    TRY(capturing(s, &cap));
+    if (cap) return LRES_OK;
     LRES_CUDA_TRY(cudaEventRecord(c->ev[2 * which + end], s));
     c->ev_used[which] = true;
     return LRES_OK;
@@ -839,7 +852,7 @@ bool counts_from_k(lres_ctx* c) {
 
 // K of the current Hamiltonian, from the trace rows where there are any.
 int ensure_k(lres_ctx* c, cudaStream_t s) {
-    if (c->k_ready) return LRES_OK;
+    if (c->k_ready && !c->replayable) return LRES_OK;
     if (!c->d_K) TRY(dalloc(&c->d_K, c->sizeC));
     const bool tr = c->have_trace;
     TRY(gram_product(c, static_cast<const double*>(tr ? c->d_Ytr : c->d_Yown), tr, c->d_K, s));
@@ -1389,7 +1402,10 @@ extern "C" int lres_set_potential(lres_ctx* c, const double* v, int v_on_device,
         LRES_CUDA_TRY(cudaMemcpyAsync(c->d_v, v, sizeof(double) * c->ng, cudaMemcpyHostToDevice, s));
         dv = c->d_v;
     }
-    c->h_from_v = c->sp.sval32 != nullptr;
+    bool cap = false;
+    TRY(capturing(s, &cap));
+    if (cap) c->replayable = true;               // (H_W changes when the graph runs, not now)
+    else c->h_from_v = c->sp.sval32 != nullptr;
     TRY(mark(c, 2, 0, s));
     if (c->sp.sval32)
         // (v is kept: the mixed adjoint assembles H(v) again in FP64)
@@ -1945,8 +1961,15 @@ extern "C" int lres_set_windows(lres_ctx* c, const double* HW, const double* SW,
     cudaStream_t s = (cudaStream_t)stream;
     const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     c->h32_dense = false;                // the FP32 windows, if any, are of the previous H
+    bool cap = false;
+    TRY(capturing(s, &cap));
     if (HW) LRES_CUDA_TRY(cudaMemcpyAsync(c->d_HW, HW, sizeof(double) * c->sizeC, kind, s));
-    if (HW) c->h_from_v = false;
+    if (cap) {
+        c->replayable = true;
+        if (HW) c->hw_replayable = true;
+    } else if (HW) {
+        c->h_from_v = false;
+    }
     if (SW) {
         LRES_CUDA_TRY(cudaMemcpyAsync(c->d_SW, SW, sizeof(double) * c->sizeC, kind, s));
         if (needs_standard_form(c)) TRY(setup_standard_form(c, s));
@@ -2123,7 +2146,7 @@ int adj_tri_accumulate(lres_ctx* c, double mu, double e_lo, const double** Wt, c
         LRES_CUDA_TRY(cudaGetLastError());
         // H_W: where it is an FP32 H(v) again in FP64 (its 1e-8 Ha of the levels are 2e-6 of dN/dmu)
         const double* HW = c->d_HW;
-        if (c->h_from_v) {
+        if (c->h_from_v && !c->hw_replayable) {
             TRY(assemble_h(c->bp, c->sp, c->d_Tblk, c->d_v, c->dV, a.Hblk, s));
             TRY(gather_windows(c->nwin, c->nmax, c->d_gfn, c->d_gfnoff, c->d_gbtab, c->d_gbtoff, c->d_gnlg, c->d_offC,
                                c->d_n, a.Hblk, a.K, nullptr, nullptr, s));
