@@ -2378,6 +2378,7 @@ extern "C" int lres_set_trace_rows(lres_ctx* c, const int32_t* r_w, const double
     c->d_Ytr = nullptr;
     c->ri_tr.release();
     c->have_trace = false;
+    c->k_ready = false;                       // (K is of the rows that counts run over)
     if (!r_w) return LRES_OK;                 // removed
     if (!R) {
         lres_set_error("null argument");
