@@ -872,8 +872,9 @@ int tri_run_count(lres_ctx* c, cudaStream_t s) {
     return LRES_OK;
 }
 
-// The FP64 density pass through P (in place of the standard form, which the reduction has consumed).
-int tri_run_matrix(lres_ctx* c, cudaStream_t s) {
+// The FP64 density pass through P (in place of the standard form, which the reduction has consumed); count:
+// the sums only, the density is left as it is.
+int tri_run_matrix(lres_ctx* c, bool count, cudaStream_t s) {
     const int P = c->npoles;
     const lres_ctx::RowItems& ri = c->ri_own;
     const double *d = static_cast<const double*>(c->d_trid), *e = static_cast<const double*>(c->d_trie);
@@ -887,7 +888,8 @@ int tri_run_matrix(lres_ctx* c, cudaStream_t s) {
                     OzForm(false), c->d_Hhat, c->d_offC + w0, OzForm(true), c->d_V, c->d_offV + w0, 0, false,
                     c->smem_budget, s));
         TRY(tri_rowdot(w0, nb, c->max_pass_items, ri.pass, ri.first, ri.count, c->d_n, c->d_m, c->d_offN, c->d_offF,
-                       c->d_offV, c->d_offQ, c->d_Oflat, Y, c->d_V, d, e, c->d_dens, ri.part, c->d_status, s));
+                       c->d_offV, c->d_offQ, c->d_Oflat, Y, c->d_V, d, e, count ? nullptr : c->d_dens, ri.part,
+                       c->d_status, s));
     }
     TRY(mark(c, 0, 1, s));
     TRY(mark(c, 1, 0, s));
@@ -899,7 +901,7 @@ int tri_run_matrix(lres_ctx* c, cudaStream_t s) {
 // A pass at the nodes already set: the density and the windows' sums, or (count) the sums only.
 int tri_any_pass(lres_ctx* c, bool count, bool trace, cudaStream_t s) {
     if ((count || trace) && counts_from_k(c)) return tri_run_count(c, s);
-    if (!trace && c->by_matrix) return tri_run_matrix(c, s);
+    if (!trace && c->by_matrix) return tri_run_matrix(c, count, s);
     return tri_run_pass(c, count && c->precision == LRES_FP64, trace, s);
 }
 

@@ -1,4 +1,5 @@
-"""lres_count against the state that it may not rest on: trace rows exchanged after a count."""
+"""lres_count against the state that it may not rest on or touch: trace rows exchanged after a count, and the
+density array where K = Y^T Y finds no room on the device."""
 import numpy as np
 import pytest
 
@@ -40,3 +41,28 @@ def test_counts_follow_the_trace_rows():
     s.remove_trace_rows()
     assert np.array_equal(count(), own)
     s.close()
+
+
+def test_count_without_room_leaves_the_density():
+    """With 16 MB free on the device K (36 MB) does not fit: the count runs over the rows, gives the same sums (n
+    roundings of 54 windows: 1e-11) and leaves the density of the last pass where it is."""
+    import torch
+    from lresdft_gb300.autograd import device_tensor
+    warm = _solver(n=(3, 3, 3), rw=8.0)              # (every kernel loaded before the device is full)
+    want = warm.pole_pass(MU + 0.05, E_LO, want_density=False)[1:]
+    warm.pole_pass(MU, E_LO)
+    s = _solver(n=(3, 3, 3), rw=8.0)
+    dens = device_tensor(s.density_device_ptr(), s.b.cr.ng)
+    s.pole_pass(MU, E_LO)
+    before = dens.cpu().numpy().copy()
+    torch.cuda.synchronize()
+    hog = torch.empty(torch.cuda.mem_get_info()[0] - (16 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        got = s.pole_pass(MU + 0.05, E_LO, want_density=False)[1:]
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    assert np.array_equal(dens.cpu().numpy(), before)
+    assert np.allclose(got, want, rtol=1e-11, atol=0)
+    s.close()
+    warm.close()
