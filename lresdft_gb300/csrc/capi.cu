@@ -2062,7 +2062,7 @@ int adj_workspace(lres_ctx* c, size_t least, size_t want, size_t* got) {
         const size_t have = c->adjws_bytes + freeb, reserve = (size_t)4 << 30;
         const size_t budget = have > reserve ? std::min(have - reserve, have / 4 * 3) : 0;
         const size_t take = std::min(want, budget);
-        if (take < least) {
+        if (take < least && c->adjws_bytes < least) {
             lres_set_error("adjoint: the factors of one window (%zu bytes) do not fit in free device memory", least);
             return LRES_ENOMEM;
         }
@@ -2106,31 +2106,61 @@ bool adj_tri_buffers(lres_ctx* c, cudaStream_t s) {
     return a.ok();
 }
 
+// The workspace of those accumulations, as parts of d_adjws.
+struct AdjPlan {
+    int groups = 0, batch = 0;            // pole groups of a window, windows at a time
+    size_t coefb = 0, trb = 0, k32b = 0, head = 0;
+};
+
+// Room for the adjoint from the tridiagonal form; false if there is none, the adjoint then factors every
+// (window, pole).  All pole groups of a window at once take the most: with less, fewer groups run side by
+// side (one at least), each over more poles.
+bool adj_tri_room(lres_ctx* c, cudaStream_t s, AdjPlan* pl) {
+    const bool mixed = c->precision == LRES_MIXED;
+    int rc = LRES_OK;
+    if (mixed) {
+        if (!adj_tri_buffers(c, s)) return false;
+    } else {
+        if (!c->d_K) rc = dalloc(&c->d_K, c->sizeC);
+        if (!rc && !c->oz_adj.offS) rc = oz_setup_rows(c, c->n_w, c->oz_adj, s);
+        if (rc) c->oz_adj.release();
+    }
+    const int P = c->npoles;
+    pl->coefb = sizeof(double4) * tri_coef_elems(c->nwin, P, c->nmax) * (mixed ? 2 : 1);   // (and derivatives)
+    pl->trb = sizeof(double2) * (size_t)c->nwin * P;
+    pl->k32b = mixed ? (sizeof(float) * (size_t)c->sizeC + 15) / 16 * 16 : 0;
+    for (pl->groups = adj_sweep_groups(c->nwin, P); !rc; pl->groups /= 2) {
+        const size_t xb = pl->groups > 1 ? sizeof(double) * 3 * (size_t)pl->groups * c->sizeC : 0;
+        const size_t perw = (mixed ? sizeof(float2) : sizeof(double2)) * 2 * (size_t)c->nmax * c->nmax * pl->groups;
+        pl->head = pl->coefb + pl->trb + pl->k32b + xb;
+        size_t got = 0;
+        rc = adj_workspace(c, pl->head + perw, pl->head + perw * c->nwin, &got);
+        if (!rc) {
+            pl->batch = (int)std::min<size_t>(c->nwin, (got - pl->head) / perw);
+            return true;
+        }
+        cudaGetLastError();
+        if (rc == LRES_ENOMEM && pl->groups > 1) rc = LRES_OK;
+    }
+    cudaGetLastError();
+    return false;
+}
+
 // The accumulations of the adjoint from the FP64 tridiagonal form: per-window N and E_band, the density by
 // the pass, A_c in the tridiagonal basis into d_adjA, W = L^-T Q in *Wt (over the standard form, which the
 // reduction has consumed).  In mixed precision the tridiagonal form is made here (d_HW and L^-T are FP64)
 // and the sweeps run in FP32: 128 windows 89 -> 36 ms, the gradients 5e-7 off 64 bits against the
 // 2e-6 of FP32 factors.
-int adj_tri_accumulate(lres_ctx* c, double mu, double e_lo, const double** Wt, cudaStream_t s) {
+int adj_tri_accumulate(lres_ctx* c, const AdjPlan& pl, double mu, double e_lo, const double** Wt, cudaStream_t s) {
     const bool mixed = c->precision == LRES_MIXED;
     if (!c->tri_ready) TRY(tri_refresh(c, s));
     const int P = c->npoles;
-    const int groups = adj_sweep_groups(c->nwin, P);
-    const size_t coefb = sizeof(double4) * tri_coef_elems(c->nwin, P, c->nmax) * (mixed ? 2 : 1);   // (and derivatives)
-    const size_t trb = sizeof(double2) * (size_t)c->nwin * P;
-    const size_t k32b = mixed ? (sizeof(float) * (size_t)c->sizeC + 15) / 16 * 16 : 0;
-    const size_t xb = groups > 1 ? sizeof(double) * 3 * (size_t)groups * c->sizeC : 0;
-    const size_t perw = (mixed ? sizeof(float2) : sizeof(double2)) * 2 * (size_t)c->nmax * c->nmax * groups;
-    const size_t head = coefb + trb + k32b + xb;
-    size_t got = 0;
-    TRY(adj_workspace(c, head + perw, head + perw * c->nwin, &got));
-    const int batch = (int)std::min<size_t>(c->nwin, (got - head) / perw);
     char* const base = static_cast<char*>(c->d_adjws);
     double4* const coef = reinterpret_cast<double4*>(base);
-    double2* const trace = reinterpret_cast<double2*>(base + coefb);
-    float* const K32 = mixed ? reinterpret_cast<float*>(base + coefb + trb) : nullptr;
-    double* const X = reinterpret_cast<double*>(base + coefb + trb + k32b);
-    void* const ws = base + head;
+    double2* const trace = reinterpret_cast<double2*>(base + pl.coefb);
+    float* const K32 = mixed ? reinterpret_cast<float*>(base + pl.coefb + pl.trb) : nullptr;
+    double* const X = reinterpret_cast<double*>(base + pl.coefb + pl.trb + pl.k32b);
+    void* const ws = base + pl.head;
     const double2* shifts = static_cast<const double2*>(c->d_shifts);
     const double *d = static_cast<const double*>(c->d_trid), *e = static_cast<const double*>(c->d_trie);
     double *W = c->d_Hhat, *K = c->d_K;
@@ -2138,7 +2168,6 @@ int adj_tri_accumulate(lres_ctx* c, double mu, double e_lo, const double** Wt, c
     if (!mixed) {
         TRY(ensure_k(c, s));
         K = c->d_K;
-        if (!c->oz_adj.offS) TRY(oz_setup_rows(c, c->n_w, c->oz_adj, s));
         TRY(rows_fp64(c, c->oz_adj, c->d_n, c->d_LinvT, c->sizeC, W, s));
     } else {
         lres_ctx::AdjTri& a = c->at;
@@ -2178,7 +2207,7 @@ int adj_tri_accumulate(lres_ctx* c, double mu, double e_lo, const double** Wt, c
         K = a.K;
     }
     *Wt = W;
-    return adj_tri(c->nwin, P, groups, batch, c->nmax, c->d_order, c->d_n, c->d_offN, c->d_offC, c->sizeC, d, e, shifts,
+    return adj_tri(c->nwin, P, pl.groups, pl.batch, c->nmax, c->d_order, c->d_n, c->d_offN, c->d_offC, c->sizeC, d, e, shifts,
                    c->d_cw, K, K32, coef, ws, X, c->d_adjA[0], c->d_adjA[1], c->d_adjA[2], c->smem_budget, s);
 }
 
@@ -2256,17 +2285,18 @@ extern "C" int lres_adjoint(lres_ctx* c, double mu, double e_lo, double* dv, int
     }
     cudaStream_t s = (cudaStream_t)stream;
     const bool mixed = c->precision == LRES_MIXED;
-    const bool tri = c->route == LRES_ROUTE_TRIDIAG && (!mixed || adj_tri_buffers(c, s));
+    TRY(adj_prepare(c, s));
+    AdjPlan plan;
+    const bool tri = c->route == LRES_ROUTE_TRIDIAG && adj_tri_room(c, s, &plan);
     const int P = c->npoles;
     if (!tri) TRY(ensure_hhat_df(c, s));       // the LDL^T path factors the double-float standard form
-    TRY(adj_prepare(c, s));
     poles_kernel<<<(P + 63) / 64, 64, 0, s>>>(P, c->M, mu, e_lo, mixed ? 1 : 0, c->d_shifts, c->d_wq, c->d_wzq);
     LRES_CUDA_TRY(cudaGetLastError());
     TRY(adj_weights(P, c->M, mu, e_lo, c->d_cw, s));
     LRES_CUDA_TRY(cudaMemsetAsync(c->d_status, 0, sizeof(int), s));
     // the accumulations are in the basis of Wt: A_c = Wt X_c Wt^T (null: the windows' own)
     const double* Wt = mixed ? c->d_LinvT : nullptr;
-    if (tri) TRY(adj_tri_accumulate(c, mu, e_lo, &Wt, s));
+    if (tri) TRY(adj_tri_accumulate(c, plan, mu, e_lo, &Wt, s));
     else TRY(adj_ldl_accumulate(c, s));
     if (!tri || !mixed)                        // (with their accumulations otherwise)
         TRY(adj_inner(c->nwin, c->d_n, c->d_offC, Wt ? nullptr : c->d_SW, c->d_adjA[0], c->d_adjA[1], c->d_adjA[2],

@@ -1,0 +1,51 @@
+"""FP64 contexts on a device with little memory left: what the fast paths would like to have is taken as far as it
+is there, and the calls still answer.  The memory is taken by one tensor; allocations that fail are ordinary
+errors of the library."""
+import contextlib
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@contextlib.contextmanager
+def _free(nbytes):
+    """Device memory taken up to `nbytes`."""
+    import torch
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    hog = torch.empty(max(torch.cuda.mem_get_info()[0] - int(nbytes), 1), dtype=torch.uint8, device="cuda")
+    try:
+        yield
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("free_gb", [4.45, 4.2])
+def test_adjoint(free_gb):
+    """The adjoint keeps 4 GB of the device free.  One window of some 600 functions and 32 poles, all pole groups at
+    once, wants some 0.7 GB; with less it takes fewer groups at a time.  Gradients as with the whole device: the
+    same sums in another order, n roundings, 1e-10."""
+    from lresdft_gb300 import LResGPU, system
+    n, side = 600, 5
+    pos = np.array([((np.array([i, j, k]) + 0.5) * 2.0) for i in range(side) for j in range(side)
+                    for k in range(side)])[:n // 6]
+    cr = system.Crystal(pos, np.ones(len(pos)), np.full(3, 2.0 * side), (5 * side,) * 3, 1.0)
+    b = system.LCAOBasis(cr, rcut=1.3, atom_exps=[((2.0, 1.0, 0.5), (0.8,))] * len(pos))
+    s = LResGPU(b, cr.pos[:1], R_w=1e3, M=64, precision="fp64", route="tridiag", trace_rows=True)
+    s.set_potential(np.linspace(-0.4, 0.1, cr.ng))
+    lam = s.min_eig(-1.0, 0.0)                       # (some tens of levels below mu)
+    with _free(free_gb * 2 ** 30):
+        a = s.adjoint(lam + 3.0, lam - 0.3, windows=True)
+    r = LResGPU(b, cr.pos[:1], R_w=1e3, M=64, precision="fp64", route="tridiag", trace_rows=True)
+    r.set_potential(np.linspace(-0.4, 0.1, cr.ng))
+    w = r.adjoint(lam + 3.0, lam - 0.3, windows=True)
+    assert w["N"] > 1
+    for k in ("N", "E", "dNdmu", "dEdmu", "kappa"):
+        assert abs(a[k] - w[k]) <= 1e-10 * abs(w["N"])
+    for k in ("dv", "dHW", "dSW"):
+        assert np.max(np.abs(a[k] - w[k])) <= 1e-10 * np.max(np.abs(w[k])), k
+    s.close()
+    r.close()
