@@ -654,13 +654,13 @@ int oz_setup(lres_ctx* c, cudaStream_t s) {
     TRY(upload(&o.offV, offV, s));
     TRY(upload(&o.offT, offT, s));
     TRY(dalloc(&o.T, size));
-    // the workspace of every product of the context (standard form, rows, P, K, adjoint), so that none
-    // of them replaces it later under a captured pass
-    TRY(oz_reserve(c->oz, c->nwin, std::max(c->mmax, c->nmax), c->nmax, c->nmax));
-    TRY(oz_reserve(c->oz, c->nwin, c->nmax, c->nmax, std::max(c->mmax, c->nmax)));
     LRES_CUDA_TRY(cudaStreamSynchronize(s));     // the host vectors go out of scope
     return LRES_OK;
 }
+
+// The workspace of every product of the context (standard form, rows, P, K, adjoint), so that none of them
+// replaces it later under a captured pass; last of the context's buffers, it makes do with less room.
+int oz_workspace(lres_ctx* c) { return oz_reserve(c->oz, c->nwin, std::max(c->mmax, c->nmax), c->nmax); }
 
 // One row set of m[w] rows for them.
 int oz_setup_rows(lres_ctx* c, const std::vector<int>& m, OzRowSet& rs, cudaStream_t s) {
@@ -725,9 +725,36 @@ int tri_setup_matrix(lres_ctx* c, cudaStream_t s) {
     return LRES_OK;
 }
 
+void tri_release(lres_ctx* c) {
+    auto drop = [](auto*& p) {
+        if (p) cudaFree(p);
+        p = nullptr;
+    };
+    drop(c->d_triA);
+    drop(c->d_trid);
+    drop(c->d_trie);
+    drop(c->d_tritau);
+    drop(c->d_Yown);
+    drop(c->d_Ytr);
+    drop(c->d_lam);
+    drop(c->d_tstatus);
+    drop(c->d_triT);
+    c->triT_size = 0;
+    c->ri_own.release();
+    c->ri_tr.release();
+    c->ozr.release();
+    c->oz_own.release();
+    c->oz_trc.release();
+    c->oz.release();
+    drop(c->d_V);
+    drop(c->d_offV);
+    drop(c->d_coef);
+    c->by_matrix = false;
+    c->tri_alloc = c->tri_ready = c->k_ready = false;
+}
+
 // Buffers of the tridiagonal route (once per context).
-int tri_setup(lres_ctx* c, cudaStream_t s) {
-    if (c->tri_alloc) return LRES_OK;
+int tri_buffers(lres_ctx* c, cudaStream_t s) {
     const bool fp32 = c->precision == LRES_MIXED;
     const size_t el = fp32 ? sizeof(float) : sizeof(double);
     TRY(tri_pick(fp32, c->nmax, c->smem_budget, c->tri_cfg, &c->tri));
@@ -756,6 +783,18 @@ int tri_setup(lres_ctx* c, cudaStream_t s) {
             TRY(oz_setup_rows(c, mT, c->oz_trc, s));
         }
         TRY(tri_setup_matrix(c, s));
+        TRY(oz_workspace(c));
+    }
+    return LRES_OK;
+}
+
+int tri_setup(lres_ctx* c, cudaStream_t s) {
+    if (c->tri_alloc) return LRES_OK;
+    const int rc = tri_buffers(c, s);
+    if (rc) {
+        cudaGetLastError();
+        tri_release(c);
+        return rc;
     }
     c->tri_alloc = true;
     return LRES_OK;
@@ -1361,7 +1400,6 @@ extern "C" int lres_ctx_create(lres_ctx** out, const lres_system_desc* d, int pr
 
     // ---- standard form (mixed path; FP64 tridiagonal route)
     if (needs_standard_form(c.get())) TRY(setup_standard_form(c.get(), s));
-    if (c->route == LRES_ROUTE_TRIDIAG) TRY(tri_setup(c.get(), s));
 
     // ---- pass buffers
     TRY(dalloc((char**)&c->d_shifts, (size_t)c->npoles * 16));
@@ -1377,6 +1415,13 @@ extern "C" int lres_ctx_create(lres_ctx** out, const lres_system_desc* d, int pr
     c->ew_h.resize(c->nwin);
     TRY(fft3_create(&c->fft, c->shape, c->cell));
     TRY(dalloc(&c->d_fftwork, (size_t)c->shape[0] * c->shape[1] * (c->shape[2] / 2 + 1)));
+
+    // ---- buffers of the tridiagonal route; without room for them an FP64 context takes the other one
+    if (c->route == LRES_ROUTE_TRIDIAG) {
+        const int rc = tri_setup(c.get(), s);
+        if (rc == LRES_ENOMEM && precision == LRES_FP64) c->route = LRES_ROUTE_LDL;
+        else if (rc) return rc;
+    }
     LRES_CUDA_TRY(cudaStreamSynchronize(s));
     *out = c.release();
     return LRES_OK;
@@ -2095,6 +2140,7 @@ bool adj_tri_buffers(lres_ctx* c, cudaStream_t s) {
     if (!rc) rc = dalloc(&a.Hblk, c->bp.nval);
     if (!rc) rc = oz_setup(c, s);
     if (!rc) rc = oz_setup_rows(c, c->n_w, c->oz_adj, s);
+    if (!rc) rc = oz_workspace(c);
     if (!rc) rc = dalloc(&a.shifts, c->npoles);
     if (rc) {
         cudaGetLastError();

@@ -110,8 +110,10 @@ struct OzWork {
     size_t bytes = 0;
     void release();
 };
-// Workspace for products of these sizes; a product whose windows fit one by one allocates nothing.
-int oz_reserve(OzWork& wk, int nwin, int mmax, int nmax, int kmax);
+// Workspace for products of up to mmax (>= nmax) rows, nmax columns and nmax terms, or nmax rows and columns
+// and mmax terms: for all windows (up to 1 GB), or for as many at a time as the device has room for.  A
+// product whose windows fit one by one allocates nothing.
+int oz_reserve(OzWork& wk, int nwin, int mmax, int nmax);
 int oz_gemm(OzWork& wk, int nwin, int mmax, int nmax, int kmax, const int* m_w, const int* n_w, const int* k_w,
             const double* A, const long long* offA, OzForm fa, const double* B, const long long* offB, OzForm fb,
             double* C, const long long* offC, int klim, bool subtract, size_t smem_budget, cudaStream_t s);

@@ -329,18 +329,28 @@ static OzPlan oz_plan(int nwin, int mmax, int nmax, int kmax) {
     return p;
 }
 
-int oz_reserve(OzWork& wk, int nwin, int mmax, int nmax, int kmax) {
-    const OzPlan p = oz_plan(nwin, mmax, nmax, kmax);
-    const size_t need = p.perw * p.batch;
-    if (wk.bytes >= need) return LRES_OK;
+static int oz_alloc(OzWork& wk, size_t bytes) {
     wk.release();
-    if (cudaMalloc(&wk.buf, need) != cudaSuccess) {
+    if (cudaMalloc(&wk.buf, bytes) != cudaSuccess) {
         cudaGetLastError();
         wk.buf = nullptr;
-        lres_set_error("tensor-core FP64 product: allocation of %zu bytes failed", need);
+        lres_set_error("tensor-core FP64 product: allocation of %zu bytes failed", bytes);
         return LRES_ENOMEM;
     }
-    wk.bytes = need;
+    wk.bytes = bytes;
+    return LRES_OK;
+}
+
+int oz_reserve(OzWork& wk, int nwin, int mmax, int nmax) {
+    const OzPlan a = oz_plan(nwin, mmax, nmax, nmax), b = oz_plan(nwin, nmax, nmax, mmax);
+    const size_t least = std::max(a.perw, b.perw);
+    size_t bytes = std::max(a.perw * a.batch, b.perw * b.batch);
+    if (wk.bytes >= bytes) return LRES_OK;
+    // as much of it as the device has, in halves
+    while (oz_alloc(wk, bytes) != LRES_OK) {
+        if (bytes == least) return LRES_ENOMEM;
+        bytes = std::max(bytes / 2, least);
+    }
     return LRES_OK;
 }
 
@@ -356,7 +366,7 @@ int oz_gemm(OzWork& wk, int nwin, int mmax, int nmax, int kmax, const int* m_w, 
     // window does not fit
     const OzPlan p = oz_plan(nwin, mmax, nmax, kmax);
     if (wk.bytes < p.perw)
-        if (int rc = oz_reserve(wk, nwin, mmax, nmax, kmax)) return rc;
+        if (int rc = oz_alloc(wk, p.perw * p.batch)) return rc;
     const int Rp = p.Rp, Cp = p.Cp, Kp = p.Kp, batch = (int)std::min<size_t>(p.batch, wk.bytes / p.perw);
     unsigned short* const da = static_cast<unsigned short*>(wk.buf);
     // (a Gram product has one operand)

@@ -8,6 +8,8 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
+MU, E_LO = 0.02, -0.9
+
 
 @contextlib.contextmanager
 def _free(nbytes):
@@ -21,6 +23,52 @@ def _free(nbytes):
     finally:
         del hog
         torch.cuda.empty_cache()
+
+
+def _crystal():
+    from lresdft_gb300 import system
+    cr = system.jittered_h2((3, 3, 3), pts_per_cell=8, seed=5)
+    return system.LCAOBasis(cr), cr
+
+
+def test_creation_and_passes():
+    """A context of 54 windows of some 290 functions with less room than its digits' workspace (some 200 MB) would
+    take at its full size: fewer windows go at a time, the results are the same bit for bit.  With less than the
+    tridiagonal route's buffers need at all, the automatic choice is the other route."""
+    import torch
+
+    from lresdft_gb300 import LResGPU
+    b, cr = _crystal()
+    v = np.linspace(-0.4, 0.1, cr.ng)
+
+    def make():
+        s = LResGPU(b, cr.pos, R_w=8.0, M=16, precision="fp64", trace_rows=False)
+        s.set_potential(v)
+        return s, s.pole_pass(MU, E_LO)
+    warm, want = make()                              # (kernels loaded; the set-up's own temporaries measured away)
+    ldl = LResGPU(b, cr.pos, R_w=8.0, M=16, precision="fp64", trace_rows=False, route="ldl")
+    ldl.set_potential(v)
+    dl, Nl, El = ldl.pole_pass(MU, E_LO)
+    ldl.close()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    free0 = torch.cuda.mem_get_info()[0]
+    s, _ = make()
+    size = free0 - torch.cuda.mem_get_info()[0]
+    s.close()
+    with _free(size - (100 << 20)):
+        s, got = make()
+        assert s.route == "tridiag"
+    assert np.array_equal(got[0], want[0]) and got[1:] == want[1:]
+    s.close()
+    warm.close()
+    with _free(size - (290 << 20)):                  # (its own buffers: 235 MB less without V and digits; the other route: 350)
+        s = LResGPU(b, cr.pos, R_w=8.0, M=16, precision="fp64", trace_rows=False)
+        assert s.route == "ldl"
+    s.set_potential(v)                               # (its workspace is taken by the first pass)
+    dl1, Nl1, El1 = s.pole_pass(MU, E_LO)
+    assert np.array_equal(dl1, dl) and (Nl1, El1) == (Nl, El)
+    s.close()
 
 
 @pytest.mark.parametrize("free_gb", [4.45, 4.2])
