@@ -36,6 +36,7 @@ int dalloc(T** p, size_t count) {
     if (count == 0) count = 1;
     cudaError_t e = cudaMalloc((void**)p, sizeof(T) * count);
     if (e != cudaSuccess) {
+        cudaGetLastError();              // (or the next launch would be taken for failed)
         lres_set_error("cudaMalloc of %zu bytes failed: %s", sizeof(T) * count, cudaGetErrorString(e));
         return LRES_ENOMEM;
     }

@@ -134,6 +134,7 @@ enum : int {
     do {                                                                             \
         cudaError_t _e = (expr);                                                     \
         if (_e != cudaSuccess) {                                                     \
+            cudaGetLastError();   /* or the next launch would be taken for failed */ \
             ::lres_set_error("%s:%d: %s: %s", __FILE__, __LINE__, #expr,             \
                              cudaGetErrorString(_e));                                \
             return LRES_ECUDA;                                                       \

@@ -83,6 +83,7 @@ int fft3_create(FFT3** out, const int64_t shape[3], const double cell[3]) {
         cudaMalloc(&f->d_k, sizeof(double) * total) != cudaSuccess ||
         cudaMemcpy(f->d_tw, tw.data(), sizeof(double2) * total, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(f->d_k, kv.data(), sizeof(double) * total, cudaMemcpyHostToDevice) != cudaSuccess) {
+        cudaGetLastError();
         fft3_destroy(f);
         lres_set_error("FFT plan allocation failed");
         return LRES_ENOMEM;

@@ -71,6 +71,17 @@ def test_creation_and_passes():
     s.close()
 
 
+def test_a_refused_context_leaves_nothing():
+    """The failed allocation of one call is not the next one's error."""
+    from lresdft_gb300 import LResGPU, _lib
+    b, cr = _crystal()
+    with _free(48 << 20):
+        with pytest.raises(_lib.LResError, match="out of memory"):
+            LResGPU(b, cr.pos, R_w=8.0, M=16, precision="fp64", trace_rows=False)
+        owner = _lib.voronoi_owner(cr.shape, cr.cell, cr.pos)
+    assert owner.size == cr.ng
+
+
 @pytest.mark.parametrize("free_gb", [4.45, 4.2])
 def test_adjoint(free_gb):
     """The adjoint keeps 4 GB of the device free.  One window of some 600 functions and 32 poles, all pole groups at
