@@ -183,13 +183,14 @@ def roofline_of(name, ms, nW, mW, P, nnz_h, peaks):
             "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)" if peaks else "fallback"}
 
 
-def oz_launches(nwin, m, n, k, gram=False):
-    """Launches of one FP64 product of all windows on the tensor cores (csrc/oz_gemm.cu): the digits
-    of both operands (one of a Gram product) and the product, per batch of 1 GB of digits."""
+def oz_launches(nwin, m, n, k, gram=False, balance=False):
+    """Launches of one FP64 product of all windows on the tensor cores (csrc/oz_gemm.cu): the balance
+    of the terms (standard form), the digits of both operands (one of a Gram product) and the product,
+    per batch of 1 GB of digits."""
     up = lambda x, t: -(-max(x, 1) // t) * t
-    per_window = 18 * (up(m, 64) + up(n, 64)) * up(k, 32) + 4 * (up(m, 64) + up(n, 64))
+    per_window = 18 * (up(m, 64) + up(n, 64)) * up(k, 32) + 4 * (up(m, 64) + up(n, 64) + up(k, 32))
     batch = min(nwin, max((1 << 30) // per_window, 1))
-    return (2 if gram else 3) * -(-nwin // batch)
+    return ((2 if gram else 3) + balance) * -(-nwin // batch)
 
 
 def launches_per_step(route, precision, tile_config=0, standard_form="simt", nW=(), mW=()):
@@ -206,7 +207,7 @@ def launches_per_step(route, precision, tile_config=0, standard_form="simt", nW=
         # FP64: assemble_h, gather, reduction, T factors, pole nodes, diagonals of G, P, rows' sums
         # (V a batch of windows at a time, 1 GB), window sums; the products: 2 of the standard form,
         # V^T V and 3 of the rows per panel of 128 reflectors, V = Y P
-        total = 9 + 2 * oz_launches(nwin, n, n, n)
+        total = 9 + 2 * oz_launches(nwin, n, n, n, balance=True)
         for j0 in range(0, n - 2, 128):
             q, r = min(128, n - 2 - j0), n - 1 - j0
             total += oz_launches(nwin, q, q, r, gram=True) + oz_launches(nwin, m, q, r)

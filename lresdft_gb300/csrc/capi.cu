@@ -404,10 +404,12 @@ int transform_f32(lres_ctx* c, cudaStream_t s) {
     return LRES_OK;
 }
 
-// FP64 product of window matrices (n x n, column-major): C = op(A) op(B), (at) A^T B, (not bk) A B^T.
-int square_gemm(lres_ctx* c, const double* A, bool at, const double* B, bool bk, double* C, int klim, cudaStream_t s) {
+// FP64 product of window matrices (n x n, column-major): C = op(A) op(B), (at) A^T B, (not bk) A B^T; balance
+// where the sum runs over basis functions, which may differ in size.
+int square_gemm(lres_ctx* c, const double* A, bool at, const double* B, bool bk, double* C, int klim, bool balance,
+                cudaStream_t s) {
     return oz_gemm(c->oz, c->nwin, c->nmax, c->nmax, c->nmax, c->d_n, c->d_n, c->d_n, A, c->d_offC, OzForm(at),
-                   B, c->d_offC, OzForm(bk), C, c->d_offC, klim, false, c->smem_budget, s);
+                   B, c->d_offC, OzForm(bk), C, c->d_offC, klim, false, balance, c->smem_budget, s);
 }
 
 // FP64 (the FP64 tridiagonal route); the product H LinvT lives in the working blocks of the
@@ -418,8 +420,8 @@ int transform_fp64(lres_ctx* c, cudaStream_t s) {
         lres_set_error("FP64 standard form without the tridiagonal buffers");
         return LRES_ESTATE;
     }
-    TRY(square_gemm(c, c->d_HW, false, c->d_LinvT, true, Y, 1, s));
-    TRY(square_gemm(c, c->d_LinvT, true, Y, true, c->d_Hhat, 2, s));
+    TRY(square_gemm(c, c->d_HW, false, c->d_LinvT, true, Y, 1, true, s));
+    TRY(square_gemm(c, c->d_LinvT, true, Y, true, c->d_Hhat, 2, true, s));
     return LRES_OK;
 }
 
@@ -874,7 +876,7 @@ int tri_run_pass(lres_ctx* c, bool count, bool trace, cudaStream_t s) {
 int gram_product(lres_ctx* c, const double* R, bool trace, double* C, cudaStream_t s) {
     const long long* off = trace ? c->d_offFT : c->d_offF;
     return oz_gemm(c->oz, c->nwin, c->nmax, c->nmax, trace ? c->mmaxT : c->mmax, c->d_n, c->d_n, trace ? c->d_mT : c->d_m,
-                   R, off, OzForm(true), R, off, OzForm(true), C, c->d_offC, 0, false, c->smem_budget, s);
+                   R, off, OzForm(true), R, off, OzForm(true), C, c->d_offC, 0, false, false, c->smem_budget, s);
 }
 
 // Trials of the chemical potential need no rows when K = Y^T Y is there (FP64); where its buffers do
@@ -926,7 +928,7 @@ int tri_run_matrix(lres_ctx* c, bool count, cudaStream_t s) {
         const int w0 = c->vbatch[i], nb = c->vbatch[i + 1] - w0;
         TRY(oz_gemm(c->oz, nb, c->mmax, c->nmax, c->nmax, c->d_m + w0, c->d_n + w0, c->d_n + w0, Y, c->d_offF + w0,
                     OzForm(false), c->d_Hhat, c->d_offC + w0, OzForm(true), c->d_V, c->d_offV + w0, 0, false,
-                    c->smem_budget, s));
+                    false, c->smem_budget, s));
         TRY(tri_rowdot(w0, nb, c->max_pass_items, ri.pass, ri.first, ri.count, c->d_n, c->d_m, c->d_offN, c->d_offF,
                        c->d_offV, c->d_offQ, c->d_Oflat, Y, c->d_V, d, e, count ? nullptr : c->d_dens, ri.part,
                        c->d_status, s));
@@ -2230,8 +2232,8 @@ int adj_tri_accumulate(lres_ctx* c, const AdjPlan& pl, double mu, double e_lo, c
                                c->d_n, a.Hblk, a.K, nullptr, nullptr, s));
             HW = a.K;
         }
-        TRY(square_gemm(c, HW, false, c->d_LinvT, true, a.A, 1, s));
-        TRY(square_gemm(c, c->d_LinvT, true, a.A, true, a.H, 2, s));
+        TRY(square_gemm(c, HW, false, c->d_LinvT, true, a.A, 1, true, s));
+        TRY(square_gemm(c, c->d_LinvT, true, a.A, true, a.H, 2, true, s));
         TRY(tri_reduce(false, c->nwin, c->d_order_w, c->d_counter, c->d_n, c->d_offC, c->d_offA, c->d_offN, a.H, a.A, a.d,
                        a.e, a.tau, c->d_status, pk, c->nmax, c->smem_budget, s));
         TRY(oz_tfactors(c->oz, c->ozr, c->nwin, c->nmax, c->d_n, a.A, a.tau, c->d_offN, c->smem_budget, s));
@@ -2239,8 +2241,8 @@ int adj_tri_accumulate(lres_ctx* c, const AdjPlan& pl, double mu, double e_lo, c
         TRY(oz_rows(c->oz, c->ozr, c->oz_adj, c->nwin, c->nmax, c->d_n, c->d_n, a.A, a.H, c->smem_budget, s));
         // K = W^T (F^T F) W
         TRY(gram_product(c, c->have_trace ? c->d_FT : c->d_F, c->have_trace, a.K, s));
-        TRY(square_gemm(c, a.K, false, a.H, true, c->d_adjA[0], 0, s));
-        TRY(square_gemm(c, a.H, true, c->d_adjA[0], true, a.K, 0, s));
+        TRY(square_gemm(c, a.K, false, a.H, true, c->d_adjA[0], 0, true, s));
+        TRY(square_gemm(c, a.H, true, c->d_adjA[0], true, a.K, 0, true, s));
         TRY(tri_count(c->nwin, P, c->nmax, c->d_n, c->d_offN, c->d_offC, a.d, a.e, a.K, a.shifts, c->d_wq, c->d_wzq, c->dV,
                       coef, trace, c->d_nw, c->d_ew, c->d_status, c->smem_budget, s));
         // the inner products <S, A_c> = tr(X_c) in FP64 (the FP32 X_c leave 1e-6 of N in dN/dmu)
@@ -2386,8 +2388,8 @@ extern "C" int lres_adjoint(lres_ctx* c, double mu, double e_lo, double* dv, int
         for (int which = 0; which < 2; ++which) {
             const double* B = which ? c->d_adjA[2] : c->d_adjA[0];
             double* D = which ? c->d_dSW : c->d_dHW;
-            TRY(square_gemm(c, Wt, false, B, true, c->d_adjA[1], 0, s));
-            TRY(square_gemm(c, c->d_adjA[1], false, Wt, false, D, 0, s));
+            TRY(square_gemm(c, Wt, false, B, true, c->d_adjA[1], 0, false, s));
+            TRY(square_gemm(c, c->d_adjA[1], false, Wt, false, D, 0, false, s));
         }
     } else {
         TRY(adj_combine(c->sizeC, c->d_adjA[0], c->d_adjA[1], c->d_adjA[2], kappa, sc, -sc, c->d_dHW, c->d_dSW,

@@ -98,7 +98,8 @@ int build_F(int nwin, const long long* Xp, const int* Xi, const double* Xv, cons
             const long long* offF, const int* m_w, int mmax, double* F, cudaStream_t s);
 // FP64 products on the tensor cores (oz_gemm.cu): C_w = op(A_w) op(B_w) (or C_w -= it), C_w m_w x n_w
 // column-major at offC, K = k_w terms.  klim 1: op(B) upper triangular, 2: op(A) lower triangular and
-// the lower triangle of C only.  The workspace grows on demand.
+// the lower triangle of C only.  balance: the terms' factors are brought to one size first (operands whose
+// elements vary along k; plain storage).  The workspace grows on demand.
 struct OzForm {                       // how an operand is stored
     bool k_contig;                    // op(A)(i, k) at A[k + i ld] (op(B)(k, j) at B[k + j ld]), else at A[i + k ld] (B[j + k ld])
     const int* ld = nullptr;          // leading dimension ld[w] rounded up to 4; none: that of a dense block
@@ -116,7 +117,8 @@ struct OzWork {
 int oz_reserve(OzWork& wk, int nwin, int mmax, int nmax);
 int oz_gemm(OzWork& wk, int nwin, int mmax, int nmax, int kmax, const int* m_w, const int* n_w, const int* k_w,
             const double* A, const long long* offA, OzForm fa, const double* B, const long long* offB, OzForm fb,
-            double* C, const long long* offC, int klim, bool subtract, size_t smem_budget, cudaStream_t s);
+            double* C, const long long* offC, int klim, bool subtract, bool balance, size_t smem_budget,
+            cudaStream_t s);
 int batched_gram(int nwin, const int* n_w, const int* m_w, const long long* offF, const long long* offK, int nmax,
                  const double* F, double* K, cudaStream_t s);
 int batched_gemm_rect_upper(int nwin, const int* n_w, const int* m_w, const long long* offA, const long long* offU,

@@ -5,12 +5,17 @@
 // digits of 7 bits, exact in bf16 (the error-free splitting of Ozaki, Ogita, Oishi and Rump, Numer.
 // Algorithms 59 (2012) 95-118).  Products of digits sum exactly in the FP32 accumulators: 64 x 64 x
 // 9 pairs x 448 terms < 2^24 (longer sums are taken in runs of 448).  The 45 digit pairs s + t <= 8
-// are kept, summed by s + t in 9 accumulators and joined with two roundings.  What is dropped is below
-// 2^-62 of the row's and the column's largest value per term: 9 bits less than FP64's rounding of
-// the largest elements, so that the smaller ones keep FP64's accuracy too (8 digits: 2^-55, a fifth
-// less time, and the density of 54 windows 2.1e-14 off 64 bits against 1.6e-14, the FP64 pipe's error).
+// are kept, summed by s + t in 9 accumulators and joined with two roundings.
 //
-// Two kernels: oz_slice_kernel writes the digits of an operand ([digit][row][k], k contiguous), each
+// Error: per term at most 2^-58, as a rule 2^-62, of the product of the row's and the column's largest element
+// (the eight pairs s + t = 9 that are dropped first, 64 x 64 each at most, in units of 2^-73), where the
+// FP64 pipe errs by 2^-53 of the term itself: more accurate where the terms are of one size, less where a term
+// lies more than 2^-5 to 2^-9 below that product and matters all the same.  What makes them so in the sums over
+// basis functions, functions of different size, is taken out first (oz_balance_kernel).
+// (8 digits: 2^-51 and 2^-55, a fifth less time, and the density of 54 windows 2.1e-14 off 64 bits against
+// 1.6e-14, the FP64 pipe's error.)
+//
+// Kernels: oz_slice_kernel writes the digits of an operand ([digit][row][k], k contiguous), each
 // element once; oz_gemm_kernel, one CTA per 64 x 64 tile, stages 32 terms of all digits of both
 // operands by cp.async (three stages of 72 KB) and issues 45 m16n8k16 products per warp tile and 16
 // terms, 8 warps of 32 x 16.  The digit pairs bound it: 45 x 4096 flops per 2048 multiply-adds at
@@ -39,6 +44,7 @@ constexpr int kOzStages = 3;
 constexpr int kOzNT = 256;
 constexpr int kOzRun = 448;                   // terms that sum exactly: kDig 64 64 kOzRun <= 2^24
 constexpr int kOzBad = 1 << 20;               // exponent of a row with a non-finite value
+constexpr int kOzNone = -(1 << 13);           // that of a row of zeros
 constexpr int kStageBytes = 2 * kDig * kOzT * kOzK * 2;
 constexpr int kOzSmem = kOzStages * kStageBytes;
 
@@ -58,8 +64,51 @@ __device__ __forceinline__ int ilogb_bits(double x) {
     return e == 0 ? -1022 : e - 1023;
 }
 
-// Digits of 32 rows of one window: dig[((slot * kDig + s) * Rp + r) * Kp + k], ex[slot * Rp + r].
-__global__ void __launch_bounds__(256) oz_slice_kernel(int w0, Operand o, int Rp, int Kp, unsigned short* dig, int* ex) {
+// A digit's place is fixed by the largest element of its row, so an operand whose elements grow along k against a
+// partner that falls (H_W and L^-T of basis functions of different size) would keep few bits of the terms
+// that matter.  Term k is therefore taken as (a 2^s) (b 2^-s), s the exponent of its largest b: what is dropped
+// then lies below the largest term of the product's row, and scaling the basis functions by powers of two
+// changes no digit.  Non-finite elements are left out (their columns are given up anyway).  One read of B (the
+// standard form's two products of 54 windows of 290 functions 0.76 -> 0.81 ms, of 432 5.6 -> 5.9 ms).
+__global__ void __launch_bounds__(256) oz_balance_kernel(int w0, Operand b, int Kp, int* sk) {
+    __shared__ int top[32];
+    const int slot = blockIdx.y, w = w0 + slot, k0 = blockIdx.x * 32;
+    const int R = b.rows[w], K = b.cols[w];
+    if (k0 >= K) return;
+    const double* const X = b.X + b.off[w];
+    const long long ld = b.f.ld ? (b.f.ld[w] + 3) & ~3 : b.f.k_contig ? K : R;
+    const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
+    auto exponent = [](double x) {
+        const int e = ilogb_bits(x);
+        return x != 0.0 && e < 1024 ? e : kOzNone;
+    };
+    if (tid < 32) top[tx] = kOzNone;
+    __syncthreads();
+    if (b.f.k_contig) {
+        int e = kOzNone;
+        if (k0 + tx < K) {
+#pragma unroll 8
+            for (int r = ty; r < R; r += 8) e = max(e, exponent(X[k0 + tx + r * ld]));
+        }
+        atomicMax(&top[tx], e);
+    } else {
+        for (int k = ty; k < 32; k += 8) {
+            int e = kOzNone;
+            if (k0 + k < K)
+                for (int r = tx; r < R; r += 32) e = max(e, exponent(X[r + (k0 + k) * ld]));
+            e = __reduce_max_sync(0xffffffffu, e);
+            if (tx == 0) top[k] = e;
+        }
+    }
+    __syncthreads();
+    if (tid < 32) sk[(size_t)slot * Kp + k0 + tx] = max(top[tx], -2400);   // (b zero throughout: a is put out of the way)
+}
+
+// Digits of 32 rows of one window: dig[((slot * kDig + s) * Rp + r) * Kp + k], ex[slot * Rp + r]; element (r, k)
+// times 2^(sign sk[slot Kp + k]), sign 0, 1 or -1.
+template <int SIGN>
+__global__ void __launch_bounds__(256) oz_slice_kernel(int w0, Operand o, int Rp, int Kp, const int* sk,
+                                                       unsigned short* dig, int* ex) {
     __shared__ double tile[32][33];
     __shared__ int emax[32];
     const int slot = blockIdx.y, w = w0 + slot, r0 = blockIdx.x * 32;
@@ -72,32 +121,31 @@ __global__ void __launch_bounds__(256) oz_slice_kernel(int w0, Operand o, int Rp
         if (o.f.refl && i <= l) return i == l ? 1.0 : 0.0;
         return X[i + l * ld];
     };
+    const int* const sw = SIGN ? sk + (size_t)slot * Kp : nullptr;
+    auto exponent = [&](double x, int k) {
+        const int e = ilogb_bits(x);
+        return x == 0.0 ? kOzNone : e == 1024 ? kOzBad : SIGN ? e + SIGN * sw[k] : e;
+    };
     const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
-    if (tid < 32) emax[tid] = -1100;
+    if (tid < 32) emax[tid] = kOzNone;
     __syncthreads();
     // the largest exponent of every row
     if (o.f.k_contig) {
         for (int r = ty; r < 32; r += 8) {
-            int e = -1100;
+            int e = kOzNone;
             if (r0 + r < R)
-                for (int k = tx; k < K; k += 32) {
-                    const double x = at(r0 + r, k);
-                    if (x != 0.0) e = max(e, ilogb_bits(x));
-                }
+                for (int k = tx; k < K; k += 32) e = max(e, exponent(at(r0 + r, k), k));
             e = __reduce_max_sync(0xffffffffu, e);
             if (tx == 0) emax[r] = e;
         }
     } else {
-        int e = -1100;
+        int e = kOzNone;
         if (r0 + tx < R)
-            for (int k = ty; k < K; k += 8) {
-                const double x = at(r0 + tx, k);
-                if (x != 0.0) e = max(e, ilogb_bits(x));
-            }
+            for (int k = ty; k < K; k += 8) e = max(e, exponent(at(r0 + tx, k), k));
         atomicMax(&emax[tx], e);
     }
     __syncthreads();
-    if (tid < 32) ex[(size_t)slot * Rp + r0 + tid] = emax[tid] == 1024 ? kOzBad : emax[tid];
+    if (tid < 32) ex[(size_t)slot * Rp + r0 + tid] = emax[tid];
     const int r = tid >> 3, kq = (tid & 7) * 4;                     // this thread: row r, 4 terms
     const int E = emax[r];
     for (int k0 = 0; k0 < Kp; k0 += 32) {
@@ -121,7 +169,8 @@ __global__ void __launch_bounds__(256) oz_slice_kernel(int w0, Operand o, int Rp
             const int ef = (int)((b >> 52) & 0x7ff);
             long long m = b & 0xfffffffffffffLL;
             if (ef) m |= 1LL << 52;
-            const int sh = (ef ? ef - 1023 : -1022) - E + kTop;     // q = x 2^(52 + kTop - E) < 2^62
+            const int s2 = SIGN && k0 + kq + u < K ? SIGN * sw[k0 + kq + u] : 0;
+            const int sh = (ef ? ef - 1023 : -1022) + s2 - E + kTop;   // q = x 2^(52 + kTop + s2 - E) < 2^62
             long long q = 0;
             if (m == 0) q = 0;
             else if (sh >= 0) q = m << sh;                           // (sh <= kTop)
@@ -176,7 +225,7 @@ __device__ __forceinline__ double oz_join(const float (&a)[kDig]) {
 }
 
 // KLIM: 1, B upper triangular (k <= column); 2, A lower triangular (k <= row) and the
-// lower triangle of C only.  LONG: sums of more than 512 terms.
+// lower triangle of C only.  LONG: sums of more than kOzRun terms.
 template <int KLIM, bool LONG>
 __global__ void __launch_bounds__(kOzNT, 1) oz_gemm_kernel(int w0, const int* m_w, const int* n_w, const int* k_w,
                                                            int Rp, int Cp, int Kp, const unsigned short* da,
@@ -324,7 +373,7 @@ static OzPlan oz_plan(int nwin, int mmax, int nmax, int kmax) {
     p.Rp = (mmax + kOzT - 1) / kOzT * kOzT;
     p.Cp = (nmax + kOzT - 1) / kOzT * kOzT;
     p.Kp = (std::max(kmax, 1) + kOzK - 1) / kOzK * kOzK;
-    p.perw = sizeof(unsigned short) * kDig * (size_t)(p.Rp + p.Cp) * p.Kp + sizeof(int) * (size_t)(p.Rp + p.Cp);
+    p.perw = sizeof(unsigned short) * kDig * (size_t)(p.Rp + p.Cp) * p.Kp + sizeof(int) * (size_t)(p.Rp + p.Cp + p.Kp);
     p.batch = (int)std::min<size_t>({(size_t)nwin, std::max<size_t>(((size_t)1 << 30) / p.perw, 1), (size_t)65535});
     return p;
 }
@@ -356,7 +405,7 @@ int oz_reserve(OzWork& wk, int nwin, int mmax, int nmax) {
 
 int oz_gemm(OzWork& wk, int nwin, int mmax, int nmax, int kmax, const int* m_w, const int* n_w, const int* k_w,
             const double* A, const long long* offA, OzForm fa, const double* B, const long long* offB, OzForm fb,
-            double* C, const long long* offC, int klim, bool subtract, size_t smem_budget, cudaStream_t s) {
+            double* C, const long long* offC, int klim, bool subtract, bool balance, size_t smem_budget, cudaStream_t s) {
     if (nwin < 1 || mmax < 1 || nmax < 1) return LRES_OK;
     if ((size_t)kOzSmem > smem_budget) {
         lres_set_error("tensor-core FP64 product needs %d B of shared memory", kOzSmem);
@@ -375,6 +424,7 @@ int oz_gemm(OzWork& wk, int nwin, int mmax, int nmax, int kmax, const int* m_w, 
     unsigned short* const db = same ? da : da + (size_t)batch * kDig * Rp * Kp;
     int* const ea = reinterpret_cast<int*>(da + (size_t)batch * kDig * (Rp + Cp) * Kp);
     int* const eb = same ? ea : ea + (size_t)batch * Rp;
+    int* const sk = balance && !same ? ea + (size_t)batch * (Rp + Cp) : nullptr;
     const bool lng = kmax > kOzRun;
     int per_sm = 0;
     auto launch = [&](auto kern, int w0, int nb) {
@@ -383,9 +433,11 @@ int oz_gemm(OzWork& wk, int nwin, int mmax, int nmax, int kmax, const int* m_w, 
     };
     for (int w0 = 0; w0 < nwin; w0 += batch) {
         const int nb = std::min(batch, nwin - w0);
-        oz_slice_kernel<<<dim3(Rp / 32, nb), 256, 0, s>>>(w0, Operand{A, offA, m_w, k_w, fa}, Rp, Kp, da, ea);
+        const Operand oa{A, offA, m_w, k_w, fa}, ob{B, offB, n_w, k_w, fb};
+        if (sk) oz_balance_kernel<<<dim3(Kp / 32, nb), 256, 0, s>>>(w0, ob, Kp, sk);
+        (sk ? oz_slice_kernel<1> : oz_slice_kernel<0>)<<<dim3(Rp / 32, nb), 256, 0, s>>>(w0, oa, Rp, Kp, sk, da, ea);
         if (!same)
-            oz_slice_kernel<<<dim3(Cp / 32, nb), 256, 0, s>>>(w0, Operand{B, offB, n_w, k_w, fb}, Cp, Kp, db, eb);
+            (sk ? oz_slice_kernel<-1> : oz_slice_kernel<0>)<<<dim3(Cp / 32, nb), 256, 0, s>>>(w0, ob, Cp, Kp, sk, db, eb);
         LRES_CUDA_TRY(cudaGetLastError());
 #define OZ_RUN(KL, LG)                                                                  \
     do {                                                                                \
@@ -486,7 +538,7 @@ int oz_tfactors(OzWork& wk, const OzRows& o, int nwin, int nmax, const int* n_w,
         const int *q = o.q + (size_t)p * nwin, *r = o.r + (size_t)p * nwin;
         const long long *offV = o.offV + (size_t)p * nwin, *offT = o.offT + (size_t)p * nwin;
         const OzForm v(true, n_w, true);
-        if (int rc = oz_gemm(wk, nwin, qm, qm, rm, q, q, r, A, offV, v, A, offV, v, o.T, offT, 0, false, smem_budget, s))
+        if (int rc = oz_gemm(wk, nwin, qm, qm, rm, q, q, r, A, offV, v, A, offV, v, o.T, offT, 0, false, false, smem_budget, s))
             return rc;
     }
     if (o.panels) {
@@ -508,13 +560,13 @@ int oz_rows(OzWork& wk, const OzRows& o, const OzRowSet& rs, int nwin, int nmax,
         const long long *offV = o.offV + (size_t)p * nwin, *offT = o.offT + (size_t)p * nwin;
         const long long* offY = rs.offY + (size_t)p * nwin;
         if (int rc = oz_gemm(wk, nwin, rs.mmax, qm, rm, m_w, q, r, Y, offY, OzForm(false), A, offV,
-                             OzForm(true, n_w, true), rs.S, rs.offS, 0, false, smem_budget, s))
+                             OzForm(true, n_w, true), rs.S, rs.offS, 0, false, false, smem_budget, s))
             return rc;
         if (int rc = oz_gemm(wk, nwin, rs.mmax, qm, qm, m_w, q, q, rs.S, rs.offS, OzForm(false), o.T, offT,
-                             OzForm(true), rs.S2, rs.offS, 1, false, smem_budget, s))
+                             OzForm(true), rs.S2, rs.offS, 1, false, false, smem_budget, s))
             return rc;
         if (int rc = oz_gemm(wk, nwin, rs.mmax, rm, qm, m_w, r, q, rs.S2, rs.offS, OzForm(false), A, offV,
-                             OzForm(false, n_w, true), Y, offY, 0, true, smem_budget, s))
+                             OzForm(false, n_w, true), Y, offY, 0, true, false, smem_budget, s))
             return rc;
     }
     return LRES_OK;
