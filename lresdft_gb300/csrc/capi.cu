@@ -97,6 +97,7 @@ struct lres_ctx {
     float *d_LinvT32 = nullptr, *d_Linv32 = nullptr;   // L^-T and L^-1 in FP32 (mixed tridiagonal route)
     bool hhat_df = false;                // d_Hhat32 holds the double-float transform of the current H_W
     double *d_Fhat64 = nullptr, *d_FhatT64 = nullptr;   // FP64 standard-form rows (FP64 tridiagonal route)
+    bool sf_stale = false;               // FP64: S_W or the trace rows changed on the LDL^T route
     long long sizeC = 0, sizeF = 0;
     // multi-shift tridiagonal route (tridiag.cu): T = Q^T H^ Q per window once per Hamiltonian,
     // rows Y = F^ Q, then each pass is one fused shifted-solve + pole-sum kernel
@@ -1671,7 +1672,8 @@ extern "C" int lres_set_route(lres_ctx* c, int32_t route, void* stream) {
     const int old = c->route;
     c->route = route;
     int rc = LRES_OK;
-    if (c->precision != LRES_MIXED && !c->d_LinvT) rc = setup_standard_form(c, s);
+    if (c->precision != LRES_MIXED && (!c->d_LinvT || c->sf_stale)) rc = setup_standard_form(c, s);
+    if (!rc) c->sf_stale = false;
     if (!rc) rc = tri_setup(c, s);
     if (!rc && c->have_h) {
         rc = window_transform(c, s);           // the route's standard form of the current H
@@ -2022,8 +2024,12 @@ extern "C" int lres_set_windows(lres_ctx* c, const double* HW, const double* SW,
     }
     if (SW) {
         LRES_CUDA_TRY(cudaMemcpyAsync(c->d_SW, SW, sizeof(double) * c->sizeC, kind, s));
-        if (needs_standard_form(c)) TRY(setup_standard_form(c, s));
-        else TRY(check_overlaps(c, s));
+        if (needs_standard_form(c)) {
+            TRY(setup_standard_form(c, s));
+        } else {
+            c->sf_stale = true;
+            TRY(check_overlaps(c, s));
+        }
     }
     if (needs_standard_form(c)) TRY(window_transform(c, s));
     if (c->route == LRES_ROUTE_TRIDIAG) TRY(tri_prepare(c, s));
@@ -2495,6 +2501,8 @@ extern "C" int lres_set_trace_rows(lres_ctx* c, const int32_t* r_w, const double
     } else if (needs_standard_form(c)) {
         TRY(dalloc(&c->d_FhatT64, c->sizeFT));
         TRY(trace_standard_form(c, s));
+    } else {
+        c->sf_stale = true;
     }
     if (c->tri_alloc) {
         TRY(build_row_items(c, m, c->ri_tr, s));
