@@ -63,8 +63,9 @@ enum { LRES_FP64 = 0, LRES_MIXED = 1 };
  *                       tridiagonal LDL^T of z I - T and one forward sweep per row (O(n)):
  *                       the mu trials of a density call cost O(P m n) each (tridiag.cu).
  * Both evaluate the same resolvent quadratic forms; the default is the tridiagonal route
- * unless the windows are too large for its shared-memory panels or the context has fewer
- * than 4 of them (in FP64: fewer than 4, and under 8 poles or over 512 functions). */
+ * unless the windows are too large for its shared-memory panels, the poles are more than 256
+ * or the context has fewer than 4 windows (in FP64: fewer than 4, and under 8 poles or over 512
+ * functions). */
 enum { LRES_ROUTE_LDL = 0, LRES_ROUTE_TRIDIAG = 1 };
 
 typedef struct lres_ctx lres_ctx;
@@ -155,7 +156,7 @@ int lres_autotune(lres_ctx* ctx, double mu, double e_lo, int32_t force_config, i
 
 /* Route of the pole solves (LRES_ROUTE_LDL or LRES_ROUTE_TRIDIAG, see above).  Switching
  * to the tridiagonal route allocates its buffers and, when a Hamiltonian is set, reduces
- * it (LRES_EINVAL if the windows are too large for the reduction); the tile configuration
+ * it (LRES_EINVAL if the windows are too large for the reduction or the poles more than 256); the tile configuration
  * of lres_autotune applies to the LDL^T kernel.  On the tridiagonal route lres_inertia and
  * lres_min_eig count by Sturm sequences of T - sigma, T being congruent to the pencil
  * (H_W, S_W) (for LRES_MIXED: of the FP32 standard form). */

@@ -761,7 +761,7 @@ void tri_release(lres_ctx* c) {
 int tri_buffers(lres_ctx* c, cudaStream_t s) {
     const bool fp32 = c->precision == LRES_MIXED;
     const size_t el = fp32 ? sizeof(float) : sizeof(double);
-    TRY(tri_pick(fp32, c->nmax, c->smem_budget, c->tri_cfg, &c->tri));
+    TRY(tri_pick(fp32, c->nmax, c->npoles, c->smem_budget, c->tri_cfg, &c->tri));
     TRY(ensure_tfactors(c));
     TRY(dalloc((char**)&c->d_triA, el * (size_t)c->sizeA));
     TRY(dalloc((char**)&c->d_trid, el * (size_t)c->sizeN));
@@ -1393,7 +1393,7 @@ extern "C" int lres_ctx_create(lres_ctx** out, const lres_system_desc* d, int pr
     TRY(upload(&c->d_order_w, c->order, s));
     {
         TriPick pk;
-        const bool fits = tri_pick(precision == LRES_MIXED, c->nmax, c->smem_budget, 0, &pk) == LRES_OK;
+        const bool fits = tri_pick(precision == LRES_MIXED, c->nmax, c->npoles, c->smem_budget, 0, &pk) == LRES_OK;
         lres_set_error("");
         // a few FP64 windows: the dense factorisations of 8 or more poles cost more than one CTA's
         // reduction (one window of 96 functions, 4096 points: a warm call 32 ms against 7.5 ms; its
@@ -1580,7 +1580,7 @@ extern "C" int lres_autotune(lres_ctx* c, double mu, double e_lo, int32_t force_
         // Hamiltonian (reduction + rows per configuration)
         auto apply_cfg = [&](int cfg) -> int {
             TriPick pk;
-            TRY(tri_pick(c->precision == LRES_MIXED, c->nmax, c->smem_budget, cfg, &pk));
+            TRY(tri_pick(c->precision == LRES_MIXED, c->nmax, c->npoles, c->smem_budget, cfg, &pk));
             c->tri_cfg = cfg;
             c->tri = pk;
             if (c->tri_alloc) {
@@ -1668,7 +1668,7 @@ extern "C" int lres_set_route(lres_ctx* c, int32_t route, void* stream) {
         return LRES_OK;
     }
     TriPick pk;
-    TRY(tri_pick(c->precision == LRES_MIXED, c->nmax, c->smem_budget, c->tri_cfg, &pk));
+    TRY(tri_pick(c->precision == LRES_MIXED, c->nmax, c->npoles, c->smem_budget, c->tri_cfg, &pk));
     const int old = c->route;
     c->route = route;
     int rc = LRES_OK;
@@ -2139,7 +2139,7 @@ bool adj_tri_buffers(lres_ctx* c, cudaStream_t s) {
     if (a.tried) return a.ok();
     a.tried = true;
     TriPick pk;
-    int rc = tri_pick(false, c->nmax, c->smem_budget, 0, &pk);
+    int rc = tri_pick(false, c->nmax, c->npoles, c->smem_budget, 0, &pk);
     if (!rc) rc = dalloc(&a.A, c->sizeA);
     if (!rc) rc = dalloc(&a.d, c->sizeN);
     if (!rc) rc = dalloc(&a.e, c->sizeN);
@@ -2227,7 +2227,7 @@ int adj_tri_accumulate(lres_ctx* c, const AdjPlan& pl, double mu, double e_lo, c
     } else {
         lres_ctx::AdjTri& a = c->at;
         TriPick pk;
-        TRY(tri_pick(false, c->nmax, c->smem_budget, 0, &pk));
+        TRY(tri_pick(false, c->nmax, c->npoles, c->smem_budget, 0, &pk));
         poles_kernel<<<(P + 63) / 64, 64, 0, s>>>(P, c->M, mu, e_lo, 0, a.shifts, c->d_wq, c->d_wzq);
         LRES_CUDA_TRY(cudaGetLastError());
         // H_W: where it is an FP32 H(v) again in FP64 (its 1e-8 Ha of the levels are 2e-6 of dN/dmu)

@@ -142,7 +142,8 @@ int pole_sums(int nwin, const long long* offQ, const int* m_w, const long long* 
               double* dens, double* n_w, double* e_w, cudaStream_t s);
 
 // Multi-shift tridiagonal route (tridiag.cu): R = float (fp32) or double.
-// Tile configuration of the tridiagonal route for windows of at most nmax functions.
+// Tile configuration of the tridiagonal route for windows of at most nmax functions and P poles; LRES_EINVAL
+// where they are too large or too many for its kernels.
 struct TriPick {
     int nb = 0, nt = 0;        // reduction panel width and threads
     int reg = 0;               // 1: the reduction holds each window on its SM (FP32, tridiag_reg.cu)
@@ -152,7 +153,7 @@ struct TriPick {
     int ldv = 0;               // shared vector length (multiple of 32, >= nmax)
     long long tstride = 0;     // T-factor elements per window (resident application)
 };
-int tri_pick(bool fp32, int nmax, size_t smem_budget, int cfg, TriPick* out);
+int tri_pick(bool fp32, int nmax, int P, size_t smem_budget, int cfg, TriPick* out);
 int tri_reduce(bool fp32, int nwin, const int* order, int* counter, const int* n_w, const long long* offC,
                const long long* offA, const long long* offN, const void* H, void* A, void* d, void* e, void* tau,
                int* status, const TriPick& pk, int nmax, size_t smem_budget, cudaStream_t s);

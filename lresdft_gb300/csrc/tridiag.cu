@@ -1907,7 +1907,11 @@ static const TriCfg kTriCfg[6] = {{16, 512, 32, 1, 1, 1, 128}, {16, 512, 32, 1, 
                                   {16, 512, 32, 1, 0, 0, 0},    {16, 512, 16, 1, 1, 0, 64},
                                   {16, 512, 32, 1, 1, 1, 32},   {8, 512, 32, 1, 1, 0, 128}};
 
-int tri_pick(bool fp32, int nmax, size_t smem_budget, int cfg, TriPick* out) {
+int tri_pick(bool fp32, int nmax, int P, size_t smem_budget, int cfg, TriPick* out) {
+    if (tri_rows_per_item(fp32, P) < 1) {
+        lres_set_error("the tridiagonal route takes at most %d poles (got %d)", kPassNT, P);
+        return LRES_EINVAL;
+    }
     const int el = fp32 ? 4 : 8;
     TriPick r;
     r.ldv = (std::max(nmax, 1) + 31) / 32 * 32;
