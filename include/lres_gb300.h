@@ -64,8 +64,8 @@ enum { LRES_FP64 = 0, LRES_MIXED = 1 };
  *                       the mu trials of a density call cost O(P m n) each (tridiag.cu).
  * Both evaluate the same resolvent quadratic forms; the default is the tridiagonal route
  * unless the windows are too large for its shared-memory panels, the poles are more than 256
- * or the context has fewer than 4 windows (in FP64: fewer than 4, and under 8 poles or over 512
- * functions). */
+ * or the context has fewer than 4 windows (in FP64: fewer than 4, and under 8 poles, over 512
+ * functions or few owned points, under 1000 for 30 functions, 200 for 100). */
 enum { LRES_ROUTE_LDL = 0, LRES_ROUTE_TRIDIAG = 1 };
 
 typedef struct lres_ctx lres_ctx;

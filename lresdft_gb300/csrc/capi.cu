@@ -1395,10 +1395,14 @@ extern "C" int lres_ctx_create(lres_ctx** out, const lres_system_desc* d, int pr
         TriPick pk;
         const bool fits = tri_pick(precision == LRES_MIXED, c->nmax, c->npoles, c->smem_budget, 0, &pk) == LRES_OK;
         lres_set_error("");
-        // a few FP64 windows: the dense factorisations of 8 or more poles cost more than one CTA's
-        // reduction (one window of 96 functions, 4096 points: a warm call 32 ms against 7.5 ms; its
-        // cost grows as n^3 on one SM, 15 ms at 512)
-        const bool few = precision == LRES_FP64 && c->npoles >= 8 && c->nmax <= 512;
+        // a few FP64 windows: a Hamiltonian and a pass take some 420 + 15 n us here (n launches' and columns'
+        // latency) and 180 + 5 n + 6e-4 m n^2 us by dense factorisations, all poles side by side.  So there where
+        // the rows are few: 3 windows of 24 functions and 200, 360 points 0.77 ms here against 0.46, 0.58, one of
+        // 512, 1000, 1728 points 0.72, 0.98, 1.44; 3 of 48 and 360, 595 points 1.10 against 0.94, 1.26; of 96 and
+        // 720 1.75 against 4.6, of 510 and 6875 24 against 635 ms.  (Further passes of the same Hamiltonian cost
+        // 0.1 to 0.8 ms here.)
+        const double n = c->nmax, m = c->mmax;
+        const bool few = precision == LRES_FP64 && c->npoles >= 8 && c->nmax <= 512 && m * n * n >= 4e5 + 17500.0 * n;
         c->route = (fits && (c->nwin >= 4 || few)) ? LRES_ROUTE_TRIDIAG : LRES_ROUTE_LDL;
     }
 
