@@ -124,8 +124,8 @@ int lres_pass(lres_ctx* ctx, double mu, double e_lo, double* dens, int dens_on_d
 
 /* N(mu) and E_band as lres_pass's out (and lres_window_sums), without a density: on the tridiagonal
  * route in FP64 as traces tr((z_k - T)^-1 Y^T Y) with Y^T Y formed once per Hamiltonian, the context's
- * density array left as it was (where Y^T Y does not fit the device, by a pass over the rows); otherwise the
- * same as lres_pass with dens == NULL. */
+ * density array left as it was (by a pass over the rows where Y^T Y does not fit the device, or the rows are
+ * fewer than 32 a window and the windows many); otherwise the same as lres_pass with dens == NULL. */
 int lres_count(lres_ctx* ctx, double mu, double e_lo, double* out, void* stream);
 
 /* The pass of lres_pass without any host synchronisation or host memory: pole nodes and

@@ -688,18 +688,30 @@ int oz_setup_rows(lres_ctx* c, const std::vector<int>& m, OzRowSet& rs, cudaStre
     return LRES_OK;
 }
 
-// Buffers of the FP64 density pass through P, where that is the cheaper one: 2.5 n^2 FP64 instructions
-// a pole and a product of m n^2 multiply-adds on the tensor cores (16 times the FP64 rate) against
-// 11 m n a pole.  Every size of the benchmark and the tests is on this side except windows of one
-// or two atoms' points.
+// Is the FP64 density pass through P the faster one?  Both in us, of the largest window (n functions, m rows) and
+// their number.  Over the rows: 4.3 us a function and wave of work items (half of it below 4 poles, which leave
+// most of an item's threads idle), an item holding 1024 / P rows of a window, 256 at most; a wave is an SM's
+// item, windows of more than some 128 functions fill one.  Through P: two chains of n steps, then per window
+// 1.4e-2 n^2 for every 32 poles or part of them (its warps hold 32), the product V = Y P and the rows'
+// two inner products, in tiles of 32.  Measured at 155 forms, n 6 to 312, m 41 to 4096, P 1 to 64, 1 to 432
+// windows (us, rows against P): 54 windows of 300 functions and 286 rows, 8 poles 1320, 1897, 16 poles 2475,
+// 1724, 32 poles 4770, 1689; the same with 41 rows, 64 poles 1316, 1993; 432 windows of 138 and 304, 2 poles
+// 1380, 2387, 8 poles 4002, 2267; 54 windows of 6 and 286, 8 poles 112, 156, 32 poles 212, 151.  The choice is
+// at most 3 % slower there than the rows, which every pass ran over once, and at most 17 % than the better one.
+bool pass_by_matrix(int nwin, int nmax, int mmax, int P) {
+    const double n = nmax, m = mmax, tiles = std::max(nmax, 32);
+    const int per_item = tri_rows_per_item(false, P);
+    const double w = (double)nwin * ((mmax + per_item - 1) / per_item) / 152;
+    const double waves = std::max(1.0, 0.75 * w + (nmax >= 128 ? 0.25 : -0.25));
+    const double rows = 60 + (4.3 * n + 25) * waves * (P < 4 ? 0.55 : 1.0);
+    const double matrix = 100 + 2.4 * n + nwin / 152.0 * (0.0144 * tiles * tiles * ((P + 31) / 32) +
+                                                         m * (0.008 * tiles + 1.6e-5 * tiles * tiles));
+    return matrix <= 0.9 * rows && nwin <= 65535;
+}
+
+// Buffers of that pass.
 int tri_setup_matrix(lres_ctx* c, cudaStream_t s) {
-    double rows = 0.0, mat = 0.0;
-    for (int w = 0; w < c->nwin; ++w) {
-        const double n = c->n_w[w], m = c->m_w[w];
-        rows += 11.0 * c->npoles * m * n;
-        mat += 2.5 * c->npoles * n * n + m * n * n / 16 + 12.0 * m * n;
-    }
-    if (mat > rows || c->nwin > 65535) return LRES_OK;
+    if (!pass_by_matrix(c->nwin, c->nmax, c->mmax, c->npoles)) return LRES_OK;
     const long long most = std::max<long long>((long long)1 << 27, 1);       // 1 GB of V
     std::vector<long long> offV(c->nwin, 0);
     long long size = 0, cur = 0;
@@ -881,9 +893,14 @@ int gram_product(lres_ctx* c, const double* R, bool trace, double* C, cudaStream
 }
 
 // Trials of the chemical potential need no rows when K = Y^T Y is there (FP64); where its buffers do
-// not fit, the trials run over the rows.
+// not fit, the trials run over the rows.  So they do where a window has fewer than 32 rows (trace rows of windows
+// of a few functions) and there are 1024 (window, pole) CTAs or more, each of them mostly idle: 432 windows of
+// 6 functions and rows, 8 poles 149 us from K, 167 over the rows, 32 poles 359 and 176; 27 of 12, 32 poles 125
+// and 139; 54 of 66, 32 poles 248 and 359.
 bool counts_from_k(lres_ctx* c) {
     if (c->route != LRES_ROUTE_TRIDIAG || c->precision != LRES_FP64 || c->no_room_for_k) return false;
+    const long long rows = c->have_trace ? c->nptsT : c->npts;
+    if (rows < 32LL * c->nwin && (long long)c->nwin * c->npoles >= 1024) return false;
     const size_t items = (size_t)c->nwin * c->npoles;
     if ((c->d_K || !dalloc(&c->d_K, c->sizeC)) && (c->d_coef || !dalloc(&c->d_coef, tri_coef_elems(c->nwin, c->npoles, c->nmax))) &&
         (c->d_tr || !dalloc(&c->d_tr, items)))
