@@ -149,7 +149,8 @@ int lres_density_ptr(lres_ctx* ctx, const double** d_dens);
  * copy in L2, or with LRES_MIXED the window's lower triangle on its SM), the row
  * application (rows resident in shared memory with LRES_MIXED, or one row per thread), their
  * panel widths and rows per item (six measured variants, each capped by the shared memory),
- * timed as reduction + rows (mu, e_lo unused).
+ * timed as reduction + rows (mu, e_lo unused); in LRES_FP64 all six are the same kernels, timed once
+ * and left at configuration 0.
  * *chosen (may be NULL) receives the choice, ms_per_config[6] (may be NULL) the measured times. */
 int lres_autotune(lres_ctx* ctx, double mu, double e_lo, int32_t force_config, int32_t* chosen,
                   double* ms_per_config, void* stream);

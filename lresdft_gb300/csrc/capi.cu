@@ -1625,11 +1625,11 @@ extern "C" int lres_autotune(lres_ctx* c, double mu, double e_lo, int32_t force_
             lres_set_error("lres_autotune before a Hamiltonian was set");
             return LRES_ESTATE;
         }
-        double best = 1e300;
+        double best = 1e300, ms = 0.0;
         int arg = 0;
         for (int cfg = 0; cfg < kLeftConfigs; ++cfg) {
-            double ms = 0.0;
-            for (int rep = 0; rep < 2; ++rep) {          // first repetition warms up
+            const bool same = c->precision == LRES_FP64 && cfg;      // (one set of kernels there)
+            for (int rep = 0; rep < 2 && !same; ++rep) {             // first repetition warms up
                 TRY(apply_cfg(cfg));
                 double t[8];
                 TRY(lres_timings(c, t, 8));

@@ -494,7 +494,8 @@ class LResGPU:
 
     def autotune(self, mu, e_lo, config=-1):
         """Pick the tile configuration of the route (-1: time all six on the current
-        Hamiltonian and keep the fastest; on the LDL^T route with full passes at (mu, e_lo)).
+        Hamiltonian and keep the fastest; on the LDL^T route with full passes at (mu, e_lo); the FP64
+        tridiagonal route has one).
         Returns (chosen, ms per config)."""
         chosen = C.c_int32()
         ms = np.full(6, -1.0)
