@@ -241,10 +241,13 @@ int lres_window_ptrs(lres_ctx* ctx, const double** d_HW, const double** d_SW);
 
 /* Adjoint of the band energy at fixed electron number (e_lo fixed), at (mu, e_lo) on the
  * current window matrices.  The reference has no gradient code; its finite-M
- * Hellmann-Feynman check (tests/test_lrft.py:59-79) is the template.  Runs one pole pass
- * whose factors are kept (pole batches of whole windows, as many as free device memory
- * admits), back-substitutes Z_k = (z_k S_W - H_W)^-1 F_W^T, accumulates Re sum_k c_k Z_k Z_k^T
- * for c in {w, w z, w z^2} and returns, each optional:
+ * Hellmann-Feynman check (tests/test_lrft.py:59-79) is the template.  It accumulates
+ * A_c = Re sum_k c_k G_k K G_k, c in {w, w z, w z^2}, G_k = (z_k S_W - H_W)^-1, K = F_W^T F_W: on the
+ * tridiagonal route from the tridiagonal form of every window in FP64 (LRES_MIXED makes one for the
+ * adjoint, from H(v) assembled in FP64 where H_W is H(v), and sweeps in FP32), as many pole groups and
+ * windows at a time as free device memory admits; on the LDL^T route, or without room for that, from the
+ * factors of every (window, pole), back-substituted for the rows F_W, in batches of whole windows.  N and
+ * E_band are by the same form, the density by one pass.  Returns, each optional:
  *   dv[ng]           dE_band/dv(r) at fixed N (the grid local potential through
  *                    H = T + X^T diag(v) X dV, lrft/lcao3d.py:98-100);
  *   dHW, dSW[sizeC]  dE_band/dH_W and dE_band/dS_W at fixed N, window layout as

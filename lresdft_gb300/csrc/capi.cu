@@ -2226,7 +2226,9 @@ bool adj_tri_room(lres_ctx* c, cudaStream_t s, AdjPlan* pl) {
 // the pass, A_c in the tridiagonal basis into d_adjA, W = L^-T Q in *Wt (over the standard form, which the
 // reduction has consumed).  In mixed precision the tridiagonal form is made here (d_HW and L^-T are FP64)
 // and the sweeps run in FP32: 128 windows 89 -> 36 ms, the gradients 5e-7 off 64 bits against the
-// 2e-6 of FP32 factors.
+// 2e-6 of FP32 factors, and dN/dmu 1e-13 against 2e-6.  Small windows of few poles pay for that accuracy: the
+// reduction's chain of columns takes longer than all factors side by side (16 windows of 84 functions, 4 poles
+// 1.96 ms by factors, 2.96 here, 32 poles 2.60 and 3.12; 128 of 138, 4 poles 5.7 and 6.7).
 int adj_tri_accumulate(lres_ctx* c, const AdjPlan& pl, double mu, double e_lo, const double** Wt, cudaStream_t s) {
     const bool mixed = c->precision == LRES_MIXED;
     if (!c->tri_ready) TRY(tri_refresh(c, s));

@@ -145,7 +145,7 @@ int pole_sums(int nwin, const long long* offQ, const int* m_w, const long long* 
 // Tile configuration of the tridiagonal route for windows of at most nmax functions and P poles; LRES_EINVAL
 // where they are too large or too many for its kernels.
 struct TriPick {
-    int nb = 0, nt = 0;        // reduction panel width and threads
+    int nb = 0;                // reduction panel width
     int reg = 0;               // 1: the reduction holds each window on its SM (FP32, tridiag_reg.cu)
     int nb_apply = 0;          // row application panel width
     int rpt = 1;               // rows per thread of the row-per-thread application; 0: resident rows
@@ -199,13 +199,13 @@ int tri_count(int nwin, int P, int nmax, const int* n_w, const long long* offN, 
               const double* e, const double* K, const double2* shifts, const double2* wq, const double2* wzq,
               double dV, double4* coef, double2* trace, double* nw, double* ew, int* status, size_t smem_budget,
               cudaStream_t s);
-// P = Re sum_k w_k (z_k - T)^-1 of every window (FP64), and the rows' n, e from V = Y P for windows
 // u[c * nwin + w] = Re sum_k cw[c P + k] tr(G_k K G_k), c = 0, 1, 2, after tri_count: its coef, dcoef as coef,
 // slope nwin * P elements.
 int tri_slopes(int nwin, int P, int nmax, const int* n_w, const long long* offN, const long long* offC, const double* d,
                const double* e, const double* K, const double2* shifts, const double2* cw, const double4* coef,
                double4* dcoef, double2* slope, double* u, cudaStream_t s);
-// w0 .. w0 + nwin - 1 (V of window w at offV[w], maxitems pass items of a window at most)
+// P = Re sum_k w_k (z_k - T)^-1 of every window (FP64); the rows' n, e from V = Y P for windows w0 ..
+// w0 + nwin - 1 (V of window w at offV[w], maxitems pass items of a window at most).
 int tri_pmat(int nwin, int P, int nmax, const int* n_w, const long long* offN, const long long* offC, const double* d,
              const double* e, const double2* shifts, const double2* wq, double4* coef, double* Pm, cudaStream_t s);
 int tri_rowdot(int w0, int nwin, int maxitems, const int4* items, const int* first, const int* count, const int* n_w,

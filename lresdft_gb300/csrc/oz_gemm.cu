@@ -483,7 +483,7 @@ constexpr int kTLd = kOzPanel + 8;            // (four columns of eight rows in 
 // functions 2.54 -> 1.17 ms, 54 windows 0.43 -> 0.20 ms).
 __global__ void __launch_bounds__(kTNT) oz_tfactor_kernel(int nwin, const int* q_w, const long long* offT,
                                                           const long long* offN, const double* tau, int qmax, double* T) {
-    extern __shared__ __align__(16) unsigned char smem[];
+    extern __shared__ __align__(128) unsigned char smem[];
     double* const Ts = reinterpret_cast<double*>(smem);             // [qmax][kTLd]
     double* const Gs = Ts + (size_t)qmax * kTLd;                    // (a, b), a <= b at b (b + 1) / 2 + a
     const int w = blockIdx.x % nwin, p = blockIdx.x / nwin, a = threadIdx.x >> 2, part = threadIdx.x & 3;

@@ -160,21 +160,18 @@ __device__ __forceinline__ void st_cluster(double* dst, unsigned rank, double x)
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(a), "r"(rank));
     asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(x) : "memory");
 }
-__device__ __forceinline__ void st_cluster(float* dst, unsigned rank, float x) {
-    unsigned a = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(a), "r"(rank));
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(x) : "memory");
-}
 
 // In FP64 every warp instruction holds its quarter of the SM for 80 clocks, so nothing is computed twice that
 // one warp can publish: the root and divisions of the reflector run in the last warp beside the others' A x,
 // the sum of p^T v in the warps that own rows only (in every warp, the same bits: a third of the FP64
 // instructions; 54 windows 7.6 -> 5.55 ms, one of 96 functions 1.64 -> 1.03 ms; with panels of 8 5.17 and 0.92).
 //
-// CL = 2: a cluster of two CTAs per window, for fewer windows than half the SMs (FP64, 54 windows of 276-300
-// functions 9.2 -> 7.6 ms, before the above; one window of 96, where the barriers outweigh the work, 1.64 -> 1.84 ms).  Both form the columns, reflectors and vectors (the same bits); the row quads of q = A x and the
-// blocks of the trailing update, which hold the FP64 pipe, are dealt to them, q exchanged through
-// distributed shared memory (two buffers by column parity: the other CTA may be a phase ahead).
+// CL = 2: a cluster of two CTAs per window, for fewer windows than half the SMs.  Both form the columns, reflectors
+// and vectors (the same bits); the row quads of q = A x and the blocks of the trailing update, which hold the
+// FP64 pipe, are dealt to them, q exchanged through distributed shared memory (two buffers by column parity:
+// the other CTA may be a phase ahead).  One and two CTAs, 1 to 54 windows (the same time): 48 functions 0.50 and
+// 0.65 ms, 96 0.91 and 1.11, where the barriers outweigh the work, 160 1.86 and 1.93, 192 2.58 and 2.43, 240
+// 4.08 and 3.45, 300 6.87 and 5.17, 384 12.7 and 8.5, 510 27.3 and 16.7.
 template <class R, int NT, int CL = 1>
 __global__ void __launch_bounds__(NT, reduce_min_ctas(NT, sizeof(R))) tri_reduce_kernel(TriReduceParams<R> p) {
     constexpr int NW = NT / 32;
@@ -1896,16 +1893,16 @@ __global__ void tri_mineig_kernel(int nwin, const int* n_w, const long long* off
 // the rows stay resident in shared memory (res; FP32 only).  Panel widths are capped by
 // what fits the shared memory at windows of nmax.
 struct TriCfg {
-    int nb, nt, nba, rpt, res, reg;      // reg: the reduction with the window on its SM (tridiag_reg.cu)
+    int nb, nba, rpt, res, reg;          // reg: the reduction with the window on its SM (tridiag_reg.cu)
     int rows;                            // resident application: rows per item at most
 };
 // Measured at 1024 electrons (mixed): reduction 3.5 ms with the window on its SM, 6.7 ms with the
 // L2-resident working copy (nb 16, 512 threads, two CTAs per SM; nb 8 6.75 ms, nb 32 7.35 ms; 256
 // threads at four CTAs per SM and 384 at three 7.8 ms); row application 2.0 ms with resident rows
 // (NB 32), 6.3 ms one row per thread.
-static const TriCfg kTriCfg[6] = {{16, 512, 32, 1, 1, 1, 128}, {16, 512, 32, 1, 1, 0, 128},
-                                  {16, 512, 32, 1, 0, 0, 0},    {16, 512, 16, 1, 1, 0, 64},
-                                  {16, 512, 32, 1, 1, 1, 32},   {8, 512, 32, 1, 1, 0, 128}};
+static const TriCfg kTriCfg[6] = {{16, 32, 1, 1, 1, 128}, {16, 32, 1, 1, 0, 128}, {16, 32, 1, 0, 0, 0},
+                                  {16, 16, 1, 1, 0, 64},  {16, 32, 1, 1, 1, 32},  {8, 32, 1, 1, 0, 128}};
+constexpr int kReduceNT = 512;           // threads of the reduction (256 where FP64 CTAs go in pairs)
 
 int tri_pick(bool fp32, int nmax, int P, size_t smem_budget, int cfg, TriPick* out) {
     if (tri_rows_per_item(fp32, P) < 1) {
@@ -1917,14 +1914,13 @@ int tri_pick(bool fp32, int nmax, int P, size_t smem_budget, int cfg, TriPick* o
     r.ldv = (std::max(nmax, 1) + 31) / 32 * 32;
     if (cfg < 0 || cfg >= 6) cfg = 0;
     const TriCfg& t = kTriCfg[cfg];
-    r.nt = t.nt;
     r.reg = t.reg && fp32;
     // FP64: panels of 8, the pending updates cost instructions of its pipe and the L2 traffic of more frequent
     // updates does not bound it (54 windows: panels of 4, 8, 16 take 5.21, 5.17, 5.56 ms; 432 windows 19.6,
     // 18.3, 19.4 to 20.7 ms; one window of 96 functions 0.88, 0.92, 1.03 ms)
     const int nbmax = fp32 ? t.nb : std::min(t.nb, 8);
     for (int b : {32, 16, 8, 4})
-        if (b <= nbmax && !r.nb && reduce_smem_elems(b, r.ldv, t.nt) * el <= smem_budget) r.nb = b;
+        if (b <= nbmax && !r.nb && reduce_smem_elems(b, r.ldv, kReduceNT) * el <= smem_budget) r.nb = b;
     if (t.res && fp32)
         for (int b : {32, 16})
             for (int rows = std::min(kResRows, t.rows); rows >= 32 && !r.nb_apply; rows -= 32)
@@ -1966,7 +1962,7 @@ static int launch_reduce(const TriReduceParams<R>& p, size_t smem_budget, cudaSt
 
 // Two CTAs per window.
 static int launch_reduce_cluster(const TriReduceParams<double>& p, cudaStream_t s) {
-    constexpr int NT = 512;
+    constexpr int NT = kReduceNT;
     const size_t smem = reduce_smem_elems(p.nb, p.ldv, NT, 2) * sizeof(double);
     int per_sm = 0;
     if (int rc = prepare_kernel<tri_reduce_kernel<double, NT, 2>>(NT, smem, &per_sm)) return rc;
@@ -1989,7 +1985,7 @@ int tri_reduce(bool fp32, int nwin, const int* order, int* counter, const int* n
                const long long* offA, const long long* offN, const void* H, void* A, void* d, void* e, void* tau,
                int* status, const TriPick& pk, int nmax, size_t smem_budget, cudaStream_t s) {
     if (!nwin) return LRES_OK;
-    const int nb = pk.nb, nt = pk.nt, ldv = pk.ldv;
+    const int nb = pk.nb, ldv = pk.ldv;
     LRES_CUDA_TRY(cudaMemsetAsync(counter, 0, sizeof(int), s));
     if (fp32) {
         TriReduceParams<float> p{nwin, order, counter, n_w, offC, offA, offN, (const float*)H, (float*)A,
@@ -1998,28 +1994,24 @@ int tri_reduce(bool fp32, int nwin, const int* order, int* counter, const int* n
             // windows beyond the resident size: their first columns from the L2-resident copy
             if (nmax > kTriRegMax) {
                 p.keep = kTriRegMax;
-                if (int rc = nt == 512 ? launch_reduce<float, 512>(p, smem_budget, s)
-                                       : launch_reduce<float, 256>(p, smem_budget, s))
-                    return rc;
+                if (int rc = launch_reduce<float, kReduceNT>(p, smem_budget, s)) return rc;
             }
             return tri_reduce_reg(nwin, order, counter, n_w, offC, offA, offN, (const float*)H, (float*)A, (float*)d,
                                   (float*)e, (float*)tau, status, nb, nmax, smem_budget, s);
         }
-        return nt == 512 ? launch_reduce<float, 512>(p, smem_budget, s) : launch_reduce<float, 256>(p, smem_budget, s);
+        return launch_reduce<float, kReduceNT>(p, smem_budget, s);
     }
     TriReduceParams<double> p{nwin, order, counter, n_w, offC, offA, offN, (const double*)H, (double*)A,
                               (double*)d, (double*)e, (double*)tau, status, nb, ldv, 0};
-    if (nt == 512) {
-        // two CTAs per window while they find an SM each and the windows are large enough to share; one
-        // CTA of 512 threads while the windows find one;
-        // beyond, two of 256 threads per SM, which fill each other's barriers (432 windows 19.7 -> 18.3 ms)
-        if (2 * nwin <= device_sms() && nmax >= 192 && reduce_smem_elems(nb, ldv, 512, 2) * sizeof(double) <= smem_budget)
-            return launch_reduce_cluster(p, s);
-        if (nwin > device_sms() && 2 * (reduce_smem_elems(nb, ldv, 256) * sizeof(double) + 1024) <= smem_budget + 1024)
-            return launch_reduce<double, 256>(p, smem_budget, s);
-        return launch_reduce<double, 512>(p, smem_budget, s);
-    }
-    return launch_reduce<double, 256>(p, smem_budget, s);
+    // two CTAs per window while they find an SM each and the windows are large enough to share (the line lies
+    // between 160 and 192 functions, see the kernel); one CTA of 512 threads while the windows find one; beyond,
+    // two of 256 threads per SM, which fill each other's barriers (432 windows 19.7 -> 18.3 ms)
+    if (2 * nwin <= device_sms() && nmax >= 192 &&
+        reduce_smem_elems(nb, ldv, kReduceNT, 2) * sizeof(double) <= smem_budget)
+        return launch_reduce_cluster(p, s);
+    if (nwin > device_sms() && 2 * (reduce_smem_elems(nb, ldv, 256) * sizeof(double) + 1024) <= smem_budget + 1024)
+        return launch_reduce<double, 256>(p, smem_budget, s);
+    return launch_reduce<double, kReduceNT>(p, smem_budget, s);
 }
 
 template <class R, int NB, int RPT>
@@ -2139,7 +2131,7 @@ int tri_count(int nwin, int P, int nmax, const int* n_w, const long long* offN, 
               cudaStream_t s) {
     if (!nwin) return LRES_OK;
     // four poles a CTA share the reads of K and the broadcasts; one where that leaves SMs without a CTA (one
-    // window of 96 functions, 32 poles: 85 -> COUNT1 us)
+    // window of 96 functions, 32 poles: 85 -> 35 us)
     const int np = (long long)nwin * ((P + 3) / 4) < device_sms() ? 1 : 4;
     const size_t smem = sizeof(double2) * np * (size_t)nmax;
     if (smem > smem_budget) {
