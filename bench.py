@@ -204,10 +204,10 @@ def launches_per_step(route, precision, tile_config=0, standard_form="simt", nW=
         # of windows beyond 384 functions
         if precision == "mixed":
             return 10 + 2 * (tile_config != 2) + (standard_form == "simt") + (tile_config in (0, 4) and n > 384)
-        # FP64: assemble_h, gather, reduction, T factors, pole nodes, diagonals of G, P, rows' sums
+        # FP64: assemble_h, gather, symmetric part, reduction, T factors, pole nodes, diagonals of G, P, rows' sums
         # (V a batch of windows at a time, 1 GB), window sums; the products: 2 of the standard form,
         # V^T V and 3 of the rows per panel of 128 reflectors, V = Y P
-        total = 9 + 2 * oz_launches(nwin, n, n, n, balance=True)
+        total = 10 + 2 * oz_launches(nwin, n, n, n, balance=True)
         for j0 in range(0, n - 2, 128):
             q, r = min(128, n - 2 - j0), n - 1 - j0
             total += oz_launches(nwin, q, q, r, gram=True) + oz_launches(nwin, m, q, r)

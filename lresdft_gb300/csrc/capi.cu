@@ -413,6 +413,16 @@ int square_gemm(lres_ctx* c, const double* A, bool at, const double* B, bool bk,
                    B, c->d_offC, OzForm(bk), C, c->d_offC, klim, false, balance, c->smem_budget, s);
 }
 
+// The lower triangle of L^-1 H L^-T in FP64 into Hhat, Y for the product H L^-T between; H may be asymmetric to
+// rounding, as sums in the order of its rows leave it, and only its symmetric part counts: one triangle of the
+// product would hold the other part too, times the condition of S_W (one window of 96 functions, H_W asymmetric
+// by 3e-15: the density 2.1e-14 off extended precision, 2e-15 this way, the error of the dense factorisations).
+int standard_form_fp64(lres_ctx* c, const double* H, double* Y, double* Hhat, cudaStream_t s) {
+    TRY(symmetrise_windows(c->nwin, c->nmax, c->d_n, c->d_offC, H, Hhat, s));
+    TRY(square_gemm(c, Hhat, false, c->d_LinvT, true, Y, 1, true, s));
+    return square_gemm(c, c->d_LinvT, true, Y, true, Hhat, 2, true, s);
+}
+
 // FP64 (the FP64 tridiagonal route); the product H LinvT lives in the working blocks of the
 // reduction (at least sizeC elements), which the reduction overwrites afterwards.
 int transform_fp64(lres_ctx* c, cudaStream_t s) {
@@ -421,9 +431,7 @@ int transform_fp64(lres_ctx* c, cudaStream_t s) {
         lres_set_error("FP64 standard form without the tridiagonal buffers");
         return LRES_ESTATE;
     }
-    TRY(square_gemm(c, c->d_HW, false, c->d_LinvT, true, Y, 1, true, s));
-    TRY(square_gemm(c, c->d_LinvT, true, Y, true, c->d_Hhat, 2, true, s));
-    return LRES_OK;
+    return standard_form_fp64(c, c->d_HW, Y, c->d_Hhat, s);
 }
 
 int window_transform(lres_ctx* c, cudaStream_t s) {
@@ -2261,8 +2269,7 @@ int adj_tri_accumulate(lres_ctx* c, const AdjPlan& pl, double mu, double e_lo, c
                                c->d_n, a.Hblk, a.K, nullptr, nullptr, s));
             HW = a.K;
         }
-        TRY(square_gemm(c, HW, false, c->d_LinvT, true, a.A, 1, true, s));
-        TRY(square_gemm(c, c->d_LinvT, true, a.A, true, a.H, 2, true, s));
+        TRY(standard_form_fp64(c, HW, a.A, a.H, s));
         TRY(tri_reduce(false, c->nwin, c->d_order_w, c->d_counter, c->d_n, c->d_offC, c->d_offA, c->d_offN, a.H, a.A, a.d,
                        a.e, a.tau, c->d_status, pk, c->nmax, c->smem_budget, s));
         TRY(oz_tfactors(c->oz, c->ozr, c->nwin, c->nmax, c->d_n, a.A, a.tau, c->d_offN, c->smem_budget, s));

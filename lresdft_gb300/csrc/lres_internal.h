@@ -93,6 +93,8 @@ int assemble_h32(const BlockPattern& bp, const Supports& sp, const double* Tblk,
 int gather_windows(int nwin, int nmax, const int* fn, const long long* fnoff, const int* btab, const long long* btoff,
                    const int* nlg, const long long* offC, const int* n_w, const double* blk, double* dense,
                    const float* blk32, float* dense32, cudaStream_t s);
+// B_w = (A_w + A_w^T) / 2 (n_w x n_w)
+int symmetrise_windows(int nwin, int nmax, const int* n_w, const long long* offC, const double* A, double* B, cudaStream_t s);
 int build_F(int nwin, const long long* Xp, const int* Xi, const double* Xv, const int* group_of_fn,
             const int* gptr, const int* gloc, int ngroups, const long long* Ooff, const long long* Oflat,
             const long long* offF, const int* m_w, int mmax, double* F, cudaStream_t s);

@@ -13,7 +13,7 @@
 // lies more than 2^-5 to 2^-9 below that product and matters all the same.  What makes them so in the sums over
 // basis functions, functions of different size, is taken out first (oz_balance_kernel).
 // (8 digits: 2^-51 and 2^-55, a fifth less time, and the density of 54 windows 2.1e-14 off 64 bits against
-// 1.6e-14, the FP64 pipe's error.)
+// 1.6e-14, both with the asymmetry of H_W in them, which alone is most of the 1.6e-14.)
 //
 // Kernels: oz_slice_kernel writes the digits of an operand ([digit][row][k], k contiguous), each
 // element once; oz_gemm_kernel, one CTA per 64 x 64 tile, stages 32 terms of all digits of both
@@ -22,8 +22,8 @@
 // ~600 TFLOP/s is 21 FP64 multiply-adds per clock and SM.  The windows go in batches, so that the
 // digits take at most ~1 GB whatever the context's size.
 //
-// Measured (432 windows of 270-306 functions): the standard form's two products 23.5 -> 5.6 ms (54
-// windows 3.7 -> 0.79).
+// Measured (432 windows of 270-306 functions): the standard form's two products 23.5 -> 5.9 ms (54
+// windows 3.7 -> 0.81), with the balance.
 #include "common.cuh"
 #include "launch.cuh"
 #include "lres_internal.h"
@@ -390,17 +390,19 @@ static int oz_alloc(OzWork& wk, size_t bytes) {
     return LRES_OK;
 }
 
-int oz_reserve(OzWork& wk, int nwin, int mmax, int nmax) {
-    const OzPlan a = oz_plan(nwin, mmax, nmax, nmax), b = oz_plan(nwin, nmax, nmax, mmax);
-    const size_t least = std::max(a.perw, b.perw);
-    size_t bytes = std::max(a.perw * a.batch, b.perw * b.batch);
-    if (wk.bytes >= bytes) return LRES_OK;
-    // as much of it as the device has, in halves
+// `bytes`, or as much of it as the device has, in halves.
+static int oz_grow(OzWork& wk, size_t bytes, size_t least) {
     while (oz_alloc(wk, bytes) != LRES_OK) {
         if (bytes == least) return LRES_ENOMEM;
         bytes = std::max(bytes / 2, least);
     }
     return LRES_OK;
+}
+
+int oz_reserve(OzWork& wk, int nwin, int mmax, int nmax) {
+    const OzPlan a = oz_plan(nwin, mmax, nmax, nmax), b = oz_plan(nwin, nmax, nmax, mmax);
+    const size_t bytes = std::max(a.perw * a.batch, b.perw * b.batch);
+    return wk.bytes >= bytes ? LRES_OK : oz_grow(wk, bytes, std::max(a.perw, b.perw));
 }
 
 int oz_gemm(OzWork& wk, int nwin, int mmax, int nmax, int kmax, const int* m_w, const int* n_w, const int* k_w,
@@ -415,7 +417,7 @@ int oz_gemm(OzWork& wk, int nwin, int mmax, int nmax, int kmax, const int* m_w, 
     // window does not fit
     const OzPlan p = oz_plan(nwin, mmax, nmax, kmax);
     if (wk.bytes < p.perw)
-        if (int rc = oz_alloc(wk, p.perw * p.batch)) return rc;
+        if (int rc = oz_grow(wk, p.perw * p.batch, p.perw)) return rc;
     const int Rp = p.Rp, Cp = p.Cp, Kp = p.Kp, batch = (int)std::min<size_t>(p.batch, wk.bytes / p.perw);
     unsigned short* const da = static_cast<unsigned short*>(wk.buf);
     // (a Gram product has one operand)
