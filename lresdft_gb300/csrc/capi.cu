@@ -639,6 +639,27 @@ int ensure_tfactors(lres_ctx* c) {
     return LRES_OK;
 }
 
+// Do FP64 reductions go two to an SM (256 threads each) rather than one (512)?  Two fill each other's barriers, but a
+// window then takes up to 1.8 times as long (t, in ms, one to an SM), which decides where the largest one outlasts
+// the rest.  One against two to an SM: 250 windows of 222-366 functions 13.9 and 19.4 ms, of 264-306 12.8 and 13.0,
+// 360 of these 19.0 and 17.2, 432 19.4 and 21.2, 504 25.4 and 22.5, 1024 44.6 and 39.7, 216 of 324 16.7 and 15.4,
+// 1024 of 60-186 9.1 and 5.9.  (The line cost 7 % at one of 34 such forms, 250 of 60-168, and 9 % at 432.)
+bool reduce_in_pairs(const lres_ctx* c) {
+    if (c->nwin <= c->nsm) return false;
+    auto t = [](double n) { return 9e-3 * n + 1.55e-7 * n * n * n; };
+    double sum = 0.0;
+    for (int n : c->n_w) sum += t(n);
+    const double slower = std::clamp(1.05 + 0.0036 * (c->nmax - 84), 1.0, 1.8);
+    return slower * t(c->nmax) <= 1.4 * sum / c->nsm;
+}
+
+// Configuration `cfg` of the tridiagonal route for the context's windows.
+int pick_config(const lres_ctx* c, bool fp32, int cfg, TriPick* pk) {
+    TRY(tri_pick(fp32, c->nmax, c->npoles, c->smem_budget, cfg, pk));
+    pk->pairs = !fp32 && reduce_in_pairs(c);
+    return LRES_OK;
+}
+
 // Panels of the FP64 rows on the tensor cores (once per context).
 int oz_setup(lres_ctx* c, cudaStream_t s) {
     OzRows& o = c->ozr;
@@ -781,7 +802,7 @@ void tri_release(lres_ctx* c) {
 int tri_buffers(lres_ctx* c, cudaStream_t s) {
     const bool fp32 = c->precision == LRES_MIXED;
     const size_t el = fp32 ? sizeof(float) : sizeof(double);
-    TRY(tri_pick(fp32, c->nmax, c->npoles, c->smem_budget, c->tri_cfg, &c->tri));
+    TRY(pick_config(c, fp32, c->tri_cfg, &c->tri));
     TRY(ensure_tfactors(c));
     TRY(dalloc((char**)&c->d_triA, el * (size_t)c->sizeA));
     TRY(dalloc((char**)&c->d_trid, el * (size_t)c->sizeN));
@@ -1418,7 +1439,7 @@ extern "C" int lres_ctx_create(lres_ctx** out, const lres_system_desc* d, int pr
     TRY(upload(&c->d_order_w, c->order, s));
     {
         TriPick pk;
-        const bool fits = tri_pick(precision == LRES_MIXED, c->nmax, c->npoles, c->smem_budget, 0, &pk) == LRES_OK;
+        const bool fits = pick_config(c.get(), precision == LRES_MIXED, 0, &pk) == LRES_OK;
         lres_set_error("");
         // a few FP64 windows: a Hamiltonian and a pass take some 420 + 15 n us here (n launches' and columns'
         // latency) and 180 + 5 n + 6e-4 m n^2 us by dense factorisations, all poles side by side.  So there where
@@ -1609,7 +1630,7 @@ extern "C" int lres_autotune(lres_ctx* c, double mu, double e_lo, int32_t force_
         // Hamiltonian (reduction + rows per configuration)
         auto apply_cfg = [&](int cfg) -> int {
             TriPick pk;
-            TRY(tri_pick(c->precision == LRES_MIXED, c->nmax, c->npoles, c->smem_budget, cfg, &pk));
+            TRY(pick_config(c, c->precision == LRES_MIXED, cfg, &pk));
             c->tri_cfg = cfg;
             c->tri = pk;
             if (c->tri_alloc) {
@@ -1697,7 +1718,7 @@ extern "C" int lres_set_route(lres_ctx* c, int32_t route, void* stream) {
         return LRES_OK;
     }
     TriPick pk;
-    TRY(tri_pick(c->precision == LRES_MIXED, c->nmax, c->npoles, c->smem_budget, c->tri_cfg, &pk));
+    TRY(pick_config(c, c->precision == LRES_MIXED, c->tri_cfg, &pk));
     const int old = c->route;
     c->route = route;
     int rc = LRES_OK;
@@ -2168,7 +2189,7 @@ bool adj_tri_buffers(lres_ctx* c, cudaStream_t s) {
     if (a.tried) return a.ok();
     a.tried = true;
     TriPick pk;
-    int rc = tri_pick(false, c->nmax, c->npoles, c->smem_budget, 0, &pk);
+    int rc = pick_config(c, false, 0, &pk);
     if (!rc) rc = dalloc(&a.A, c->sizeA);
     if (!rc) rc = dalloc(&a.d, c->sizeN);
     if (!rc) rc = dalloc(&a.e, c->sizeN);
@@ -2258,7 +2279,7 @@ int adj_tri_accumulate(lres_ctx* c, const AdjPlan& pl, double mu, double e_lo, c
     } else {
         lres_ctx::AdjTri& a = c->at;
         TriPick pk;
-        TRY(tri_pick(false, c->nmax, c->npoles, c->smem_budget, 0, &pk));
+        TRY(pick_config(c, false, 0, &pk));
         poles_kernel<<<(P + 63) / 64, 64, 0, s>>>(P, c->M, mu, e_lo, 0, a.shifts, c->d_wq, c->d_wzq);
         LRES_CUDA_TRY(cudaGetLastError());
         // H_W: where it is an FP32 H(v) again in FP64 (its 1e-8 Ha of the levels are 2e-6 of dN/dmu)

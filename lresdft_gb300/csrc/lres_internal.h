@@ -148,6 +148,7 @@ int pole_sums(int nwin, const long long* offQ, const int* m_w, const long long* 
 // where they are too large or too many for its kernels.
 struct TriPick {
     int nb = 0;                // reduction panel width
+    bool pairs = false;        // FP64: reductions two to an SM, beyond an SM for each
     int reg = 0;               // 1: the reduction holds each window on its SM (FP32, tridiag_reg.cu)
     int nb_apply = 0;          // row application panel width
     int rpt = 1;               // rows per thread of the row-per-thread application; 0: resident rows

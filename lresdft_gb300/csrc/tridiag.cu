@@ -1916,8 +1916,8 @@ int tri_pick(bool fp32, int nmax, int P, size_t smem_budget, int cfg, TriPick* o
     const TriCfg& t = kTriCfg[cfg];
     r.reg = t.reg && fp32;
     // FP64: panels of 8, the pending updates cost instructions of its pipe and the L2 traffic of more frequent
-    // updates does not bound it (54 windows: panels of 4, 8, 16 take 5.21, 5.17, 5.56 ms; 432 windows 19.6,
-    // 18.3, 19.4 to 20.7 ms; one window of 96 functions 0.88, 0.92, 1.03 ms)
+    // updates does not bound it (54 windows: panels of 4, 8, 16 take 5.23, 5.19, 5.58 ms; 432 windows 20.9,
+    // 20.9, 22.5 ms; one window of 96 functions 0.88, 0.91, 1.03 ms)
     const int nbmax = fp32 ? t.nb : std::min(t.nb, 8);
     for (int b : {32, 16, 8, 4})
         if (b <= nbmax && !r.nb && reduce_smem_elems(b, r.ldv, kReduceNT) * el <= smem_budget) r.nb = b;
@@ -2004,12 +2004,11 @@ int tri_reduce(bool fp32, int nwin, const int* order, int* counter, const int* n
     TriReduceParams<double> p{nwin, order, counter, n_w, offC, offA, offN, (const double*)H, (double*)A,
                               (double*)d, (double*)e, (double*)tau, status, nb, ldv, 0};
     // two CTAs per window while they find an SM each and the windows are large enough to share (the line lies
-    // between 160 and 192 functions, see the kernel); one CTA of 512 threads while the windows find one; beyond,
-    // two of 256 threads per SM, which fill each other's barriers (432 windows 19.7 -> 18.3 ms)
+    // between 160 and 192 functions, see the kernel); else one CTA of 512 threads, or two of 256 per SM (TriPick)
     if (2 * nwin <= device_sms() && nmax >= 192 &&
         reduce_smem_elems(nb, ldv, kReduceNT, 2) * sizeof(double) <= smem_budget)
         return launch_reduce_cluster(p, s);
-    if (nwin > device_sms() && 2 * (reduce_smem_elems(nb, ldv, 256) * sizeof(double) + 1024) <= smem_budget + 1024)
+    if (pk.pairs && 2 * (reduce_smem_elems(nb, ldv, 256) * sizeof(double) + 1024) <= smem_budget + 1024)
         return launch_reduce<double, 256>(p, smem_budget, s);
     return launch_reduce<double, kReduceNT>(p, smem_budget, s);
 }
