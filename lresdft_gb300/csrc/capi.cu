@@ -2497,12 +2497,7 @@ extern "C" int lres_owned_gram(lres_ctx* c, double* K, int on_device, void* stre
     return rc;
 }
 
-extern "C" int lres_set_trace_rows(lres_ctx* c, const int32_t* r_w, const double* R, void* stream) {
-    if (!c) {
-        lres_set_error("null argument");
-        return LRES_EINVAL;
-    }
-    cudaStream_t s = (cudaStream_t)stream;
+static int set_trace_rows(lres_ctx* c, const int32_t* r_w, const double* R, cudaStream_t s) {
     LRES_CUDA_TRY(cudaStreamSynchronize(s));
     for (void* p : {(void*)c->d_mT, (void*)c->d_offFT, (void*)c->d_offQT, (void*)c->d_FT, (void*)c->d_FhatT32,
                     c->d_qT, (void*)c->d_FhatT64, c->d_Ytr})
@@ -2563,4 +2558,14 @@ extern "C" int lres_set_trace_rows(lres_ctx* c, const int32_t* r_w, const double
     }
     LRES_CUDA_TRY(cudaStreamSynchronize(s));
     return LRES_OK;
+}
+
+extern "C" int lres_set_trace_rows(lres_ctx* c, const int32_t* r_w, const double* R, void* stream) {
+    if (!c) {
+        lres_set_error("null argument");
+        return LRES_EINVAL;
+    }
+    const int rc = set_trace_rows(c, r_w, R, (cudaStream_t)stream);
+    if (rc) c->have_trace = false;       // (half of their buffers may be there: passes run over the owned rows)
+    return rc;
 }

@@ -82,6 +82,22 @@ def test_a_refused_context_leaves_nothing():
     assert owner.size == cr.ng
 
 
+def test_refused_trace_rows_leave_none():
+    """Trace rows that find no room: the passes run over the owned rows, as before them."""
+    from lresdft_gb300 import LResGPU, _lib
+    b, cr = _crystal()
+    s = LResGPU(b, cr.pos, R_w=8.0, M=16, precision="fp64", route="tridiag", trace_rows=False)
+    s.set_potential(np.linspace(-0.4, 0.1, cr.ng))
+    want = s.pole_pass(MU, E_LO, want_density=False)[1:]
+    with _free(48 << 20):                            # (the factors take 26 MB each, four times)
+        with pytest.raises(_lib.LResError, match="out of memory"):
+            s.install_trace_rows()
+    assert s.pole_pass(MU, E_LO, want_density=False)[1:] == want
+    s.set_potential(np.linspace(-0.4, 0.1, cr.ng))
+    assert s.pole_pass(MU, E_LO, want_density=False)[1:] == want
+    s.close()
+
+
 @pytest.mark.parametrize("free_gb", [4.45, 4.2])
 def test_adjoint(free_gb):
     """The adjoint keeps 4 GB of the device free.  One window of some 600 functions and 32 poles, all pole groups at
